@@ -14,6 +14,7 @@
 #include "../agl_field.cuh"
 #include "sha256.hpp"
 #include "host_field.hpp"
+#include "monolith_avx512.hpp"
 
 namespace mbhost {
 namespace aglm {
@@ -78,7 +79,7 @@ inline void concrete(uint64_t* s, const uint64_t* rc) {
 }
 
 // In place; any 64-bit words in, canonical residues out (crypto/monolith.rs:201-208).
-inline void permute(uint64_t* s) {
+inline void permute_portable(uint64_t* s) {
     static const uint64_t(*const rc)[WIDTH] = round_constants();
     concrete(s, rc[0]);
     for (int r = 1; r <= N_ROUNDS; r++) {
@@ -90,6 +91,14 @@ inline void permute(uint64_t* s) {
         concrete(s, rc[r]);
     }
     for (int i = 0; i < WIDTH; i++) s[i] = s[i] >= agl::P ? s[i] - agl::P : s[i];
+}
+
+inline void permute(uint64_t* s) {
+#if defined(__x86_64__)
+    static const uint64_t(*const rc)[WIDTH] = round_constants();
+    if (mono512::available) return mono512::permute<mono512::Agl>(s, rc);
+#endif
+    permute_portable(s);
 }
 
 class Transcript {

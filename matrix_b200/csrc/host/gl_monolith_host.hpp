@@ -6,6 +6,7 @@
 #include <cstdint>
 #include "../gl_monolith.cuh"
 #include "host_field.hpp"
+#include "monolith_avx512.hpp"
 
 namespace mbhost {
 namespace monohost {
@@ -22,7 +23,7 @@ static inline void concrete(uint64_t* s, const uint64_t* rc) {
 }
 
 // In place; any 64-bit words in, canonical residues out.
-static inline void permute(uint64_t* s) {
+static inline void permute_portable(uint64_t* s) {
     concrete(s, nullptr);
     for (int r = 1; r <= gl::MONO_ROUNDS; r++) {
         for (int i = 0; i < 4; i++) s[i] = gl::mono_bar(hf::gl_canon(s[i]));   // bars act on the canonical word
@@ -33,6 +34,13 @@ static inline void permute(uint64_t* s) {
         concrete(s, r < gl::MONO_ROUNDS ? gl::h_mono_rc[r] : nullptr);
     }
     for (int i = 0; i < 12; i++) s[i] = hf::gl_canon(s[i]);
+}
+
+static inline void permute(uint64_t* s) {
+#if defined(__x86_64__)
+    if (mono512::available) return mono512::permute<mono512::Gl>(s, gl::h_mono_rc);
+#endif
+    permute_portable(s);
 }
 
 }  // namespace monohost

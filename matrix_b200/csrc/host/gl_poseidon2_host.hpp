@@ -45,8 +45,8 @@ static inline void external_linear(uint64_t* s, const uint64_t* rc) {
     }
 }
 
-// In place; any 64-bit words in, canonical residues out.
-static inline void permute(uint64_t* s) {
+// In place, for any host core.
+static inline void permute_portable(uint64_t* s) {
     const uint64_t(*rc_ext)[8] = gl::h_p2_rc_ext;
     const uint64_t* rc_int = gl::h_p2_rc_int;
     const uint64_t* diag = gl::h_p2_diag;
@@ -77,6 +77,103 @@ static inline void permute(uint64_t* s) {
         external_linear(s, r < 7 ? rc_ext[r + 1] : nullptr);
     }
     for (int i = 0; i < 8; i++) s[i] = s[i] >= gl::P ? s[i] - gl::P : s[i];
+}
+
+#if defined(__x86_64__)
+// The same permutation for an x86-64 core with BMI2, the products and reductions in assembly. The compiled form above
+// is bound by its micro-operations (about 14 per product and reduction, and the spills between them); here a product
+// and its reduction are nine: the borrow of lo - hi_hi is a jump that is taken once in 2^32 products, hi_lo (2^32 - 1)
+// is one multiplication, and only the last carry (a coin flip) is repaired without a branch. 0.85 -> 0.57 us a
+// permutation on a 16-core Sapphire-Rapids-class host. In the internal rounds (d_0 + 1) x x^2 is formed beside x^3 and x^4, so that lane 0's
+// next value is three products after this one instead of four, and the other lanes' sum is one round behind it.
+#define MB_P2_RED                                                                                                     \
+    "mov %k[hi], %k[t]\n\timul %[eps], %[t]\n\tshr $32, %[hi]\n\tsub %[hi], %[lo]\n\tjb 2f\n1:\tadd %[t], %[lo]\n\t"  \
+    "sbb %k[t], %k[t]\n\tadd %[t], %[lo]\n\t.subsection 1\n2:\tsub %[eps], %[lo]\n\tjmp 1b\n\t.previous"
+namespace bmi2 {
+// a b, a b + c and a b + c + d mod p, loose ((2^64 - 1)^2 + 2 (2^64 - 1) < 2^128)
+static inline uint64_t mul(uint64_t a, uint64_t b) {
+    uint64_t lo, hi, t;
+    asm("mulx %[b], %[lo], %[hi]\n\t" MB_P2_RED
+        : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t) : [eps] "r"(EPS), "d"(a), [b] "rm"(b) : "cc");
+    return lo;
+}
+static inline uint64_t mul_add(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t lo, hi, t;
+    asm("mulx %[b], %[lo], %[hi]\n\tadd %[c], %[lo]\n\tadc $0, %[hi]\n\t" MB_P2_RED
+        : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t) : [eps] "r"(EPS), "d"(a), [b] "rm"(b), [c] "r"(c) : "cc");
+    return lo;
+}
+static inline uint64_t mul_add2(uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+    uint64_t lo, hi, t;
+    asm("mulx %[b], %[lo], %[hi]\n\tadd %[c], %[lo]\n\tadc $0, %[hi]\n\tadd %[d], %[lo]\n\tadc $0, %[hi]\n\t" MB_P2_RED
+        : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t)
+        : [eps] "r"(EPS), "d"(a), [b] "rm"(b), [c] "r"(c), [d] "rm"(d) : "cc");
+    return lo;
+}
+// hi 2^64 + lo mod p, loose, for hi < 2^32 (the wrapped sum is below hi EPS, so the repair cannot carry)
+static inline uint64_t red_small(uint64_t lo, uint64_t hi) {
+    uint64_t u = (hi << 32) - hi;
+    asm("add %[u], %[lo]\n\tsbb %k[u], %k[u]\n\tadd %[u], %[lo]" : [lo] "+r"(lo), [u] "+r"(u) : : "cc");
+    return lo;
+}
+static inline uint64_t red_small(u128 x) { return red_small((uint64_t)x, (uint64_t)(x >> 64)); }
+static inline uint64_t sbox7(uint64_t x) {
+    const uint64_t x2 = mul(x, x), x4 = mul(x2, x2), x3 = mul(x2, x);
+    return mul(x4, x3);
+}
+static inline void full_round(uint64_t* s, const uint64_t* rc) {   // rc: the next round's constants
+    s[0] = sbox7(s[0]); s[1] = sbox7(s[1]); s[2] = sbox7(s[2]); s[3] = sbox7(s[3]);   // unrolled by hand
+    s[4] = sbox7(s[4]); s[5] = sbox7(s[5]); s[6] = sbox7(s[6]); s[7] = sbox7(s[7]);
+    u128 a[4], b[4];
+    mat4(s, a);
+    mat4(s + 4, b);
+    const auto out = [&](int i) {
+        const u128 sum = a[i] + b[i];
+        s[i] = red_small(a[i] + sum + rc[i]);
+        s[i + 4] = red_small(b[i] + sum + rc[i + 4]);
+    };
+    out(0); out(1); out(2); out(3);
+}
+static inline void permute(uint64_t* st) {
+    const uint64_t(*rc_ext)[8] = gl::h_p2_rc_ext;
+    const uint64_t *rc_int = gl::h_p2_rc_int, *diag = gl::h_p2_diag;
+    static const uint64_t none[8] = {};
+    uint64_t s[8];
+    for (int i = 0; i < 8; i++) s[i] = red_small((u128)st[i] + rc_ext[0][i]);
+    for (int r = 0; r < 4; r++) full_round(s, r < 3 ? rc_ext[r + 1] : none);
+    const uint64_t d0p1 = diag[0] + 1;
+    uint64_t x = red_small((u128)s[0] + rc_int[0]);
+    u128 sum = 0;
+    for (int i = 1; i < 8; i++) sum += s[i];
+    uint64_t rest = red_small(sum);   // sum of lanes 1 .. 7
+    for (int r = 0; r < 22; r++) {
+        const uint64_t x2 = mul(x, x), w = mul(x, d0p1), x4 = mul(x2, x2), w3 = mul(w, x2), x3 = mul(x2, x);
+        x = mul_add2(x4, w3, rest, r < 21 ? rc_int[r + 1] : 0);
+        const uint64_t all = red_small((u128)mul(x3, x4) + rest);
+        uint64_t lo = 0, hi = 0;
+        const auto lane = [&](int i) {
+            const uint64_t v = s[i] = mul_add(s[i], diag[i], all);
+            asm("add %[v], %[lo]\n\tadc $0, %[hi]" : [lo] "+r"(lo), [hi] "+r"(hi) : [v] "r"(v) : "cc");
+        };
+        lane(1); lane(2); lane(3); lane(4); lane(5); lane(6); lane(7);
+        rest = red_small(lo, hi);
+    }
+    s[0] = x;
+    for (int i = 0; i < 8; i++) s[i] = red_small((u128)s[i] + rc_ext[4][i]);
+    for (int r = 4; r < 8; r++) full_round(s, r < 7 ? rc_ext[r + 1] : none);
+    for (int i = 0; i < 8; i++) st[i] = s[i] >= gl::P ? s[i] - gl::P : s[i];
+}
+}  // namespace bmi2
+#undef MB_P2_RED
+static const bool have_bmi2 = [] { __builtin_cpu_init(); return __builtin_cpu_supports("bmi2") != 0; }();
+#endif
+
+// In place; any 64-bit words in, canonical residues out.
+static inline void permute(uint64_t* s) {
+#if defined(__x86_64__)
+    if (have_bmi2) return bmi2::permute(s);
+#endif
+    permute_portable(s);
 }
 
 }  // namespace p2host

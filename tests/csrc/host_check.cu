@@ -63,6 +63,7 @@ void hc_mcm_key_block(const uint32_t* seed, uint32_t kind, uint32_t row, uint64_
 void hc_poseidon2(uint64_t* s) { gl::poseidon2_permute(s); }
 // the host-side form (transcripts, tree tops) and the reductions underneath both host permutations
 void hc_poseidon2_host(uint64_t* s) { mbhost::p2host::permute(s); }
+void hc_poseidon2_host_portable(uint64_t* s) { mbhost::p2host::permute_portable(s); }
 // host-form extension arithmetic (the last rounds of a sumcheck): o = a * b, a + b, a - b on canonical words
 void hc_hf_e2(int agl_field, const uint64_t* a, const uint64_t* b, uint64_t* o) {
     using namespace mbhost::hf;
@@ -108,6 +109,8 @@ void hc_tree_top(int hash, const uint64_t* nodes, size_t count, uint64_t* upper,
     mbhost::host_hash_top(hash, nodes, count, upper, root);
 }
 void hc_gl_monolith_host(uint64_t* s) { mbhost::monohost::permute(s); }
+void hc_gl_monolith_host_portable(uint64_t* s) { mbhost::monohost::permute_portable(s); }
+void hc_agl_monolith_portable(uint64_t* s) { mbhost::aglm::permute_portable(s); }
 void hc_agl_monolith(uint64_t* s) { mbhost::aglm::permute(s); }
 uint64_t hc_agl_reduce_limb_sums(uint64_t L, uint64_t H) { return agl::reduce_limb_sums(L, H); }
 
