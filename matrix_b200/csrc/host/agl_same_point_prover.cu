@@ -14,40 +14,19 @@
 // width 12) and is advanced exactly as the reference's prover advances it, so proofs are interchangeable with
 // the CPU prover's (heterogeneous arities stay on that path, as in the reference).
 //
-// Device side: two ping-pong buffers of M x (eq | f) tables; the eq tables of all leaves are built in two launches.
-// A binary witness is never lifted: round 0 reads the packed bits, afterwards everything is an extension table.
-// Per round: ONE pass over the tables (the fold on the challenge and the per-leaf sums of the next round in the
-// same kernel; the reference folds, then reads the folded tables again), one small launch that adds the blocks'
-// partial sums, a 48-byte-per-leaf read-back into page-locked memory, the host combination with the powers of
-// alpha and the transcript. The header of the transcript (every claim point) is absorbed while the device builds
-// the tables and the first message.
+// Device side (same_point_kernels.cuh): the eq polynomials stay factored, and one pass over a table serves up to four
+// rounds (six for the packed witness): it returns 2^B eq-weighted sums per leaf, on which the host runs the messages
+// and folds of B rounds, and the next pass folds the B challenges at once. The first pass is queued before the header of
+// the transcript (every claim point, label by label), which the host absorbs while the device works: after the pass
+// that header is the longest part of a proof. The reference launches a message and a fold kernel per round over eq and f
+// tables; with one fused pass per round over both tables, arity 22 and 42 binary leaves took 7.4 ms and 11 GB.
 #include <vector>
-#include "../agl_traits.cuh"
-#include "../eq_kernels.cuh"
+#include "../same_point_kernels.cuh"
 #include "agl_transcript.hpp"
+#include "host_field.hpp"
 
 using namespace mb;
 using namespace mb::sc;
-
-extern "C" {
-int aext2_sumcheck_batched_round_message_ffi(const uint64_t* d_polys, uint64_t* d_partial, size_t original_size, size_t half,
-                                             int num_leaves, int num_blocks_x);
-int aext2_sumcheck_batched_fold_ffi(const uint64_t* d_input, uint64_t* d_output, uint64_t challenge_c0, uint64_t challenge_c1,
-                                    size_t original_size, size_t half, int num_leaves);
-int aext2_sumcheck_batched_round0_binary_msg_ffi(const uint64_t* d_polys, const uint64_t* d_packed, uint64_t* d_partial,
-                                                 size_t original_size, size_t half, int num_leaves, int num_blocks_x,
-                                                 size_t packed_size_u64);
-int aext2_sumcheck_batched_round0_binary_fold_ffi(const uint64_t* d_polys, const uint64_t* d_packed, uint64_t* d_output,
-                                                  uint64_t challenge_c0, uint64_t challenge_c1, size_t original_size, size_t half,
-                                                  int num_leaves, size_t packed_size_u64);
-int aext2_sumcheck_batched_fold_message_ffi(const uint64_t* d_input, uint64_t* d_output, uint64_t challenge_c0, uint64_t challenge_c1,
-                                            size_t original_size, size_t half, int num_leaves, int num_blocks_x, uint64_t* d_partial);
-int aext2_sumcheck_batched_round0_binary_fold_message_ffi(const uint64_t* d_polys, const uint64_t* d_packed, uint64_t* d_output,
-                                                          uint64_t challenge_c0, uint64_t challenge_c1, size_t original_size, size_t half,
-                                                          int num_leaves, int num_blocks_x, size_t packed_size_u64, uint64_t* d_partial);
-int aext2_batched_lift_ternary_single_ffi(const uint64_t* d_pos, const uint64_t* d_neg, uint64_t* d_polys, size_t original_size,
-                                          int num_leaves, size_t packed_size_u64);
-}
 
 namespace mbhost {
 
@@ -67,30 +46,6 @@ inline E2 challenge(AglTranscript& t, const uint8_t* l, size_t n) {
     uint64_t w[2];
     t.challenge_vector(l, n, w, 2);   // the label once, two squeezes (transcript.rs:120-125)
     return E2{w[0], w[1]};
-}
-
-// sums[leaf][c][2] = sum over the blocks of partial[block][leaf][c][2]: one thread per output word
-__global__ void add_blocks_kernel(const uint64_t* __restrict__ partial, int blocks, int words, uint64_t* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= words) return;
-    uint64_t s = 0;
-    for (int b = 0; b < blocks; b++) s = agl::add(s, partial[(size_t)b * words + k]);
-    out[k] = agl::canon(s);
-}
-
-// out[leaf][2] = element 0 of every leaf's f table
-__global__ void first_f_kernel(const uint64_t* __restrict__ polys, size_t n, int leaves, uint64_t* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < 2 * leaves) out[k] = polys[(size_t)(k >> 1) * 4 * n + 2 * n + (k & 1)];
-}
-
-// dense witness: the caller's [leaf][n][2] tables into the f halves of the interleaved buffer
-__global__ void place_dense_kernel(const uint64_t* __restrict__ src, uint64_t* __restrict__ polys, size_t n) {
-    const size_t step = (size_t)gridDim.x * blockDim.x;
-    const uint64_t* s = src + (size_t)blockIdx.y * 2 * n;
-    uint64_t* d = polys + (size_t)blockIdx.y * 4 * n + 2 * n;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
-        agl::e2_store(d + 2 * i, E2{agl::canon(s[2 * i]), agl::canon(s[2 * i + 1])});
 }
 
 void header(AglTranscript& t, int M, int arity, const uint64_t* pts, const uint64_t* vals) {   // same_point_sumcheck.rs:78-87
@@ -116,42 +71,57 @@ E2 eq_eval(const uint64_t* a, const E2* b, int n) {   // same_point_sumcheck.rs:
     return acc;
 }
 
-struct Buffers {
-    uint64_t *a = nullptr, *b = nullptr, *partial = nullptr, *sums = nullptr, *pts = nullptr, *scratch = nullptr;
-    ~Buffers() { pool_free(a); pool_free(b); pool_free(partial); pool_free(sums); pool_free(pts); pool_free(scratch); }
+// ---- the rounds of one pass on the host -------------------------------------------------------
+E2 mul(E2 a, E2 b) {   // canonical words in and out, on the host core's multiplier
+    E2 r;
+    hf::e2_mul<hf::AglE2Ops>(a.c0, a.c1, b.c0, b.c1, r.c0, r.c1);
+    return r;
+}
+E2 add(E2 a, E2 b) { return E2{hf::agl_add(a.c0, b.c0), hf::agl_add(a.c1, b.c1)}; }
+E2 sub(E2 a, E2 b) { return E2{hf::agl_sub(a.c0, b.c0), hf::agl_sub(a.c1, b.c1)}; }
+// sum of products, reduced once
+struct Dot {
+    struct Wide {
+        hf::u128 s = 0;
+        uint64_t top = 0;
+        void mac(uint64_t x, uint64_t y) {
+            const hf::u128 p = (hf::u128)x * y;
+            s += p;
+            top += s < p;
+        }
+        // 2^128 = 63 2^32 + 992 (mod q)
+        uint64_t red() const { return hf::agl_red((hf::u128)top * (63ULL * (1ULL << 32) + 992ULL) + hf::agl_red(s)); }
+    };
+    Wide p00, p11, p01;
+    void mac(E2 a, E2 b) {
+        p00.mac(a.c0, b.c0);
+        p11.mac(a.c1, b.c1);
+        p01.mac(a.c0, b.c1);
+        p01.mac(a.c1, b.c0);
+    }
+    E2 value() const {
+        return E2{hf::agl_canon(hf::agl_red((hf::u128)p11.red() * 3 + p00.red())), hf::agl_canon(p01.red())};
+    }
 };
 
-// Device state of M leaves of 2^arity points: eq tables from the claim points, and the f tables unless the
-// witness is binary (round 0 reads the packed bits).
-int setup(Buffers& buf, int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool two_buffers,
-          int& blocks) {
-    const size_t n = (size_t)1 << arity, words = arity >= 6 ? n >> 6 : 1;
-    blocks = (int)(n / 2 >= (size_t)256 * 64 ? 64 : (n / 2 + 255) / 256 > 0 ? (n / 2 + 255) / 256 : 1);
-    const int sum_words = 6 * M;
-    MB_CUDA(pool_alloc((void**)&buf.a, sizeof(uint64_t) * 4 * n * (size_t)M));
-    if (two_buffers) MB_CUDA(pool_alloc((void**)&buf.b, sizeof(uint64_t) * 4 * n * (size_t)M));
-    MB_CUDA(pool_alloc((void**)&buf.partial, sizeof(uint64_t) * (size_t)blocks * sum_words));
-    MB_CUDA(pool_alloc((void**)&buf.sums, sizeof(uint64_t) * sum_words));
-    MB_CUDA(pool_alloc((void**)&buf.pts, sizeof(uint64_t) * 2 * (size_t)arity * M));
-    MB_CUDA(pool_alloc((void**)&buf.scratch,
-                       sizeof(uint64_t) * 2 * (size_t)M * (((size_t)1 << (arity / 2)) + ((size_t)1 << (arity - arity / 2)))));
-    MB_CUDA(cudaMemcpyAsync(buf.pts, h_pts, sizeof(uint64_t) * 2 * (size_t)arity * M, cudaMemcpyHostToDevice, MB_STREAM));
-    // eq tables from the claim points, on the device, into the eq halves: all leaves in two launches
-    int rc = eq::build_batched<AglExt2>(buf.pts, 2 * (size_t)arity, buf.a, 4 * n, buf.scratch, arity, M, MB_STREAM);
-    if (rc != MB_OK) return rc;
-    if (kind == 1) {
-        rc = aext2_batched_lift_ternary_single_ffi(d_w0, d_w1, buf.a, n, M, words);
-    } else if (kind == 2) {
-        MB_KERNEL("same_point_place");
-        dim3 grid(grid_for(n, 256, 8), M);
-        place_dense_kernel<<<grid, 256, 0, MB_STREAM>>>(d_w0, buf.a, n);
-        rc = finish_async();
-    }
-    return rc;
-}
+// A block of rounds from variable `first` on, and what the pass before it reads.
+enum Source { FROM_WITNESS, FROM_WORD_SUMS, FROM_WORDS, FROM_TABLE };
+struct Stage {
+    int first, rounds;
+    Source source;
+    size_t wl = 0, wh = 0;
+};
 
-// Page-locked landing zone of the calling thread for the per-leaf sums (grown on demand, kept between calls): a
-// read-back into it is asynchronous, so the host can work while the device finishes the round.
+struct Buffers {
+    uint64_t *pts = nullptr, *tabs = nullptr, *partial = nullptr, *g6 = nullptr, *t0 = nullptr, *t1 = nullptr;
+    unsigned* counter = nullptr;
+    ~Buffers() {
+        pool_free(pts); pool_free(tabs); pool_free(partial); pool_free(g6); pool_free(t0); pool_free(t1); pool_free(counter);
+    }
+};
+
+// Page-locked landing zone of the calling thread for the sums (grown on demand, kept between calls): the last block of
+// a pass writes them there.
 uint64_t* pinned_words(size_t words) {
     struct Holder {
         uint64_t* p = nullptr;
@@ -169,61 +139,180 @@ uint64_t* pinned_words(size_t words) {
     return h.p;
 }
 
-inline int blocks_for(size_t pairs, int blocks) { return (int)((pairs + 255) / 256 < (size_t)blocks ? (pairs + 255) / 256 : blocks); }
-
-// Adds the blocks' partial sums and queues the read-back of sums[leaf][3][2] into h_sums.
-int queue_sums(Buffers& buf, int M, int bx, uint64_t* h_sums) {
-    const int sum_words = 6 * M;
-    {
-        MB_KERNEL("same_point_add_blocks");
-        add_blocks_kernel<<<(sum_words + 127) / 128, 128, 0, MB_STREAM>>>(buf.partial, bx, sum_words, buf.sums);
+class SamePointDevice {
+public:
+    // Stages of the proof, eq tables of all passes, and the first pass, all queued; the sums of the first stage are in
+    // sums() after a stream synchronisation. claims_only: nothing after the first pass will be asked for.
+    int init(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool claims_only) {
+        M_ = M; k_ = arity; kind_ = kind; w0_ = d_w0; w1_ = d_w1;
+        const int inside = kind == 2 ? 0 : (arity < sp::BITS ? arity : sp::BITS);
+        words_ = arity >= 6 ? (size_t)1 << (arity - 6) : 1;
+        if (inside) {
+            const int b0 = (inside + 1) / 2;
+            stages_.push_back({0, b0, FROM_WITNESS});
+            if (inside > b0) stages_.push_back({b0, inside - b0, FROM_WORD_SUMS});
+        }
+        const int rest = arity - inside, parts = (rest + sp::MAX_B - 1) / sp::MAX_B;
+        for (int i = 0, at = inside; i < parts; i++) {
+            const int b = (arity - at + (parts - i) - 1) / (parts - i);
+            stages_.push_back({at, b, at == inside ? (inside ? FROM_WORDS : FROM_WITNESS) : FROM_TABLE});
+            at += b;
+        }
+        // eq tables: per pass over the variables the thread index and the loop counter stand for
+        sp::TableSet set;
+        int nt = 0;
+        const auto table = [&](int first, int bits) {
+            set.d[nt].first = first;
+            set.d[nt].bits = bits;
+            set.d[nt].off = leaf_words_;
+            leaf_words_ += (size_t)4 << bits;
+            return set.d[nt++].off;
+        };
+        size_t low_off = 0;
+        const int lo_bits = rest < 8 ? rest : 8;
+        for (Stage& s : stages_) {
+            if (s.source == FROM_WITNESS && inside) {
+                s.wl = table(inside, lo_bits);
+                s.wh = table(inside + lo_bits, rest - lo_bits);
+                low_off = table(s.rounds, inside - s.rounds);
+            } else if (s.source != FROM_WORD_SUMS) {
+                const int v = arity - s.first, tb = v < 8 ? v : 8;
+                s.wl = table(s.first + s.rounds, tb - s.rounds);
+                s.wh = table(s.first + tb, v - tb);
+            }
+            if (claims_only) break;
+        }
+        const int cap = sm_count() * 8 / M > 1 ? sm_count() * 8 / M : 1;
+        max_blocks_ = cap;
+        MB_CUDA(pool_alloc((void**)&b_.pts, sizeof(uint64_t) * 2 * (size_t)arity * M));
+        MB_CUDA(pool_alloc((void**)&b_.tabs, sizeof(uint64_t) * leaf_words_ * M));
+        MB_CUDA(pool_alloc((void**)&b_.partial, sizeof(uint64_t) * 2 * 64 * (size_t)cap * M));
+        MB_CUDA(pool_alloc((void**)&b_.counter, sizeof(unsigned) * M));
+        if (inside) MB_CUDA(pool_alloc((void**)&b_.g6, sizeof(uint64_t) * 2 * 64 * (size_t)M));
+        // staging: the points go up from page-locked memory, the sums come back behind them
+        const size_t pt_words = 2 * (size_t)arity * M;
+        uint64_t* pin = pinned_words(pt_words + ((size_t)2 << sp::MAX_B) * M);
+        if (!pin) return MB_ERR_CUDA;
+        for (size_t i = 0; i < pt_words; i++) pin[i] = h_pts[i];
+        h_sums_ = pin + pt_words;
+        MB_CUDA(cudaMemcpyAsync(b_.pts, pin, sizeof(uint64_t) * pt_words, cudaMemcpyHostToDevice, MB_STREAM));
+        MB_CUDA(cudaMemsetAsync(b_.counter, 0, sizeof(unsigned) * M, MB_STREAM));
+        {
+            MB_KERNEL("same_point_eq_tables");
+            sp::eq_tables_kernel<<<dim3(nt, M), sp::BLK, 0, MB_STREAM>>>(set, b_.pts, arity, b_.tabs, leaf_words_);
+        }
+        if (!inside) return fold(0, nullptr, 0);
+        sp::BitsArgs a;
+        a.pos = d_w0; a.neg = d_w1; a.words = words_;
+        a.lo_bits = lo_bits; a.hi_bits = rest - lo_bits; a.in_bits = inside; a.first_bits = stages_[0].rounds;
+        a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = stages_[0].wl; a.wh_off = stages_[0].wh; a.low_off = low_off;
+        a.partial = b_.partial; a.g6 = b_.g6; a.counter = b_.counter; a.out = h_sums_;
+        // eight warps a block, a warp per high index: a power of two of blocks, so that no warp has more of them
+        int gx = 1;
+        while (2 * gx <= cap && (size_t)16 * gx <= ((size_t)1 << a.hi_bits)) gx *= 2;
+        {
+            MB_KERNEL("same_point_bits");
+            if (kind == 1) sp::bits_pass_kernel<true><<<dim3(gx, M), sp::BLK, 0, MB_STREAM>>>(a);
+            else sp::bits_pass_kernel<false><<<dim3(gx, M), sp::BLK, 0, MB_STREAM>>>(a);
+        }
+        return finish_async();
     }
-    MB_CUDA(cudaMemcpyAsync(h_sums, buf.sums, sizeof(uint64_t) * sum_words, cudaMemcpyDeviceToHost, MB_STREAM));
-    return MB_OK;
-}
+    // The pass before stage i: folds the challenges r[0 .. count) that bind the variables the pass consumes (all six of
+    // a word for the first extension table, those of the stage before otherwise) and queues the sums of stage i.
+    int fold(size_t i, const E2* r, int count) {
+        const Stage& s = stages_[i];
+        sp::FoldArgs a{};
+        a.v = k_ - s.first;
+        a.next = s.rounds;
+        if (s.source == FROM_WORD_SUMS) a.v = s.rounds;   // the other variables are summed already
+        a.t_bits = a.v < 8 ? a.v : 8;
+        a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = s.wl; a.wh_off = s.wh;
+        a.partial = b_.partial; a.counter = b_.counter; a.out = h_sums_;
+        const size_t iters = (size_t)1 << (a.v - a.t_bits);
+        const int half = (max_blocks_ + 1) / 2, gx = iters < (size_t)half ? (int)iters : half;
+        const dim3 grid(gx, M_);
+        if (s.source == FROM_WORD_SUMS) {
+            a.in = b_.g6; a.in_stride = 2 * 64;
+        } else if (s.source == FROM_WORDS) {
+            a.in = w0_; a.neg = w1_; a.in_stride = words_;
+        } else {   // the caller's extension tables serve the first two passes
+            a.in = kind_ == 2 && i <= 1 ? w0_ : cur_;
+            a.in_stride = (size_t)2 << (a.v + count);
+        }
+        // a table is stored only for a pass that will read it
+        if (i + 1 < stages_.size() && s.source != FROM_WITNESS && s.source != FROM_WORD_SUMS) {
+            uint64_t*& t = flip_ ? b_.t1 : b_.t0;
+            if (!t) MB_CUDA(pool_alloc((void**)&t, sizeof(uint64_t) * ((size_t)2 << a.v) * M_));
+            a.table = cur_ = t;
+            flip_ = !flip_;
+        }
+        if (s.source == FROM_WORDS) {
+            sp::WordWeights w;
+            eq_vector(r, count, w.w);
+            for (int j = 1 << count; j < 64; j++) w.w[j] = E2{0, 0};
+            MB_KERNEL("same_point_words");
+            constexpr int lut = 8 * 256 * 16;
+            if (kind_ == 1) sp::fold_pass_kernel<0, 2, sp::WordWeights><<<grid, sp::BLK, lut, MB_STREAM>>>(a, w);
+            else sp::fold_pass_kernel<0, 1, sp::WordWeights><<<grid, sp::BLK, lut, MB_STREAM>>>(a, w);
+            return finish_async();
+        }
+        sp::FoldWeights w;
+        E2 e[1 << sp::MAX_B];
+        eq_vector(r, count, e);
+        for (int j = 0; j < (1 << count); j++) w.w[j] = agl::e2_pre(e[j]);
+        MB_KERNEL("same_point_fold");
+        switch (count) {
+            case 0: sp::fold_pass_kernel<0, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+            case 1: sp::fold_pass_kernel<1, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+            case 2: sp::fold_pass_kernel<2, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+            case 3: sp::fold_pass_kernel<3, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+            default: sp::fold_pass_kernel<4, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+        }
+        return finish_async();
+    }
+    const std::vector<Stage>& stages() const { return stages_; }
+    const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the stage queued last
 
-// Per-leaf T_i(0), T_i(1), T_i(2) of the current round into h_sums[leaf][3][2] (page-locked): launches and the
-// read-back are queued; the caller synchronises the stream before it reads h_sums.
-int leaf_messages(Buffers& buf, const uint64_t* cur, int M, size_t n, size_t half, int blocks, bool bits, const uint64_t* d_packed,
-                  size_t words, uint64_t* h_sums) {
-    const int bx = blocks_for(half, blocks);
-    int rc = bits ? aext2_sumcheck_batched_round0_binary_msg_ffi(cur, d_packed, buf.partial, n, half, M, bx, words)
-                  : aext2_sumcheck_batched_round_message_ffi(cur, buf.partial, n, half, M, bx);
-    if (rc != MB_OK) return rc;
-    return queue_sums(buf, M, bx, h_sums);
-}
-
-// The fold on r fused with the per-leaf sums of the next round (input half >= 2); h_sums as above.
-int fold_and_next_messages(Buffers& buf, const uint64_t* cur, uint64_t* other, E2 r, int M, size_t n, size_t half, int blocks, bool bits,
-                           const uint64_t* d_packed, size_t words, uint64_t* h_sums) {
-    const int bx = blocks_for(half / 2, blocks);
-    int rc = bits ? aext2_sumcheck_batched_round0_binary_fold_message_ffi(cur, d_packed, other, r.c0, r.c1, n, half, M, bx, words, buf.partial)
-                  : aext2_sumcheck_batched_fold_message_ffi(cur, other, r.c0, r.c1, n, half, M, bx, buf.partial);
-    if (rc != MB_OK) return rc;
-    return queue_sums(buf, M, bx, h_sums);
-}
+private:
+    // out[x] = prod_k (x_k ? r_k : 1 - r_k)
+    static void eq_vector(const E2* r, int n, E2* out) {
+        out[0] = E2{1, 0};
+        for (int b = 0; b < n; b++)
+            for (int x = 0; x < (1 << b); x++) {
+                const E2 hi = mul(out[x], r[b]);
+                out[x + (1 << b)] = hi;
+                out[x] = sub(out[x], hi);
+            }
+    }
+    int M_ = 0, k_ = 0, kind_ = 0, max_blocks_ = 1;
+    size_t words_ = 1, leaf_words_ = 0;
+    const uint64_t *w0_ = nullptr, *w1_ = nullptr;
+    uint64_t *h_sums_ = nullptr, *cur_ = nullptr;
+    bool flip_ = false;
+    std::vector<Stage> stages_;
+    Buffers b_;
+};
 
 }  // namespace
 
 // y_i = f_i(r_i) for every leaf: the claims the protocol starts from (FoldData::evaluate_at_ext2,
-// zk-torch-4/src/fold/mod.rs:107-110), as sum_x eq(r_i, x) f_i(x) = T_i(0) + T_i(1) of the first round.
+// zk-torch-4/src/fold/mod.rs:107-110), as sum_m eq(r_i[0 .. B), m) G_i(m) over the sums of the first stage.
 int same_point_claims(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, uint64_t* h_vals) {
     if (M < 1 || M > 4096 || arity < 1 || arity > 32 || !h_pts || !d_w0 || kind < 0 || kind > 2 || (kind == 1 && !d_w1) || !h_vals)
         return MB_ERR_ARG;
-    const size_t n = (size_t)1 << arity, words = arity >= 6 ? n >> 6 : 1;
-    Buffers buf;
-    int blocks = 1;
-    int rc = setup(buf, M, arity, h_pts, kind, d_w0, d_w1, false, blocks);
-    if (rc != MB_OK) return rc;
-    uint64_t* h_sums = pinned_words(6 * (size_t)M);
-    if (!h_sums) return MB_ERR_CUDA;
-    rc = leaf_messages(buf, buf.a, M, n, n / 2, blocks, kind == 0, d_w0, words, h_sums);
+    SamePointDevice dev;
+    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, true);
     if (rc != MB_OK) return rc;
     MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+    const int b = dev.stages()[0].rounds;
     for (int i = 0; i < M; i++) {
-        const E2 y = e2c(agl::e2_add(ld(h_sums + 6 * (size_t)i), ld(h_sums + 6 * (size_t)i + 2)));
-        h_vals[2 * i] = y.c0;
-        h_vals[2 * i + 1] = y.c1;
+        E2 g[1 << sp::MAX_B];
+        for (int m = 0; m < (1 << b); m++) g[m] = ld(dev.sums() + 2 * (((size_t)i << b) + m));
+        for (int j = 0; j < b; j++)
+            for (int m = 0; m < (1 << (b - j - 1)); m++)
+                g[m] = add(g[2 * m], mul(ld(h_pts + 2 * ((size_t)i * arity + j)), sub(g[2 * m + 1], g[2 * m])));
+        h_vals[2 * i] = g[0].c0;
+        h_vals[2 * i + 1] = g[0].c1;
     }
     return MB_OK;
 }
@@ -236,79 +325,107 @@ int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_
     if (M < 1 || M > 4096 || arity < 1 || arity > 32 || !h_pts || !h_vals || !d_w0 || kind < 0 || kind > 2 || (kind == 1 && !d_w1) ||
         !h_round_msgs || !h_f_evals || !h_final_eval)
         return MB_ERR_ARG;
-    const size_t n = (size_t)1 << arity, words = arity >= 6 ? n >> 6 : 1;
-    Buffers buf;
-    int blocks = 1;
-    const int sum_words = 6 * M;
-    uint64_t* h_sums = pinned_words(sum_words);
-    if (!h_sums) return MB_ERR_CUDA;
-    // the tables and the first round's per-leaf sums do not depend on alpha: they are queued first, and the
-    // header of the transcript (every claim point, label by label: the longest host step of the proof) is
-    // absorbed while the device works
-    int rc = setup(buf, M, arity, h_pts, kind, d_w0, d_w1, true, blocks);
-    if (rc != MB_OK) return rc;
-    rc = leaf_messages(buf, buf.a, M, n, n / 2, blocks, kind == 0, d_w0, words, h_sums);
+    // the first pass does not depend on alpha: it is queued first, and the header of the transcript (every claim
+    // point, label by label) is absorbed while the device works
+    SamePointDevice dev;
+    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, false);
     if (rc != MB_OK) return rc;
     header(t, M, arity, h_pts, h_vals);
     const E2 alpha = challenge(t, SP_LABEL(L_ALPHA));
-    std::vector<E2> alphas(M);
+    // scale_i = alpha^i eq(r_i[0 .. j), R[0 .. j))
+    std::vector<E2> scale(M);
     E2 pw{1, 0};
-    for (int i = 0; i < M; i++) { alphas[i] = pw; pw = e2c(agl::e2_mul(pw, alpha)); }
+    for (int i = 0; i < M; i++) { scale[i] = pw; pw = mul(pw, alpha); }
 
-    std::vector<E2> R(arity);
+    std::vector<E2> R(arity), g((size_t)M << sp::MAX_B), up(M), down(M);
+    // suffix eq tables of the block's variables, per leaf: 2^(rounds - 1 - j) entries for round j, back to back
+    std::vector<E2> suffix((size_t)M << sp::MAX_B);
     bool label_absorbed = false;
-    uint64_t* cur = buf.a;
-    uint64_t* other = buf.b;
-    for (int round = 0; round < arity; round++) {
-        const size_t half = n >> (round + 1);
-        const bool bits = kind == 0 && round == 0;
-        // this round's sums were queued with the setup (round 0) or by the fold of the round before
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        E2 msg[3] = {{0, 0}, {0, 0}, {0, 0}};
-        for (int i = 0; i < M; i++)
-            for (int c = 0; c < 3; c++) msg[c] = agl::e2_add(msg[c], agl::e2_mul(alphas[i], ld(h_sums + (size_t)i * 6 + 2 * c)));
-        for (int c = 0; c < 3; c++) {
-            msg[c] = e2c(msg[c]);
-            if (c > 0 || !label_absorbed) t.begin_append(SP_LABEL(L_MSG));
-            t.finish_append_ext2(msg[c].c0, msg[c].c1);
-            h_round_msgs[((size_t)round * 3 + c) * 2] = msg[c].c0;
-            h_round_msgs[((size_t)round * 3 + c) * 2 + 1] = msg[c].c1;
+    for (size_t si = 0; si < dev.stages().size(); si++) {
+        const Stage st = dev.stages()[si];
+        if (si > 0) {
+            // the challenges that the pass consumes: all of a word's for the first extension table
+            const int from = st.source == FROM_WORDS ? 0 : dev.stages()[si - 1].first;
+            rc = dev.fold(si, R.data() + from, st.first - from);
+            if (rc != MB_OK) return rc;
         }
-        const E2 r = challenge(t, SP_LABEL(L_CH));
-        R[round] = r;
-        if (h_challenges) { h_challenges[2 * round] = r.c0; h_challenges[2 * round + 1] = r.c1; }
-        if (half >= 2)
-            rc = fold_and_next_messages(buf, cur, other, r, M, n, half, blocks, bits, d_w0, words, h_sums);
-        else
-            rc = bits ? aext2_sumcheck_batched_round0_binary_fold_ffi(cur, d_w0, other, r.c0, r.c1, n, half, M, words)
-                      : aext2_sumcheck_batched_fold_ffi(cur, other, r.c0, r.c1, n, half, M);
-        if (rc != MB_OK) return rc;
-        // the next message's first label is absorbed while the fold runs
-        label_absorbed = round + 1 < arity;
-        if (label_absorbed) t.begin_append(SP_LABEL(L_MSG));
-        uint64_t* tmp = cur; cur = other; other = tmp;
+        if (si > 0) {   // while the pass runs
+            t.begin_append(SP_LABEL(L_MSG));
+            label_absorbed = true;
+        }
+        const int B = st.rounds, size = 1 << B;
+        for (int i = 0; i < M; i++) {
+            // tables for rounds B - 1, B - 2, ..: each from the one before by its lowest variable
+            E2* w = suffix.data() + ((size_t)i << B);
+            w[0] = E2{1, 0};
+            int at = 0;
+            for (int j = B - 2; j >= 0; j--) {
+                const E2 rj = ld(h_pts + 2 * ((size_t)i * arity + st.first + j + 1));
+                const int n = 1 << (B - 2 - j);
+                for (int y = 0; y < n; y++) {
+                    const E2 hi = mul(w[at + y], rj);
+                    w[at + n + 2 * y + 1] = hi;
+                    w[at + n + 2 * y] = sub(w[at + y], hi);
+                }
+                at += n;
+            }
+        }
+        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        for (size_t x = 0; x < (size_t)M * size; x++) g[x] = E2{dev.sums()[2 * x], dev.sums()[2 * x + 1]};
+        for (int j = 0; j < B; j++) {
+            const int round = st.first + j, half = size >> (j + 1);
+            // T_i(c) = scale_i ((1 - r)(1 - c) + r c) (A + c (B - A)) with A, B the weighted even and odd sums;
+            // with u = scale (1 - r), v = scale r: T(0) = u A, T(1) = v B, T(2) = (2 v - u)(2 B - A)
+            Dot m0, m1, m2;
+            for (int i = 0; i < M; i++) {
+                const E2* w = suffix.data() + ((size_t)i << B) + (half - 1);
+                const E2* gi = g.data() + (size_t)i * size;
+                E2 a = gi[0], b = gi[1];
+                if (half > 1) {
+                    Dot da, db;
+                    for (int y = 0; y < half; y++) { da.mac(w[y], gi[2 * y]); db.mac(w[y], gi[2 * y + 1]); }
+                    a = da.value();
+                    b = db.value();
+                }
+                up[i] = mul(scale[i], ld(h_pts + 2 * ((size_t)i * arity + round)));
+                down[i] = sub(scale[i], up[i]);
+                m0.mac(down[i], a);
+                m1.mac(up[i], b);
+                m2.mac(sub(add(up[i], up[i]), down[i]), sub(add(b, b), a));
+            }
+            const E2 msg[3] = {m0.value(), m1.value(), m2.value()};
+            for (int c = 0; c < 3; c++) {
+                if (c > 0 || !label_absorbed) t.begin_append(SP_LABEL(L_MSG));
+                t.finish_append_ext2(msg[c].c0, msg[c].c1);
+                h_round_msgs[((size_t)round * 3 + c) * 2] = msg[c].c0;
+                h_round_msgs[((size_t)round * 3 + c) * 2 + 1] = msg[c].c1;
+            }
+            label_absorbed = false;
+            const E2 r = challenge(t, SP_LABEL(L_CH));
+            R[round] = r;
+            if (h_challenges) { h_challenges[2 * round] = r.c0; h_challenges[2 * round + 1] = r.c1; }
+            const bool last = si + 1 == dev.stages().size();
+            for (int i = 0; i < M; i++) {
+                scale[i] = add(down[i], mul(r, sub(up[i], down[i])));
+                if (j + 1 == B && !last) continue;   // the next pass folds
+                E2* gi = g.data() + (size_t)i * size;
+                for (int y = 0; y < half; y++) gi[y] = add(gi[2 * y], mul(r, sub(gi[2 * y + 1], gi[2 * y])));
+            }
+        }
+        if (si + 1 == dev.stages().size())
+            for (int i = 0; i < M; i++) {   // nothing is left to sum over: the folded sums are the reveals f_i(R)
+                h_f_evals[2 * i] = g[(size_t)i * size].c0;
+                h_f_evals[2 * i + 1] = g[(size_t)i * size].c1;
+            }
     }
-    // reveals f_i(R): element 0 of every leaf's f table
-    std::vector<uint64_t> fe(2 * (size_t)M);
-    {
-        MB_KERNEL("same_point_reveals");
-        first_f_kernel<<<(2 * M + 127) / 128, 128, 0, MB_STREAM>>>(cur, n, M, buf.sums);
-    }
-    MB_CUDA(cudaMemcpyAsync(fe.data(), buf.sums, sizeof(uint64_t) * 2 * (size_t)M, cudaMemcpyDeviceToHost, MB_STREAM));
-    MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-    E2 fin{0, 0};
+    Dot fin;
     for (int i = 0; i < M; i++) {
-        t.append_ext2(SP_LABEL(L_FEVAL), fe[2 * i], fe[2 * i + 1]);
-        h_f_evals[2 * i] = fe[2 * i];
-        h_f_evals[2 * i + 1] = fe[2 * i + 1];
+        t.append_ext2(SP_LABEL(L_FEVAL), h_f_evals[2 * i], h_f_evals[2 * i + 1]);
+        fin.mac(scale[i], E2{h_f_evals[2 * i], h_f_evals[2 * i + 1]});   // scale_i = alpha^i eq(r_i, R)
     }
-    for (int i = 0; i < M; i++) {
-        const E2 eq_i = eq_eval(h_pts + 2 * (size_t)arity * i, R.data(), arity);
-        fin = agl::e2_add(fin, agl::e2_mul(alphas[i], e2c(agl::e2_mul(eq_i, ld(fe.data() + 2 * i)))));
-    }
-    fin = e2c(fin);
-    h_final_eval[0] = fin.c0;
-    h_final_eval[1] = fin.c1;
+    const E2 v = fin.value();
+    h_final_eval[0] = v.c0;
+    h_final_eval[1] = v.c1;
     return MB_OK;
 }
 
@@ -377,7 +494,8 @@ extern "C" {
 // device: kind 0 binary packed (d_w0[num_leaves][words], words = max(1, 2^(arity - 6))), 1 ternary single chunk
 // (d_w0 = +1 masks, d_w1 = -1 masks), 2 extension tables (d_w0[num_leaves][2^arity][2]). `transcript`: a handle
 // from agl_transcript_create, advanced by the proof. Host outputs: round_msgs[arity][3][2], challenges[arity][2]
-// (may be null), f_evals[num_leaves][2], final_eval[2]. Needs 2 x num_leaves x 2^arity x 32 bytes of device memory.
+// (may be null), f_evals[num_leaves][2], final_eval[2]. Device memory beyond the caller's: about
+// num_leaves x 2^(arity - 6) x 17 bytes for packed witnesses, num_leaves x 2^(arity - 4) x 17 for extension tables.
 int agl_same_point_prove_device_ffi(int num_leaves, int arity, const uint64_t* h_claim_pts, const uint64_t* h_claim_vals, int kind,
                                     const uint64_t* d_w0, const uint64_t* d_w1, void* transcript, uint64_t* h_round_msgs,
                                     uint64_t* h_challenges, uint64_t* h_f_evals, uint64_t* h_final_eval) {
