@@ -12,9 +12,16 @@
 // caller's: it depends on the equation and the shapes only (matrix_b200/layer_trace.py builds it once).
 #include <vector>
 #include "../agl_traits.cuh"
+#include "../gl_sumcheck_launch.cuh"
 #include "../eq_kernels.cuh"
 #include "../fused_peval_kernels.cuh"
 #include "../peval_kernels.cuh"
+#include "agl_transcript.hpp"
+
+namespace mbhost {
+int prove_pair_with_eq(const uint64_t* d_a, const uint64_t* d_b, bool base, int num_var, const uint64_t* eq_pt, int eq_vars,
+                       aglm::Transcript& t, uint64_t* round_msgs, uint64_t* challenges, uint64_t* final_evals, uint64_t* final_eval);
+}
 
 using namespace mb;
 using namespace mb::sc;
@@ -137,9 +144,18 @@ int agl_einsum_prove_device_ffi(int num_operands, const mb_einsum_operand* ops, 
     h_small[w++] = 1;
     h_small[w++] = 0;
 
+    // two operands: the third table is the eq polynomial (or ones), which the pair prover never forms
+    const bool pair = num_operands == 2 && rounds > 0;
+    auto& tr = *static_cast<mbhost::aglm::Transcript*>(transcript);
+    // nothing to evaluate or tile: the operands are the tables, base field words as they are
+    const auto plain = [&](const mb_einsum_operand& o) { return !o.d_lut_lo && o.m == 0 && o.n == rounds && aligned16(o.d_src); };
+    if (pair && plain(ops[0]) && plain(ops[1]))
+        return mbhost::prove_pair_with_eq(ops[0].d_src, ops[1].d_src, true, rounds, h_small + shared_off, num_shared, tr, round_msgs,
+                                          challenges, final_evals, final_eval);
+
     Scratch sc;
     uint64_t* d_small = sc.get(small_words);
-    uint64_t* tables = sc.get((size_t)d * size * 2);
+    uint64_t* tables = sc.get((size_t)(pair ? 2 : d) * size * 2);
     if (!d_small || !tables) return MB_ERR_CUDA;
     MB_CUDA(cudaMemcpyAsync(d_small, h_small, sizeof(uint64_t) * small_words, cudaMemcpyHostToDevice, MB_STREAM));
 
@@ -176,6 +192,9 @@ int agl_einsum_prove_device_ffi(int num_operands, const mb_einsum_operand* ops, 
         rc = tile(dst, mine, rounds);
         if (rc != MB_OK) return rc;
     }
+    if (pair)
+        return mbhost::prove_pair_with_eq(tables, tables + 2 * size, false, rounds, h_small + shared_off, num_shared, tr, round_msgs,
+                                          challenges, final_evals, final_eval);
     uint64_t* last = tables + (size_t)(d - 1) * size * 2;
     if (num_shared) {
         uint64_t* eqs = sc.get(2 * (((size_t)1 << (num_shared / 2)) + ((size_t)1 << (num_shared - num_shared / 2))));

@@ -91,6 +91,67 @@ static int prove_linear(const uint64_t* d_tables, int d, int num_var, bool base_
     return MB_OK;
 }
 
+// The same protocol for the three tables a, b, eq(t, x) (extended by copies over the variables from eq_vars on; a
+// table of ones when eq_vars is 0) without forming the third: several rounds per pass (pair_sumcheck.cuh). base: a and
+// b are base field words. Messages are those of the three-table prover, P(0..3).
+int prove_pair_with_eq(const uint64_t* d_a, const uint64_t* d_b, bool base, int num_var, const uint64_t* eq_pt, int eq_vars,
+                       AglTranscript& t, uint64_t* round_msgs, uint64_t* challenges, uint64_t* final_evals, uint64_t* final_eval) {
+    using Pair = PairSumcheck<pr::AglF, PairAgl>;
+    using H = Pair::H;
+    using E2 = agl::E2;
+    Pair st;
+    int rc = st.init(d_a, d_b, 0, 1, num_var, base, eq_pt, eq_vars);
+    if (rc != MB_OK) return rc;
+    t.append_u64(L_NUM_VAR, sizeof(L_NUM_VAR) - 1, (uint64_t)num_var);
+    t.append_u64(L_NUM_POLY, sizeof(L_NUM_POLY) - 1, 3);
+    for (int round = 0; round < num_var; round++) {
+        t.begin_append(L_MSG, sizeof(L_MSG) - 1);   // the first label goes in while a pass runs
+        E2 t0, t1, t2;
+        rc = st.sums(t0, t1, t2);
+        if (rc != MB_OK) return rc;
+        const E2 s12 = H::add(t1, t2), p2 = H::sub(H::add(s12, s12), t0);                        // 2 t1 + 2 t2 - t0
+        const E2 t22 = H::add(t2, t2), p3 = H::add(H::sub(H::add(p2, t1), t0), H::add(t22, t22));   // 3 t1 + 6 t2 - 2 t0
+        E2 msg[4] = {t0, t1, p2, p3};
+        if (eq_vars > 0) {
+            E2 lam = st.eq_scale(), step{0, 0};
+            if (round < eq_vars) {
+                const E2 c = st.eq_coord(round), one{1, 0};
+                step = H::mul(lam, H::sub(H::add(c, c), one));
+                lam = H::mul(lam, H::sub(one, c));
+            }
+            for (int c = 0; c < 4; c++) {
+                msg[c] = H::mul(lam, msg[c]);
+                lam = H::add(lam, step);
+            }
+        }
+        for (int c = 0; c < 4; c++) {
+            if (c > 0) t.begin_append(L_MSG, sizeof(L_MSG) - 1);
+            t.finish_append_ext2(msg[c].c0, msg[c].c1);
+            round_msgs[((size_t)round * 4 + c) * 2] = msg[c].c0;
+            round_msgs[((size_t)round * 4 + c) * 2 + 1] = msg[c].c1;
+        }
+        const Ext2 r = challenge_ext2(t);
+        if (challenges) {
+            challenges[2 * round] = r.c0;
+            challenges[2 * round + 1] = r.c1;
+        }
+        rc = st.fold(E2{r.c0, r.c1});
+        if (rc != MB_OK) return rc;
+    }
+    E2 f[3];
+    rc = st.finals(&f[0], &f[1]);
+    if (rc != MB_OK) return rc;
+    f[2] = st.eq_scale();
+    for (int i = 0; i < 3 && final_evals; i++) {
+        final_evals[2 * i] = f[i].c0;
+        final_evals[2 * i + 1] = f[i].c1;
+    }
+    const E2 prod = H::mul(H::mul(f[0], f[1]), f[2]);
+    final_eval[0] = prod.c0;
+    final_eval[1] = prod.c1;
+    return MB_OK;
+}
+
 // Lagrange interpolation through x = 0..n-1, evaluated at x (verifier.rs:91-113).
 static Ext2 interpolate_and_evaluate(const Ext2* evals, int n, Ext2 x) {
     Ext2 result{0, 0};

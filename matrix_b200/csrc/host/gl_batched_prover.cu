@@ -14,260 +14,115 @@
 #include <cstdlib>
 #include <cstring>
 #include <vector>
-#include "../batched_kernels.cuh"
-#include "../eq_kernels.cuh"
 #include "exchange.hpp"
 #include "gl_transcript.hpp"
+#include "../gl_sumcheck_launch.cuh"
+#include "pair_sumcheck.cuh"
 
 using namespace mb;
 using namespace mb::sc;
 
 namespace mbhost {
 
+constexpr int BATCHED_MAX_K = 64;
+
+// The round polynomials of sum_x eq(t, x) sum_k alpha^k a_k(x) b_k(x) factor: m(c) = lambda(c) T(c) with
+// lambda(c) = (1 - t_i) + c (2 t_i - 1) times the eq value of the variables bound before, and T quadratic. T comes from
+// the several-rounds-per-pass engine (pair_sumcheck.cuh): the first pass is independent of alpha and gives every
+// instance its own matrix, from which the claims are read and, once alpha is known, the first rounds run; the eq table
+// (as large as an instance) is never formed.
 class BatchedEqAbState {
 public:
-    ~BatchedEqAbState() { release(); }
+    using Pair = PairSumcheck<pr::GlF, PairGl>;
+    using H = PairHost<pr::GlF, PairGl>;
+    using E2 = gl::E2;
 
+    // threads: the handle may be used from other host threads than this one, so every call ends with the work it
+    // queued (another thread's stream knows nothing of this one's)
     int init(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* h_point_low, const uint64_t* h_eq_scale, int K,
-             int n_loc) {
-        if (!d_a || !d_b || !h_eq_scale || K < 1 || K > bt::MAX_K || n_loc < 1 || n_loc > 34) return MB_ERR_ARG;
-        if (n_loc > 0 && !h_point_low) return MB_ERR_ARG;
-        K_ = K; n_loc_ = n_loc; n_ = (size_t)1 << n_loc; round_ = 0; have_msg_ = false; have_alpha_ = false; have_inst_ = false;
-        pt_.assign(h_point_low, h_point_low + 2 * (size_t)n_loc);
-        a0_ = d_a;  // the caller's tables are read in place during round 0 and never written
-        b0_ = d_b;
-        size_t half = n_ / 2, quarter = n_ >= 4 ? n_ / 4 : 1;
-        MB_CUDA(pool_alloc((void**)&eq0_, 16 * n_));
-        MB_CUDA(pool_alloc((void**)&eq_a_, 16 * half));
-        MB_CUDA(pool_alloc((void**)&eq_b_, 16 * quarter));
-        MB_CUDA(pool_alloc((void**)&ab_a_, 16 * 2 * K * half));
-        MB_CUDA(pool_alloc((void**)&ab_b_, 16 * 2 * K * quarter));
-        grid_max_ = grid_for(half, 256, 4);
-        // round-0 kernel: lane groups of Kp lanes, two output pairs per lane and step
-        Kp_ = 1;
-        while (Kp_ < K && Kp_ < 32) Kp_ *= 2;
-        const size_t per_step = (size_t)2 * (32 / Kp_);
-        grid_inst_ = grid_for(((half + per_step - 1) / per_step) * 32, 256, 3);
-        size_t partial_words = 2 * (size_t)bt::NC * (size_t)grid_max_;
-        if (partial_words < 2 * (size_t)bt::NC * K * grid_inst_) partial_words = 2 * (size_t)bt::NC * K * grid_inst_;
-        MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * partial_words));
-        MB_CUDA(pool_alloc((void**)&small_, sizeof(uint64_t) * (16 + 2 * bt::MAX_K + 2 * 40 + 2 + 4 * bt::MAX_K + 8 * bt::MAX_K)));
-        msg_dev_ = small_;                      // 8 words
-        counter_ = reinterpret_cast<unsigned int*>(small_ + 8);
-        alpha_dev_ = small_ + 16;               // 2 * MAX_K words
-        uint64_t* point_dev = alpha_dev_ + 2 * bt::MAX_K;  // 2 * 40 words
-        uint64_t* scale_dev = point_dev + 80;               // 2 words
-        wtab_dev_ = scale_dev + 2;                          // 4 * MAX_K words
-        inst_dev_ = wtab_dev_ + 4 * bt::MAX_K;              // 8 * MAX_K words
-        MB_CUDA(cudaMemsetAsync(small_, 0, 16 * sizeof(uint64_t), MB_STREAM));
-        MB_CUDA(cudaMemcpyAsync(point_dev, h_point_low, 16 * (size_t)n_loc, cudaMemcpyHostToDevice, MB_STREAM));
-        MB_CUDA(cudaMemcpyAsync(scale_dev, h_eq_scale, 16, cudaMemcpyHostToDevice, MB_STREAM));
-        // eq slice scaled by eq(t_top, shard); ab_a_ is free until the first fold and serves as scratch
-        int rc = eq::build<GlExt2>(point_dev, eq0_, ab_a_, n_loc, MB_STREAM, scale_dev);
-        if (rc != MB_OK) return rc;
-        // the table build and the copies above are complete before the handle is handed out, so that the
-        // first call on it may come from another host thread (whose stream knows nothing of this one)
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        return MB_OK;
+             int n_loc, bool threads) {
+        if (!d_a || !d_b || !h_eq_scale || K < 1 || K > BATCHED_MAX_K || n_loc < 1 || n_loc > 34) return MB_ERR_ARG;
+        if (!h_point_low || !aligned16(d_a) || !aligned16(d_b)) return MB_ERR_ARG;
+        K_ = K; n_loc_ = n_loc; threads_ = threads;
+        shard_ = H::canon(E2{h_eq_scale[0], h_eq_scale[1]});
+        // the caller's base-field tables are read in place until the first fold and never written
+        int rc = pair_.init(d_a, d_b, (size_t)1 << n_loc, K, n_loc, true, h_point_low, n_loc);
+        return rc == MB_OK ? finish_call() : rc;
     }
-
-    // Per-instance round-0 messages m_k(0..3) of this shard, one pass over the caller's tables.
-    int instance_messages() {
-        if (have_inst_) return MB_OK;
-        const size_t half = n_ / 2;
-        dim3 grid(grid_inst_, (K_ + 31) / 32);
-        const size_t smem = sizeof(uint64_t) * 8 * 2 * (size_t)(2 * (32 / Kp_)) * 2;
-        if (smem > 48 * 1024)
-            MB_CUDA(cudaFuncSetAttribute(bt::instance_messages_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        {
-            MB_KERNEL("batched_instance_messages");
-            bt::instance_messages_kernel<<<grid, 256, smem, MB_STREAM>>>(eq0_, a0_, b0_, K_, Kp_, n_, half, partial_);
-        }
-        {
-            MB_KERNEL("reduce_partials");
-            reduce_partials_kernel<256, GlAdd, GlCanon><<<1, 256, 0, MB_STREAM>>>(partial_, grid_inst_, 2 * bt::NC * K_, inst_dev_);
-        }
-        inst_.resize(2 * (size_t)bt::NC * K_);
-        MB_CUDA(cudaMemcpyAsync(inst_.data(), inst_dev_, sizeof(uint64_t) * inst_.size(), cudaMemcpyDeviceToHost, MB_STREAM));
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        have_inst_ = true;
-        return MB_OK;
-    }
-
-    // m(0..3) = lambda(c) T(c) from T(0), T(1) and the leading coefficient T2 (six words) for the
-    // variable bound in `round`: lambda(c) = (1 - t) + c (2 t - 1), T(2) = 2 T(1) + 2 T2 - T(0),
-    // T(3) = 3 T(1) + 6 T2 - 2 T(0).
-    void expand_message(const uint64_t* t6, int round, gl::E2 (&out)[4]) const {
-        const gl::E2 T0{t6[0], t6[1]}, T1{t6[2], t6[3]}, T2{t6[4], t6[5]};
-        const gl::E2 t{gl::canon(pt_[2 * (size_t)round]), gl::canon(pt_[2 * (size_t)round + 1])};
-        const gl::E2 s12 = gl::e2_add(T1, T2), s122 = gl::e2_add(s12, T2);
-        gl::E2 T[4] = {T0, T1, gl::e2_sub(gl::e2_add(s12, s12), T0),
-                       gl::e2_sub(gl::e2_sub(gl::e2_add(gl::e2_add(s122, s122), s122), T0), T0)};
-        gl::E2 lam = gl::e2_sub(gl::E2{1, 0}, t);                 // lambda(0) = 1 - t
-        const gl::E2 step = gl::e2_sub(gl::e2_add(t, t), gl::E2{1, 0});  // 2 t - 1
-        for (int c = 0; c < 4; c++) {
-            out[c] = gl::e2_canon(gl::e2_mul(lam, T[c]));
-            lam = gl::e2_add(lam, step);
-        }
-    }
-
-    // Local share of the per-instance claims s_k = m_k(0) + m_k(1) (K extension elements).
+    // Local share of the per-instance claims sum_x eq a_k b_k (K extension elements).
     int claims(uint64_t* h_out) {
-        int rc = instance_messages();
+        std::vector<E2> c(K_);
+        if (round_ != 0) return MB_ERR_ARG;
+        int rc = pair_.claims(c.data());
         if (rc != MB_OK) return rc;
         for (int k = 0; k < K_; k++) {
-            gl::E2 m[4];
-            expand_message(inst_.data() + 2 * bt::NC * (size_t)k, 0, m);
-            const gl::E2 s = gl::e2_canon(gl::e2_add(m[0], m[1]));
-            h_out[2 * k] = s.c0;
-            h_out[2 * k + 1] = s.c1;
+            c[k] = H::mul(c[k], shard_);
+            h_out[2 * k] = c[k].c0;
+            h_out[2 * k + 1] = c[k].c1;
         }
         return MB_OK;
     }
-
     int set_alpha(Ext2 alpha) {
-        std::vector<uint64_t>& pows = pows_;
-        pows.resize(2 * (size_t)K_);
-        gl::E2 p{1, 0}, a{gl::canon(alpha.c0), gl::canon(alpha.c1)};
+        alphas_.resize(K_);
+        E2 p{1, 0};
+        const E2 a = H::canon(E2{alpha.c0, alpha.c1});
         for (int k = 0; k < K_; k++) {
-            pows[2 * k] = p.c0;
-            pows[2 * k + 1] = p.c1;
-            p = gl::e2_canon(gl::e2_mul(p, a));
+            alphas_[k] = p;
+            p = H::mul(p, a);
         }
-        MB_CUDA(cudaMemcpyAsync(alpha_dev_, pows.data(), 16 * (size_t)K_, cudaMemcpyHostToDevice, MB_STREAM));
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        have_alpha_ = true;
-        return MB_OK;
+        return pair_.set_scale(alphas_.data());
     }
-
-    // Local share of m(0..3) for the current round.
+    // Local share of m(0..3) for the current round: T(2) = 2 T(1) + 2 T2 - T(0), T(3) = 3 T(1) + 6 T2 - 2 T(0).
     int round_message(uint64_t* h_msg) {
-        if (!have_alpha_ || round_ >= n_loc_) return MB_ERR_ARG;
-        if (round_ == 0) {
-            // sum_k alpha^k m_k(c) from the per-instance messages
-            int rc = instance_messages();
-            if (rc != MB_OK) return rc;
-            gl::E2 acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-            for (int k = 0; k < K_; k++) {
-                gl::E2 m[4];
-                expand_message(inst_.data() + 2 * bt::NC * (size_t)k, 0, m);
-                const gl::E2 w{pows_[2 * k], pows_[2 * k + 1]};
-                for (int c = 0; c < 4; c++) acc[c] = gl::e2_add(acc[c], gl::e2_mul(w, m[c]));
-            }
-            for (int c = 0; c < 4; c++) {
-                acc[c] = gl::e2_canon(acc[c]);
-                h_msg[2 * c] = acc[c].c0;
-                h_msg[2 * c + 1] = acc[c].c1;
-            }
-            return MB_OK;
-        }
-        if (!have_msg_) return MB_ERR_ARG;
-        uint64_t* h = landing_;
-        if (h) {
-            // the fold kernel's last block wrote the six words straight into pinned host memory
-            MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        } else {
-            h = pinned_scratch();   // the calling thread's landing zone, not the creating thread's
-            if (!h) return MB_ERR_CUDA;
-            MB_CUDA(cudaMemcpyAsync(h, msg_dev_, 16 * bt::NC, cudaMemcpyDeviceToHost, MB_STREAM));
-            MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        }
-        gl::E2 m[4];
-        expand_message(h, round_, m);
+        if (alphas_.empty() || round_ >= n_loc_) return MB_ERR_ARG;
+        E2 t0, t1, t2;
+        int rc = pair_.sums(t0, t1, t2);
+        if (rc != MB_OK) return rc;
+        const E2 s12 = H::add(t1, t2), d = H::sub(H::add(s12, s12), t0);      // T(2)
+        const E2 t22 = H::add(t2, t2), s = H::add(H::sub(H::add(d, t1), t0), H::add(t22, t22));   // T(3)
+        const E2 T[4] = {t0, t1, d, s};
+        const E2 t = pair_.eq_coord(round_), one{1, 0}, w = H::mul(shard_, pair_.eq_scale());
+        E2 lam = H::mul(w, H::sub(one, t));
+        const E2 step = H::mul(w, H::sub(H::add(t, t), one));
         for (int c = 0; c < 4; c++) {
-            h_msg[2 * c] = m[c].c0;
-            h_msg[2 * c + 1] = m[c].c1;
+            const E2 m = H::mul(lam, T[c]);
+            h_msg[2 * c] = m.c0;
+            h_msg[2 * c + 1] = m.c1;
+            lam = H::add(lam, step);
         }
         return MB_OK;
     }
-
     int fold(Ext2 ch) {
-        if (!have_alpha_ || round_ >= n_loc_) return MB_ERR_ARG;
-        gl::E2 r{gl::canon(ch.c0), gl::canon(ch.c1)};
-        size_t live = n_ >> round_, quarter = live / 4;
-        bool first = round_ == 0;
-        const uint64_t* eq_in = first ? eq0_ : eq_cur_;
-        const uint64_t* ab_in = first ? a0_ : ab_cur_;
-        size_t stride_in = first ? n_ : ab_stride_;
-        bool to_a = first || ab_cur_ == ab_b_;
-        uint64_t* eq_out = to_a ? eq_a_ : eq_b_;
-        uint64_t* ab_out = to_a ? ab_a_ : ab_b_;
-        size_t stride_out = to_a ? n_ / 2 : (n_ >= 4 ? n_ / 4 : 1);
-        if (quarter >= 1) {
-            int grid = grid_for(quarter, 256, 4);
-            if (first) {
-                // per instance: alpha^k and alpha^k r
-                std::vector<uint64_t> wt(4 * (size_t)K_);
-                for (int k = 0; k < K_; k++) {
-                    gl::E2 w{pows_[2 * k], pows_[2 * k + 1]}, wr = gl::e2_canon(gl::e2_mul(w, r));
-                    wt[4 * k] = w.c0; wt[4 * k + 1] = w.c1; wt[4 * k + 2] = wr.c0; wt[4 * k + 3] = wr.c1;
-                }
-                MB_CUDA(cudaMemcpyAsync(wtab_dev_, wt.data(), sizeof(uint64_t) * wt.size(), cudaMemcpyHostToDevice, MB_STREAM));
-                MB_CUDA(cudaStreamSynchronize(MB_STREAM));  // wt leaves scope
-            }
-            MB_KERNEL("batched_fold_message");
-            uint64_t* msg_out = landing_ ? landing_ : msg_dev_;
-            if (first)
-                bt::fold_message_kernel<true><<<grid, 256, 0, MB_STREAM>>>(
-                    eq_in, eq_out, ab_in, b0_, ab_out, wtab_dev_, r, K_, stride_in, stride_out, quarter, partial_, counter_, msg_out);
-            else
-                bt::fold_message_kernel<false><<<grid, 256, 0, MB_STREAM>>>(
-                    eq_in, eq_out, ab_in, b0_, ab_out, wtab_dev_, r, K_, stride_in, stride_out, quarter, partial_, counter_, msg_out);
-            have_msg_ = true;
-        } else {
-            MB_KERNEL("batched_final_fold");
-            int threads = 2 * K_ + 1;
-            if (first)
-                bt::final_fold_kernel<GlBase, GlExt2, true><<<(threads + 127) / 128, 128, 0, MB_STREAM>>>(
-                    eq_in, eq_out, ab_in, b0_, ab_out, alpha_dev_, r, K_, stride_in, stride_out);
-            else
-                bt::final_fold_kernel<GlBase, GlExt2, false><<<(threads + 127) / 128, 128, 0, MB_STREAM>>>(
-                    eq_in, eq_out, ab_in, b0_, ab_out, alpha_dev_, r, K_, stride_in, stride_out);
-            have_msg_ = false;
-        }
-        if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
-        eq_cur_ = eq_out;
-        ab_cur_ = ab_out;
-        ab_stride_ = stride_out;
+        if (alphas_.empty() || round_ >= n_loc_) return MB_ERR_ARG;
         round_++;
-        return MB_OK;
+        int rc = pair_.fold(H::canon(E2{ch.c0, ch.c1}));
+        return rc == MB_OK ? finish_call() : rc;
     }
-
-    // Round messages land in `pinned` (six words of page-locked host memory of the calling thread) instead of
-    // being copied back: a round is then one launch and one stream synchronisation. Used by the whole-proof loop,
-    // which stays on one thread; the per-round C-ABI keeps the copy because its callers may change threads.
-    void set_landing(uint64_t* pinned) { landing_ = pinned; }
-
-    // After n_loc folds: eq, then alpha^k a_k, b_k for every k: (2K + 1) extension elements.
-    int finals(uint64_t* h_out) {
+    // After n_loc folds: eq (with the shard's factor), a_k, b_k: (2K + 1) extension elements; scaled: alpha^k a_k.
+    int finals(uint64_t* h_out, bool scaled) {
         if (round_ != n_loc_) return MB_ERR_ARG;
-        MB_CUDA(cudaMemcpyAsync(h_out, eq_cur_, 16, cudaMemcpyDeviceToHost, MB_STREAM));
-        for (int t = 0; t < 2 * K_; t++) {
-            int k = t >> 1, which = t & 1;  // output order: a'_0 .. a'_{K-1}, b_0 .. b_{K-1}
-            uint64_t* dst = h_out + 2 + 2 * (size_t)(which * K_ + k);
-            MB_CUDA(cudaMemcpyAsync(dst, ab_cur_ + (size_t)t * ab_stride_ * 2, 16, cudaMemcpyDeviceToHost, MB_STREAM));
+        std::vector<E2> v(2 * (size_t)K_ + 1);
+        v[0] = H::mul(shard_, pair_.eq_scale());
+        int rc = pair_.finals(v.data() + 1, v.data() + 1 + K_);
+        if (rc != MB_OK) return rc;
+        for (int k = 0; k < K_ && scaled; k++) v[1 + k] = H::mul(alphas_[k], v[1 + k]);
+        for (size_t i = 0; i < v.size(); i++) {
+            h_out[2 * i] = v[i].c0;
+            h_out[2 * i + 1] = v[i].c1;
         }
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
         return MB_OK;
     }
 
 private:
-    void release() {
-        pool_free(eq0_); pool_free(eq_a_); pool_free(eq_b_); pool_free(ab_a_); pool_free(ab_b_);
-        pool_free(partial_); pool_free(small_);
-        eq0_ = eq_a_ = eq_b_ = ab_a_ = ab_b_ = partial_ = small_ = nullptr;
+    int finish_call() {
+        if (threads_) MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        return MB_OK;
     }
-    int K_ = 0, Kp_ = 1, n_loc_ = 0, round_ = 0, grid_max_ = 0, grid_inst_ = 0;
-    bool have_inst_ = false;
-    std::vector<uint64_t> inst_, pows_, pt_;
-    uint64_t *wtab_dev_ = nullptr, *inst_dev_ = nullptr;
-    size_t n_ = 0, ab_stride_ = 0;
-    bool have_msg_ = false, have_alpha_ = false;
-    const uint64_t *a0_ = nullptr, *b0_ = nullptr;
-    uint64_t *eq0_ = nullptr, *eq_a_ = nullptr, *eq_b_ = nullptr, *ab_a_ = nullptr, *ab_b_ = nullptr;
-    uint64_t *partial_ = nullptr, *small_ = nullptr, *msg_dev_ = nullptr, *alpha_dev_ = nullptr, *eq_cur_ = nullptr, *ab_cur_ = nullptr;
-    unsigned int* counter_ = nullptr;
-    uint64_t* landing_ = nullptr;
+    int K_ = 0, n_loc_ = 0, round_ = 0;
+    bool threads_ = false;
+    E2 shard_{1, 0};
+    std::vector<E2> alphas_;
+    Pair pair_;
 };
 
 }  // namespace mbhost
@@ -311,7 +166,7 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
                           const uint64_t* h_point, const uint8_t* label, size_t label_len, uint64_t* h_claims,
                           uint64_t* h_alpha, uint64_t* h_round_msgs, uint64_t* h_challenges, uint64_t* h_finals,
                           uint64_t* h_final_eval, uint64_t* h_transcript_state, double* h_round_us) {
-    if (!ex || !d_a || !d_b || !h_point || (!label && label_len) || K < 1 || K > bt::MAX_K) return MB_ERR_ARG;
+    if (!ex || !d_a || !d_b || !h_point || (!label && label_len) || K < 1 || K > BATCHED_MAX_K) return MB_ERR_ARG;
     const int world = ex->world, rank = ex->rank;
     int g_bits = 0;
     while ((1 << g_bits) < world) g_bits++;
@@ -326,14 +181,12 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
         scale = e2c(gl::e2_mul(scale, (rank >> i) & 1 ? t : gl::e2_sub(E2{1, 0}, t)));
     }
     const uint64_t scale_w[2] = {scale.c0, scale.c1};
-    uint64_t* pin = pinned_scratch();
-    if (!pin) return MB_ERR_CUDA;
 
     BatchedEqAbState st;
-    int rc = st.init(d_a, d_b, h_point, scale_w, K, n_loc);
+    int rc = st.init(d_a, d_b, h_point, scale_w, K, n_loc, false);
     if (rc != MB_OK) return rc;
-    st.set_landing(pin);
 
+    using H = BatchedEqAbState::H;
     const int T = 2 * K + 1;
     std::vector<uint64_t> mine((size_t)2 * (T > 4 ? T : 4)), all((size_t)world * mine.size());
     std::vector<E2> claims(K);
@@ -395,9 +248,9 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
             label_absorbed = true;
         }
     }
-    // one value per table and rank: eq, alpha^k a_k, b_k; the top variables are finished on the host
+    // one value per table and rank: eq, a_k, b_k; the top variables are finished on the host
     clock.start();
-    rc = st.finals(mine.data());
+    rc = st.finals(mine.data(), false);
     if (rc != MB_OK) return rc;
     clock.stop(clock.kernel);
     rc = ex->all_gather_host(ex->ctx, mine.data(), 2 * (size_t)T, all.data());
@@ -406,6 +259,14 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
     std::vector<std::vector<E2>> tab(T, std::vector<E2>(world));
     for (int g = 0; g < world; g++)
         for (int i = 0; i < T; i++) tab[i][g] = e2_load(all.data() + ((size_t)g * T + i) * 2);
+    std::vector<E2> alphas(K);
+    {
+        E2 pw{1, 0};
+        for (int k = 0; k < K; k++) {
+            alphas[k] = pw;
+            pw = H::mul(pw, E2{alpha.c0, alpha.c1});
+        }
+    }
     for (int size = world; size > 1; size /= 2) {
         const int half = size / 2;
         E2 msg[4];
@@ -417,7 +278,8 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
                     return e2c(gl::e2_add(t[2 * y], gl::e2_mul(cc, gl::e2_sub(t[2 * y + 1], t[2 * y]))));
                 };
                 E2 inner{0, 0};
-                for (int k = 0; k < K; k++) inner = gl::e2_add(inner, gl::e2_mul(at(tab[1 + k]), at(tab[1 + K + k])));
+                for (int k = 0; k < K; k++)
+                    inner = gl::e2_add(inner, gl::e2_mul(alphas[k], e2c(gl::e2_mul(at(tab[1 + k]), at(tab[1 + K + k])))));
                 tot = gl::e2_add(tot, gl::e2_mul(at(tab[0]), e2c(inner)));
             }
             msg[c] = e2c(tot);
@@ -427,22 +289,15 @@ int batched_prove_sharded(const mb_exchange* ex, const uint64_t* d_a, const uint
         for (auto& t : tab)
             for (int y = 0; y < half; y++) t[y] = e2c(gl::e2_add(t[2 * y], gl::e2_mul(r, gl::e2_sub(t[2 * y + 1], t[2 * y]))));
     }
-    // a_k(R) is reported without the alpha^k factor the shards carry
     std::vector<E2> fin(T);
-    fin[0] = tab[0][0];
-    E2 pw{1, 0}, acc{0, 0};
-    const E2 al{alpha.c0, alpha.c1};
-    for (int k = 0; k < K; k++) {
-        fin[1 + k] = e2c(gl::e2_mul(tab[1 + k][0], gl::e2_inv(pw)));
-        acc = gl::e2_add(acc, gl::e2_mul(tab[1 + k][0], tab[1 + K + k][0]));
-        pw = e2c(gl::e2_mul(pw, al));
-        fin[1 + K + k] = tab[1 + K + k][0];
-    }
+    E2 acc{0, 0};
+    for (int i = 0; i < T; i++) fin[i] = tab[i][0];
+    for (int k = 0; k < K; k++) acc = H::add(acc, H::mul(alphas[k], H::mul(fin[1 + k], fin[1 + K + k])));
     for (int i = 0; i < T; i++) {
         tr.append_ext2("sp_f_eval", Ext2{fin[i].c0, fin[i].c1});
         if (h_finals) { h_finals[2 * i] = fin[i].c0; h_finals[2 * i + 1] = fin[i].c1; }
     }
-    const E2 fe = e2c(gl::e2_mul(tab[0][0], e2c(acc)));
+    const E2 fe = H::mul(fin[0], acc);
     if (h_final_eval) { h_final_eval[0] = fe.c0; h_final_eval[1] = fe.c1; }
     if (h_transcript_state) std::memcpy(h_transcript_state, tr.state(), 64);
     clock.stop(clock.host);
@@ -471,7 +326,7 @@ int gl_batched_state_create(const uint64_t* d_a, const uint64_t* d_b, const uint
                             const uint64_t* h_eq_scale, int K, int n_loc, void** state) {
     if (!state) return MB_ERR_ARG;
     auto* s = new BatchedEqAbState;
-    int rc = s->init(d_a, d_b, h_point_low, h_eq_scale, K, n_loc);
+    int rc = s->init(d_a, d_b, h_point_low, h_eq_scale, K, n_loc, true);
     if (rc != MB_OK) { delete s; return rc; }
     *state = s;
     return MB_OK;
@@ -481,7 +336,7 @@ int gl_batched_state_claims(void* state, uint64_t* h_claims) { return static_cas
 int gl_batched_state_set_alpha(void* state, uint64_t c0, uint64_t c1) { return static_cast<BatchedEqAbState*>(state)->set_alpha(Ext2{c0, c1}); }
 int gl_batched_state_round_message(void* state, uint64_t* h_msg) { return static_cast<BatchedEqAbState*>(state)->round_message(h_msg); }
 int gl_batched_state_fold(void* state, uint64_t c0, uint64_t c1) { return static_cast<BatchedEqAbState*>(state)->fold(Ext2{c0, c1}); }
-int gl_batched_state_finals(void* state, uint64_t* h_out) { return static_cast<BatchedEqAbState*>(state)->finals(h_out); }
+int gl_batched_state_finals(void* state, uint64_t* h_out) { return static_cast<BatchedEqAbState*>(state)->finals(h_out, true); }
 
 // ---- the whole proof over the shards of an exchange (world = 1: an mb_exchange_local_create(1) object) ----
 // d_a, d_b: this rank's slices [K][2^(num_vars - log2 world)]; h_point: num_vars (c0, c1) pairs, the same on every

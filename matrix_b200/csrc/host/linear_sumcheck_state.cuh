@@ -14,16 +14,19 @@
 //    after a fold only reads (d+1) extension elements back.
 // Base / Ext are the field traits of sumcheck_kernels.cuh (GlBase, GlExt2) or
 // agl_traits.cuh (AglBase, AglExt2).
+//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh); the other counts a round per pass:
 //  * once a table is down to host_tail(d) elements the live tables are read back and the remaining rounds run on
 //    the host: a round on the device costs a launch and a synchronisation (about 20 us) whatever its size, the
 //    same round on a few hundred elements takes a host core less (about 7 ns per extension product). The field
 //    arithmetic is exact, so the messages are the same words.
 #pragma once
+#include <memory>
 #include <vector>
 #include "../agl_field.cuh"
 #include "../gl_sumcheck_launch.cuh"
 #include "ext2_words.hpp"
 #include "host_field.hpp"
+#include "pair_sumcheck.cuh"
 
 namespace mbhost {
 
@@ -45,6 +48,9 @@ template <class T, class F> struct HostExtOps {
 };
 template <> struct HostExt<gl::E2> : HostExtOps<gl::E2, hf::GlE2Ops> {};
 template <> struct HostExt<agl::E2> : HostExtOps<agl::E2, hf::AglE2Ops> {};
+template <class T> struct PairOf;
+template <> struct PairOf<gl::E2> { using type = PairSumcheck<pr::GlF, PairGl>; };
+template <> struct PairOf<agl::E2> { using type = PairSumcheck<pr::AglF, PairAgl>; };
 
 // Live elements per table at which the rounds move to the host: a host round costs live / 2 x (d^2 - 1 + d)
 // extension products, about 9 us at 512 elements of two tables and 10 us at 256 elements of three.
@@ -68,6 +74,11 @@ public:
         round_ = 0;
         cur_ = nullptr;
         host_mode_ = false;
+        if (d == 2 && num_vars > 0 && aligned16(d_tables)) {
+            pair_.reset(new typename PairOf<typename Ext::T>::type);
+            const size_t words = n_ * (base_field ? 1 : 2);
+            return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0);
+        }
         size_t cap_a = n_ >= 2 ? n_ / 2 : 1, cap_b = n_ >= 4 ? n_ / 4 : 1;
         stride_a_ = cap_a;
         stride_b_ = cap_b;
@@ -90,6 +101,19 @@ public:
     // Evaluations P(0..d) of the current round polynomial, canonical.
     int compute_round_message(std::vector<Ext2>& out) {
         if (round_ >= num_vars_) return MB_ERR_ARG;
+        if (pair_) {
+            // P(2) = 2 P(1) - P(0) + 2 S2
+            using H = HostExt<typename Ext::T>;
+            typename Ext::T s0, s1, s2;
+            int rc = pair_->sums(s0, s1, s2);
+            if (rc != MB_OK) return rc;
+            const typename Ext::T p2 = H::sub(H::add(H::add(s1, s1), H::add(s2, s2)), s0);
+            out.resize(3);
+            out[0].c0 = s0.c0; out[0].c1 = s0.c1;
+            out[1].c0 = s1.c0; out[1].c1 = s1.c1;
+            out[2].c0 = p2.c0; out[2].c1 = p2.c1;
+            return MB_OK;
+        }
         size_t live = n_ >> round_, half = live / 2;
         if (host_mode_) return host_message(out, half);
         if (!have_msg_) {
@@ -124,6 +148,10 @@ public:
         size_t live = n_ >> round_, half = live / 2, quarter = live / 4;
         const typename Ext::WordCanon canon;
         typename Ext::T r{canon(challenge.c0), canon(challenge.c1)};
+        if (pair_) {
+            round_++;
+            return pair_->fold(r);
+        }
         if (!host_mode_ && round_ >= 1 && live <= host_tail(d_)) {
             int rc = to_host(live);
             if (rc != MB_OK) return rc;
@@ -174,6 +202,14 @@ public:
     int final_evaluations(std::vector<Ext2>& out) {
         if (round_ != num_vars_) return MB_ERR_ARG;
         out.resize(d_);
+        if (pair_) {
+            typename Ext::T a, b;
+            int rc = pair_->finals(&a, &b);
+            if (rc != MB_OK) return rc;
+            out[0].c0 = a.c0; out[0].c1 = a.c1;
+            out[1].c0 = b.c0; out[1].c1 = b.c1;
+            return MB_OK;
+        }
         if (host_mode_) {
             for (int i = 0; i < d_; i++) {
                 const typename Ext::T v = host_tab_[(size_t)i * host_stride_];
@@ -265,6 +301,7 @@ private:
     bool host_mode_ = false;
     size_t host_stride_ = 0;
     std::vector<typename Ext::T> host_tab_;
+    std::unique_ptr<typename PairOf<typename Ext::T>::type> pair_;
 };
 
 }  // namespace mbhost

@@ -1,0 +1,449 @@
+// Host side of the several-rounds-per-pass sumcheck over products of two tables (pair_kernels.cuh):
+//     sum_x w(x) sum_k s_k a_k(x) b_k(x),   w = 1 or eq(t, x) on the first eq_vars variables,
+// for K instances whose factors s_k may be chosen after the first pass (powers of a challenge). The object plans the
+// blocks of rounds, queues the passes and runs the rounds of a block on the matrices they return; the last rounds, on
+// tables of at most 512 elements together, run on the host altogether. The caller owns the transcript.
+//
+//   rounds per block  4 while a pass has at most 2^17 elements, 3 up to 2^19 (2^21 of the base field), then 2: a round more
+//                     doubles the products per element (2^B), which pays while a launch and a synchronisation (about
+//                     12 us) cost more than they do; bounded too by what the host then has to fold, K 4^B entries.
+//   host tables       2^t elements per table with K 2^t <= 512: the rest of a proof on them takes a core about as long
+//                     as one more pass and its synchronisation.
+//   all on the host   base-field tables of at most 2^10 elements: the copy and the rounds (35 us) cost less than two passes.
+#pragma once
+#include <vector>
+#include "../common.cuh"
+#include "../pair_kernels.cuh"
+#include "host_field.hpp"
+#include "pinned_pool.hpp"
+
+namespace mbhost {
+
+using namespace mb;
+
+// Host arithmetic by field: canonical words in and out.
+struct PairGl : hf::GlE2Ops {
+    static constexpr uint64_t TOP = 0xFFFFFFFE00000001ULL;                       // 2^128 mod p = -2^32 mod p
+};
+struct PairAgl : hf::AglE2Ops {
+    static constexpr uint64_t TOP = 63ULL * (1ULL << 32) + 992ULL;               // 2^128 mod q
+};
+template <class F, class O>
+struct PairHost {
+    using E2 = typename F::E2;
+    static E2 mul(E2 a, E2 b) {
+        E2 r;
+        hf::e2_mul<O>(a.c0, a.c1, b.c0, b.c1, r.c0, r.c1);
+        return r;
+    }
+    static E2 add(E2 a, E2 b) { return E2{O::add(a.c0, b.c0), O::add(a.c1, b.c1)}; }
+    static E2 sub(E2 a, E2 b) { return E2{O::sub(a.c0, b.c0), O::sub(a.c1, b.c1)}; }
+    static E2 fold(E2 a, E2 b, E2 r) { return add(a, mul(r, sub(b, a))); }
+    static E2 canon(E2 a) { return E2{O::canon(a.c0), O::canon(a.c1)}; }
+    // sum of products, reduced once
+    struct Wide {
+        hf::u128 s = 0;
+        uint64_t top = 0;
+        void mac(uint64_t x, uint64_t y) {
+            const hf::u128 p = (hf::u128)x * y;
+            s += p;
+            top += s < p;
+        }
+        uint64_t red() const { return O::red((hf::u128)top * O::TOP + O::red(s)); }
+    };
+    struct Dot {
+        Wide p00, p11, p01;
+        void mac(E2 a, E2 b) {
+            p00.mac(a.c0, b.c0);
+            p11.mac(a.c1, b.c1);
+            p01.mac(a.c0, b.c1);
+            p01.mac(a.c1, b.c0);
+        }
+        E2 value() const { return E2{O::canon(O::red((hf::u128)p11.red() * O::W + p00.red())), O::canon(p01.red())}; }
+    };
+    // out[x] = prod_j (x_j ? r_j : 1 - r_j)
+    static void eq_vector(const E2* r, int n, E2* out) {
+        out[0] = E2{1, 0};
+        for (int b = 0; b < n; b++)
+            for (int x = 0; x < (1 << b); x++) {
+                const E2 hi = mul(out[x], r[b]);
+                out[x + (1 << b)] = hi;
+                out[x] = sub(out[x], hi);
+            }
+    }
+};
+
+template <class F, class O>
+class PairSumcheck {
+public:
+    using H = PairHost<F, O>;
+    using E2 = typename F::E2;
+    ~PairSumcheck() {
+        if (pin_) {
+            cudaStreamSynchronize(MB_STREAM);   // nothing may still be writing the block
+            PinnedPool::give(pin_);
+        }
+        pool_free(t0_);
+        pool_free(t1_);
+        pool_free(tabs_);
+        pool_free(partial_);
+        pool_free(counter_);
+    }
+    // a, b: instance 0's device tables of 2^n elements (never written), instances inst_stride words apart; base: base
+    // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. Queues the first pass.
+    int init(const uint64_t* a, const uint64_t* b, size_t inst_stride, int K, int n, bool base, const uint64_t* eq_pt, int eq_vars) {
+        a_ = a; b_ = b; stride_ = inst_stride; K_ = K; n_ = n; base_ = base;
+        pt_.resize(eq_vars);
+        for (int i = 0; i < eq_vars; i++) pt_[i] = H::canon(E2{eq_pt[2 * i], eq_pt[2 * i + 1]});
+        int t = 0;
+        while (t < 9 && ((size_t)K << (t + 1)) <= 512) t++;
+        if (base && ((size_t)K << n) <= 1024 && n > t) t = n;
+        for (int v = n; v > t;) {
+            const size_t size = (size_t)K << v;
+            const bool first = v == n;
+            int g = size <= (1u << 17) ? 4 : size <= (first && base && eq_vars == 0 ? 1u << 21 : 1u << 19) ? 3 : 2;
+            while (g > 1 && ((size_t)K << (2 * g)) > 1024) g--;
+            if (g > v - t) g = v - t;
+            blocks_.push_back(Block{n - v, g, 0, 0, 0, 63, 0});
+            v -= g;
+        }
+        tail_first_ = n - (n > t ? t : n);
+        pin_ = PinnedPool::take();
+        if (!pin_) return MB_ERR_CUDA;
+        if (!blocks_.empty()) {
+            cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;
+            MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 2 * 256 * (size_t)cap_ * K));
+            MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned) * K));
+            MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * K, MB_STREAM));
+            int rc = tables();
+            if (rc != MB_OK) return rc;
+        }
+        r_.resize(n);
+        return pass();
+    }
+    // The instances' factors (K = 1: not needed). sums() and fold() may be called from then on.
+    int set_scale(const E2* s) {
+        scale_.assign(s, s + K_);
+        return MB_OK;
+    }
+    // sum_x w(x) a_k(x) b_k(x) of every instance, before the first fold
+    int claims(E2* out) {
+        int rc = wait();
+        if (rc != MB_OK) return rc;
+        if (host_) {
+            suffix(0, n_);
+            for (int k = 0; k < K_; k++) out[k] = total(k);
+            return MB_OK;
+        }
+        const int g = blocks_[0].rounds, G = 1 << g;
+        std::vector<E2> w(G, E2{1, 0});
+        const int we = (int)pt_.size() < g ? (int)pt_.size() : g;
+        if (we) H::eq_vector(pt_.data(), we, w.data());
+        for (int x = 1 << we; x < G; x++) w[x] = w[x & ((1 << we) - 1)];
+        for (int k = 0; k < K_; k++) {
+            typename H::Dot d;
+            for (int m = 0; m < G; m++) d.mac(w[m], entry(k, m, m));
+            out[k] = d.value();
+        }
+        return MB_OK;
+    }
+    // T(0), T(1) and the leading coefficient of this round's sum without the round's own eq factor: the round polynomial
+    // is eq_scale() ((1 - t)(1 - c) + t c) T(c) while the round is below eq_vars, eq_scale() T(c) from then on.
+    int sums(E2& s0, E2& s1, E2& s2) {
+        int rc = wait();
+        if (rc != MB_OK) return rc;
+        if (host_) { host_sums(s0, s1, s2); return MB_OK; }
+        if (m_.empty()) combine();
+        const int half = side_ / 2;
+        s0 = s1 = E2{0, 0};
+        E2 cross{0, 0};
+        if (half > 1 && weighted_) {
+            typename H::Dot d0, d1, dc;
+            const E2* w = weights(half);
+            for (int m = 0; m < half; m++) {
+                d0.mac(w[m], at(2 * m, 2 * m));
+                d1.mac(w[m], at(2 * m + 1, 2 * m + 1));
+                dc.mac(w[m], H::add(at(2 * m, 2 * m + 1), at(2 * m + 1, 2 * m)));
+            }
+            s0 = d0.value(); s1 = d1.value(); cross = dc.value();
+        } else {
+            for (int m = 0; m < half; m++) {
+                s0 = H::add(s0, at(2 * m, 2 * m));
+                s1 = H::add(s1, at(2 * m + 1, 2 * m + 1));
+                cross = H::add(cross, H::add(at(2 * m, 2 * m + 1), at(2 * m + 1, 2 * m)));
+            }
+        }
+        s2 = H::sub(H::add(s0, s1), cross);
+        return MB_OK;
+    }
+    int fold(E2 r) {
+        const int round = round_++;
+        r_[round] = r;
+        if (round < (int)pt_.size()) {
+            const E2 t = pt_[round], tr = H::mul(t, r);   // (1 - t)(1 - r) + t r = 1 - t - r + 2 t r
+            eq_scale_ = H::mul(eq_scale_, H::add(H::sub(H::sub(E2{1, 0}, t), r), H::add(tr, tr)));
+        }
+        if (host_) { host_fold(r); return MB_OK; }
+        const Block& bl = blocks_[block_];
+        if (round + 1 == bl.first + bl.rounds) {
+            block_++;
+            return pass();
+        }
+        const int half = side_ / 2;   // rows, then columns
+        for (int i = 0; i < half; i++)
+            for (int j = 0; j < side_; j++) at(i, j) = H::fold(at(2 * i, j), at(2 * i + 1, j), r);
+        for (int i = 0; i < half; i++)
+            for (int j = 0; j < half; j++) at(i, j) = H::fold(at(i, 2 * j), at(i, 2 * j + 1), r);
+        side_ = half;
+        return MB_OK;
+    }
+    // a_k(R), b_k(R) after the last fold
+    int finals(E2* a, E2* b) {
+        int rc = wait();
+        if (rc != MB_OK) return rc;
+        for (int k = 0; k < K_; k++) { a[k] = ta_[(size_t)k * tn_]; b[k] = tb_[(size_t)k * tn_]; }
+        return MB_OK;
+    }
+    E2 eq_scale() const { return eq_scale_; }
+    E2 eq_coord(int round) const { return pt_[round]; }
+
+private:
+    struct Block {
+        int first, rounds;
+        size_t wl, wh;      // word offsets of the eq tables
+        int lo, row_shift;
+        size_t row_mask;
+    };
+    // eq tables of the passes: over the variables above a block, those of WL first
+    int tables() {
+        const int ne = (int)pt_.size();
+        pr::TableSet set;
+        int nt = 0;
+        size_t words = 0;
+        const auto table = [&](int first, int bits) {
+            set.d[nt].first = first;
+            set.d[nt].bits = bits;
+            set.d[nt].off = words;
+            words += (size_t)4 << bits;
+            return set.d[nt++].off;
+        };
+        for (Block& b : blocks_) {
+            const int above = ne - b.first - b.rounds;
+            if (above <= 0) continue;
+            b.lo = above < pr::ROW_BITS ? above : pr::ROW_BITS;
+            b.wl = table(b.first + b.rounds, b.lo);
+            b.wh = table(b.first + b.rounds + b.lo, above - b.lo);
+            if (above > b.lo) {
+                b.row_shift = b.lo + b.rounds;
+                b.row_mask = ((size_t)1 << (above - b.lo)) - 1;
+            }
+        }
+        if (!nt) return MB_OK;
+        MB_CUDA(pool_alloc((void**)&tabs_, sizeof(uint64_t) * (words + 2 * (size_t)ne)));
+        uint64_t* d_pt = tabs_ + words;
+        uint64_t* h = pin_ + PinnedPool::WORDS - 2 * (size_t)ne;   // the end of the block: no pass writes there
+        for (int i = 0; i < ne; i++) { h[2 * i] = pt_[i].c0; h[2 * i + 1] = pt_[i].c1; }
+        MB_CUDA(cudaMemcpyAsync(d_pt, h, 16 * (size_t)ne, cudaMemcpyHostToDevice, MB_STREAM));
+        MB_KERNEL("pair_eq_tables");
+        pr::eq_tables_kernel<F><<<nt, pr::BLK, 0, MB_STREAM>>>(set, d_pt, tabs_);
+        return finish_async();
+    }
+    // The pass before block block_ (or, after the last one, before the host tables): folds the challenges of the block
+    // before and queues the matrices of this one.
+    int pass() {
+        const int from = block_ > 0 ? blocks_[block_ - 1].first : 0, fb = block_ > 0 ? blocks_[block_ - 1].rounds : 0;
+        const bool last = block_ == blocks_.size();
+        pr::FoldWeights<F> fw;
+        E2 e[1 << pr::MAX_B];
+        H::eq_vector(r_.data() + from, fb, e);
+        for (int i = 0; i < (1 << fb); i++)
+            fw.w[i] = typename F::Pre{e[i].c0, e[i].c1, O::canon(O::red((hf::u128)e[i].c1 * O::W))};
+        pr::PairArgs p{};
+        p.fb = fb;
+        p.a = a_; p.b = b_; p.in_stride = stride_;
+        p.v = n_ - (last ? tail_first_ : blocks_[block_].first);
+        if (last) {
+            p.out = pin_;
+            tn_ = (size_t)1 << p.v;
+            if (fb == 0) return copy_tables();   // everything on the host
+        } else if (fb) {
+            uint64_t*& t = flip_ ? t1_ : t0_;
+            if (!t) MB_CUDA(pool_alloc((void**)&t, sizeof(uint64_t) * ((size_t)4 << p.v) * K_));
+            p.out = t;
+            flip_ = !flip_;
+        }
+        const int gb = last ? 0 : blocks_[block_].rounds;
+        bool weighted = false;
+        if (!last) {
+            const Block& b = blocks_[block_];
+            weighted = (int)pt_.size() > b.first + b.rounds;
+            p.lo = b.lo; p.row_shift = b.row_shift; p.row_mask = b.row_mask;
+            p.wl = tabs_ + b.wl; p.wh = tabs_ + b.wh;
+        }
+        p.partial = partial_; p.counter = counter_; p.sums = pin_;
+        const size_t tiles = (((size_t)1 << p.v) + pr::BLK - 1) / pr::BLK;
+        const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);
+        {
+            MB_KERNEL("pair_pass");
+            if (fb) base_ ? launch<true, true>(gb, weighted, grid, p, fw) : launch<true, false>(gb, weighted, grid, p, fw);
+            else base_ ? launch<false, true>(gb, weighted, grid, p, fw) : launch<false, false>(gb, weighted, grid, p, fw);
+        }
+        if (p.out && !last) {   // the folded tables are the next pass's input
+            a_ = p.out;
+            b_ = p.out + ((size_t)2 << p.v);
+            stride_ = (size_t)4 << p.v;
+        }
+        if (fb) base_ = false;
+        pending_ = true;
+        m_.clear();
+        return finish_async();
+    }
+    template <bool FOLD, bool BASE, int GB>
+    static void launch_w(bool weighted, dim3 grid, const pr::PairArgs& p, const pr::FoldWeights<F>& fw) {
+        if (weighted) pr::pair_pass_kernel<F, FOLD, GB, BASE, true><<<grid, pr::BLK, sizeof(uint64_t) * ((size_t)3 << p.lo), MB_STREAM>>>(p, fw);
+        else pr::pair_pass_kernel<F, FOLD, GB, BASE, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
+    }
+    template <bool FOLD, bool BASE>
+    static void launch(int gb, bool weighted, dim3 grid, const pr::PairArgs& p, const pr::FoldWeights<F>& fw) {
+        switch (gb) {
+            case 0: pr::pair_pass_kernel<F, true, 0, BASE, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw); break;
+            case 1: launch_w<FOLD, BASE, 1>(weighted, grid, p, fw); break;
+            case 2: launch_w<FOLD, BASE, 2>(weighted, grid, p, fw); break;
+            case 3: launch_w<FOLD, BASE, 3>(weighted, grid, p, fw); break;
+            default: launch_w<FOLD, BASE, 4>(weighted, grid, p, fw); break;
+        }
+    }
+    int copy_tables() {
+        const size_t w = tn_ * (base_ ? 1 : 2);
+        if (2 * w * K_ > PinnedPool::WORDS) return MB_ERR_UNSUPPORTED;
+        for (int k = 0; k < K_; k++)
+            for (int s = 0; s < 2; s++)
+                MB_CUDA(cudaMemcpyAsync(pin_ + (2 * k + s) * w, (s ? b_ : a_) + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
+        pending_ = true;
+        return MB_OK;
+    }
+    // Results of the pass queued last.
+    int wait() {
+        if (!pending_) return MB_OK;
+        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        pending_ = false;
+        if (block_ < blocks_.size()) return MB_OK;
+        host_ = true;
+        const size_t nw = base_ ? 1 : 2;
+        ta_.resize(tn_ * K_);
+        tb_.resize(tn_ * K_);
+        for (int k = 0; k < K_; k++)
+            for (size_t x = 0; x < tn_; x++) {
+                const uint64_t *p = pin_ + ((2 * (size_t)k) * tn_ + x) * nw, *q = p + tn_ * nw;
+                ta_[k * tn_ + x] = H::canon(E2{p[0], nw == 2 ? p[1] : 0});
+                tb_[k * tn_ + x] = H::canon(E2{q[0], nw == 2 ? q[1] : 0});
+            }
+        live_ = tn_;
+        return MB_OK;
+    }
+    // ---- the rounds of a block on the matrix ----
+    E2 entry(int k, int i, int j) const {
+        const int g = blocks_[block_].rounds;
+        const uint64_t* p = pin_ + 2 * (((size_t)k << (2 * g)) + ((size_t)i << g) + j);
+        return E2{p[0], p[1]};
+    }
+    E2& at(int i, int j) { return m_[(size_t)i * width_ + j]; }
+    void combine() {
+        const Block& b = blocks_[block_];
+        side_ = width_ = 1 << b.rounds;
+        m_.resize((size_t)width_ * width_);
+        for (int i = 0; i < width_; i++)
+            for (int j = 0; j < width_; j++) {
+                if (scale_.empty()) {
+                    at(i, j) = entry(0, i, j);
+                } else {
+                    typename H::Dot d;
+                    for (int k = 0; k < K_; k++) d.mac(scale_[k], entry(k, i, j));
+                    at(i, j) = d.value();
+                }
+            }
+        weighted_ = (int)pt_.size() > b.first + 1;
+        if (weighted_) suffix(b.first, b.first + b.rounds);
+    }
+    // eq over the variables above each round of [first, last): for round last - 1 one entry, then 2, 4, .. , back to
+    // back; variables without a coordinate weigh 1
+    void suffix(int first, int last) {
+        w_.assign((size_t)1 << (last - first), E2{1, 0});
+        size_t at = 0;
+        for (int j = last - 2; j >= first; j--) {
+            const size_t n = (size_t)1 << (last - 2 - j);
+            const bool has = j + 1 < (int)pt_.size();
+            for (size_t y = 0; y < n; y++) {
+                const E2 lo = w_[at + y], hi = has ? H::mul(lo, pt_[j + 1]) : lo;
+                w_[at + n + 2 * y] = has ? H::sub(lo, hi) : lo;
+                w_[at + n + 2 * y + 1] = hi;
+            }
+            at += n;
+        }
+    }
+    const E2* weights(size_t half) const { return w_.data() + (half - 1); }
+    // ---- host tables ----
+    E2 total(int k) {   // before any fold: sum over the whole cube
+        const E2 *a = ta_.data() + k * tn_, *b = tb_.data() + k * tn_;
+        typename H::Dot d;
+        const bool has = !pt_.empty();
+        const E2* w = weights(tn_ / 2);
+        for (size_t y = 0; 2 * y < tn_; y++) {
+            E2 x0 = H::mul(a[2 * y], b[2 * y]), x1 = H::mul(a[2 * y + 1], b[2 * y + 1]);
+            const E2 v = has ? H::add(x0, H::mul(pt_[0], H::sub(x1, x0))) : H::add(x0, x1);
+            d.mac(w[y], v);
+        }
+        return d.value();
+    }
+    void host_sums(E2& s0, E2& s1, E2& s2) {
+        const size_t half = live_ / 2;
+        const bool weigh = (int)pt_.size() > round_ + 1;
+        if (weigh && !have_w_) suffix(round_, n_);
+        have_w_ = true;
+        typename H::Dot d0, d1, d2;
+        for (int k = 0; k < K_; k++) {
+            const E2 *a = ta_.data() + k * tn_, *b = tb_.data() + k * tn_;
+            typename H::Dot e0, e1, e2;
+            typename H::Dot &f0 = scale_.empty() ? d0 : e0, &f1 = scale_.empty() ? d1 : e1, &f2 = scale_.empty() ? d2 : e2;
+            for (size_t y = 0; y < half; y++) {
+                E2 a0 = a[2 * y], a1 = a[2 * y + 1];
+                if (weigh) {
+                    const E2 w = weights(half)[y];
+                    a0 = H::mul(w, a0);
+                    a1 = H::mul(w, a1);
+                }
+                f0.mac(a0, b[2 * y]);
+                f1.mac(a1, b[2 * y + 1]);
+                f2.mac(H::sub(a1, a0), H::sub(b[2 * y + 1], b[2 * y]));
+            }
+            if (!scale_.empty()) {
+                d0.mac(scale_[k], e0.value());
+                d1.mac(scale_[k], e1.value());
+                d2.mac(scale_[k], e2.value());
+            }
+        }
+        s0 = d0.value(); s1 = d1.value(); s2 = d2.value();
+    }
+    void host_fold(E2 r) {
+        const size_t half = live_ / 2;
+        for (int k = 0; k < K_; k++)
+            for (E2* t : {ta_.data() + k * tn_, tb_.data() + k * tn_})
+                for (size_t y = 0; y < half; y++) t[y] = H::fold(t[2 * y], t[2 * y + 1], r);
+        live_ = half;
+    }
+
+    const uint64_t *a_ = nullptr, *b_ = nullptr;
+    size_t stride_ = 0;
+    int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0;
+    bool base_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false;
+    std::vector<Block> blocks_;
+    size_t block_ = 0;
+    std::vector<E2> pt_, r_, scale_, m_, w_, ta_, tb_;
+    int side_ = 0, width_ = 0;
+    size_t tn_ = 0, live_ = 0;
+    E2 eq_scale_{1, 0};
+    uint64_t *pin_ = nullptr, *t0_ = nullptr, *t1_ = nullptr, *tabs_ = nullptr, *partial_ = nullptr;
+    unsigned* counter_ = nullptr;
+};
+
+}  // namespace mbhost

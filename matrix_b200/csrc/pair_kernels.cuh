@@ -1,0 +1,281 @@
+// Several rounds of a sumcheck over products of two tables per pass.
+//
+// For sum_x w(x) a(x) b(x) (w = 1, or an eq polynomial) B consecutive rounds, which bind the low B variables, need
+// nothing of the tables but the 2^B x 2^B matrix
+//     M[i][j] = sum_y w'(y) a(i + 2^B y) b(j + 2^B y),          w' = w over the variables above the low B,
+// because folding and evaluating the round polynomials only combine rows and columns: the host runs the B rounds on
+// M. One pass over the tables folds the F challenges of the block of rounds before (a dot product with their eq
+// vector, reduced once), stores the folded tables and accumulates M from them. Per element that is 2^F products for
+// the fold and 2^B for M, against one read and write of the tables, one launch and one synchronisation per round when
+// every round has its own pass; B grows as the tables shrink (what bounds a large table is its traffic and products,
+// a small one the launch).
+//
+// A block takes tiles of 256 folded elements per table: thread t folds element t of a and of b into shared memory,
+// then thread t = (y group, i, j) adds its entry of M over the tile, 2^B products. Weights: w'(y) = WL[y mod 2^lo]
+// WH[y >> lo]; a is multiplied by WL before it enters shared memory, and a thread's sum by WH whenever the row ends.
+#pragma once
+#include "agl_traits.cuh"
+
+namespace mb {
+namespace pr {
+
+constexpr int BLK = 256;
+constexpr int MAX_B = 4;
+constexpr int ROW_BITS = 10;   // variables of WL
+
+// ---- fields --------------------------------------------------------------------------------------
+struct GlF {
+    using E2 = gl::E2;
+    using Pre = gl::E2Pre;
+    static constexpr uint32_t W = 7;
+    static __device__ __forceinline__ uint64_t canon(uint64_t x) { return gl::canon(x); }
+    static __device__ __forceinline__ uint64_t red(const gl::Acc& s) { return gl::acc_reduce(s); }
+    static __device__ __forceinline__ uint64_t redw(const gl::Acc& s) { return gl::acc_reduce_wide(s); }
+    static __device__ __forceinline__ uint64_t times_w(uint64_t x) { return gl::mul_small(x, W); }
+    static __device__ __forceinline__ E2 add(E2 a, E2 b) { return gl::e2_add(a, b); }
+    static __device__ __forceinline__ E2 sub(E2 a, E2 b) { return gl::e2_sub(a, b); }
+    static __device__ __forceinline__ E2 mul(E2 a, E2 b) { return gl::e2_mul_lazy(a, b); }
+    static __device__ __forceinline__ E2 fma(Pre w, E2 x, E2 a) { return gl::e2_fma_pre(w, x, a); }
+};
+struct AglF {
+    using E2 = agl::E2;
+    using Pre = agl::E2Pre;
+    static constexpr uint32_t W = 3;
+    static __device__ __forceinline__ uint64_t canon(uint64_t x) { return agl::canon(x); }
+    static __device__ __forceinline__ uint64_t red(const gl::Acc& s) { return agl::acc_reduce(s); }
+    static __device__ __forceinline__ uint64_t redw(const gl::Acc& s) { return agl::acc_reduce_wide(s); }
+    static __device__ __forceinline__ uint64_t times_w(uint64_t x) { return agl::mul_small(x, W); }
+    static __device__ __forceinline__ E2 add(E2 a, E2 b) { return agl::e2_add(a, b); }
+    static __device__ __forceinline__ E2 sub(E2 a, E2 b) { return agl::e2_sub(a, b); }
+    static __device__ __forceinline__ E2 mul(E2 a, E2 b) { return agl::e2_mul_lazy(a, b); }
+    static __device__ __forceinline__ E2 fma(Pre w, E2 x, E2 a) { return agl::e2_fma_pre(w, x, a); }
+};
+template <class E2>
+__device__ __forceinline__ E2 load2(const uint64_t* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return E2{v.x, v.y};
+}
+__device__ __forceinline__ void store2(uint64_t* p, uint64_t c0, uint64_t c1) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(c0, c1);
+}
+
+// ---- eq tables: entries (c0, c1, W c1, 0) over variables [first, first + bits) of the point -----------
+struct TableDesc {
+    int first, bits;
+    size_t off;   // words
+};
+constexpr int MAX_TABLES = 48;
+struct TableSet {
+    TableDesc d[MAX_TABLES];
+};
+template <class F>
+__global__ void __launch_bounds__(BLK)
+eq_tables_kernel(const __grid_constant__ TableSet set, const uint64_t* __restrict__ pt, uint64_t* __restrict__ tabs) {
+    using E2 = typename F::E2;
+    const TableDesc d = set.d[blockIdx.x];
+    uint64_t* out = tabs + d.off;
+    if (threadIdx.x == 0) store2(out, 1, 0);
+    __syncthreads();
+    for (int b = 0; b < d.bits; b++) {
+        const E2 rb = load2<E2>(pt + 2 * (d.first + b));
+        const size_t half = (size_t)1 << b;
+        for (size_t j = threadIdx.x; j < half; j += BLK) {
+            const E2 a = load2<E2>(out + 4 * j), ar = F::mul(a, rb), s = F::sub(a, ar);
+            store2(out + 4 * j, F::canon(s.c0), F::canon(s.c1));
+            store2(out + 4 * (j + half), F::canon(ar.c0), F::canon(ar.c1));
+        }
+        __syncthreads();
+    }
+    for (size_t j = threadIdx.x; j < ((size_t)1 << d.bits); j += BLK)
+        store2(out + 4 * j + 2, F::canon(F::times_w(out[4 * j + 1])), 0);
+}
+template <class F>
+__device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(p);
+    return typename F::Pre{a.x, a.y, p[2]};
+}
+
+// Sums the threads' values by t mod 2^bits over the block and then over the gridDim.x blocks of blockIdx.y; true in
+// the block that finishes last, with the sums (canonical) in sm[0 .. 2^bits). partial: gridDim.x * 2^bits elements of
+// this blockIdx.y; counter: zero before and after.
+template <class F>
+__device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F::E2* sm, uint64_t* partial, unsigned* counter) {
+    using E2 = typename F::E2;
+    __shared__ bool last;
+    const int t = threadIdx.x, n = 1 << bits;
+    const auto block_sum = [&](E2 x) {
+        __syncthreads();
+        sm[t] = x;
+        __syncthreads();
+        for (int s = BLK / 2; s >= n; s >>= 1) {
+            if (t < s) sm[t] = F::add(sm[t], sm[t + s]);
+            __syncthreads();
+        }
+        if (t < n) sm[t] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
+        __syncthreads();
+    };
+    block_sum(v);
+    if (gridDim.x == 1) return true;
+    if (t < n) {
+        store2(partial + 2 * ((size_t)blockIdx.x * n + t), sm[t].c0, sm[t].c1);
+        __threadfence();
+    }
+    __syncthreads();
+    if (t == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    E2 x{0, 0};
+    for (unsigned b = t >> bits; b < gridDim.x; b += BLK >> bits) {
+        const uint64_t* p = partial + 2 * ((size_t)b * n + (t & (n - 1)));
+        x = F::add(x, E2{__ldcg(p), __ldcg(p + 1)});
+    }
+    block_sum(x);
+    if (t == 0) *counter = 0;
+    return true;
+}
+
+// ---- the pass -----------------------------------------------------------------------------------------
+struct PairArgs {
+    int fb;                   // challenges to fold
+    const uint64_t *a, *b;    // instance 0's tables: 2^(v + fb) elements, base field words or (c0, c1)
+    size_t in_stride;         // words from one instance to the next
+    uint64_t* out;            // [instance][a, b][2^v][2] folded tables, or null
+    int v;                    // variables left after the fold
+    int lo;                   // weighted passes: variables of WL; y's next variables index WH
+    int row_shift;            // log2 of the elements between two entries of WH (63: WH is a single 1)
+    size_t row_mask;
+    const uint64_t *wl, *wh;
+    uint64_t* partial;        // [instance][gridDim.x][4^B][2]
+    unsigned* counter;        // per instance
+    uint64_t* sums;           // pinned: [instance][4^B][2]
+};
+template <class F>
+struct FoldWeights {
+    typename F::Pre w[1 << MAX_B];   // eq vector of the challenges to fold, bit k: challenge k
+};
+
+// element y of the folded table: a dot product with the eq vector of fb challenges (two or more inputs, read in pairs)
+template <class F, bool FOLD, bool BASE>
+__device__ __forceinline__ typename F::E2 fold_element(const uint64_t* p, size_t y, int fb, const FoldWeights<F>& fw) {
+    using E2 = typename F::E2;
+    if constexpr (!FOLD) {
+        if constexpr (BASE) return E2{p[y], 0};
+        else return load2<E2>(p + 2 * y);
+    } else {
+        gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
+        const uint64_t* q = p + ((BASE ? y : 2 * y) << fb);
+#pragma unroll 2
+        for (int m = 0; m < (1 << fb); m += 2) {
+            if constexpr (BASE) {
+                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(q + m);
+                gl::acc_mul(s0, fw.w[m].c0, x.x);
+                gl::acc_mul(s1, fw.w[m].c1, x.x);
+                gl::acc_mul(s0, fw.w[m + 1].c0, x.y);
+                gl::acc_mul(s1, fw.w[m + 1].c1, x.y);
+            } else {
+                const E2 x = load2<E2>(q + 2 * m), z = load2<E2>(q + 2 * m + 2);
+                gl::acc_mul(s0, fw.w[m].c0, x.c0);
+                gl::acc_mul(s0, fw.w[m].c1w, x.c1);
+                gl::acc_mul(s1, fw.w[m].c0, x.c1);
+                gl::acc_mul(s1, fw.w[m].c1, x.c0);
+                gl::acc_mul(s0, fw.w[m + 1].c0, z.c0);
+                gl::acc_mul(s0, fw.w[m + 1].c1w, z.c1);
+                gl::acc_mul(s1, fw.w[m + 1].c0, z.c1);
+                gl::acc_mul(s1, fw.w[m + 1].c1, z.c0);
+            }
+        }
+        return E2{F::canon(F::red(s0)), F::canon(F::red(s1))};
+    }
+}
+
+// FOLD: there are challenges to fold (a.fb of them); GB: rounds of the next block (0: fold and store only). BASE: input
+// words of the base field.
+template <class F, bool FOLD, int GB, bool BASE, bool WEIGHTED>
+__global__ void __launch_bounds__(BLK)
+pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
+    using E2 = typename F::E2;
+    constexpr bool RAW = BASE && !FOLD;                  // b stays a base field element, and a too without weights
+    constexpr int E = 1 << (2 * GB);                       // entries of M
+    extern __shared__ uint64_t wl_sm[];                    // WEIGHTED: c0[2^lo], c1[2^lo], W c1[2^lo]
+    __shared__ E2 sa[BLK], sb[BLK];
+    __shared__ uint64_t sbw[BLK];
+    const int t = threadIdx.x, k = blockIdx.y;
+    const uint64_t *pa = a.a + a.in_stride * k, *pb = a.b + a.in_stride * k;
+    uint64_t* oa = a.out ? a.out + ((size_t)4 << a.v) * k : nullptr;
+    const size_t n = (size_t)1 << a.v, tiles = (n + BLK - 1) / BLK;
+    const size_t per = (tiles + gridDim.x - 1) / gridDim.x, first = per * blockIdx.x;
+    const size_t end = first + per < tiles ? first + per : tiles;
+    if constexpr (WEIGHTED && GB > 0) {
+        const int nl = 1 << a.lo;
+        for (int j = t; j < nl; j += BLK) {
+            wl_sm[j] = a.wl[4 * j];
+            wl_sm[nl + j] = a.wl[4 * j + 1];
+            wl_sm[2 * nl + j] = a.wl[4 * j + 2];
+        }
+        __syncthreads();
+    }
+    gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
+    E2 sum{0, 0};
+    const int e = t & (E - 1), ei = (e >> GB) & ((1 << GB) - 1), ej = e & ((1 << GB) - 1), y0 = t >> (2 * GB);
+    for (size_t tile = first; tile < end; tile++) {
+        const size_t x = tile * BLK + t;
+        E2 fa{0, 0}, fb{0, 0};
+        if (x < n) {
+            fa = fold_element<F, FOLD, BASE>(pa, x, a.fb, fw);
+            fb = fold_element<F, FOLD, BASE>(pb, x, a.fb, fw);
+            if (oa != nullptr) {
+                store2(oa + 2 * x, fa.c0, fa.c1);
+                store2(oa + 2 * (n + x), fb.c0, fb.c1);
+            }
+        }
+        if constexpr (GB > 0) {
+            if constexpr (WEIGHTED) {
+                const int nl = 1 << a.lo, y = (int)((x >> GB) & (nl - 1));
+                const typename F::Pre w{wl_sm[y], wl_sm[nl + y], wl_sm[2 * nl + y]};
+                gl::Acc c0 = gl::acc_zero(), c1 = gl::acc_zero();
+                gl::acc_mul(c0, w.c0, fa.c0);
+                gl::acc_mul(c1, w.c1, fa.c0);
+                if constexpr (!RAW) {
+                    gl::acc_mul(c0, w.c1w, fa.c1);
+                    gl::acc_mul(c1, w.c0, fa.c1);
+                }
+                fa = E2{F::red(c0), F::red(c1)};
+            }
+            __syncthreads();   // the tile before has been read
+            sa[t] = fa;
+            sb[t] = fb;
+            if constexpr (!RAW) sbw[t] = F::times_w(fb.c1);
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < (1 << GB); q++) {
+                const int y = (y0 + q * (BLK >> (2 * GB))) << GB;
+                const E2 u = sa[y + ei];
+                const uint64_t v0 = sb[y + ej].c0;
+                gl::acc_mul(s0, u.c0, v0);
+                if constexpr (!RAW || WEIGHTED) gl::acc_mul(s1, u.c1, v0);
+                if constexpr (!RAW) {
+                    gl::acc_mul(s0, u.c1, sbw[y + ej]);
+                    gl::acc_mul(s1, u.c0, sb[y + ej].c1);
+                }
+            }
+            if constexpr (WEIGHTED) {
+                // the row's WH when the row or the block's share ends
+                const size_t row = (tile * BLK) >> a.row_shift;
+                if (tile + 1 == end || ((tile + 1) * BLK) >> a.row_shift != row) {
+                    sum = F::fma(load_weight<F>(a.wh + 4 * (row & a.row_mask)), E2{F::redw(s0), F::redw(s1)}, sum);
+                    s0 = gl::acc_zero();
+                    s1 = gl::acc_zero();
+                }
+            }
+        }
+    }
+    if constexpr (GB > 0) {
+        if constexpr (!WEIGHTED) sum = E2{F::redw(s0), F::redw(s1)};
+        if (!grid_sum<F>(sum, 2 * GB, sa, a.partial + ((size_t)(2 * gridDim.x) << (2 * GB)) * k, a.counter + k)) return;
+        if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), sa[t].c0, sa[t].c1);
+    }
+}
+
+}  // namespace pr
+}  // namespace mb
