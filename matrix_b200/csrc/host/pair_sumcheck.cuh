@@ -111,10 +111,10 @@ public:
         pin_ = PinnedPool::take();
         if (!pin_) return MB_ERR_CUDA;
         if (!blocks_.empty()) {
-            cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;
-            MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 2 * 256 * (size_t)cap_ * K));
-            MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned) * K));
-            MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * K, MB_STREAM));
+            cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;   // a wave: four blocks of at most 64 registers fit an SM
+            MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 4 * 256 * (size_t)cap_ * K));
+            MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned) * (pr::GROUPS + 1) * K));
+            MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * (pr::GROUPS + 1) * K, MB_STREAM));
             int rc = tables();
             if (rc != MB_OK) return rc;
         }

@@ -28,18 +28,30 @@ namespace mk {
 constexpr int BLOCK = 128;
 constexpr int TAIL_NODES = 64;  // layers of at most this many nodes are finished by one block
 
-// Hash policies. COOP: an 8-lanes-per-permutation variant exists for small layers.
+// Hash policies. COOP: an 8-lanes-per-permutation variant exists for small layers. permute(load): the permutation of the
+// state that load(s) writes (it may be asked for again).
 struct HashPoseidon2 {
     static constexpr int WIDTH = 8;
     static constexpr bool COOP = true;
-    static __device__ __forceinline__ void permute(uint64_t* s) { gl::poseidon2_permute(s); }
+    template <class Load>
+    static __device__ __forceinline__ void permute(uint64_t* s, Load load) {
+        load(s);
+        if (!gl::poseidon2_permute_throughput(s)) {
+            load(s);
+            gl::poseidon2_permute(s);
+        }
+    }
     static const char* leaves_name() { return "hash_leaves"; }
     static const char* layer_name() { return "compress_layer"; }
 };
 struct HashMonolith {
     static constexpr int WIDTH = 12;
     static constexpr bool COOP = false;
-    static __device__ __forceinline__ void permute(uint64_t* s) { gl::monolith_permute(s); }
+    template <class Load>
+    static __device__ __forceinline__ void permute(uint64_t* s, Load load) {
+        load(s);
+        gl::monolith_permute(s);
+    }
     static const char* leaves_name() { return "monolith_hash_leaves"; }
     static const char* layer_name() { return "monolith_compress_layer"; }
 };
@@ -50,42 +62,47 @@ __device__ __forceinline__ void store_digest(uint64_t* out, const uint64_t* s) {
 }
 
 template <class H, bool EXT2>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, H::COOP ? 9 : 1)
 hash_leaves_kernel(const uint64_t* __restrict__ cw, uint64_t* __restrict__ digests, size_t num_leaves) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < num_leaves; k += step) {
-        uint64_t s[H::WIDTH];
-        if (EXT2) {
-            ulonglong2 a = *reinterpret_cast<const ulonglong2*>(cw + 4 * k);
-            ulonglong2 b = *reinterpret_cast<const ulonglong2*>(cw + 4 * k + 2);
-            s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
-        } else {
-            ulonglong2 a = *reinterpret_cast<const ulonglong2*>(cw + 2 * k);
-            s[0] = a.x; s[1] = a.y; s[2] = 0; s[3] = 0;
-        }
+        uint64_t st[H::WIDTH];
+        H::permute(st, [&](uint64_t* s) {
+            if (EXT2) {
+                ulonglong2 a = *reinterpret_cast<const ulonglong2*>(cw + 4 * k);
+                ulonglong2 b = *reinterpret_cast<const ulonglong2*>(cw + 4 * k + 2);
+                s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
+            } else {
+                ulonglong2 a = *reinterpret_cast<const ulonglong2*>(cw + 2 * k);
+                s[0] = a.x; s[1] = a.y; s[2] = 0; s[3] = 0;
+            }
 #pragma unroll
-        for (int i = 4; i < H::WIDTH; i++) s[i] = 0;
-        H::permute(s);
-        store_digest(digests + 4 * k, s);
+            for (int i = 4; i < H::WIDTH; i++) s[i] = 0;
+        });
+        store_digest(digests + 4 * k, st);
     }
 }
 
+// eight words in front of zeros
 template <class H>
-__device__ __forceinline__ void compress_node(const uint64_t* in, uint64_t* out) {
-    uint64_t s[H::WIDTH];
-    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(in);
-    ulonglong2 a = p[0], b = p[1], c = p[2], d = p[3];
+__device__ __forceinline__ void load_pair(const uint64_t* l, const uint64_t* r, uint64_t* s) {
+    const ulonglong2 *p = reinterpret_cast<const ulonglong2*>(l), *q = reinterpret_cast<const ulonglong2*>(r);
+    const ulonglong2 a = p[0], b = p[1], c = q[0], d = q[1];
     s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
     s[4] = c.x; s[5] = c.y; s[6] = d.x; s[7] = d.y;
 #pragma unroll
     for (int i = 8; i < H::WIDTH; i++) s[i] = 0;
-    H::permute(s);
-    store_digest(out, s);
+}
+template <class H>
+__device__ __forceinline__ void compress_node(const uint64_t* in, uint64_t* out) {
+    uint64_t st[H::WIDTH];
+    H::permute(st, [&](uint64_t* s) { load_pair<H>(in, in + 4, s); });
+    store_digest(out, st);
 }
 
 // out[k] = compress(in[2k], in[2k+1]) for k < n
 template <class H>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, H::COOP ? 9 : 1)
 compress_layer_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += step) compress_node<H>(in + 8 * k, out + 4 * k);
@@ -97,15 +114,9 @@ compress_pairs_kernel(const uint64_t* __restrict__ left, const uint64_t* __restr
                       uint64_t* __restrict__ out, size_t n) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += step) {
-        uint64_t s[8];
-        ulonglong2 a = *reinterpret_cast<const ulonglong2*>(left + 4 * k);
-        ulonglong2 b = *reinterpret_cast<const ulonglong2*>(left + 4 * k + 2);
-        ulonglong2 c = *reinterpret_cast<const ulonglong2*>(right + 4 * k);
-        ulonglong2 d = *reinterpret_cast<const ulonglong2*>(right + 4 * k + 2);
-        s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
-        s[4] = c.x; s[5] = c.y; s[6] = d.x; s[7] = d.y;
-        gl::poseidon2_permute(s);
-        store_digest(out + 4 * k, s);
+        uint64_t st[8];
+        HashPoseidon2::permute(st, [&](uint64_t* s) { load_pair<HashPoseidon2>(left + 4 * k, right + 4 * k, s); });
+        store_digest(out + 4 * k, st);
     }
 }
 
@@ -248,18 +259,14 @@ tree_up_coop_kernel(uint64_t* layer, size_t size, int levels, uint64_t* last_out
 }
 
 // Full permutation of n width-8 states (poseidon2_hash_batch_ffi).
-static __global__ void __launch_bounds__(BLOCK)
+static __global__ void __launch_bounds__(BLOCK, 9)
 permute_batch_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += step) {
-        uint64_t s[8];
-        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(in + 8 * k);
-        ulonglong2 a = p[0], b = p[1], c = p[2], d = p[3];
-        s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
-        s[4] = c.x; s[5] = c.y; s[6] = d.x; s[7] = d.y;
-        gl::poseidon2_permute(s);
-        store_digest(out + 8 * k, s);
-        store_digest(out + 8 * k + 4, s + 4);
+        uint64_t st[8];
+        HashPoseidon2::permute(st, [&](uint64_t* s) { load_pair<HashPoseidon2>(in + 8 * k, in + 8 * k + 4, s); });
+        store_digest(out + 8 * k, st);
+        store_digest(out + 8 * k + 4, st + 4);
     }
 }
 

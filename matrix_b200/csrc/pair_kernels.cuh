@@ -96,10 +96,13 @@ __device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
 }
 
 // Sums the threads' values by t mod 2^bits over the block and then over the gridDim.x blocks of blockIdx.y; true in
-// the block that finishes last, with the sums (canonical) in sm[0 .. 2^bits). partial: gridDim.x * 2^bits elements of
-// this blockIdx.y; counter: zero before and after.
+// the block that finishes last, with the sums (canonical) in sm[0 .. 2^bits). partial: 2 gridDim.x * 2^bits elements of
+// this blockIdx.y; counters: GROUPS + 1 of this blockIdx.y, zero before and after.
+// A block that reads hundreds of rows one after another waits for L2 each time (512 rows: 70 us), so rows are summed in
+// groups of about sqrt(gridDim.x) by each group's last block, then the groups by the last of those.
+constexpr int GROUPS = 64;
 template <class F>
-__device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F::E2* sm, uint64_t* partial, unsigned* counter) {
+__device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F::E2* sm, uint64_t* partial, unsigned* counters) {
     using E2 = typename F::E2;
     __shared__ bool last;
     const int t = threadIdx.x, n = 1 << bits;
@@ -114,24 +117,41 @@ __device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F:
         if (t < n) sm[t] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
         __syncthreads();
     };
+    // writes sm to row `row`, takes a ticket of `counter`; true in the block that takes the last of `of`
+    const auto publish = [&](size_t row, unsigned* counter, unsigned of) {
+        if (t < n) {
+            store2(partial + 2 * (row * n + t), sm[t].c0, sm[t].c1);
+            __threadfence();
+        }
+        __syncthreads();
+        if (t == 0) {
+            last = atomicAdd(counter, 1u) == of - 1;
+            if (last) *counter = 0;
+        }
+        __syncthreads();
+        return last;
+    };
+    const auto rows_sum = [&](size_t first, unsigned count) {
+        __threadfence();
+        E2 x{0, 0};
+#pragma unroll 8
+        for (unsigned b = t >> bits; b < count; b += BLK >> bits) {
+            const uint64_t* p = partial + 2 * ((first + b) * n + (t & (n - 1)));
+            x = F::add(x, E2{__ldcg(p), __ldcg(p + 1)});
+        }
+        block_sum(x);
+    };
     block_sum(v);
     if (gridDim.x == 1) return true;
-    if (t < n) {
-        store2(partial + 2 * ((size_t)blockIdx.x * n + t), sm[t].c0, sm[t].c1);
-        __threadfence();
-    }
-    __syncthreads();
-    if (t == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    E2 x{0, 0};
-    for (unsigned b = t >> bits; b < gridDim.x; b += BLK >> bits) {
-        const uint64_t* p = partial + 2 * ((size_t)b * n + (t & (n - 1)));
-        x = F::add(x, E2{__ldcg(p), __ldcg(p + 1)});
-    }
-    block_sum(x);
-    if (t == 0) *counter = 0;
+    unsigned per = 8;   // rows per group
+    while (per * per < gridDim.x || (gridDim.x + per - 1) / per > GROUPS) per += 8;
+    const unsigned groups = (gridDim.x + per - 1) / per, g = blockIdx.x / per;
+    const unsigned members = (g + 1) * per <= gridDim.x ? per : gridDim.x - g * per;
+    if (!publish(blockIdx.x, counters + 1 + g, members)) return false;
+    rows_sum((size_t)g * per, members);
+    if (groups == 1) return true;
+    if (!publish(gridDim.x + g, counters, groups)) return false;
+    rows_sum(gridDim.x, groups);
     return true;
 }
 
@@ -146,8 +166,8 @@ struct PairArgs {
     int row_shift;            // log2 of the elements between two entries of WH (63: WH is a single 1)
     size_t row_mask;
     const uint64_t *wl, *wh;
-    uint64_t* partial;        // [instance][gridDim.x][4^B][2]
-    unsigned* counter;        // per instance
+    uint64_t* partial;        // [instance][2 gridDim.x][4^B][2]
+    unsigned* counter;        // [instance][GROUPS + 1]
     uint64_t* sums;           // pinned: [instance][4^B][2]
 };
 template <class F>
@@ -218,16 +238,30 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
     gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
     E2 sum{0, 0};
     const int e = t & (E - 1), ei = (e >> GB) & ((1 << GB) - 1), ej = e & ((1 << GB) - 1), y0 = t >> (2 * GB);
+    // without a fold the next tile's elements are loaded before this tile's products
+    E2 na{0, 0}, nb{0, 0};
+    const auto prefetch = [&](size_t tile) {
+        const size_t x = tile * BLK + t;
+        if (!FOLD && tile < end && x < n) {
+            na = fold_element<F, FOLD, BASE>(pa, x, 0, fw);
+            nb = fold_element<F, FOLD, BASE>(pb, x, 0, fw);
+        }
+    };
+    prefetch(first);
     for (size_t tile = first; tile < end; tile++) {
         const size_t x = tile * BLK + t;
-        E2 fa{0, 0}, fb{0, 0};
-        if (x < n) {
-            fa = fold_element<F, FOLD, BASE>(pa, x, a.fb, fw);
-            fb = fold_element<F, FOLD, BASE>(pb, x, a.fb, fw);
-            if (oa != nullptr) {
-                store2(oa + 2 * x, fa.c0, fa.c1);
-                store2(oa + 2 * (n + x), fb.c0, fb.c1);
+        E2 fa = na, fb = nb;
+        if constexpr (FOLD) {
+            if (x < n) {
+                fa = fold_element<F, FOLD, BASE>(pa, x, a.fb, fw);
+                fb = fold_element<F, FOLD, BASE>(pb, x, a.fb, fw);
+                if (oa != nullptr) {
+                    store2(oa + 2 * x, fa.c0, fa.c1);
+                    store2(oa + 2 * (n + x), fb.c0, fb.c1);
+                }
             }
+        } else {
+            prefetch(tile + 1);
         }
         if constexpr (GB > 0) {
             if constexpr (WEIGHTED) {
@@ -272,7 +306,7 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
     }
     if constexpr (GB > 0) {
         if constexpr (!WEIGHTED) sum = E2{F::redw(s0), F::redw(s1)};
-        if (!grid_sum<F>(sum, 2 * GB, sa, a.partial + ((size_t)(2 * gridDim.x) << (2 * GB)) * k, a.counter + k)) return;
+        if (!grid_sum<F>(sum, 2 * GB, sa, a.partial + ((size_t)(4 * gridDim.x) << (2 * GB)) * k, a.counter + (GROUPS + 1) * k)) return;
         if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), sa[t].c0, sa[t].c1);
     }
 }
