@@ -153,19 +153,37 @@ int prove_pair_with_eq(const uint64_t* d_a, const uint64_t* d_b, bool base, int 
 }
 
 // Lagrange interpolation through x = 0..n-1, evaluated at x (verifier.rs:91-113).
+// The denominators are products of small integers: their inverses are formed once per node count.
 static Ext2 interpolate_and_evaluate(const Ext2* evals, int n, Ext2 x) {
-    Ext2 result{0, 0};
-    for (int i = 0; i < n; i++) {
-        Ext2 basis{1, 0};
-        for (int j = 0; j < n; j++) {
-            if (j == i) continue;
-            Ext2 num = aext2_sub_host(x, Ext2{(uint64_t)j, 0});
-            Ext2 den = aext2_sub_host(Ext2{(uint64_t)i, 0}, Ext2{(uint64_t)j, 0});
-            basis = aext2_mul_host(basis, aext2_mul_host(num, aext2_inv_host(den)));
+    using H = PairHost<pr::AglF, PairAgl>;
+    using E2 = agl::E2;
+    struct Table {
+        uint64_t inv[MAX_D + 2][MAX_D + 1];
+        Table() {
+            for (int m = 1; m <= MAX_D + 1; m++)
+                for (int i = 0; i < m; i++) {
+                    uint64_t den = 1;
+                    for (int j = 0; j < m; j++)
+                        if (j != i) den = agl::mul(den, agl::sub((uint64_t)i, (uint64_t)j));
+                    inv[m][i] = agl::canon(agl::inv(den));
+                }
         }
-        result = aext2_add_host(result, aext2_mul_host(basis, evals[i]));
+    };
+    static const Table table;
+    // prefix and suffix products of x - j
+    E2 d[MAX_D + 1], pre[MAX_D + 2], suf[MAX_D + 2];
+    pre[0] = suf[n] = E2{1, 0};
+    for (int j = 0; j < n; j++) d[j] = H::sub(E2{x.c0, x.c1}, E2{(uint64_t)j, 0});
+    for (int j = 0; j < n; j++) pre[j + 1] = H::mul(pre[j], d[j]);
+    for (int j = n - 1; j >= 0; j--) suf[j] = H::mul(suf[j + 1], d[j]);
+    typename H::Dot sum;
+    for (int i = 0; i < n; i++) {
+        const E2 e{evals[i].c0, evals[i].c1};
+        const uint64_t w = table.inv[n][i];
+        sum.mac(E2{PairAgl::canon(PairAgl::red((hf::u128)e.c0 * w)), PairAgl::canon(PairAgl::red((hf::u128)e.c1 * w))}, H::mul(pre[i], suf[i + 1]));
     }
-    return result;
+    const E2 r = sum.value();
+    return Ext2{r.c0, r.c1};
 }
 
 }  // namespace mbhost

@@ -67,23 +67,37 @@ static int prove_linear(const uint64_t* d_tables, int d, int num_var, bool base_
 
 // Lagrange interpolation through x = 0..n-1, evaluated at x (zk-torch-3/src/sumcheck/verifier.rs: the next claim is
 // P_round(r)).
+// The denominators are products of small integers: their inverses are formed once per node count.
 static Ext2 interpolate_and_evaluate(const Ext2* evals, int n, Ext2 x) {
-    gl::E2 result{0, 0};
-    const gl::E2 xx{x.c0, x.c1};
-    for (int i = 0; i < n; i++) {
-        gl::E2 num{1, 0};
-        uint64_t den = 1;
-        for (int j = 0; j < n; j++) {
-            if (j == i) continue;
-            num = gl::e2_canon(gl::e2_mul(num, gl::e2_sub(xx, gl::E2{(uint64_t)j, 0})));
-            den = gl::mul(den, gl::sub((uint64_t)i, (uint64_t)j));
+    using H = PairHost<pr::GlF, PairGl>;
+    using E2 = gl::E2;
+    struct Table {
+        uint64_t inv[MAX_D + 2][MAX_D + 1];
+        Table() {
+            for (int m = 1; m <= MAX_D + 1; m++)
+                for (int i = 0; i < m; i++) {
+                    uint64_t den = 1;
+                    for (int j = 0; j < m; j++)
+                        if (j != i) den = gl::mul(den, gl::sub((uint64_t)i, (uint64_t)j));
+                    inv[m][i] = gl::canon(gl::inv(den));
+                }
         }
-        const uint64_t inv = gl::canon(gl::inv(den));
-        const gl::E2 basis{gl::mul(num.c0, inv), gl::mul(num.c1, inv)};
-        result = gl::e2_add(result, gl::e2_mul(gl::E2{evals[i].c0, evals[i].c1}, basis));
+    };
+    static const Table table;
+    // prefix and suffix products of x - j
+    E2 d[MAX_D + 1], pre[MAX_D + 2], suf[MAX_D + 2];
+    pre[0] = suf[n] = E2{1, 0};
+    for (int j = 0; j < n; j++) d[j] = H::sub(E2{x.c0, x.c1}, E2{(uint64_t)j, 0});
+    for (int j = 0; j < n; j++) pre[j + 1] = H::mul(pre[j], d[j]);
+    for (int j = n - 1; j >= 0; j--) suf[j] = H::mul(suf[j + 1], d[j]);
+    typename H::Dot sum;
+    for (int i = 0; i < n; i++) {
+        const E2 e{evals[i].c0, evals[i].c1};
+        const uint64_t w = table.inv[n][i];
+        sum.mac(E2{PairGl::canon(PairGl::red((hf::u128)e.c0 * w)), PairGl::canon(PairGl::red((hf::u128)e.c1 * w))}, H::mul(pre[i], suf[i + 1]));
     }
-    result = gl::e2_canon(result);
-    return Ext2{result.c0, result.c1};
+    const E2 r = sum.value();
+    return Ext2{r.c0, r.c1};
 }
 
 }  // namespace mbhost

@@ -19,6 +19,14 @@ constexpr uint64_t GL_EPS = 0xFFFFFFFFULL;   // 2^64 mod p
 // x = lo - hi_hi + hi_lo (2^32 - 1). A borrow is repaired by - EPS (the wrapped value is above 2^64 - 2^32), a
 // carry by + EPS (the wrapped value is below hi_lo EPS < 2^64 - 2^33).
 static inline uint64_t gl_red(u128 x) {
+#if defined(__x86_64__)
+    // seven micro-operations: hi_lo (2^32 - 1) is one multiplication, the borrow (once in 2^32 random words) a jump
+    uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64), t;
+    asm("mov %k[hi], %k[t]\n\timul %[eps], %[t]\n\tshr $32, %[hi]\n\tsub %[hi], %[lo]\n\tjb 2f\n1:\tadd %[t], %[lo]\n\t"
+        "sbb %k[t], %k[t]\n\tadd %[t], %[lo]\n\t.subsection 1\n2:\tsub %[eps], %[lo]\n\tjmp 1b\n\t.previous"
+        : [lo] "+r"(lo), [hi] "+r"(hi), [t] "=&r"(t) : [eps] "r"(GL_EPS) : "cc");
+    return lo;
+#else
     const uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64);
     const uint64_t hh = hi >> 32, hl = hi & GL_EPS, t1 = (hl << 32) - hl;
     uint64_t t0 = lo - hh;
@@ -26,6 +34,7 @@ static inline uint64_t gl_red(u128 x) {
     uint64_t r = t0 + t1;
     r += (0 - (uint64_t)(r < t1)) & GL_EPS;
     return r;
+#endif
 }
 static inline uint64_t gl_canon(uint64_t x) { return x >= GL_P ? x - GL_P : x; }
 // canonical in, canonical out
@@ -52,9 +61,18 @@ static inline uint64_t agl_red_small(u128 x) {
 }
 // Any 128-bit value: two folds of the high word (2^64 = c) bring it below 2^34 and then below 8.
 static inline uint64_t agl_red(u128 x) {
+#if defined(__x86_64__)
+    // the same two folds in registers; the last carry (h 2^64 for h below 8 leaves a word near 2^64 only once in 2^28) a jump
+    uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64), a = hi;
+    asm("mul %[c]\n\tadd %%rax, %[lo]\n\tadc $0, %%rdx\n\tmov %%rdx, %%rax\n\tmul %[c]\n\tadd %%rax, %[lo]\n\tadc $0, %%rdx\n\t"
+        "imul %[c], %%rdx\n\tadd %%rdx, %[lo]\n\tjc 2f\n1:\n\t.subsection 1\n2:\tadd %[c], %[lo]\n\tjmp 1b\n\t.previous"
+        : [lo] "+r"(lo), "+a"(a), "=&d"(hi) : [c] "r"(AGL_C) : "cc");
+    return lo;
+#else
     x = (u128)(uint64_t)(x >> 64) * AGL_C + (uint64_t)x;
     x = (u128)(uint64_t)(x >> 64) * AGL_C + (uint64_t)x;
     return agl_red_small(x);
+#endif
 }
 static inline uint64_t agl_canon(uint64_t x) { return x >= AGL_P ? x - AGL_P : x; }
 static inline uint64_t agl_add(uint64_t a, uint64_t b) {

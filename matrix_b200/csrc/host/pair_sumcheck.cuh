@@ -316,10 +316,14 @@ private:
     int copy_tables() {
         const size_t w = tn_ * (base_ ? 1 : 2);
         if (2 * w * K_ > PinnedPool::WORDS) return MB_ERR_UNSUPPORTED;
+        pending_ = true;
+        if (K_ == 1 && b_ == a_ + w) {
+            MB_CUDA(cudaMemcpyAsync(pin_, a_, 16 * w, cudaMemcpyDeviceToHost, MB_STREAM));
+            return MB_OK;
+        }
         for (int k = 0; k < K_; k++)
             for (int s = 0; s < 2; s++)
                 MB_CUDA(cudaMemcpyAsync(pin_ + (2 * k + s) * w, (s ? b_ : a_) + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
-        pending_ = true;
         return MB_OK;
     }
     // Results of the pass queued last.
@@ -339,6 +343,7 @@ private:
                 tb_[k * tn_ + x] = H::canon(E2{q[0], nw == 2 ? q[1] : 0});
             }
         live_ = tn_;
+        words_ = nw == 1;
         return MB_OK;
     }
     // ---- the rounds of a block on the matrix ----
@@ -400,6 +405,17 @@ private:
         const bool weigh = (int)pt_.size() > round_ + 1;
         if (weigh && !have_w_) suffix(round_, n_);
         have_w_ = true;
+        if (words_ && !weigh && scale_.empty()) {   // base field words still: one product instead of four
+            typename H::Wide p0, p1, p2;
+            for (size_t y = 0; y < half; y++) {
+                const uint64_t a0 = ta_[2 * y].c0, a1 = ta_[2 * y + 1].c0, b0 = tb_[2 * y].c0, b1 = tb_[2 * y + 1].c0;
+                p0.mac(a0, b0);
+                p1.mac(a1, b1);
+                p2.mac(O::sub(a1, a0), O::sub(b1, b0));
+            }
+            s0 = E2{O::canon(p0.red()), 0}; s1 = E2{O::canon(p1.red()), 0}; s2 = E2{O::canon(p2.red()), 0};
+            return;
+        }
         typename H::Dot d0, d1, d2;
         for (int k = 0; k < K_; k++) {
             const E2 *a = ta_.data() + k * tn_, *b = tb_.data() + k * tn_;
@@ -428,14 +444,22 @@ private:
         const size_t half = live_ / 2;
         for (int k = 0; k < K_; k++)
             for (E2* t : {ta_.data() + k * tn_, tb_.data() + k * tn_})
-                for (size_t y = 0; y < half; y++) t[y] = H::fold(t[2 * y], t[2 * y + 1], r);
+                for (size_t y = 0; y < half; y++) {
+                    if (words_) {
+                        const uint64_t x = t[2 * y].c0, d = O::sub(t[2 * y + 1].c0, x);
+                        t[y] = E2{O::canon(O::red((hf::u128)r.c0 * d + x)), O::canon(O::red((hf::u128)r.c1 * d))};
+                    } else {
+                        t[y] = H::fold(t[2 * y], t[2 * y + 1], r);
+                    }
+                }
+        words_ = false;
         live_ = half;
     }
 
     const uint64_t *a_ = nullptr, *b_ = nullptr;
     size_t stride_ = 0;
     int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0;
-    bool base_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false;
+    bool base_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;
     std::vector<E2> pt_, r_, scale_, m_, w_, ta_, tb_;
