@@ -15,6 +15,7 @@
 //  * reductions use warp shuffles and finish on the device.
 // All outputs are canonical.
 #pragma once
+#include "codeword_fold.cuh"
 #include "sumcheck_kernels.cuh"
 
 namespace mb {
@@ -106,7 +107,61 @@ struct CodeOp {
     }
 };
 
-// One pass applies Op on index bits [bit_lo, bit_lo + nbits). A tile holds
+// Interp then Code on one bit: (a, b) -> (b, 2 a - b). Both are maps of single bits, so the evaluations become the codeword
+// in one set of passes.
+struct InterpCodeOp {
+    static __device__ __forceinline__ void apply(uint64_t& a, uint64_t& b) {
+        const uint64_t d = gl::add(a, gl::sub(a, b));
+        a = b;
+        b = d;
+    }
+};
+
+// One pass over tiles of 2^12 elements: Op on index bits [bit_lo, bit_lo + nbits), a tile being 2^nbits rows (stride
+// 2^bit_lo) of 2^(12 - nbits) consecutive elements. A thread takes sixteen elements through four bits in registers, so
+// shared memory is read and written once per four bits (bit by bit it was the bound: 167 us a pass at 2^24 elements);
+// one padding word per sixteen keeps the strided accesses apart.
+template <class Op>
+__global__ void __launch_bounds__(BLOCK)
+bit_pass_kernel(const uint64_t* in, uint64_t* out, int log_n, int bit_lo, int nbits) {
+    extern __shared__ uint64_t tile[];
+    constexpr int N = 1 << TILE_LOG;
+    const int cbits = TILE_LOG - nbits, mid_bits = bit_lo - cbits, t = threadIdx.x;
+    const auto pad = [](int e) { return e + (e >> 4); };
+    const size_t num_tiles = (size_t)1 << (log_n - TILE_LOG);
+    for (size_t k = blockIdx.x; k < num_tiles; k += gridDim.x) {
+        const size_t mid = k & (((size_t)1 << mid_bits) - 1), high = k >> mid_bits;
+        const size_t base = (high << (bit_lo + nbits)) | (mid << cbits);
+        const auto addr = [&](int e) { return base | ((size_t)(e >> cbits) << bit_lo) | (size_t)(e & ((1 << cbits) - 1)); };
+#pragma unroll 8
+        for (int e = t; e < N; e += BLOCK) tile[pad(e)] = in[addr(e)];
+        for (int q = cbits; q < TILE_LOG; q += 4) {
+            const int left = TILE_LOG - q < 4 ? TILE_LOG - q : 4;   // bits of this group
+            // sixteen elements: the bits [p, p + 4) of the index, p + 4 never above the tile
+            const int p = q + 4 <= TILE_LOG ? q : TILE_LOG - 4;
+            const int e0 = ((t >> p) << (p + 4)) | (t & ((1 << p) - 1));
+            uint64_t v[16];
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[j] = tile[pad(e0 | (j << p))];
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                if (b < 4 - left) continue;   // a short last group: its bits are the upper ones
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (!(j & (1 << b))) Op::apply(v[j], v[j | (1 << b)]);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; j++) tile[pad(e0 | (j << p))] = v[j];
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int e = t; e < N; e += BLOCK) out[addr(e)] = gl::canon(tile[pad(e)]);
+        __syncthreads();
+    }
+}
+
+// The same for arrays smaller than a tile of bit_pass_kernel, and any split: one pass applies Op on index bits [bit_lo, bit_lo + nbits). A tile holds
 // 2^nbits rows (stride 2^bit_lo) of 2^cbits consecutive elements, nbits + cbits
 // <= TILE_LOG and cbits <= bit_lo (cbits = 0 when bit_lo = 0). `in` may equal `out`.
 template <class Op>
@@ -162,22 +217,18 @@ static __global__ void fold_mixed_kernel(const uint64_t* __restrict__ cw, const 
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += step) {
         ulonglong2 v = *reinterpret_cast<const ulonglong2*>(cw + 2 * i);
         ulonglong2 e = *reinterpret_cast<const ulonglong2*>(table + 2 * i);
-        uint64_t dw = gl::mul(gl::sub(v.y, v.x), e.y);
-        gl::E2 cx{gl::sub(r.c0, e.x), r.c1};
-        gl::E2 res{gl::add(v.x, gl::mul(cx.c0, dw)), gl::mul(cx.c1, dw)};
-        gl::e2_store(out + 2 * i, gl::e2_canon(res));
+        gl::e2_store(out + 2 * i, fold_pair_base(v, e, r));
     }
 }
 
 static __global__ void fold_ext2_kernel(const uint64_t* __restrict__ cw, const uint64_t* __restrict__ table, gl::E2 r,
                                  uint64_t* __restrict__ out, size_t pairs) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
+    const uint64_t r1w = gl::mul_small(r.c1, 7);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += step) {
         gl::E2 v0 = gl::e2_load(cw + 4 * i), v1 = gl::e2_load(cw + 4 * i + 2);
         ulonglong2 e = *reinterpret_cast<const ulonglong2*>(table + 2 * i);
-        gl::E2 dw = gl::e2_mul_base(gl::e2_sub(v1, v0), e.y);
-        gl::E2 cx{gl::sub(r.c0, e.x), r.c1};
-        gl::e2_store(out + 2 * i, gl::e2_canon(gl::e2_add(v0, gl::e2_mul(cx, dw))));
+        gl::e2_store(out + 2 * i, fold_pair_ext(v0, v1, e, r, r1w));
     }
 }
 

@@ -25,6 +25,24 @@ int run_layers(const uint64_t* in, uint64_t* out, int log_n, int first_bit, int 
         return MB_OK;
     }
     const int tile_log = log_n < TILE_LOG ? log_n : TILE_LOG;
+    if (log_n >= TILE_LOG && first_bit == 0) {
+        // twelve bits in the first pass (contiguous tiles), then eight at most, so that rows are runs of 128 bytes
+        const size_t tiles = (size_t)1 << (log_n - TILE_LOG);
+        const int grid = (int)(tiles < (size_t)sm_count() * 6 ? tiles : (size_t)sm_count() * 6);
+        const size_t smem = sizeof(uint64_t) * ((1 << TILE_LOG) + (1 << (TILE_LOG - 4)));
+        while (left > 0) {
+            const int most = bit == 0 ? TILE_LOG : 8, passes = (left + most - 1) / most;
+            const int nbits = bit == 0 ? (left < most ? left : most) : (left + passes - 1) / passes;
+            if (TILE_LOG - nbits > bit) break;   // a first pass of fewer bits than a tile
+            {
+                MB_KERNEL_ON("bit_layers", st);
+                bit_pass_kernel<Op><<<grid, BLOCK, smem, st>>>(src, out, log_n, bit, nbits);
+            }
+            src = out;
+            bit += nbits;
+            left -= nbits;
+        }
+    }
     while (left > 0) {
         // Row bits first (as many layers per pass as the tile allows), but keep
         // runs of at least 4 consecutive elements (one 32-byte sector) when the
@@ -87,6 +105,18 @@ int encode_async(const uint64_t* d_coeffs, uint64_t* d_work, uint64_t* d_codewor
     int rc = run_layers<CodeOp>(d_coeffs, d_work, nv, 0, nv, st);
     if (rc != MB_OK) return rc;
     return bit_reverse_out_of_place(d_work, d_codeword, nv, 1 << lr, st);
+}
+
+// evaluations -> codeword of 2^(nv+lr) in one set of passes (interpolation and code layers fused bit by bit); d_work: 2^nv
+// words.
+int evals_to_codeword_async(const uint64_t* d_evals, uint64_t* d_work, uint64_t* d_codeword, int nv, int lr, cudaStream_t st) {
+    if (nv < 0 || lr < 0 || nv + lr > 32 || !d_evals || !d_work || !d_codeword) return MB_ERR_ARG;
+    int rc = run_layers<InterpCodeOp>(d_evals, d_work, nv, 0, nv, st);
+    if (rc != MB_OK) return rc;
+    return bit_reverse_out_of_place(d_work, d_codeword, nv, 1 << lr, st);
+}
+int bit_reverse_async(const uint64_t* d_in, uint64_t* d_out, int log_n, cudaStream_t st) {
+    return bit_reverse_out_of_place(d_in, d_out, log_n, 1, st);
 }
 
 }  // namespace bf

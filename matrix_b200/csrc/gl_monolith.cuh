@@ -109,4 +109,42 @@ GLF void monolith_permute(uint64_t* s) {
     }
 }
 
+#ifdef __CUDACC__
+// ---- one permutation spread over 16 lanes ----------------------------------------
+// For layers too small to fill the machine, where the latency of a permutation is what counts: lane i < 12 holds word i.
+// A linear layer is twelve shuffles of each half against the lane's row of the circulant (two chains of twelve
+// multiply-adds instead of 288), the bars run in lanes 0..3, the bricks take the neighbour's word by a shuffle. About 2 us
+// instead of 15 to 20 us for a permutation in one thread. All 32 lanes of the warp must call; lane16 = lane & 15.
+static __device__ const uint64_t g_mono_rc[MONO_ROUNDS + 1][MONO_W] = GLMONO_RC_INIT;   // per-lane reads
+// C[(j - i) mod 12] = g_mono_row[12 - i + j]
+static __device__ const uint32_t g_mono_row[2 * MONO_W] = {7, 23, 8, 26, 13, 10, 9, 7, 6, 22, 21, 8, 7, 23, 8, 26, 13, 10, 9, 7, 6, 22, 21, 8};
+__device__ __forceinline__ uint64_t mono_concrete_coop(uint64_t x, const uint32_t (&m)[MONO_W], uint64_t rc) {
+    uint64_t L = lo32(rc), H = hi32(rc);
+    const uint32_t xl = lo32(x), xh = hi32(x);
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) {
+        L = madwide(__shfl_sync(0xffffffffu, xl, j, 16), m[j], L);
+        H = madwide(__shfl_sync(0xffffffffu, xh, j, 16), m[j], H);
+    }
+    return reduce_limb_sums(L, H);
+}
+__device__ __forceinline__ uint64_t monolith_permute_coop16(uint64_t x, int lane16) {
+    const bool live = lane16 < MONO_W;
+    uint32_t m[MONO_W];   // the lane's row of the circulant
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) m[j] = live ? g_mono_row[MONO_W - lane16 + j] : 0;
+    x = mono_concrete_coop(x, m, 0);
+#pragma unroll 1
+    for (int r = 1; r <= MONO_ROUNDS; r++) {
+        const uint64_t b = mono_bar(canon(x));
+        x = lane16 < 4 ? b : x;
+        const uint64_t prev = pack64(__shfl_up_sync(0xffffffffu, lo32(x), 1, 16), __shfl_up_sync(0xffffffffu, hi32(x), 1, 16));
+        const uint64_t y = mul_add(prev, prev, x);
+        x = lane16 > 0 ? y : x;
+        x = mono_concrete_coop(x, m, (live && r < MONO_ROUNDS) ? g_mono_rc[r][lane16] : 0);
+    }
+    return x;
+}
+#endif
+
 }  // namespace gl

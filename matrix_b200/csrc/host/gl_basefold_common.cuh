@@ -14,11 +14,13 @@
 #include "../merkle_kernels.cuh"
 #include "host_tree_top.hpp"
 #include "gl_transcript.hpp"
+#include "pair_sumcheck.cuh"
+#include "pinned_pool.hpp"
 
 namespace mb {
 namespace bf {
-int interpolate_async(const uint64_t*, uint64_t*, uint64_t*, int, cudaStream_t);
-int encode_async(const uint64_t*, uint64_t*, uint64_t*, int, int, cudaStream_t);
+int evals_to_codeword_async(const uint64_t*, uint64_t*, uint64_t*, int, int, cudaStream_t);
+int bit_reverse_async(const uint64_t*, uint64_t*, int, cudaStream_t);
 }  // namespace bf
 }  // namespace mb
 
@@ -150,6 +152,202 @@ open_round_kernel(const uint64_t* __restrict__ eq_in, const uint64_t* __restrict
     oracle_finish(a0, a1, a2, partial, counter, final_out);
 }
 
+// ---- the opening's inner sumcheck, several rounds per pass --------------------------------------
+// sum_x eq(t, x) bh(x) with eq factored (pair_kernels.cuh has the idea, here with one table): B rounds need the 2^B sums
+//     S(m) = sum_s w(s) f(m, s)
+// over the variables that are not among the next B. The table is the commitment's bit-reversed evaluations, in which the
+// variable bound first is the top index bit: m and the challenges to fold select whole runs of the array, every access
+// is coalesced, and the evaluations need not be put back into natural order. blockIdx.y = m. w(s) = WL[t] WH[h] for
+// s = 256 h + t. Replaces an eq table, a reversed copy and one pass over both tables per round (1.1 ms of an opening at
+// 2^24, and 10 us of every round of a small one).
+struct OpenPassArgs {
+    const uint64_t* in;      // 2^(v + fb) elements
+    uint64_t* out;           // 2^v folded elements, or null
+    int fb, v, rounds;       // challenges to fold; variables left after that; rounds of the next block
+    const uint64_t *wl, *wh; // eq over the s variables: the low 8 (or fewer), and the others
+    uint64_t* partial;       // [2^rounds][2 gridDim.x][2]
+    unsigned* counter;       // [2^rounds][GROUPS + 1]
+    uint64_t* sums;          // pinned: [2^rounds][2]
+};
+template <bool FOLD, bool BASE>
+__global__ void __launch_bounds__(pr::BLK)
+open_pass_kernel(const OpenPassArgs a, const __grid_constant__ pr::FoldWeights<pr::GlF> fw) {
+    using F = pr::GlF;
+    __shared__ gl::E2 sm[pr::BLK];
+    const int t = threadIdx.x, m = blockIdx.y, sb = a.v - a.rounds;
+    const size_t ns = (size_t)1 << sb, n = (size_t)1 << a.v;
+    gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
+    gl::E2 x{0, 0};
+    for (size_t h = blockIdx.x; h * pr::BLK < ns; h += gridDim.x) {
+        const size_t s = h * pr::BLK + t;
+        if (s >= ns) break;
+        const size_t y = (size_t)m * ns + s;
+        gl::E2 f;
+        if constexpr (!FOLD) {
+            f = BASE ? gl::E2{a.in[y], 0} : gl::e2_load(a.in + 2 * y);
+        } else {
+            gl::Acc c0 = gl::acc_zero(), c1 = gl::acc_zero();
+#pragma unroll 4
+            for (int j = 0; j < (1 << a.fb); j++) {
+                const size_t i = ((size_t)j << a.v) + y;
+                if (BASE) {
+                    const uint64_t v = a.in[i];
+                    gl::acc_mul(c0, fw.w[j].c0, v);
+                    gl::acc_mul(c1, fw.w[j].c1, v);
+                } else {
+                    const gl::E2 v = gl::e2_load(a.in + 2 * i);
+                    gl::acc_mul(c0, fw.w[j].c0, v.c0);
+                    gl::acc_mul(c0, fw.w[j].c1w, v.c1);
+                    gl::acc_mul(c1, fw.w[j].c0, v.c1);
+                    gl::acc_mul(c1, fw.w[j].c1, v.c0);
+                }
+            }
+            f = gl::e2_canon(gl::E2{gl::acc_reduce(c0), gl::acc_reduce(c1)});
+            if (a.out != nullptr) gl::e2_store(a.out + 2 * y, f);
+        }
+        if (ns <= pr::BLK) {
+            x = f;
+        } else {
+            const gl::E2Pre w = pr::load_weight<F>(a.wh + 4 * h);
+            gl::acc_mul(s0, w.c0, f.c0);
+            gl::acc_mul(s1, w.c1, f.c0);
+            if constexpr (FOLD || !BASE) {
+                gl::acc_mul(s0, w.c1w, f.c1);
+                gl::acc_mul(s1, w.c0, f.c1);
+            }
+        }
+    }
+    if (ns > pr::BLK) x = gl::E2{gl::acc_reduce_wide(s0), gl::acc_reduce_wide(s1)};
+    if (sb > 0 && (size_t)t < ns) x = F::fma(pr::load_weight<F>(a.wl + 4 * t), x, gl::E2{0, 0});
+    if (!pr::grid_sum<F>(x, 0, sm, a.partial + 4 * (size_t)gridDim.x * m, a.counter + (pr::GROUPS + 1) * m)) return;
+    if (t == 0) pr::store2(a.sums + 2 * m, sm[0].c0, sm[0].c1);
+}
+
+class OpenSumcheck {
+public:
+    using H = PairHost<pr::GlF, PairGl>;
+    using E2 = gl::E2;
+    // bh: 2^nv bit-reversed evaluations on the device; point: nv (c0, c1) pairs; pinned: 32 words for the passes' sums
+    // and 2 nv for the point's upload. Queues the first pass.
+    int init(const uint64_t* bh, int nv, const uint64_t* point, uint64_t* sums, uint64_t* upload) {
+        nv_ = nv; in_ = bh; sums_ = sums;
+        pt_.resize(nv);
+        r_.resize(nv);
+        for (int i = 0; i < nv; i++) pt_[i] = H::canon(E2{point[2 * i], point[2 * i + 1]});
+        const int parts = (nv + pr::MAX_B - 1) / pr::MAX_B;
+        pr::TableSet set;
+        int nt = 0;
+        size_t words = 0;
+        for (int i = 0, at = 0; i < parts; i++) {
+            Stage s;
+            s.first = at;
+            s.rounds = (nv - at + (parts - i) - 1) / (parts - i);
+            const int sb = nv - at - s.rounds, lo = sb < 8 ? sb : 8;   // index bit j of s goes with variable nv - 1 - j
+            s.wl = words; set.d[nt].first = 0; set.d[nt].bits = lo; set.d[nt++].off = words; words += (size_t)4 << lo;
+            s.wh = words; set.d[nt].first = lo; set.d[nt].bits = sb - lo; set.d[nt++].off = words; words += (size_t)4 << (sb - lo);
+            stages_.push_back(s);
+            at += s.rounds;
+        }
+        int rc = tabs_.alloc(words + 2 * (size_t)nv);
+        if (rc == MB_OK) rc = partial_.alloc(4 * (size_t)GX * 16);
+        if (rc == MB_OK) rc = counter_.alloc((16 * (pr::GROUPS + 1) + 1) / 2);
+        if (rc != MB_OK) return rc;
+        for (int i = 0; i < nv; i++) { upload[2 * i] = pt_[nv - 1 - i].c0; upload[2 * i + 1] = pt_[nv - 1 - i].c1; }
+        MB_CUDA(cudaMemcpyAsync(tabs_.p + words, upload, 16 * (size_t)nv, cudaMemcpyHostToDevice, MB_STREAM));
+        MB_CUDA(cudaMemsetAsync(counter_.p, 0, 8 * counter_.words, MB_STREAM));
+        {
+            MB_KERNEL_ON("open_eq_tables", MB_STREAM);
+            pr::eq_tables_kernel<pr::GlF><<<nt, pr::BLK, 0, MB_STREAM>>>(set, tabs_.p + words, tabs_.p);
+        }
+        return pass();
+    }
+    // The oracle of the current round, c0 c1 c2 (six words); the stream must have been synchronised since the last call that
+    // queued a pass (init or fold).
+    void oracle(uint64_t* out6) {
+        const Stage& st = stages_[stage_];
+        if (g_.empty()) {
+            const int B = st.rounds;
+            g_.resize((size_t)1 << B);
+            for (int m = 0; m < (1 << B); m++) {   // the top bit of m is the variable bound first
+                int i = 0;
+                for (int k = 0; k < B; k++) i |= ((m >> (B - 1 - k)) & 1) << k;
+                g_[i] = E2{sums_[2 * m], sums_[2 * m + 1]};
+            }
+        }
+        // eq of the block's later variables
+        const int later = st.first + st.rounds - round_ - 1;
+        E2 w[1 << pr::MAX_B];
+        H::eq_vector(pt_.data() + round_ + 1, later, w);
+        typename H::Dot da, db;
+        for (int y = 0; y < (1 << later); y++) { da.mac(w[y], g_[2 * y]); db.mac(w[y], g_[2 * y + 1]); }
+        const E2 a = da.value(), d = H::sub(db.value(), a), t = pt_[round_], one{1, 0};
+        const E2 e0 = H::mul(scale_, H::sub(one, t)), e1 = H::mul(scale_, H::sub(H::add(t, t), one));
+        const E2 c0 = H::mul(e0, a), c1 = H::add(H::mul(e0, d), H::mul(e1, a)), c2 = H::mul(e1, d);
+        out6[0] = c0.c0; out6[1] = c0.c1; out6[2] = c1.c0; out6[3] = c1.c1; out6[4] = c2.c0; out6[5] = c2.c1;
+    }
+    int fold(E2 r) {
+        const E2 t = pt_[round_], tr = H::mul(t, r);
+        scale_ = H::mul(scale_, H::add(H::sub(H::sub(E2{1, 0}, t), r), H::add(tr, tr)));
+        r_[round_++] = r;
+        const Stage& st = stages_[stage_];
+        if (round_ == st.first + st.rounds) {
+            stage_++;
+            g_.clear();
+            return stage_ < stages_.size() ? pass() : MB_OK;
+        }
+        for (size_t y = 0; y < g_.size() / 2; y++) g_[y] = H::fold(g_[2 * y], g_[2 * y + 1], r);
+        g_.resize(g_.size() / 2);
+        return MB_OK;
+    }
+
+private:
+    struct Stage {
+        int first, rounds;
+        size_t wl, wh;
+    };
+    static constexpr int GX = 148;   // blocks per sum at most: eight per SM with sixteen sums
+    int pass() {
+        const Stage& st = stages_[stage_];
+        const int fb = stage_ ? stages_[stage_ - 1].rounds : 0;
+        OpenPassArgs a;
+        a.fb = fb; a.v = nv_ - st.first; a.rounds = st.rounds;
+        a.wl = tabs_.p + st.wl; a.wh = tabs_.p + st.wh;
+        a.partial = partial_.p; a.counter = reinterpret_cast<unsigned*>(counter_.p); a.sums = sums_;
+        a.in = in_; a.out = nullptr;
+        if (fb && stage_ + 1 < stages_.size()) {
+            DevBuf& t = tables_[stage_ & 1];
+            int rc = t.alloc((size_t)2 << a.v);
+            if (rc != MB_OK) return rc;
+            a.out = t.p;
+        }
+        pr::FoldWeights<pr::GlF> fw;
+        if (fb) {   // index bit fb - 1 - k goes with challenge k
+            E2 rev[pr::MAX_B], e[1 << pr::MAX_B];
+            for (int k = 0; k < fb; k++) rev[k] = r_[st.first - 1 - k];
+            H::eq_vector(rev, fb, e);
+            for (int j = 0; j < (1 << fb); j++) fw.w[j] = gl::e2_pre(e[j]);
+        }
+        const size_t rows = (((size_t)1 << (a.v - a.rounds)) + pr::BLK - 1) / pr::BLK;
+        const dim3 grid(rows < GX ? (unsigned)rows : GX, 1u << a.rounds);
+        {
+            MB_KERNEL_ON("open_pass", MB_STREAM);
+            if (!fb) open_pass_kernel<false, true><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
+            else if (stage_ == 1) open_pass_kernel<true, true><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
+            else open_pass_kernel<true, false><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
+        }
+        if (a.out) in_ = a.out;
+        return finish_async();
+    }
+    int nv_ = 0, round_ = 0;
+    size_t stage_ = 0;
+    const uint64_t* in_ = nullptr;
+    uint64_t* sums_ = nullptr;
+    E2 scale_{1, 0};
+    std::vector<Stage> stages_;
+    std::vector<E2> pt_, r_, g_;
+    DevBuf tabs_, partial_, counter_, tables_[2];
+};
+
 // Query phase: every value pair and authentication path of every query in
 // one launch. Block q handles query q; out is the per-query part of the proof.
 struct QueryLevels {
@@ -265,14 +463,14 @@ public:
         num_vars = nv; log_rate = lr;
         hash = g_merkle_hash.load();
         size_t n = (size_t)1 << nv, cw_len = (size_t)1 << (nv + lr);
-        DevBuf coeffs;
-        int rc = coeffs.alloc(n);
+        DevBuf work;
+        int rc = work.alloc(n);
         if (rc == MB_OK) rc = d_bh_evals.alloc(n);
         if (rc == MB_OK) rc = d_codeword.alloc(cw_len);
         if (rc == MB_OK) rc = d_tree.alloc(4 * (cw_len - 1));
         if (rc != MB_OK) return rc;
-        rc = bf::interpolate_async(d_evals, coeffs.p, d_bh_evals.p, nv, MB_STREAM);
-        if (rc == MB_OK) rc = bf::encode_async(coeffs.p, coeffs.p, d_codeword.p, nv, lr, MB_STREAM);
+        rc = bf::bit_reverse_async(d_evals, d_bh_evals.p, nv, MB_STREAM);
+        if (rc == MB_OK) rc = bf::evals_to_codeword_async(d_evals, work.p, d_codeword.p, nv, lr, MB_STREAM);
         if (rc == MB_OK)
             rc = hash ? mk::build_tree_periodic<mk::HashMonolith>(d_codeword.p, d_tree.p, cw_len / 2, (size_t)1 << lr, MB_STREAM)
                       : mk::build_tree_periodic<mk::HashPoseidon2>(d_codeword.p, d_tree.p, cw_len / 2, (size_t)1 << lr, MB_STREAM);
@@ -287,6 +485,30 @@ public:
 };
 
 // ---- host hashing of tree tops: host_tree_top.hpp -------------------------------------------
+// A pinned block for the length of a scope (nothing may still be writing it when the scope ends).
+struct PinnedBlock {
+    uint64_t* p = PinnedPool::take();
+    PinnedBlock() = default;
+    PinnedBlock(const PinnedBlock&) = delete;
+    PinnedBlock& operator=(const PinnedBlock&) = delete;
+    ~PinnedBlock() {
+        if (!p) return;
+        cudaStreamSynchronize(MB_STREAM);
+        PinnedPool::give(p);
+    }
+};
+
+// One round's codeword fold and the tree over the folded codeword, queued; the layer of min(leaves, host_top) digests
+// goes to `nodes` (pinned). f: source, table level, target and challenge of the fold; mixed: the source is base field.
+inline int queue_fold_tree(int hash, bool mixed, const mk::FoldSource& f, uint64_t* d_tree, size_t leaves, uint64_t* nodes) {
+    const size_t stop = host_top(hash);
+    if (hash)
+        return mixed ? mk::fold_tree<mk::HashMonolith, true>(f, d_tree, leaves, MB_STREAM, nodes, stop)
+                     : mk::fold_tree<mk::HashMonolith, false>(f, d_tree, leaves, MB_STREAM, nodes, stop);
+    return mixed ? mk::fold_tree<mk::HashPoseidon2, true>(f, d_tree, leaves, MB_STREAM, nodes, stop)
+                 : mk::fold_tree<mk::HashPoseidon2, false>(f, d_tree, leaves, MB_STREAM, nodes, stop);
+}
+
 // nodes: the layer of `count` digests (a power of two, at most HOST_TOP) the device left; upper: pinned staging for
 // count - 1 digests that stays untouched until the stream has run the upload; d_tree: the tree of num_leaves
 // leaves (2 num_leaves - 1 digests, layers back to back). root receives the root.

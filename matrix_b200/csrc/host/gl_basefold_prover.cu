@@ -11,11 +11,10 @@
 // The protocol order, every transcript interaction and every value that enters
 // the proof are the reference's. The work between them is organised for the
 // B200: the claimed value is read off the first oracle (eval = p(0) + p(1), one
-// pass fewer), the inner sumcheck keeps its tables as plain values and folds
-// them in the same pass that accumulates the next oracle, partial sums are
-// finished on the device, each round issues its sumcheck pass, codeword fold and
-// Merkle tree back to back and synchronises once, and the query phase is one
-// gather kernel and one copy.
+// pass fewer), the inner sumcheck runs several rounds per pass over the
+// bit-reversed evaluations (OpenSumcheck), the codeword is folded by the kernels
+// that hash its leaves, each round issues them back to back and synchronises
+// once, and the query phase is one gather kernel and one copy.
 #include "gl_basefold_common.cuh"
 
 namespace mbhost {
@@ -39,53 +38,18 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     t.observe_hash(cm.root);
     for (int i = 0; i < nv; i++) t.observe_ext2(Ext2{point[2 * i], point[2 * i + 1]});
 
-    // device state
-    DevBuf eq_a, eq_b, bh_fp, bh_a, bh_b, d_point, partial, small, stage;
-    const int grid_max = grid_for(n / 2, 256, 4);
-    int rc = eq_a.alloc(2 * n);
-    if (rc == MB_OK) rc = eq_b.alloc(n);
-    if (rc == MB_OK) rc = bh_fp.alloc(n);
-    if (rc == MB_OK) rc = bh_a.alloc(n);
-    if (rc == MB_OK) rc = bh_b.alloc(n / 2 > 2 ? n / 2 : 2);
-    if (rc == MB_OK) rc = d_point.alloc(2 * (size_t)nv);
-    if (rc == MB_OK) rc = partial.alloc(6 * (size_t)grid_max);
-    if (rc == MB_OK) rc = small.alloc(16);  // [0..6) oracle words, [8] ticket counter
+    PinnedBlock pin;   // sums of the inner sumcheck (32 words), a tree's last device layer (from word 64)
+    uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv + 2 * (size_t)nv);   // host-hashed tree tops on their way up
+    if (!pin.p || !top_staging) return MB_ERR_CUDA;
+    uint64_t* nodes = pin.p + 64;
+    OpenSumcheck sc;
+    int rc = sc.init(cm.d_bh_evals.p, nv, point, pin.p, top_staging + 4 * (HOST_TOP - 1) * (size_t)nv);
     if (rc != MB_OK) return rc;
-    unsigned int* counter = reinterpret_cast<unsigned int*>(small.p + 8);
-    MB_CUDA(cudaMemsetAsync(small.p, 0, 16 * sizeof(uint64_t), MB_STREAM));
-    uint64_t* h_small = pinned_scratch();  // landing zone: 6 oracle words, then (from word 8) the tree's last device layer
-    uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv);   // host-hashed tree tops on their way up
-    if (!h_small || !top_staging) return MB_ERR_CUDA;
-
-    MB_CUDA(cudaMemcpyAsync(d_point.p, point, sizeof(uint64_t) * 2 * nv, cudaMemcpyHostToDevice, MB_STREAM));
-    // eq table; bh_a doubles as scratch for the two small tables (free until round 0 writes it)
-    rc = eq::build<sc::GlExt2>(d_point.p, eq_a.p, bh_a.p, nv, MB_STREAM);
-    if (rc != MB_OK) return rc;
-    // evaluations back in natural order (basefold.rs:600-602)
-    if (nv >= 12) {
-        size_t tiles = (size_t)1 << (nv - 12);
-        int g = (int)(tiles < (size_t)sm_count() * 4 ? tiles : (size_t)sm_count() * 4);
-        {
-            MB_KERNEL_ON("bit_reverse_tiled", MB_STREAM);
-            bf::bit_reverse_tiled_kernel<<<g, 256, 0, MB_STREAM>>>(cm.d_bh_evals.p, bh_fp.p, nv, 1);
-        }
-    } else {
-        {
-            MB_KERNEL_ON("bit_reverse_copy", MB_STREAM);
-            bf::bit_reverse_copy_kernel<<<grid_for(n, 256, 8), 256, 0, MB_STREAM>>>(cm.d_bh_evals.p, bh_fp.p, nv, 1);
-        }
-    }
-
-    // oracle 0 and the claimed value eval = p(0) + p(1) = 2 c0 + c1 + c2
-    {
-        MB_KERNEL_ON("oracle0", MB_STREAM);
-        oracle0_kernel<<<grid_for(n / 2, 256, 4), 256, 0, MB_STREAM>>>(eq_a.p, bh_fp.p, n / 2, partial.p, counter, small.p);
-    }
-    MB_CUDA(cudaMemcpyAsync(h_small, small.p, 48, cudaMemcpyDeviceToHost, MB_STREAM));
     MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-    std::memcpy(p_oracles, h_small, 48);
+    // oracle 0 and the claimed value eval = p(0) + p(1) = 2 c0 + c1 + c2
+    sc.oracle(p_oracles);
     {
-        gl::E2 c0{h_small[0], h_small[1]}, c1{h_small[2], h_small[3]}, c2{h_small[4], h_small[5]};
+        gl::E2 c0{p_oracles[0], p_oracles[1]}, c1{p_oracles[2], p_oracles[3]}, c2{p_oracles[4], p_oracles[5]};
         gl::E2 ev = gl::e2_canon(gl::e2_add(gl::e2_add(c0, c0), gl::e2_add(c1, c2)));
         p_eval[0] = ev.c0;
         p_eval[1] = ev.c1;
@@ -109,66 +73,28 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
         }
     }
 
-    const uint64_t *eq_cur = eq_a.p, *bh_cur = bh_fp.p;
-    uint64_t *eq_nxt = eq_b.p, *bh_nxt = bh_a.p;
-    size_t live = n;            // current length of the sumcheck tables
     size_t cw_pairs = cw_len / 2;
     for (int round = 0; round < nv - 1; round++) {
         Ext2 ch = t.sample_challenge_ext2();
         gl::E2 r{ch.c0, ch.c1};
-        size_t quarter = live / 4;
-        int g = grid_for(quarter, 256, 4);
-        // the last block of the round kernel writes the finished oracle straight into pinned host memory, the last
-        // block of the tree its root: a round is its launches and one stream synchronisation, no copy command
-        if (round == 0) {
-            {
-                MB_KERNEL_ON("open_round", MB_STREAM);
-                open_round_kernel<true><<<g, 256, 0, MB_STREAM>>>(eq_cur, bh_cur, r, eq_nxt, bh_nxt, quarter, partial.p,
-                                                                  counter, h_small);
-            }
-        } else {
-            {
-                MB_KERNEL_ON("open_round", MB_STREAM);
-                open_round_kernel<false><<<g, 256, 0, MB_STREAM>>>(eq_cur, bh_cur, r, eq_nxt, bh_nxt, quarter, partial.p,
-                                                                   counter, h_small);
-            }
-        }
-        if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
-        // codeword fold with this round's table level, then its tree
-        const uint64_t* level = table.device_level_ptr(round);
-        int gf = grid_for(cw_pairs, 256, 8);
-        if (round == 0) {
-            {
-                MB_KERNEL_ON("fold_mixed", MB_STREAM);
-                bf::fold_mixed_kernel<<<gf, 256, 0, MB_STREAM>>>(cm.d_codeword.p, level, r, fcw[0]->p, cw_pairs);
-            }
-        } else {
-            {
-                MB_KERNEL_ON("fold_ext2", MB_STREAM);
-                bf::fold_ext2_kernel<<<gf, 256, 0, MB_STREAM>>>(fcw[round - 1]->p, level, r, fcw[round]->p, cw_pairs);
-            }
-        }
-        if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
-        // the device stops at the layer of HOST_TOP digests; the host hashes the levels above it
+        // kernels write their results straight into pinned host memory: a round is its launches and one stream
+        // synchronisation, no copy command
+        rc = sc.fold(r);
+        if (rc != MB_OK) return rc;
+        // codeword fold with this round's table level, and its tree up to the layer the host takes over
         const size_t leaves = cw_pairs / 2;
-        rc = cm.hash ? mk::build_tree<mk::HashMonolith, true>(fcw[round]->p, ftree[round]->p, leaves, MB_STREAM, h_small + 8, HOST_TOP)
-                     : mk::build_tree<mk::HashPoseidon2, true>(fcw[round]->p, ftree[round]->p, leaves, MB_STREAM, h_small + 8, HOST_TOP);
+        const mk::FoldSource f{round == 0 ? cm.d_codeword.p : fcw[round - 1]->p, table.device_level_ptr(round), fcw[round]->p, r};
+        rc = queue_fold_tree(cm.hash, round == 0, f, ftree[round]->p, leaves, nodes);
         if (rc != MB_OK) return rc;
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
         uint64_t* po = p_oracles + 6 * (size_t)(round + 1);
-        std::memcpy(po, h_small, 48);
-        rc = host_finish_top(cm.hash, h_small + 8, leaves < HOST_TOP ? leaves : HOST_TOP, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
+        sc.oracle(po);
+        const size_t top = host_top(cm.hash);
+        rc = host_finish_top(cm.hash, nodes, leaves < top ? leaves : top, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
                              ftree[round]->p, leaves, p_roots + 4 * (size_t)round, MB_STREAM);
         if (rc != MB_OK) return rc;
         for (int k = 0; k < 3; k++) t.observe_ext2(Ext2{po[2 * k], po[2 * k + 1]});
         t.observe_hash(p_roots + 4 * (size_t)round);
-
-        // ping-pong: eq between eq_b and eq_a, bh between bh_a and bh_b
-        eq_cur = eq_nxt;
-        bh_cur = bh_nxt;
-        eq_nxt = (eq_nxt == eq_b.p) ? eq_a.p : eq_b.p;
-        bh_nxt = (bh_nxt == bh_a.p) ? bh_b.p : bh_a.p;
-        live /= 2;
         cw_pairs /= 2;
     }
 

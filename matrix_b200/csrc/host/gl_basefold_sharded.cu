@@ -222,7 +222,8 @@ int prove_sharded(const uint64_t* d_evals, int nv, int lr, const uint64_t* point
     uint64_t* p_queries = p_final + ((size_t)2 << lr);
 
     std::vector<uint64_t> h_mine, h_all;
-    uint64_t* h_small = pinned_scratch();   // words 0..5 oracle, 6..9 subtree root, 16..47 the subtree's last device layer
+    PinnedBlock pin;
+    uint64_t* h_small = pin.p;   // words 0..5 oracle, 6..9 subtree root, from 16 the subtree's last device layer
     uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv);
     if (!h_small || !top_staging) return MB_ERR_CUDA;
 
@@ -242,9 +243,8 @@ int prove_sharded(const uint64_t* d_evals, int nv, int lr, const uint64_t* point
     rc = ex->all_to_all_device(ex->ctx, send.p, slice.p, piece);
     if (rc != MB_OK) return rc;
     pc.lap(0);
-    // the remaining nv - m bits: coefficients in `send`, butterflies in place, reversal into `slice`
-    rc = bf::interpolate_async(slice.p, send.p, nullptr, nv - m, MB_STREAM);
-    if (rc == MB_OK) rc = bf::encode_async(send.p, send.p, slice.p, nv - m, 0, MB_STREAM);
+    // the remaining nv - m bits into `send`, reversal back into `slice`
+    rc = bf::evals_to_codeword_async(slice.p, send.p, slice.p, nv - m, 0, MB_STREAM);
     if (rc != MB_OK) return rc;
     // this rank's part of the commitment tree: 1 / 2^lr of the slice's leaves
     {
@@ -418,22 +418,13 @@ int prove_sharded(const uint64_t* d_evals, int nv, int lr, const uint64_t* point
         // (the kernel's last block and the tree's last block write into the pinned landing zone themselves)
         // codeword fold on this rank's pairs with its entries of the round's table level, then the tree
         const uint64_t* level = table.device_level_ptr(round) + (distributed ? 2 * (size_t)g * cw_pairs : 0);
-        const int gf = grid_for(cw_pairs, 256, 8);
-        if (round == 0) {
-            MB_KERNEL_ON("fold_mixed", MB_STREAM);
-            bf::fold_mixed_kernel<<<gf, 256, 0, MB_STREAM>>>(slice.p, level, r, fcw[0]->p, cw_pairs);
-        } else {
-            MB_KERNEL_ON("fold_ext2", MB_STREAM);
-            bf::fold_ext2_kernel<<<gf, 256, 0, MB_STREAM>>>(cw_prev, level, r, fcw[round]->p, cw_pairs);
-        }
-        if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
-        // the device stops at the layer of HOST_TOP digests of this rank's (sub)tree; the host hashes the levels above
-        const size_t leaves = cw_pairs / 2;
-        rc = hash ? mk::build_tree<mk::HashMonolith, true>(fcw[round]->p, ftree[round]->p, leaves, MB_STREAM, h_small + 16, HOST_TOP)
-                  : mk::build_tree<mk::HashPoseidon2, true>(fcw[round]->p, ftree[round]->p, leaves, MB_STREAM, h_small + 16, HOST_TOP);
+        // the device stops at the layer of host_top digests of this rank's (sub)tree; the host hashes the levels above
+        const size_t leaves = cw_pairs / 2, top = host_top(hash);
+        const mk::FoldSource f{round == 0 ? slice.p : cw_prev, level, fcw[round]->p, r};
+        rc = queue_fold_tree(hash, round == 0, f, ftree[round]->p, leaves, h_small + 16);
         if (rc != MB_OK) return rc;
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        rc = host_finish_top(hash, h_small + 16, leaves < HOST_TOP ? leaves : HOST_TOP, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
+        rc = host_finish_top(hash, h_small + 16, leaves < top ? leaves : top, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
                              ftree[round]->p, leaves, h_small + 6, MB_STREAM);
         if (rc != MB_OK) return rc;
         uint64_t* po = p_oracles + 6 * (size_t)(round + 1);

@@ -1,10 +1,10 @@
 // Host hashing of the top of a Merkle tree (Poseidon2 or Monolith over Goldilocks, as the device trees).
 //
-// The last levels of a tree are bound by the latency of one permutation per level on the device (about 10 us with
-// the 8-lane Poseidon2, a whole single-thread permutation with Monolith); a host core runs a permutation in about
-// 1 us. So a round's tree stops on the device at a layer of HOST_TOP digests (mk::build_tree's `stop`), which the
-// kernel leaves in pinned memory, and the host hashes the three levels above: seven permutations, then one small
-// upload puts them into the device tree for the query phase (host_finish_top, gl_basefold_common.cuh).
+// The last levels of a tree are bound by the latency of one permutation per level on the device (about 8 us with the
+// 8-lane Poseidon2, 2 us with the 16-lane Monolith); a host core runs a permutation in 0.6 or 0.2 us. So a round's
+// tree stops on the device at a layer of host_top(hash) digests (mk::build_tree's `stop`), which the kernel leaves in pinned
+// memory, and the host hashes the levels above: 15 or 31 permutations, then one small upload puts them into the device tree
+// for the query phase (host_finish_top, gl_basefold_common.cuh).
 #pragma once
 #include <cstdint>
 #include <cstring>
@@ -27,7 +27,9 @@ inline Digest host_compress(int hash, const uint64_t* l, const uint64_t* r) {
 }
 inline Digest host_compress(int hash, const Digest& l, const Digest& r) { return host_compress(hash, l.w, r.w); }
 
-constexpr size_t HOST_TOP = 8;
+// where a level costs the device as long as its nodes cost the host
+constexpr size_t host_top(int hash) { return hash ? 32 : 16; }
+constexpr size_t HOST_TOP = 32;   // the largest of them
 
 // nodes: a layer of `count` digests (a power of two). upper receives the count - 1 digests of the layers above it,
 // layer by layer as the tree stores them (count / 2, count / 4, ..., 1); root receives the last one.
