@@ -98,30 +98,28 @@ constexpr int TC_PASS_PLANES = TC_MAX_PLANES;   // one MMA covers all planes of 
 
 template <int SRC, int NP>
 int launch_tc_np(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T, const int8_t* d_digits, uint64_t N, int p0,
-                 uint64_t col_offset, uint64_t* partial, int* d_err, uint8_t* materialize, size_t chunks, int chunk_cols) {
+                 uint64_t col_offset, uint64_t* partial, int* err, uint8_t* materialize, size_t chunks, int chunk_cols) {
     dim3 grid((unsigned)chunks, 3);
     if (materialize) {   // the matrix as byte planes in operand order: the builder of the single-phase kernel, no MMAs
         const size_t smem = tc_pipe_smem_bytes(NP);
         if (cudaFuncSetAttribute(commit_tc_pipe_kernel<SRC, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return MB_ERR_CUDA;
-        commit_tc_pipe_kernel<SRC, NP><<<grid, TCP_THREADS, smem, MB_STREAM>>>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err,
+        commit_tc_pipe_kernel<SRC, NP><<<grid, TCP_THREADS, smem, MB_STREAM>>>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err,
                                                                                  materialize, chunk_cols);
         return MB_OK;
     }
     const size_t smem = tc_ws_smem_bytes(SRC, NP);
     if (cudaFuncSetAttribute(commit_tc_ws_kernel<SRC, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return MB_ERR_CUDA;
-    commit_tc_ws_kernel<SRC, NP><<<grid, ws_threads(SRC), smem, MB_STREAM>>>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err, chunk_cols);
+    commit_tc_ws_kernel<SRC, NP><<<grid, ws_threads(SRC), smem, MB_STREAM>>>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err, chunk_cols);
     return MB_OK;
 }
 // Columns per CTA (a multiple of the four columns of an MMA stage, at most 512): one CTA runs per SM at a time
 // and a grid has three CTAs per chunk, so the chunk width is chosen to make the grid a whole number of waves:
-// as few waves as 512-column chunks allow (two at least, so that a short witness still spreads over every SM),
-// then the widest chunks that fill them. 2^18 columns: 542 chunks of 484 columns = 1626 CTAs = 10.99 waves of
-// 148 instead of 512 chunks = 10.4 waves, of which the last is two fifths full.
+// as few waves as 512-column chunks allow, then the widest chunks that fill them. 2^18 columns: 542 chunks of 484
+// columns = 1626 CTAs = 10.99 waves of 148 instead of 512 chunks = 10.4 waves, of which the last is two fifths full.
 inline int tc_chunk_cols(uint64_t N) {
     const uint64_t sms = (uint64_t)sm_count();
     const uint64_t min_chunks = (N + TC_CHUNK_COLS - 1) / TC_CHUNK_COLS;
     uint64_t waves = (3 * min_chunks + sms - 1) / sms;
-    if (waves < 2) waves = 2;
     uint64_t want_chunks = waves * sms / 3;
     if (want_chunks < 1) want_chunks = 1;
     uint64_t cols = (N + want_chunks - 1) / want_chunks;
@@ -132,12 +130,12 @@ inline int tc_chunk_cols(uint64_t N) {
 }
 template <int SRC>
 int launch_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T, const int8_t* d_digits, uint64_t N, int p0, int np,
-              uint64_t col_offset, uint64_t* partial, int* d_err, uint8_t* materialize, size_t chunks, int chunk_cols) {
+              uint64_t col_offset, uint64_t* partial, int* err, uint8_t* materialize, size_t chunks, int chunk_cols) {
     switch (np) {
-        case 1: return launch_tc_np<SRC, 1>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err, materialize, chunks, chunk_cols);
-        case 2: return launch_tc_np<SRC, 2>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err, materialize, chunks, chunk_cols);
-        case 3: return launch_tc_np<SRC, 3>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err, materialize, chunks, chunk_cols);
-        default: return launch_tc_np<SRC, 4>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, d_err, materialize, chunks, chunk_cols);
+        case 1: return launch_tc_np<SRC, 1>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err, materialize, chunks, chunk_cols);
+        case 2: return launch_tc_np<SRC, 2>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err, materialize, chunks, chunk_cols);
+        case 3: return launch_tc_np<SRC, 3>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err, materialize, chunks, chunk_cols);
+        default: return launch_tc_np<SRC, 4>(d_key, d_M, d_T, d_digits, N, p0, col_offset, partial, err, materialize, chunks, chunk_cols);
     }
 }
 
@@ -153,38 +151,35 @@ int commit_s8_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T,
     }
     const int chunk_cols = tc_chunk_cols(N);
     const size_t chunks = (N + chunk_cols - 1) / chunk_cols;
+    uint64_t* scratch = pinned_scratch();
+    if (!scratch) return MB_ERR_CUDA;
+    int* err = reinterpret_cast<int*>(scratch);   // written by the kernel only where something is wrong
+    err[0] = err[1] = 0;
     uint64_t* partial = nullptr;
-    int* d_err = nullptr;
     MB_CUDA(pool_alloc((void**)&partial, chunks * 3 * TC_MAX_PLANES * TC_ROWS * D * sizeof(uint64_t)));
-    if (pool_alloc((void**)&d_err, sizeof(int)) != cudaSuccess) { pool_free(partial); return MB_ERR_CUDA; }
     int rc = MB_OK;
-    if (cudaMemsetAsync(d_err, 0, sizeof(int), MB_STREAM) != cudaSuccess) rc = MB_ERR_CUDA;
     for (int p0 = 0; p0 < planes && rc == MB_OK; p0 += TC_PASS_PLANES) {
         const int np = planes - p0 < TC_PASS_PLANES ? planes - p0 : TC_PASS_PLANES;
         {
             MB_KERNEL(d_T ? "ajtai_commit_tc_tiled" : d_M ? "ajtai_commit_tc_premat" : "ajtai_commit_tc");
-            if (d_T) rc = launch_tc<TC_SRC_TILED>(nullptr, nullptr, d_T, d_digits, N, p0, np, 0, partial, d_err, nullptr, chunks, chunk_cols);
-            else if (d_M) rc = launch_tc<TC_SRC_COEFFS>(nullptr, d_M, nullptr, d_digits, N, p0, np, 0, partial, d_err, nullptr, chunks, chunk_cols);
-            else rc = launch_tc<TC_SRC_CHACHA>(d_key, nullptr, nullptr, d_digits, N, p0, np, col_offset, partial, d_err, nullptr, chunks, chunk_cols);
+            if (d_T) rc = launch_tc<TC_SRC_TILED>(nullptr, nullptr, d_T, d_digits, N, p0, np, 0, partial, err, nullptr, chunks, chunk_cols);
+            else if (d_M) rc = launch_tc<TC_SRC_COEFFS>(nullptr, d_M, nullptr, d_digits, N, p0, np, 0, partial, err, nullptr, chunks, chunk_cols);
+            else rc = launch_tc<TC_SRC_CHACHA>(d_key, nullptr, nullptr, d_digits, N, p0, np, col_offset, partial, err, nullptr, chunks, chunk_cols);
         }
         if (rc != MB_OK) break;
         {
             MB_KERNEL("ajtai_reduce_tc");
-            reduce_tc_partials_kernel<<<grid_for((size_t)np * plane_words, 256, 4), 256, 0, MB_STREAM>>>(
+            reduce_tc_partials_kernel<<<(unsigned)(np * plane_words / 32), 32 * TC_RED_SLICES, 0, MB_STREAM>>>(
                 partial, chunks, np, d_out + (size_t)p0 * plane_words);
         }
         rc = finish_async();
     }
-    int h_err = 0;
-    if (rc == MB_OK && cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, MB_STREAM) != cudaSuccess)
-        rc = MB_ERR_CUDA;
-    if (rc == MB_OK) rc = finish_sync();
+    const int synced = finish_sync();   // also after a failed launch: nothing may still write to err or partial
+    if (rc == MB_OK) rc = synced;
     pool_free(partial);
-    pool_free(d_err);
     if (rc != MB_OK) return rc;
-    if (h_err == TC_ERR_TIMEOUT) return MB_ERR_CUDA;
-    if (h_err == TC_ERR_DIGIT_RANGE) return MB_ERR_UNSUPPORTED;
-    return MB_OK;
+    if (err[1]) return MB_ERR_CUDA;
+    return err[0] ? MB_ERR_UNSUPPORTED : MB_OK;
 }
 }  // namespace
 

@@ -126,19 +126,19 @@ __device__ __forceinline__ void prg_ring_block(const uint32_t (&key)[8], uint32_
 
 // prg_ring_block for a thread that keeps `pre` = chacha8_columns(key, block_idx, row, high word of j) across
 // columns. A coefficient is rejected only when its high word is 0xFFFFFFFE or 0xFFFFFFFF (q = 2^64 - 2^32 - 31),
-// so one comparison per coefficient decides whether the exact path has to look.
+// so the largest high word decides whether the exact path has to look.
 __device__ __forceinline__ void prg_ring_block_pre(const uint32_t (&key)[8], ChaChaColumns& pre, uint32_t row, uint64_t j,
                                                    uint32_t block_idx, uint64_t (&out)[8]) {
     if ((uint32_t)(j >> 32) != pre.n2) chacha8_columns(key, block_idx, row, (uint32_t)(j >> 32), pre);
     uint32_t buf[16];
     chacha8_block_pre(key, pre, block_idx, row, (uint32_t)j, buf);
-    bool ok = true;
+    uint32_t top = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         out[k] = ((uint64_t)buf[2 * k + 1] << 32) | buf[2 * k];
-        ok = ok && (buf[2 * k + 1] < 0xFFFFFFFEu);
+        top = max(top, buf[2 * k + 1]);   // three-operand maxima: half the instructions of eight comparisons
     }
-    if (ok) return;
+    if (top < 0xFFFFFFFEu) return;
     prg_ring_block(key, row, j, block_idx, out);
 }
 

@@ -44,7 +44,7 @@ constexpr int TC_ROWS = 14;             // matrix rows per CTA (3 groups cover 4
 constexpr int TC_STAGE_COLS = 4;        // columns per MMA stage
 constexpr int TC_STAGE_K = TC_STAGE_COLS * D;   // 256 bytes of K per stage
 constexpr int TC_CHUNK_COLS = 512;      // most columns per accumulation (s32 exactness)
-constexpr int TC_CHUNK_MIN = 32;        // fewest columns per CTA: below that the set-up and the epilogue dominate
+constexpr int TC_CHUNK_MIN = 8;          // fewest columns per CTA: two stages
 constexpr int TC_MAX_PLANES = 4;        // digit planes per CTA: N = 64 * planes <= 256
 constexpr uint32_t TC_CORE = 128;       // bytes of one 8 x 16 core matrix
 constexpr uint32_t TC_SBO = (TC_STAGE_K / 16) * TC_CORE;  // 2048: next 8-row group
@@ -310,18 +310,18 @@ commit_tc_pipe_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __rest
 }
 
 // ---- the commit kernel: builder warps and an issuing warp ------------------------------------------------
-// Fifteen warps build operands, the sixteenth issues MMAs; they meet only at mbarriers, so a builder never
-// waits for the issue of a stage and the issuer never waits for a block-wide barrier.
+// Builder warps (those with matrix jobs and those that expand digits) and an issuing warp meet only at mbarriers, so
+// a builder never waits for the issue of a stage and the issuer never waits for a block-wide barrier.
 // A stage uses buffer b = s mod WS_NB (three buffers: the round trip builder -> issuer -> tensor pipe -> builder
 // is longer than a stage, two buffers left the pipe waiting).
-//   full[b]   (count 15)  every builder warp has finished buffer b of this stage (lane 0 arrives after a
-//                         proxy fence and a warp barrier)
+//   full[b]   (count = builder warps)  every builder warp has finished buffer b of this stage (lane 0 arrives after
+//                         a proxy fence and a warp barrier)
 //   empty[b]  (count 1)   the MMAs that read buffer b have completed (tcgen05.commit)
 //   tma[q]    (tiled)     the 28 KB image of stage s has landed in slot q = s mod ws_a_slots(NP) of the A ring
 // Work needs no other synchronisation: a (column, plane) pair's digits are fetched (asynchronous copies into a
-// ring, three stages ahead), reversed and expanded into its rows of B by one warp (pair w of the stage, and
-// w + the number of builder warps where there are more pairs than warps), and every matrix job (one ChaCha8
-// block or eight coefficients -> one 8 x 8 byte tile of A) belongs to one thread.
+// ring, three of the warp's stages ahead), reversed and expanded into its rows of B by one digit warp (pair w of the
+// stage, and w + the number of digit warps of a stage where there are more pairs than warps), and every matrix job
+// (one ChaCha8 block or eight coefficients -> one 8 x 8 byte tile of A) belongs to one thread of a job warp.
 // B is the overlapping sliding-row image described at the top of this file (1792 bytes per pair), with the
 // planes of a column interleaved by core matrix: row group o / 8 of plane p sits at group (o / 8) np + p of the
 // column's image. With a row-group stride of 128 bytes and a K-block stride of 256 np bytes one descriptor then
@@ -330,44 +330,61 @@ commit_tc_pipe_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __rest
 // pipe for about 90 cycles whatever its width up to N = 128 (and 136 cycles at N = 256): per-plane MMAs cap the
 // kernel at 37 % of the pipe's rate.
 // The small B leaves room for a deeper ring of A images, which is what the copies from HBM need.
-// TILED: the A image is not touched by threads at all: thread 0 issues one bulk copy per stage into a ring of
-// ws_a_slots(NP) slots, ws_a_slots(NP) - 2 stages ahead of the builders (the copy issued at stage s reuses the
-// slot of stage s - 2, whose MMAs the thread has just seen complete); rows 112..127 of the M = 128 operand are whatever follows the slot in shared
-// memory: they only feed accumulator rows that nobody reads.
+// TILED: the A image is not touched by threads at all: one lane issues one bulk copy per stage into a ring of
+// ws_a_slots(NP) slots; rows 112..127 of the M = 128 operand are whatever follows the slot in shared memory: they
+// only feed accumulator rows that nobody reads.
 // Every wait is bounded; a warp that gives up records TC_ERR_TIMEOUT and leaves the loop, the others then run
 // out of their own waits, and all threads meet at the barrier before the epilogue.
-// Warps: 15 builders and the issuer (512 threads) when threads generate or split the matrix (the ChaCha8 build
-// needs 120 registers). Tiled source: 16 builders (one (column, plane) pair each at four planes: with 15 the warp
-// that owned two pairs set the pace of every stage), the issuer, and a warp whose first lane issues the bulk
-// copies of the A images into their own ring, as far ahead as the ring is deep (the issuer commits every stage
-// to the B buffer's barrier and to the A slot's).
-__host__ __device__ constexpr int ws_build_warps(int src) { return src == TC_SRC_TILED ? 16 : 15; }
-__host__ __device__ constexpr int ws_threads(int src) { return src == TC_SRC_TILED ? 576 : 512; }
+// Warps. When threads generate or split the matrix: 14 job warps (448 matrix jobs, one per thread), four digit warps
+// that build B, the issuer. The kernel is bound by the pipe that does the xors, rotations and byte permutes of the
+// jobs (one warp instruction per two cycles and scheduler; the additions go to the multiply-add pipe): about 300 of
+// them a job. Warp w runs on scheduler w mod 4, so the jobs load the schedulers 4 : 4 : 3 : 3, and the digit warps are
+// the warps 14, 15, 18, 19 that sit on the two short ones (16 issues, 17 idles). 2^18 columns x 3 planes: 2356 us with
+// the pairs dealt to the job warps as well, 2130 us with the digit warps apart, 2000 us with the shifted windows below
+// (4490 instead of 5030 instructions of that pipe per stage). Dealing the 14 warp jobs of a stage to 16 warps in
+// turn levels the schedulers but pays for it in index arithmetic (2015 us).
+// Tiled source: 16 digit warps in two groups that take the stages in turn, the issuer, and a warp whose first lane
+// issues the bulk copies of the A images, as far ahead as their ring is deep (the issuer commits every stage to the B
+// buffer's barrier and to the A slot's). A digit warp's stage is a chain of about a thousand cycles (wait, read,
+// shift, write, proxy fence): with all warps on every stage that chain set the pace (2^18 columns: 1.04 ms with two
+// planes, 1.37 ms with three), with two groups and three B buffers it is 0.95 and 1.10-1.19 ms (0.86 ms: one plane,
+// the rate of HBM).
+__host__ __device__ constexpr int ws_job_warps(int src) { return src == TC_SRC_TILED ? 0 : 14; }
+__host__ __device__ constexpr int ws_digit_warps(int src) { return src == TC_SRC_TILED ? 16 : 4; }
+__host__ __device__ constexpr int ws_threads(int src) { return src == TC_SRC_TILED ? 576 : 640; }
+__host__ __device__ constexpr int ws_digit_groups(int src) { return src == TC_SRC_TILED ? 2 : 1; }
+constexpr int WS_ISSUE_WARP = 16, WS_COPY_WARP = 17;
 constexpr int WS_NB = 3;                             // operand buffers in flight (a round trip builder -> issuer ->
                                                      // tensor pipe -> builder takes about two stage times)
 constexpr int WS_A_SLOTS_MAX = 6;
-constexpr int WS_DIGIT_DEPTH = 4;                    // ring of digit stages: copies run three stages ahead
-__host__ __device__ constexpr int ws_nb(int src) { return src == TC_SRC_TILED ? 2 : WS_NB; }   // tiled: room for the A ring
-__host__ __device__ constexpr int ws_a_slots(int np) { return np <= 3 ? 6 : 5; }
+constexpr int WS_DIGIT_DEPTH = 4;                    // ring of digit stages per group: copies run three of its stages ahead
+constexpr int WS_SHIFT_STRIDE = 40, WS_SHIFT_WORDS = 4 * WS_SHIFT_STRIDE;   // words of a pair's shifted windows (8 banks apart)
+__host__ __device__ constexpr int ws_a_slots(int np) { return np <= 2 ? 6 : np == 3 ? 5 : 4; }   // what 227 KB leave
 
+// err[0] is set when a digit is -128, err[1] when a wait gave up: plain stores of one value, because the words lie in
+// page-locked host memory (nothing is written, and nothing has to be cleared or copied on the stream, without an error).
 template <int SRC, int NP>
 static __global__ void __launch_bounds__(ws_threads(SRC), 1)
 commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restrict__ d_M, const uint8_t* __restrict__ d_T,
                     const int8_t* __restrict__ d_digits, uint64_t N, int p0, uint64_t col_offset, uint64_t* __restrict__ partial,
-                    int* __restrict__ d_error, int chunk_cols) {
+                    int* __restrict__ err, int chunk_cols) {
     constexpr int np = NP;
     constexpr bool TILED = SRC == TC_SRC_TILED, PREMAT = SRC == TC_SRC_COEFFS;
     constexpr int PAIRS = TC_STAGE_COLS * np;                       // (column, plane) pairs per stage
-    constexpr int WS_BUILD_WARPS = ws_build_warps(SRC), WS_THREADS = ws_threads(SRC);
-    constexpr int PAIRS_PER_WARP = (PAIRS + WS_BUILD_WARPS - 1) / WS_BUILD_WARPS;
+    constexpr int JOB_WARPS = ws_job_warps(SRC), DIGIT_WARPS = ws_digit_warps(SRC), WS_THREADS = ws_threads(SRC);
+    constexpr int GROUPS = ws_digit_groups(SRC), GROUP_WARPS = DIGIT_WARPS / GROUPS;
+    constexpr int WS_BUILD_WARPS = JOB_WARPS + GROUP_WARPS;   // that work on one stage
+    constexpr int PAIRS_PER_WARP = (PAIRS + GROUP_WARPS - 1) / GROUP_WARPS;
+    constexpr int DIGIT_DEPTH = WS_DIGIT_DEPTH * GROUPS;
+    static_assert(PAIRS_PER_WARP <= 8, "four lanes fetch a pair's digits");
     constexpr uint32_t A_SLOT = TILED ? TCP_A_IMAGE : TC_A_BYTES;
-    constexpr int NB = ws_nb(SRC);
+    constexpr int NB = WS_NB;
     constexpr int A_SLOTS = TILED ? ws_a_slots(NP) : NB;
     constexpr uint32_t B_BYTES = PAIRS * TC_B_IMAGE;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* A_base = smem;
     uint8_t* B_base = smem + A_SLOTS * A_SLOT;
-    uint8_t* DG_base = B_base + NB * B_BYTES;                        // WS_DIGIT_DEPTH stages of digits, 64 bytes per pair
+    uint8_t* DG_base = B_base + NB * B_BYTES;                        // DIGIT_DEPTH stages of digits, 64 bytes per pair
     __shared__ __align__(8) uint64_t bar_full[WS_NB], bar_empty[WS_NB], bar_tma[WS_A_SLOTS_MAX], bar_afree[WS_A_SLOTS_MAX];
     __shared__ uint32_t tmem_base_sh;
 
@@ -417,37 +434,29 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
                      ::"r"(dst), "l"(src), "r"((uint32_t)TCP_A_IMAGE), "r"(bar) : "memory");
     };
 
-    if (warp < WS_BUILD_WARPS) {
-        // ================= builders =================
+    // the MMAs that last read the buffer of stage sidx (those of stage sidx - NB) are done: one lane polls
+    auto buffer_free = [&](int sidx) {
+        if (sidx < NB) return true;
+        uint32_t ok = 1;
+        if (lane == 0) ok = mbar_wait(smem_u32(&bar_empty[sidx % NB]), (uint32_t)((sidx / NB - 1) & 1)) ? 1u : 0u;
+        return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    };
+    auto report_full = [&](int sidx) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_full[sidx % NB])) : "memory");
+    };
+    if (warp < JOB_WARPS) {
+        // ================= matrix jobs: eight coefficients of (column jj, row il) to one 8 x 8 byte tile of A =================
+        static_assert(JOB_WARPS == 0 || JOB_WARPS * 32 == TC_STAGE_COLS * TC_ROWS * 8, "one job per thread and stage");
+        const int jj = t / (TC_ROWS * 8), rem = t % (TC_ROWS * 8), il = rem >> 3, blk = rem & 7;
         uint32_t key[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) key[k] = SRC == TC_SRC_CHACHA ? d_key[k] : 0u;
-        constexpr int JOBS = TC_STAGE_COLS * TC_ROWS * 8;   // 448 matrix jobs per stage, one per thread
         ulonglong2 creg[4];
-        // The digits of stage `stage` go into slot stage mod WS_DIGIT_DEPTH of a ring in shared memory by
-        // asynchronous copies (16 bytes per lane, four lanes per pair), WS_DIGIT_DEPTH - 1 stages ahead of their
-        // use: a global load consumed one stage later leaves every stage waiting for a full memory latency.
-        // One group is committed per stage, empty or not, so that the group count says which stage has landed.
-        auto fetch_digits = [&](int stage) {
-            const uint64_t js = j0 + (uint64_t)stage * TC_STAGE_COLS;
-            uint8_t* slot = DG_base + (stage % WS_DIGIT_DEPTH) * (PAIRS * D);
-#pragma unroll
-            for (int q = 0; q < PAIRS_PER_WARP; q++) {
-                const int cp = warp + WS_BUILD_WARPS * q;
-                if (cp < PAIRS && lane < 4) {
-                    const int jj = cp / np, p = cp % np;
-                    const bool on = stage < n_stages && js + jj < j1;
-                    const int8_t* src = d_digits + ((size_t)(p0 + p) * N + (on ? js + jj : j0)) * D + 16 * lane;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                                 ::"r"(smem_u32(slot + cp * D + 16 * lane)), "l"(src), "r"(on ? 16 : 0) : "memory");
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
         auto fetch = [&](uint64_t js) {
             if (PREMAT) {
-                const int jj = t / (TC_ROWS * 8), rem = t % (TC_ROWS * 8), il = rem >> 3, blk = rem & 7;
-                const bool on = t < JOBS && js + jj < j1;
+                const bool on = js + jj < j1;
                 const ulonglong2* src = reinterpret_cast<const ulonglong2*>(
                     d_M + ((js + jj) * (uint64_t)KAPPA + (uint64_t)(group * TC_ROWS + il)) * D + 8 * blk);
 #pragma unroll
@@ -455,102 +464,136 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
             }
         };
         if (n_stages > 0) fetch(j0);
-        for (int st = 0; st < WS_DIGIT_DEPTH - 1; st++) fetch_digits(st);
-        // this thread's matrix job has the same row and block in every stage: the quarter rounds of the first
+        // this thread's job has the same row and block in every stage: the quarter rounds of the first
         // column round that do not see the column index are computed once
         ChaChaColumns cols_pre;
         cols_pre.n2 = 0;
-        if (SRC == TC_SRC_CHACHA && t < JOBS) {
-            const int rem = t % (TC_ROWS * 8);
-            chacha8_columns(key, (uint32_t)(rem & 7), (uint32_t)(group * TC_ROWS + (rem >> 3)), (uint32_t)((col_offset + j0) >> 32), cols_pre);
-        }
+        if (SRC == TC_SRC_CHACHA)
+            chacha8_columns(key, (uint32_t)blk, (uint32_t)(group * TC_ROWS + il), (uint32_t)((col_offset + j0) >> 32), cols_pre);
+        // Bytes to planes: two 4 x 4 byte transposes per half, eight permutes each (pairs of words first, then pairs
+        // of pairs). A lane stores its planes in the order bp = b ^ rot, so that the lanes of one store cover
+        // different banks; rot's two bits pick which result of each permute level is formed first.
+        const int rot = (t >> 1) & 3;
+        const uint32_t first0 = rot & 2 ? 0x7362u : 0x5140u, first1 = first0 ^ (0x7362u ^ 0x5140u);
+        const uint32_t second0 = rot & 1 ? 0x7632u : 0x5410u, second1 = second0 ^ (0x7632u ^ 0x5410u);
+        const uint32_t kk = (uint32_t)(jj * D + 8 * blk);
+        const uint32_t job_off = (uint32_t)il * TC_SBO + (kk >> 4) * TC_CORE + (kk & 15);
         for (int sidx = 0; sidx < n_stages; sidx++) {
             const uint64_t js = j0 + (uint64_t)sidx * TC_STAGE_COLS;
-            const int buf = sidx % NB, use = sidx / NB;   // buffer and how many times it has been used before
-            uint8_t* A_sh = A_base + buf * A_SLOT;     // not used when TILED
-            uint8_t* B_sh = B_base + buf * B_BYTES;
-            // the MMAs that last read this buffer (stage sidx - NB) must be done before it is rewritten
-            if (sidx >= NB) {
-                uint32_t ok = 1;
-                if (lane == 0) ok = mbar_wait(smem_u32(&bar_empty[buf]), (uint32_t)((use - 1) & 1)) ? 1u : 0u;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) { failed = true; break; }
+            if (!buffer_free(sidx)) { failed = true; break; }
+            uint64_t c[8];
+            if (PREMAT) {
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    c[2 * x] = creg[x].x;
+                    c[2 * x + 1] = creg[x].y;
+                }
+            } else {
+                prg_ring_block_pre(key, cols_pre, (uint32_t)(group * TC_ROWS + il), col_offset + js + jj, (uint32_t)blk, c);
             }
-            // the copies of stage sidx + WS_DIGIT_DEPTH - 1 go out (their slot held stage sidx - 1, which this warp
-            // read before its last barrier); all but the newest WS_DIGIT_DEPTH - 1 groups have then landed
-            fetch_digits(sidx + WS_DIGIT_DEPTH - 1);
-            asm volatile("cp.async.wait_group %0;" ::"n"(WS_DIGIT_DEPTH - 1) : "memory");
-            __syncwarp();
-            // A: byte planes of this thread's eight coefficients
-            if (!TILED && t < JOBS) {
-                const int jj = t / (TC_ROWS * 8), rem = t % (TC_ROWS * 8), il = rem >> 3, blk = rem & 7;
-                uint64_t c[8];
-                if (PREMAT) {
+            uint8_t* dst = A_base + (sidx % NB) * A_SLOT + job_off;
 #pragma unroll
-                    for (int x = 0; x < 4; x++) {
-                        c[2 * x] = creg[x].x;
-                        c[2 * x + 1] = creg[x].y;
-                    }
-                } else {
-                    prg_ring_block_pre(key, cols_pre, (uint32_t)(group * TC_ROWS + il), col_offset + js + jj, (uint32_t)blk, c);
+            for (int h = 0; h < 2; h++) {
+                uint32_t w[8], a[4], b[4];
+#pragma unroll
+                for (int x = 0; x < 8; x++) w[x] = h ? (uint32_t)(c[x] >> 32) : (uint32_t)c[x];
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    a[x] = __byte_perm(w[2 * x], w[2 * x + 1], first0);
+                    b[x] = __byte_perm(w[2 * x], w[2 * x + 1], first1);
                 }
-                const uint32_t kk = (uint32_t)(jj * D + 8 * blk);
-                uint8_t* dst = A_sh + il * TC_SBO + (kk >> 4) * TC_CORE + (kk & 15);
-                const int rot = (t >> 1) & 3;
-#pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    const int bp = (b & 4) | ((b + rot) & 3);
-                    uint32_t w[8];
-#pragma unroll
-                    for (int x = 0; x < 8; x++) w[x] = b < 4 ? (uint32_t)c[x] : (uint32_t)(c[x] >> 32);
-                    const uint32_t sel = (uint32_t)(bp & 3) | ((4u + (uint32_t)(bp & 3)) << 4);
-                    const uint32_t lo = __byte_perm(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel), 0x5410);
-                    const uint32_t hi = __byte_perm(__byte_perm(w[4], w[5], sel), __byte_perm(w[6], w[7], sel), 0x5410);
-                    *reinterpret_cast<uint2*>(dst + bp * 16) = make_uint2(lo, hi);
-                }
-            }
-            // B: the 112 sliding rows of this warp's pairs, straight from the digits. The reversed, sign-wrapped
-            // window of a pair has words W[i] = reverse(Z[15 - i]) for i < 16 and -reverse(Z[31 - i]) for i >= 16
-            // (Z the 16 digit words); lane l < 28 reads W[l .. l + 4] and forms rows 4 l .. 4 l + 3 (byte offsets
-            // 0 .. 3 into the same five words). The four stores of a lane go out rotated by l / 2, so that the
-            // lanes of one store instruction cover eight different 16-byte slots of the banks.
-#pragma unroll
-            for (int q = 0; q < PAIRS_PER_WARP; q++) {
-                const int cp = warp + WS_BUILD_WARPS * q;
-                if (cp < PAIRS && lane < 28) {
-                    const uint32_t* Z = reinterpret_cast<const uint32_t*>(DG_base + (sidx % WS_DIGIT_DEPTH) * (PAIRS * D) + cp * D);
-                    uint32_t w[5];
-#pragma unroll
-                    for (int x = 0; x < 5; x++) {
-                        const int i = lane + x;
-                        const uint32_t z = Z[i < 16 ? 15 - i : 31 - i];
-                        if (x == 0 && lane < 16 &&
-                            (((z & 0xffu) == 0x80u) | ((z & 0xff00u) == 0x8000u) | ((z & 0xff0000u) == 0x800000u) | ((z >> 24) == 0x80u)))
-                            bad_digit = 1;
-                        const uint32_t rev = __byte_perm(z, 0, 0x0123);
-                        w[x] = i < 16 ? rev : __vneg4(rev);
-                    }
-                    // row o of plane p goes to row group (o / 8) * np + p of the column's image: the planes are
-                    // interleaved by core matrix, so that one descriptor walks all of them
-                    const int jj = cp / np, p = cp - jj * np;
-                    uint8_t* dst = B_sh + (size_t)jj * (np * TC_B_IMAGE) + p * TC_CORE + (lane >> 1) * (np * TC_CORE) + (lane & 1) * 64;
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const int kk = (k + (lane >> 1)) & 3, sh = 8 * kk;
-                        *reinterpret_cast<uint4*>(dst + 16 * kk) =
-                            make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh),
-                                       __funnelshift_r(w[3], w[4], sh));
-                    }
-                }
+                uint8_t* d = dst + 64 * h;
+                *reinterpret_cast<uint2*>(d + 16 * rot) = make_uint2(__byte_perm(a[0], a[1], second0), __byte_perm(a[2], a[3], second0));
+                *reinterpret_cast<uint2*>(d + 16 * (rot ^ 1)) = make_uint2(__byte_perm(a[0], a[1], second1), __byte_perm(a[2], a[3], second1));
+                *reinterpret_cast<uint2*>(d + 16 * (rot ^ 2)) = make_uint2(__byte_perm(b[0], b[1], second0), __byte_perm(b[2], b[3], second0));
+                *reinterpret_cast<uint2*>(d + 16 * (rot ^ 3)) = make_uint2(__byte_perm(b[0], b[1], second1), __byte_perm(b[2], b[3], second1));
             }
             // next stage's global reads go out before this warp reports the stage
             if (sidx + 1 < n_stages) fetch(js + TC_STAGE_COLS);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            report_full(sidx);
+        }
+    } else if (TILED ? warp < WS_ISSUE_WARP : (warp & 2) != 0) {
+        // ================= digits =================
+        uint32_t bad_bytes = 0;
+        const int dw = TILED ? warp : (warp & 1) + 2 * (warp >= 16);   // warps 14, 15, 18, 19
+        const int dg = dw % GROUPS, gw = dw / GROUPS;                  // stages dg, dg + GROUPS, ...; pairs gw, gw + GROUP_WARPS, ...
+        // The digits of stage `stage` go into slot stage mod DIGIT_DEPTH of a ring in shared memory by asynchronous
+        // copies (16 bytes per lane, four lanes per pair of this warp), WS_DIGIT_DEPTH - 1 of this warp's stages ahead
+        // of their use: a global load consumed one stage later leaves every stage waiting for a full memory latency.
+        // One group is committed per stage, empty or not, so that the group count says which stage has landed.
+        // (A warp that works on every second stage still never waits for a barrier more than one phase behind: it has
+        // seen the MMAs of stage s - 2 - NB done when it waits for those of s - NB, and NB >= 2.)
+        auto fetch_digits = [&](int stage) {
+            const uint64_t js = j0 + (uint64_t)stage * TC_STAGE_COLS;
+            uint8_t* slot = DG_base + (stage % DIGIT_DEPTH) * (PAIRS * D);
+            const int q = lane >> 2, piece = 16 * (lane & 3), cp = gw + GROUP_WARPS * q;
+            if (q < PAIRS_PER_WARP && cp < PAIRS) {
+                const int jj = cp / np, p = cp % np;
+                const bool on = stage < n_stages && js + jj < j1;
+                const int8_t* src = d_digits + ((size_t)(p0 + p) * N + (on ? js + jj : j0)) * D + piece;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                             ::"r"(smem_u32(slot + cp * D + piece)), "l"(src), "r"(on ? 16 : 0) : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        uint32_t* shifted = reinterpret_cast<uint32_t*>(DG_base + DIGIT_DEPTH * PAIRS * D) + dg * PAIRS * WS_SHIFT_WORDS;
+        for (int st = 0; st < WS_DIGIT_DEPTH - 1; st++) fetch_digits(dg + st * GROUPS);
+        for (int sidx = dg; sidx < n_stages; sidx += GROUPS) {
+            uint8_t* B_sh = B_base + (sidx % NB) * B_BYTES;
+            if (!buffer_free(sidx)) { failed = true; break; }
+            // the copies for this warp's stage WS_DIGIT_DEPTH - 1 further on go out (their slot held its last stage,
+            // which it read before its last barrier); all but the newest WS_DIGIT_DEPTH - 1 groups have then landed
+            fetch_digits(sidx + (WS_DIGIT_DEPTH - 1) * GROUPS);
+            asm volatile("cp.async.wait_group %0;" ::"n"(WS_DIGIT_DEPTH - 1) : "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_full[buf])) : "memory");
+            // B: the 112 sliding rows of this warp's pairs. Word i of a pair's reversed, sign-wrapped window is
+            // reverse(Z[15 - i]) for i < 16 and -reverse(Z[31 - i]) for i >= 16 (Z the 16 digit words): one word per
+            // lane. The window shifted by k = 0 .. 3 bytes goes to four word arrays in shared memory (three funnel
+            // shifts), and row o is then four consecutive words of array o & 3: lane l forms rows l, l + 32, ... with
+            // reads and 16-byte stores that meet no bank twice. Forming every row from its five window words took
+            // sixteen shifts and five negations a lane on the pipe that bounds the kernel.
+#pragma unroll
+            for (int q = 0; q < PAIRS_PER_WARP; q++) {
+                const int cp = gw + GROUP_WARPS * q;
+                if (cp < PAIRS) {
+                    const uint32_t z = reinterpret_cast<const uint32_t*>(DG_base + (sidx % DIGIT_DEPTH) * (PAIRS * D) + cp * D)[(lane & 15) ^ 15];
+                    const uint32_t x = z ^ 0x80808080u;
+                    bad_bytes |= (x - 0x01010101u) & ~x;       // bit 7 of a byte: some byte is 0x80
+                    const uint32_t rev = __byte_perm(z, 0, 0x0123);
+                    const uint32_t neg = (0x80808080u - (rev & 0x7f7f7f7fu)) ^ (~rev & 0x80808080u);   // bytewise
+                    const uint32_t w = lane < 16 ? rev : neg, next = __shfl_down_sync(0xffffffffu, w, 1);
+                    uint32_t* F = shifted + cp * WS_SHIFT_WORDS + lane;
+                    F[0] = w;
+#pragma unroll
+                    for (int k = 1; k < 4; k++) F[k * WS_SHIFT_STRIDE] = __funnelshift_r(w, next, 8 * k);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < PAIRS_PER_WARP; q++) {
+                const int cp = gw + GROUP_WARPS * q;
+                if (cp < PAIRS) {
+                    // row o of plane p goes to row group (o / 8) * np + p of the column's image: the planes are
+                    // interleaved by core matrix, so that one descriptor walks all of them
+                    const int jj = cp / np, p = cp - jj * np;
+                    const uint32_t* F = shifted + cp * WS_SHIFT_WORDS + (lane & 3) * WS_SHIFT_STRIDE + (lane >> 2);
+                    uint8_t* dst = B_sh + (size_t)jj * (np * TC_B_IMAGE) + p * TC_CORE + (lane >> 3) * (np * TC_CORE) + (lane & 7) * 16;
+                    uint32_t r[4][4];
+#pragma unroll
+                    for (int m = 0; m < 4; m++)
+#pragma unroll
+                        for (int x = 0; x < 4; x++) r[m][x] = m < 3 || lane < 16 ? F[8 * m + x] : 0u;
+#pragma unroll
+                    for (int m = 0; m < 4; m++)
+                        if (m < 3 || lane < 16)
+                            *reinterpret_cast<uint4*>(dst + m * (4 * np * TC_CORE)) = make_uint4(r[m][0], r[m][1], r[m][2], r[m][3]);
+                }
+            }
+            report_full(sidx);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");   // nothing of this warp is still in flight when it leaves
-    } else if (warp == WS_BUILD_WARPS + 1) {
+        if (bad_bytes & 0x80808080u) bad_digit = 1;
+    } else if (warp == WS_COPY_WARP) {
         // ================= copies of the A images (tiled source) =================
         if (TILED && lane == 0) {
             for (int st = 0; st < n_stages; st++) {
@@ -560,7 +603,7 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
                 copies_issued = st + 1;
             }
         }
-    } else if (lane == 0) {
+    } else if (warp == WS_ISSUE_WARP && lane == 0) {
         // ================= issuer =================
         const uint32_t idesc = umma_idesc_i8(64 * np);   // all planes in one MMA
         for (int sidx = 0; sidx < n_stages; sidx++) {
@@ -596,7 +639,7 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
         }
     }
     if (__syncthreads_or(failed)) failed = true;
-    if (TILED && failed && warp == WS_BUILD_WARPS + 1 && lane == 0) {
+    if (TILED && failed && warp == WS_COPY_WARP && lane == 0) {
         // a wait gave up somewhere: no copy of this CTA may still be in flight when it leaves (bounded waits again;
         // a landed copy's phase is complete whether or not the issuer consumed it)
         for (int st = copies_issued > A_SLOTS ? copies_issued - A_SLOTS : 0; st < copies_issued; st++)
@@ -648,16 +691,16 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
-    if (failed && lane == 0) atomicMax(d_error, (int)TC_ERR_TIMEOUT);
-    if (bad_digit) atomicMax(d_error, (int)TC_ERR_DIGIT_RANGE);
+    if (failed && lane == 0) *(volatile int*)&err[1] = 1;
+    if (bad_digit) *(volatile int*)&err[0] = 1;
 }
 
 inline size_t tc_ws_smem_bytes(int src, int np) {
     const size_t pairs = (size_t)TC_STAGE_COLS * np;
     const size_t a = src == TC_SRC_TILED ? (size_t)ws_a_slots(np) * TCP_A_IMAGE : (size_t)WS_NB * TC_A_BYTES;
-    const size_t nb = (size_t)ws_nb(src);
     // the tiled ring's last slot is read 4 KB past its image (rows 112..127 of the operand): B follows it
-    return a + nb * pairs * TC_B_IMAGE + (size_t)WS_DIGIT_DEPTH * pairs * D + 4096;
+    const size_t groups = (size_t)ws_digit_groups(src);
+    return a + WS_NB * pairs * TC_B_IMAGE + groups * pairs * (WS_DIGIT_DEPTH * D + WS_SHIFT_WORDS * sizeof(uint32_t));
 }
 
 // ---- sustained int8 rate of the tensor pipe, measured with this file's own issue loop -------------------
@@ -732,21 +775,29 @@ inline size_t tc_pipe_smem_bytes(int np) {
     return 2 * (TC_A_BYTES + (size_t)TC_STAGE_COLS * np * TC_B_IMAGE) + TC_STAGE_COLS * TC_MAX_PLANES * TC_V_STRIDE;
 }
 
-// out[p][i][r] = sum over chunks of partial[chunk][group = i / 14][p][i % 14][r]
-static __global__ void reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, int np,
-                                                 uint64_t* __restrict__ out) {
-    const size_t width = (size_t)np * KAPPA * D;
-    const size_t step = (size_t)gridDim.x * blockDim.x;
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < width; k += step) {
-        int p = (int)(k / (KAPPA * D)), i = (int)((k / D) % KAPPA), r = (int)(k % D);
-        int g = i / TC_ROWS, il = i % TC_ROWS;
-        uint64_t a = 0;
-        for (size_t c = 0; c < chunks; c++)
-            a = agl::add(a, partial[((c * 3 + g) * np + p) * (TC_ROWS * D) + il * D + r]);
+// out[p][i][r] = sum over chunks of partial[chunk][group = i / 14][p][i % 14][r]. A block owns 32 outputs and deals
+// the chunks to sixteen warps: one thread per output read its chunks one after the other on a quarter of the SMs
+// (18.5 us for 98 chunks x 3 planes, 84 us for 542 chunks).
+constexpr int TC_RED_SLICES = 16;
+static __global__ void __launch_bounds__(32 * TC_RED_SLICES)
+reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, int np, uint64_t* __restrict__ out) {
+    __shared__ uint64_t sums[TC_RED_SLICES][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const size_t k = (size_t)blockIdx.x * 32 + lane;   // 32 divides the width np * 42 * 64
+    const int p = (int)(k / (KAPPA * D)), i = (int)((k / D) % KAPPA), r = (int)(k % D);
+    const uint64_t* src = partial + ((size_t)(i / TC_ROWS) * np + p) * (TC_ROWS * D) + (i % TC_ROWS) * D + r;
+    const size_t stride = (size_t)3 * np * TC_ROWS * D;
+    uint64_t a = 0;
+#pragma unroll 8
+    for (size_t c = slice; c < chunks; c += TC_RED_SLICES) a = agl::add(a, src[c * stride]);
+    sums[slice][lane] = a;
+    __syncthreads();
+    if (slice == 0) {
+#pragma unroll
+        for (int q = 1; q < TC_RED_SLICES; q++) a = agl::add(a, sums[q][lane]);
         out[k] = agl::canon(a);
     }
 }
-
 
 }  // namespace aj
 }  // namespace mb
