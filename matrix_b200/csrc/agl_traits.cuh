@@ -96,6 +96,26 @@ struct Lazy<AglExt2> {
 };
 
 template <>
+struct NarrowLazy<AglBase> {
+    using A = gl::Acc;
+    static __device__ __forceinline__ A zero() { return gl::acc_zero(); }
+    static __device__ __forceinline__ void mul(A& s, uint64_t x, uint64_t y) { gl::acc_mul(s, x, y); }
+    static __device__ __forceinline__ uint64_t reduce(const A& s) { return agl::acc_reduce_wide(s); }
+};
+template <>
+struct NarrowLazy<AglExt2> {
+    using A = NarrowSum;
+    static __device__ __forceinline__ A zero() { return A{gl::acc_zero(), gl::acc_zero()}; }
+    static __device__ __forceinline__ void mul(A& s, agl::E2 x, agl::E2 y) {
+        gl::acc_mul(s.s0, x.c0, y.c0);
+        gl::acc_mul(s.s0, x.c1, agl::mul_small(y.c1, 3));
+        gl::acc_mul(s.s1, x.c0, y.c1);
+        gl::acc_mul(s.s1, x.c1, y.c0);
+    }
+    static __device__ __forceinline__ agl::E2 reduce(const A& s) { return agl::E2{agl::acc_reduce_wide(s.s0), agl::acc_reduce_wide(s.s1)}; }
+};
+
+template <>
 struct FoldOp<AglBase, AglExt2> {
     static __device__ __forceinline__ agl::E2 apply(uint64_t a, uint64_t b, agl::E2 r) {
         return agl::e2_fma_pre_base(agl::e2_pre(r), agl::sub(b, a), a);

@@ -41,10 +41,9 @@ int launch_round_message(const uint64_t* d_polys, uint64_t* d_partial, int d, si
     if (half < 1 || 2 * half > stride) return MB_ERR_ARG;
     if (!aligned16(d_polys) || ((stride * F::NW) & 1)) return MB_ERR_ARG;
     int threads = threads_for(half, num_blocks);
-    // launch bounds of round_message_kernel: 512 threads for two tables (register budget of the exact
-    // sums), 1024 for three, 256 for every other count (one table included); the kernels are
-    // grid-stride loops, so a smaller block only means more sweeps
-    const int bound = d == 2 ? 512 : d == 3 ? 1024 : 256;
+    // launch bounds of round_message_kernel: 512 threads for two tables, 256 for every other count (register budget of
+    // the exact sums); the kernels are grid-stride loops, so a smaller block only means more sweeps
+    const int bound = d == 2 ? 512 : 256;
     if (threads > bound) threads = bound;
     MB_KERNEL_ON("sumcheck_round_message", st);
     MB_DISPATCH_D(d, (round_message_kernel<F, D><<<num_blocks, threads, 0, st>>>(d_polys, stride, half, d_partial,
@@ -95,8 +94,10 @@ int launch_fold_lift(const uint64_t* d_in, uint64_t* d_out, typename FOut::T r, 
     return finish_async();
 }
 
-// Grid used by this library's own provers for a pass over `items` work items.
-inline int prover_grid(size_t items) { return grid_for(items, BLOCK, 6); }
+// Grid used by this library's own provers for a pass over `items` work items of d tables. The exact sums of three or four
+// tables leave room for two blocks per SM, and a block's own sums at its end cost as much as a few items a thread:
+// as many blocks as run at once.
+inline int prover_grid(size_t items, int d = 2) { return grid_for(items, BLOCK, d == 3 || d == 4 ? 2 : 6); }
 
 }  // namespace sc
 }  // namespace mb

@@ -219,7 +219,8 @@ open_pass_kernel(const OpenPassArgs a, const __grid_constant__ pr::FoldWeights<p
     }
     if (ns > pr::BLK) x = gl::E2{gl::acc_reduce_wide(s0), gl::acc_reduce_wide(s1)};
     if (sb > 0 && (size_t)t < ns) x = F::fma(pr::load_weight<F>(a.wl + 4 * t), x, gl::E2{0, 0});
-    if (!pr::grid_sum<F>(x, 0, sm, a.partial + 4 * (size_t)gridDim.x * m, a.counter + (pr::GROUPS + 1) * m)) return;
+    gl::E2 total[1] = {x};
+    if (!pr::grid_sum<F, 1>(total, 0, sm, a.partial + 4 * (size_t)gridDim.x * m, a.counter + (pr::GROUPS + 1) * m)) return;
     if (t == 0) pr::store2(a.sums + 2 * m, sm[0].c0, sm[0].c1);
 }
 

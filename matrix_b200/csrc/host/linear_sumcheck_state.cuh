@@ -14,7 +14,8 @@
 //    after a fold only reads (d+1) extension elements back.
 // Base / Ext are the field traits of sumcheck_kernels.cuh (GlBase, GlExt2) or
 // agl_traits.cuh (AglBase, AglExt2).
-//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh); the other counts a round per pass:
+//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh), and so do one, three or four tables that
+//    are small (product_sumcheck.cuh); other sizes and counts take a round per pass:
 //  * once a table is down to host_tail(d) elements the live tables are read back and the remaining rounds run on
 //    the host: a round on the device costs a launch and a synchronisation (about 20 us) whatever its size, the
 //    same round on a few hundred elements takes a host core less (about 7 ns per extension product). The field
@@ -27,6 +28,7 @@
 #include "ext2_words.hpp"
 #include "host_field.hpp"
 #include "pair_sumcheck.cuh"
+#include "product_sumcheck.cuh"
 
 namespace mbhost {
 
@@ -49,8 +51,8 @@ template <class T, class F> struct HostExtOps {
 template <> struct HostExt<gl::E2> : HostExtOps<gl::E2, hf::GlE2Ops> {};
 template <> struct HostExt<agl::E2> : HostExtOps<agl::E2, hf::AglE2Ops> {};
 template <class T> struct PairOf;
-template <> struct PairOf<gl::E2> { using type = PairSumcheck<pr::GlF, PairGl>; };
-template <> struct PairOf<agl::E2> { using type = PairSumcheck<pr::AglF, PairAgl>; };
+template <> struct PairOf<gl::E2> { using type = PairSumcheck<pr::GlF, PairGl>; using product = ProductSumcheck<pr::GlF, PairGl>; };
+template <> struct PairOf<agl::E2> { using type = PairSumcheck<pr::AglF, PairAgl>; using product = ProductSumcheck<pr::AglF, PairAgl>; };
 
 // Live elements per table at which the rounds move to the host: a host round costs live / 2 x (d^2 - 1 + d)
 // extension products, about 9 us at 512 elements of two tables and 10 us at 256 elements of three.
@@ -79,12 +81,17 @@ public:
             const size_t words = n_ * (base_field ? 1 : 2);
             return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0);
         }
+        products_ = Product::handles(d) && aligned16(d_tables) && num_vars > 0;
+        if (products_ && num_vars <= Product::limit(d)) {
+            product_.reset(new Product);
+            return product_->init(d_tables, n_ * (base_field ? 1 : 2), d, num_vars, base_field, nullptr);
+        }
         size_t cap_a = n_ >= 2 ? n_ / 2 : 1, cap_b = n_ >= 4 ? n_ / 4 : 1;
         stride_a_ = cap_a;
         stride_b_ = cap_b;
         MB_CUDA(pool_alloc((void**)&buf_a_, sizeof(uint64_t) * 2 * cap_a * d));
         MB_CUDA(pool_alloc((void**)&buf_b_, sizeof(uint64_t) * 2 * cap_b * d));
-        max_blocks_ = prover_grid(n_ / 2 > 0 ? n_ / 2 : 1);
+        max_blocks_ = prover_grid(n_ / 2 > 0 ? n_ / 2 : 1, d);
         MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 2 * (d + 1) * (size_t)max_blocks_));
         MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned int)));
         MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned int), MB_STREAM));
@@ -115,10 +122,21 @@ public:
             return MB_OK;
         }
         size_t live = n_ >> round_, half = live / 2;
+        if (product_) {
+            if (!product_->at_tail()) {
+                typename Ext::T p[5];
+                int rc = product_->message(p);
+                out.resize(d_ + 1);
+                for (int c = 0; c <= d_; c++) { out[c].c0 = p[c].c0; out[c].c1 = p[c].c1; }
+                return rc;
+            }
+            int rc = take_tables();
+            if (rc != MB_OK) return rc;
+        }
         if (host_mode_) return host_message(out, half);
         if (!have_msg_) {
             // Only round 0 gets here: every fold leaves the next message behind.
-            int grid = prover_grid(half);
+            int grid = prover_grid(half, d_);
             int rc;
             if (base_) {
                 rc = launch_round_message<Base>(src_, partial_, d_, n_, half, grid, MB_STREAM, counter_, msg_dev_);
@@ -152,6 +170,14 @@ public:
             round_++;
             return pair_->fold(r);
         }
+        if (product_) {
+            if (!product_->at_tail()) {
+                round_++;
+                return product_->fold(r);
+            }
+            int rc = take_tables();
+            if (rc != MB_OK) return rc;
+        }
         if (!host_mode_ && round_ >= 1 && live <= host_tail(d_)) {
             int rc = to_host(live);
             if (rc != MB_OK) return rc;
@@ -172,8 +198,13 @@ public:
         size_t stride_out = to_a ? stride_a_ : stride_b_;
         bool in_base = base_ && round_ == 0;
         int rc;
+        if (products_ && half <= (size_t)1 << Product::limit(d_)) {   // the tables stay where they are until the state goes
+            product_.reset(new Product);
+            round_++;
+            return product_->init(in, stride_in * (in_base ? 1 : 2), d_, num_vars_ - round_ + 1, in_base, &r);
+        }
         if (quarter >= 1) {
-            int grid = prover_grid(quarter);
+            int grid = prover_grid(quarter, d_);
             if (in_base) {
                 rc = launch_fold_message<Base, Ext>(in, out, r, nullptr, d_, stride_in, stride_out, quarter,
                                                          partial_, grid, MB_STREAM, counter_, msg_dev_);
@@ -210,6 +241,10 @@ public:
             out[1].c0 = b.c0; out[1].c1 = b.c1;
             return MB_OK;
         }
+        if (product_) {
+            int rc = take_tables();
+            if (rc != MB_OK) return rc;
+        }
         if (host_mode_) {
             for (int i = 0; i < d_; i++) {
                 const typename Ext::T v = host_tab_[(size_t)i * host_stride_];
@@ -239,6 +274,16 @@ public:
     int current_round() const { return round_; }
 
 private:
+    using Product = typename PairOf<typename Ext::T>::product;
+    // The several-rounds passes are done: the rounds continue on the host.
+    int take_tables() {
+        int rc = product_->tables(host_tab_, host_stride_);
+        if (rc != MB_OK) return rc;
+        product_.reset();
+        host_mode_ = true;
+        have_msg_ = false;
+        return MB_OK;
+    }
     // The live elements of the (extension) tables come to the host; the rounds continue there.
     int to_host(size_t live) {
         host_stride_ = live;
@@ -302,6 +347,8 @@ private:
     size_t host_stride_ = 0;
     std::vector<typename Ext::T> host_tab_;
     std::unique_ptr<typename PairOf<typename Ext::T>::type> pair_;
+    bool products_ = false;   // the several-rounds passes take over once the tables are small enough
+    std::unique_ptr<Product> product_;
 };
 
 }  // namespace mbhost

@@ -95,32 +95,43 @@ __device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
     return typename F::Pre{a.x, a.y, p[2]};
 }
 
-// Sums the threads' values by t mod 2^bits over the block and then over the gridDim.x blocks of blockIdx.y; true in
-// the block that finishes last, with the sums (canonical) in sm[0 .. 2^bits). partial: 2 gridDim.x * 2^bits elements of
-// this blockIdx.y; counters: GROUPS + 1 of this blockIdx.y, zero before and after.
-// A block that reads hundreds of rows one after another waits for L2 each time (512 rows: 70 us), so rows are summed in
-// groups of about sqrt(gridDim.x) by each group's last block, then the groups by the last of those.
+// Sums the threads' V values by t mod 2^bits over the block and then over the gridDim.x blocks of blockIdx.y; true in
+// the block that finishes last, with the sums (canonical) in sm[0 .. V 2^bits), value j of t at j 2^bits + t.
+// partial: 2 gridDim.x * V 2^bits elements of this blockIdx.y; counters: GROUPS + 1 of this blockIdx.y, zero before and after.
+// A block that reads hundreds of rows one after another waits for L2 each time (512 rows: 70 us), so beyond sixteen rows
+// a thread they are summed in groups of about sqrt(gridDim.x) by each group's last block, then the groups by the last
+// of those; up to sixteen (their loads overlap) one level is faster by a fence and an atomic.
 constexpr int GROUPS = 64;
-template <class F>
-__device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F::E2* sm, uint64_t* partial, unsigned* counters) {
+template <class F, int V>
+__device__ __forceinline__ bool grid_sum(typename F::E2 (&v)[V], int bits, typename F::E2* sm, uint64_t* partial, unsigned* counters) {
     using E2 = typename F::E2;
     __shared__ bool last;
     const int t = threadIdx.x, n = 1 << bits;
-    const auto block_sum = [&](E2 x) {
-        __syncthreads();
-        sm[t] = x;
-        __syncthreads();
-        for (int s = BLK / 2; s >= n; s >>= 1) {
-            if (t < s) sm[t] = F::add(sm[t], sm[t + s]);
+    const auto block_sum = [&]() {
+        E2 x[V];
+#pragma unroll
+        for (int j = 0; j < V; j++) {
             __syncthreads();
+            sm[t] = v[j];
+            __syncthreads();
+            for (int s = BLK / 2; s >= n; s >>= 1) {
+                if (t < s) sm[t] = F::add(sm[t], sm[t + s]);
+                __syncthreads();
+            }
+            x[j] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
         }
-        if (t < n) sm[t] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
+        __syncthreads();
+        if (t < n) {
+#pragma unroll
+            for (int j = 0; j < V; j++) sm[j * n + t] = x[j];
+        }
         __syncthreads();
     };
     // writes sm to row `row`, takes a ticket of `counter`; true in the block that takes the last of `of`
     const auto publish = [&](size_t row, unsigned* counter, unsigned of) {
         if (t < n) {
-            store2(partial + 2 * (row * n + t), sm[t].c0, sm[t].c1);
+#pragma unroll
+            for (int j = 0; j < V; j++) store2(partial + 2 * ((row * V + j) * n + t), sm[j * n + t].c0, sm[j * n + t].c1);
             __threadfence();
         }
         __syncthreads();
@@ -133,18 +144,25 @@ __device__ __forceinline__ bool grid_sum(typename F::E2 v, int bits, typename F:
     };
     const auto rows_sum = [&](size_t first, unsigned count) {
         __threadfence();
-        E2 x{0, 0};
+#pragma unroll
+        for (int j = 0; j < V; j++) v[j] = E2{0, 0};
 #pragma unroll 8
         for (unsigned b = t >> bits; b < count; b += BLK >> bits) {
-            const uint64_t* p = partial + 2 * ((first + b) * n + (t & (n - 1)));
-            x = F::add(x, E2{__ldcg(p), __ldcg(p + 1)});
+#pragma unroll
+            for (int j = 0; j < V; j++) {
+                const uint64_t* p = partial + 2 * (((first + b) * V + j) * n + (t & (n - 1)));
+                v[j] = F::add(v[j], E2{__ldcg(p), __ldcg(p + 1)});
+            }
         }
-        block_sum(x);
+        block_sum();
     };
-    block_sum(v);
+    block_sum();
     if (gridDim.x == 1) return true;
-    unsigned per = 8;   // rows per group
-    while (per * per < gridDim.x || (gridDim.x + per - 1) / per > GROUPS) per += 8;
+    unsigned per = 16 * (BLK >> bits);   // rows per group
+    if (gridDim.x > per) {
+        per = 8;
+        while (per * per < gridDim.x || (gridDim.x + per - 1) / per > GROUPS) per += 8;
+    }
     const unsigned groups = (gridDim.x + per - 1) / per, g = blockIdx.x / per;
     const unsigned members = (g + 1) * per <= gridDim.x ? per : gridDim.x - g * per;
     if (!publish(blockIdx.x, counters + 1 + g, members)) return false;
@@ -236,7 +254,7 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
         __syncthreads();
     }
     gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
-    E2 sum{0, 0};
+    E2 sum[1] = {E2{0, 0}};
     const int e = t & (E - 1), ei = (e >> GB) & ((1 << GB) - 1), ej = e & ((1 << GB) - 1), y0 = t >> (2 * GB);
     // without a fold the next tile's elements are loaded before this tile's products
     E2 na{0, 0}, nb{0, 0};
@@ -297,7 +315,7 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
                 // the row's WH when the row or the block's share ends
                 const size_t row = (tile * BLK) >> a.row_shift;
                 if (tile + 1 == end || ((tile + 1) * BLK) >> a.row_shift != row) {
-                    sum = F::fma(load_weight<F>(a.wh + 4 * (row & a.row_mask)), E2{F::redw(s0), F::redw(s1)}, sum);
+                    sum[0] = F::fma(load_weight<F>(a.wh + 4 * (row & a.row_mask)), E2{F::redw(s0), F::redw(s1)}, sum[0]);
                     s0 = gl::acc_zero();
                     s1 = gl::acc_zero();
                 }
@@ -305,8 +323,8 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
         }
     }
     if constexpr (GB > 0) {
-        if constexpr (!WEIGHTED) sum = E2{F::redw(s0), F::redw(s1)};
-        if (!grid_sum<F>(sum, 2 * GB, sa, a.partial + ((size_t)(4 * gridDim.x) << (2 * GB)) * k, a.counter + (GROUPS + 1) * k)) return;
+        if constexpr (!WEIGHTED) sum[0] = E2{F::redw(s0), F::redw(s1)};
+        if (!grid_sum<F, 1>(sum, 2 * GB, sa, a.partial + ((size_t)(4 * gridDim.x) << (2 * GB)) * k, a.counter + (GROUPS + 1) * k)) return;
         if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), sa[t].c0, sa[t].c1);
     }
 }

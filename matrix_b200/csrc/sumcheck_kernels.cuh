@@ -112,44 +112,105 @@ struct Lazy<GlExt2> {
     static __device__ __forceinline__ gl::E2 reduce(const A& s) { return gl::e2acc_reduce(s); }
 };
 
-// Round polynomial of a product of two tables from three exact sums. With a = value at 0, b = value at 1 and
-// d = b - a per table, P(c) = S0 + c S1 + c^2 S2 where S0 = sum a0 a1 = P(0), S2 = sum d0 d1 and
-// P(1) = sum b0 b1, hence P(2) = 2 P(1) - S0 + 2 S2. The three sums take one multiply-accumulate chain each per
-// pair and are reduced once per LAZY_MAX pairs, instead of three reduced products, three modular additions and
-// two rounds of value updates per pair.
+// The same with the non-residue multiplied into the second factor first, for kernels that keep several sums in registers:
+// two sums per extension element instead of three, and any number of products.
 template <class F>
-struct PairSums {
+struct NarrowLazy;
+struct NarrowSum {
+    gl::Acc s0, s1;
+};
+template <>
+struct NarrowLazy<GlBase> {
+    using A = gl::Acc;
+    static __device__ __forceinline__ A zero() { return gl::acc_zero(); }
+    static __device__ __forceinline__ void mul(A& s, uint64_t x, uint64_t y) { gl::acc_mul(s, x, y); }
+    static __device__ __forceinline__ uint64_t reduce(const A& s) { return gl::acc_reduce_wide(s); }
+};
+template <>
+struct NarrowLazy<GlExt2> {
+    using A = NarrowSum;
+    static __device__ __forceinline__ A zero() { return A{gl::acc_zero(), gl::acc_zero()}; }
+    static __device__ __forceinline__ void mul(A& s, gl::E2 x, gl::E2 y) {
+        gl::acc_mul(s.s0, x.c0, y.c0);
+        gl::acc_mul(s.s0, x.c1, gl::mul_small(y.c1, 7));
+        gl::acc_mul(s.s1, x.c0, y.c1);
+        gl::acc_mul(s.s1, x.c1, y.c0);
+    }
+    static __device__ __forceinline__ gl::E2 reduce(const A& s) {
+        return gl::E2{gl::acc_reduce_wide(s.s0), gl::acc_reduce_wide(s.s1)};
+    }
+};
+
+// Round polynomial of a product of D tables from D + 1 exact sums, one multiply-accumulate chain each per pair, reduced
+// once at the end. Written a at 0, b at 1 and b - a as the leading coefficient (the value at infinity), the
+// product of two tables takes three products (at 0, 1, infinity), and its other values are small combinations:
+//   q(-1) = 2 q(0) + 2 q(inf) - q(1),   q(2) = 2 q(1) + 2 q(inf) - q(0).
+//   D = 2: sums at 0, 1, infinity            D = 3: q times the third table at 0, 1, -1, infinity
+//   D = 4: q times the other two's product at 0, 1, -1, 2, infinity
+// Evaluating at 0 .. D takes (D + 1)(D - 1) reduced products and as many sums instead: eight against three reduced and
+// four accumulated for D = 3 (2^22 almost-Goldilocks extension elements, first round: 168 -> 102 us), fifteen against six and five for D = 4.
+template <class F, int D>
+struct RoundSums {
+    static_assert(D >= 2 && D <= 4, "see accumulate_pair for other counts");
     using T = typename F::T;
-    typename Lazy<F>::A s0, s1, s2;
-    T t0, t1, t2;
-    int pending;
+    using Sum = NarrowLazy<F>;
+    typename Sum::A s[D + 1];
+    static __device__ __forceinline__ T twice(T x) { return F::add(x, x); }
     __device__ __forceinline__ void init() {
-        s0 = Lazy<F>::zero(); s1 = Lazy<F>::zero(); s2 = Lazy<F>::zero();
-        t0 = F::zero(); t1 = F::zero(); t2 = F::zero();
-        pending = 0;
+#pragma unroll
+        for (int c = 0; c <= D; c++) s[c] = Sum::zero();
     }
-    __device__ __forceinline__ void flush() {
-        t0 = F::add(t0, Lazy<F>::reduce(s0));
-        t1 = F::add(t1, Lazy<F>::reduce(s1));
-        t2 = F::add(t2, Lazy<F>::reduce(s2));
-        s0 = Lazy<F>::zero(); s1 = Lazy<F>::zero(); s2 = Lazy<F>::zero();
-        pending = 0;
+    // lo, hi: the tables' values at 0 and 1
+    __device__ __forceinline__ void add_pair(const T (&lo)[D], const T (&hi)[D]) {
+        if constexpr (D == 2) {
+            Sum::mul(s[0], lo[0], lo[1]);
+            Sum::mul(s[1], hi[0], hi[1]);
+            Sum::mul(s[2], F::sub(hi[0], lo[0]), F::sub(hi[1], lo[1]));
+        } else {
+            const T q0 = F::mul(lo[0], lo[1]), q1 = F::mul(hi[0], hi[1]);
+            const T qi = F::mul(F::sub(hi[0], lo[0]), F::sub(hi[1], lo[1]));
+            if constexpr (D == 3) {
+                Sum::mul(s[0], q0, lo[2]);
+                Sum::mul(s[1], q1, hi[2]);
+                Sum::mul(s[2], F::sub(twice(F::add(q0, qi)), q1), F::sub(twice(lo[2]), hi[2]));
+                Sum::mul(s[3], qi, F::sub(hi[2], lo[2]));
+            } else {
+                const T u0 = F::mul(lo[2], lo[3]), u1 = F::mul(hi[2], hi[3]);
+                const T ui = F::mul(F::sub(hi[2], lo[2]), F::sub(hi[3], lo[3]));
+                Sum::mul(s[0], q0, u0);
+                Sum::mul(s[1], q1, u1);
+                Sum::mul(s[2], F::sub(twice(F::add(q0, qi)), q1), F::sub(twice(F::add(u0, ui)), u1));
+                Sum::mul(s[3], F::sub(twice(F::add(q1, qi)), q0), F::sub(twice(F::add(u1, ui)), u0));
+                Sum::mul(s[4], qi, ui);
+            }
+        }
     }
-    // a_i, b_i: the two tables' values at 0 and 1
-    __device__ __forceinline__ void add_pair(T a0, T b0, T a1, T b1) {
-        Lazy<F>::mul(s0, a0, a1);
-        Lazy<F>::mul(s1, b0, b1);
-        Lazy<F>::mul(s2, F::sub(b0, a0), F::sub(b1, a1));
-        if (++pending == LAZY_MAX) flush();
+    // acc[c] = this thread's share of P(c), c = 0 .. D; the values beyond the sums by differences of order D, which are
+    // D! times the leading coefficient
+    __device__ __forceinline__ void finish(T (&acc)[D + 1]) {
+        T total[D + 1];
+#pragma unroll
+        for (int c = 0; c <= D; c++) total[c] = Sum::reduce(s[c]);
+        acc[0] = total[0];
+        acc[1] = total[1];
+        if constexpr (D == 2) {
+            acc[2] = F::sub(twice(F::add(total[1], total[2])), total[0]);
+        } else if constexpr (D == 3) {
+            const T c6 = twice(thrice(total[3]));
+            acc[2] = F::add(F::add(thrice(F::sub(total[1], total[0])), total[2]), c6);
+            acc[3] = F::add(F::add(thrice(F::sub(acc[2], total[1])), total[0]), c6);
+        } else {
+            const T c24 = twice(twice(twice(thrice(total[4]))));
+            acc[2] = total[3];
+            acc[3] = F::add(F::sub(step4(acc[2], acc[1], acc[0]), total[2]), c24);
+            acc[4] = F::add(F::sub(step4(acc[3], acc[2], acc[1]), acc[0]), c24);
+        }
     }
-    // acc[0..2] = this thread's share of P(0), P(1), P(2)
-    __device__ __forceinline__ void finish(T (&acc)[3]) {
-        flush();
-        acc[0] = t0;
-        acc[1] = t1;
-        T twice = F::add(F::add(t1, t1), F::add(t2, t2));
-        acc[2] = F::sub(twice, t0);
-    }
+
+private:
+    static __device__ __forceinline__ T thrice(T x) { return F::add(twice(x), x); }
+    // 4 x - 6 y + 4 z
+    static __device__ __forceinline__ T step4(T x, T y, T z) { return F::sub(twice(twice(F::add(x, z))), twice(thrice(y))); }
 };
 
 // ---- block-wide sum of NV residues per thread -------------------------------
@@ -239,22 +300,22 @@ __device__ __forceinline__ void store_partials(typename F::T (&acc)[D + 1], uint
 // ---- round message ----------------------------------------------------------
 // partial[(blockIdx.x * (D+1) + c) * NW ...] = this block's share of P(c).
 template <class F, int D>
-__global__ void __launch_bounds__(D == 2 ? 512 : D == 3 ? 1024 : 256)   // D = 2 keeps exact sums in registers
+__global__ void __launch_bounds__(D == 2 ? 512 : 256, D == 3 || D == 4 ? 2 : 1)   // exact sums in registers for D = 2, 3, 4
 round_message_kernel(const uint64_t* __restrict__ polys, size_t stride, size_t half, uint64_t* __restrict__ partial,
                      unsigned int* counter, uint64_t* final_out) {
     using T = typename F::T;
     T acc[D + 1];
     const size_t step = (size_t)gridDim.x * blockDim.x;
-    if constexpr (D == 2) {
-        PairSums<F> ps;
-        ps.init();
+    if constexpr (D >= 2 && D <= 4) {
+        RoundSums<F, D> sums;
+        sums.init();
         for (size_t y = (size_t)blockIdx.x * blockDim.x + threadIdx.x; y < half; y += step) {
-            T a0, b0, a1, b1;
-            F::load2(polys, 2 * y, a0, b0);
-            F::load2(polys + stride * F::NW, 2 * y, a1, b1);
-            ps.add_pair(a0, b0, a1, b1);
+            T lo[D], hi[D];
+#pragma unroll
+            for (int i = 0; i < D; i++) F::load2(polys + (size_t)i * stride * F::NW, 2 * y, lo[i], hi[i]);
+            sums.add_pair(lo, hi);
         }
-        ps.finish(acc);
+        sums.finish(acc);
     } else {
 #pragma unroll
         for (int c = 0; c <= D; c++) acc[c] = F::zero();
@@ -319,7 +380,7 @@ struct FoldOp<GlExt2, GlExt2> {
 };
 
 template <class FIn, class FOut, int D>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, D == 3 || D == 4 ? 2 : 1)
 fold_message_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, typename FOut::T r_val,
                     const uint64_t* __restrict__ r_ptr, size_t stride_in, size_t stride_out, size_t quarter,
                     uint64_t* __restrict__ partial, unsigned int* counter, uint64_t* final_out) {
@@ -329,24 +390,24 @@ fold_message_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
     if (r_ptr != nullptr) r = FOut::load(r_ptr, 0);
     TO acc[D + 1];
     const size_t step = (size_t)gridDim.x * blockDim.x;
-    if constexpr (D == 2) {
-        PairSums<FOut> ps;
-        ps.init();
+    if constexpr (D >= 2 && D <= 4) {
+        RoundSums<FOut, D> sums;
+        sums.init();
         for (size_t y = (size_t)blockIdx.x * blockDim.x + threadIdx.x; y < quarter; y += step) {
-            TO f[2][2];
+            TO lo[D], hi[D];
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < D; i++) {
                 TI e0, e1, e2, e3;
                 const uint64_t* pin = in + (size_t)i * stride_in * FIn::NW;
                 FIn::load2(pin, 4 * y, e0, e1);
                 FIn::load2(pin, 4 * y + 2, e2, e3);
-                f[i][0] = FoldOp<FIn, FOut>::apply(e0, e1, r);
-                f[i][1] = FoldOp<FIn, FOut>::apply(e2, e3, r);
-                FOut::store2(out + (size_t)i * stride_out * FOut::NW, 2 * y, f[i][0], f[i][1]);
+                lo[i] = FoldOp<FIn, FOut>::apply(e0, e1, r);
+                hi[i] = FoldOp<FIn, FOut>::apply(e2, e3, r);
+                FOut::store2(out + (size_t)i * stride_out * FOut::NW, 2 * y, lo[i], hi[i]);
             }
-            ps.add_pair(f[0][0], f[0][1], f[1][0], f[1][1]);
+            sums.add_pair(lo, hi);
         }
-        ps.finish(acc);
+        sums.finish(acc);
     } else {
 #pragma unroll
         for (int c = 0; c <= D; c++) acc[c] = FOut::zero();
