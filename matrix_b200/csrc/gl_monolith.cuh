@@ -7,13 +7,15 @@
 //   bricks   s_i += s_{i-1}^2 for i = 11 down to 1
 //   concrete circulant MDS (first row 7 23 8 26 13 10 9 7 6 22 21 8) + constants
 //
-// The concrete layer is formed on 32-bit halves: every output is
-// sum_j m_j lo(s_j) + 2^32 sum_j m_j hi(s_j) with integer weights (row sum 160,
-// so with the constant's halves both sums stay below 161 * 2^32 < 2^40), one
-// mad.wide.u32 per term and one reduction per output instead of twelve modular
-// multiply-adds. Values are loose in [0, 2^64) between layers; words 0..3 are
-// made canonical before the bars (the S-box acts on the canonical bit pattern),
-// and the caller canonicalises what it stores.
+// The concrete layer is formed on three limbs of 22, 22 and 20 bits: the weights' row sum is 160, so the sums of a limb
+// stay below 2^30 and 32-bit arithmetic is exact. The circulant is split over Z[x] / (x^12 - 1) = (x^6 + 1)(x^3 + 1)(x^3 - 1):
+//   out_i = P_i + M_i, out_{i+6} = P_i - M_i   (i < 6; P of s_j + s_{j+6}, M of s_j - s_{j+6})
+//   P_i = A_i + B_i, P_{i+3} = A_i - B_i       (i < 3, the same once more)
+// with the halves moved into the weights, which all become powers of two: M -1 8 1 2 -4 1 (negacyclic), A 16 16 8,
+// B -8 -1 -1 (negacyclic). That is 84 additions and shift-additions a limb where the circulant on 32-bit halves took
+// 288 multiply-adds with 64-bit results, which cost the multiply pipe two to three times as much each
+// (2^19 compressions: 96 -> 61 us). Values are loose in [0, 2^64) between layers; words 0..3 are made canonical before the
+// bars (the S-box acts on the canonical bit pattern), and the caller canonicalises what it stores.
 #pragma once
 #include "gl_field.cuh"
 
@@ -65,31 +67,69 @@ GLF uint32_t mono_bar32(uint32_t x) {
 }
 GLF uint64_t mono_bar(uint64_t x) { return pack64(mono_bar32(lo32(x)), mono_bar32(hi32(x))); }
 
+// o = circulant times x, modulo 2^32.
+GLF void mono_circulant(const uint32_t (&x)[MONO_W], uint32_t (&o)[MONO_W]) {
+    uint32_t p[6], m[6], u[3], v[3], A[3], B[3], M[6];
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+        p[j] = x[j] + x[j + 6];
+        m[j] = x[j] - x[j + 6];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        u[j] = p[j] + p[j + 3];
+        v[j] = p[j] - p[j + 3];
+    }
+    const uint32_t sum16 = (u[0] + u[1] + u[2]) << 4;
+#pragma unroll
+    for (int i = 0; i < 3; i++) A[i] = sum16 - (u[(i + 2) % 3] << 3);
+    B[0] = 0u - v[1] - v[2] - (v[0] << 3);
+    B[1] = v[0] - v[2] - (v[1] << 3);
+    B[2] = v[0] + v[1] - (v[2] << 3);
+    M[0] = m[2] + m[5] - m[0] + (m[1] << 3) + (m[3] << 1) - (m[4] << 2);
+    M[1] = m[3] - m[0] - m[1] + (m[2] << 3) + (m[4] << 1) - (m[5] << 2);
+    M[2] = m[4] - m[1] - m[2] + (m[3] << 3) + (m[5] << 1) + (m[0] << 2);
+    M[3] = m[5] - m[2] - m[3] + (m[4] << 3) - (m[0] << 1) + (m[1] << 2);
+    M[4] = 0u - m[0] - m[3] - m[4] + (m[5] << 3) - (m[1] << 1) + (m[2] << 2);
+    M[5] = 0u - m[1] - m[4] - m[5] - (m[0] << 3) - (m[2] << 1) + (m[3] << 2);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const uint32_t lo = A[i] + B[i], hi = A[i] - B[i];
+        o[i] = lo + M[i];
+        o[i + 6] = lo - M[i];
+        o[i + 3] = hi + M[i + 3];
+        o[i + 9] = hi - M[i + 3];
+    }
+}
+
 // MDS times state plus the constants of `round` (`HAS_RC` false: zero constants).
 template <bool HAS_RC>
 GLF void mono_concrete(uint64_t* s, int round) {
-    constexpr uint32_t C[MONO_W] = {7, 23, 8, 26, 13, 10, 9, 7, 6, 22, 21, 8};
-    uint32_t lo[MONO_W], hi[MONO_W];
+    constexpr uint32_t MASK = (1u << 22) - 1;
+    uint32_t x[MONO_W], o[MONO_W], top[MONO_W];
+    uint64_t low[MONO_W];
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) x[j] = lo32(s[j]) & MASK;
+    mono_circulant(x, o);
 #pragma unroll
     for (int j = 0; j < MONO_W; j++) {
-        lo[j] = lo32(s[j]);
-        hi[j] = hi32(s[j]);
+        low[j] = o[j];
+        x[j] = (uint32_t)(s[j] >> 22) & MASK;
+        top[j] = hi32(s[j]) >> 12;
     }
+    mono_circulant(x, o);
 #pragma unroll
-    for (int i = 0; i < MONO_W; i++) {
-        uint64_t L = 0, H = 0;
-        if (HAS_RC) {
-            uint64_t rc = mono_rc(round, i);
-            L = lo32(rc);
-            H = hi32(rc);
-        }
+    for (int j = 0; j < MONO_W; j++) low[j] = madwide(o[j], 1u << 22, low[j]);
+    mono_circulant(top, o);
 #pragma unroll
-        for (int j = 0; j < MONO_W; j++) {
-            const uint32_t m = C[(j - i + MONO_W) % MONO_W];
-            L = madwide(lo[j], m, L);
-            H = madwide(hi[j], m, H);
+    for (int j = 0; j < MONO_W; j++) {
+        uint64_t H = (uint64_t)o[j] << 12;
+        if (HAS_RC) {   // the constant's halves: both sums stay below 2^54
+            const uint64_t rc = mono_rc(round, j);
+            low[j] += lo32(rc);
+            H += hi32(rc);
         }
-        s[i] = reduce_limb_sums(L, H);
+        s[j] = reduce_limb_sums(low[j], H);
     }
 }
 
