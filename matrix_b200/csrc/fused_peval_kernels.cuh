@@ -236,7 +236,10 @@ inline int launch(const uint64_t* d_evals, uint64_t* d_output, const uint64_t* d
             return MB_ERR_CUDA;
         // every lane takes at least 16 terms when there are that many: the lanes of a warp then read
         // neighbouring sectors of the same term instead of one far-apart sector per term
-        const int log_tq = m <= 4 ? 0 : (m - 4 < 5 ? m - 4 : 5);
+        int log_tq = m <= 4 ? 0 : (m - 4 < 5 ? m - 4 : 5);
+        // fewer terms a lane while the outputs do not fill the chip: a lane's terms are a chain of memory latencies
+        // (4096 outputs of 2^7 terms: 22 -> 11 us)
+        while (log_tq < 5 && log_tq < m && (((size_t)output_size >> 2) << log_tq) < (size_t)sm_count() * 256) log_tq++;
         int grid = grid_for(((size_t)output_size >> 2) << log_tq, 256, per_sm < 4 ? per_sm : 4);
         // 16-byte loads of the inputs need a 16-byte aligned table
         const bool aligned = (reinterpret_cast<uintptr_t>(d_evals) & 15) == 0;

@@ -5,14 +5,12 @@
 // cuda_almost_goldilocks/almost_partial_eval.cuh:22-180, one launch and one full
 // pass per variable). Here m variables take ceil(m / 4) passes and the traffic is
 // about N (1 + 2^-4) instead of about 3 N.
-//  * The first pass over a base-field table (the large one) is an inner product:
-//    out[j] = sum_b in[16 j + b] w_b with the 16 weights eq(r[0..4), b) held in
-//    registers, accumulated as exact 160-bit sums and reduced once per output
-//    (two multiply-accumulate chains per element instead of a reduced fold per
-//    level). A block stages 4096 consecutive elements in shared memory with
-//    coalesced 16-byte loads; each thread then reads its run of 16 from a padded
-//    layout without bank conflicts.
-//  * Other passes (extension tables, at most 1/16 of the data) fold a run of 2^K
+//  * The first pass over a base-field table (the large one) is an inner product with the eq vector of the variables it
+//    binds, as exact 160-bit sums (two multiply-accumulate chains per element instead of a reduced fold per level):
+//    six or more variables by warps that stream whole rows (dot_rows_kernel), fewer with the 2^K weights in shared
+//    memory (dot_levels_kernel: a block stages 4096 consecutive elements with coalesced 16-byte loads; each thread
+//    then reads its run of 2^K from a padded layout without bank conflicts).
+//  * Other passes (extension tables, what the first left) fold a run of 2^K
 //    consecutive elements through K variables in registers.
 #pragma once
 #include "sumcheck_kernels.cuh"
@@ -106,6 +104,117 @@ dot_levels_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, c
     }
 }
 
+// First pass over a base-field table: m >= 6 variables at once. Element b of a row weighs WL[b mod 64] WH[b / 64]: a lane
+// keeps elements 2 lane, 2 lane + 1 of every 64, sums them times WH (the same for the whole warp) and applies its two
+// entries of WL once at the end, so an element costs two multiply-accumulates whatever m is, and nothing between the
+// row and its output goes through memory. 2^parts_log warps of a block share a row. Bound by those products (28 us for
+// 2^24 elements) and by the latency of the loads (2^24 elements, m = 12: 55 us at the profiler's clock, where passes of
+// four variables took 43 + 11 + 8 and two more launches).
+template <class FIn, class FOut>
+__global__ void __launch_bounds__(256)
+dot_rows_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, const uint64_t* __restrict__ r, int lvl, int m,
+                int parts_log, size_t n_out) {
+    using TO = typename FOut::T;
+    using Sum = sc::NarrowLazy<FIn>;
+    extern __shared__ uint64_t wh[];   // [2^(m - 6)][2]
+    __shared__ uint64_t part_sm[8][2];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, hi_n = 1 << (m - 6), parts = 1 << parts_log;
+    if (t == 0) FOut::to_words(TO{1, 0}, wh);
+    __syncthreads();
+    for (int k = 0; k < m - 6; k++) {
+        const TO rk = FOut::load(r, lvl + 6 + k);
+        for (int j = t; j < (1 << k); j += 256) {
+            const TO w = FOut::from_words(wh + 2 * j), hi = FOut::mul(w, rk);
+            FOut::to_words(FOut::sub(w, hi), wh + 2 * j);
+            FOut::to_words(hi, wh + 2 * (j + (1 << k)));
+        }
+        __syncthreads();
+    }
+    TO wl0{1, 0};
+#pragma unroll
+    for (int k = 1; k < 6; k++) {
+        const TO rk = FOut::load(r, lvl + k), hi = FOut::mul(wl0, rk);
+        wl0 = (lane >> (k - 1)) & 1 ? hi : FOut::sub(wl0, hi);
+    }
+    const TO wl1 = FOut::mul(wl0, FOut::load(r, lvl));
+    wl0 = FOut::sub(wl0, wl1);
+    const int rows = 8 >> parts_log, part = warp & (parts - 1);
+    for (size_t row0 = (size_t)blockIdx.x * rows; row0 < n_out; row0 += (size_t)gridDim.x * rows) {
+        const size_t row = row0 + (warp >> parts_log);   // rows divides n_out
+        const uint64_t* src = in + (row << m) + 2 * lane;
+        typename Sum::A e0 = Sum::zero(), e1 = Sum::zero(), o0 = Sum::zero(), o1 = Sum::zero();
+        // the next four loads are in flight while four are used
+        const int count = hi_n >> parts_log;
+        const auto index = [&](int k) { return part + ((k & (count - 1)) << parts_log); };   // wraps where there are fewer than four
+        ulonglong2 next[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) next[u] = *reinterpret_cast<const ulonglong2*>(src + 64 * (size_t)index(u));
+        for (int k = 0; k < count; k += 4) {
+            ulonglong2 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = next[u];
+            if (k + 4 < count) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) next[u] = *reinterpret_cast<const ulonglong2*>(src + 64 * (size_t)index(k + 4 + u));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (k + u >= count) break;
+                const int i = index(k + u);
+                const uint64_t w0 = wh[2 * i], w1 = wh[2 * i + 1];
+                Sum::mul(e0, x[u].x, w0);
+                Sum::mul(e1, x[u].x, w1);
+                Sum::mul(o0, x[u].y, w0);
+                Sum::mul(o1, x[u].y, w1);
+            }
+        }
+        TO v = FOut::add(FOut::mul(TO{Sum::reduce(e0), Sum::reduce(e1)}, wl0), FOut::mul(TO{Sum::reduce(o0), Sum::reduce(o1)}, wl1));
+        uint64_t w[2];
+        FOut::to_words(v, w);
+        const typename FOut::WordAdd wadd;
+#pragma unroll
+        for (int off = 16; off; off >>= 1) {
+            w[0] = wadd(w[0], __shfl_xor_sync(0xffffffffu, w[0], off));
+            w[1] = wadd(w[1], __shfl_xor_sync(0xffffffffu, w[1], off));
+        }
+        if (parts_log == 0) {
+            if (lane == 0) FOut::store(out, row, FOut::from_words(w));
+            continue;
+        }
+        if (lane == 0) {
+            part_sm[warp][0] = w[0];
+            part_sm[warp][1] = w[1];
+        }
+        __syncthreads();
+        if (lane == 0 && part == 0) {
+            for (int q = 1; q < parts; q++) {
+                w[0] = wadd(w[0], part_sm[warp + q][0]);
+                w[1] = wadd(w[1], part_sm[warp + q][1]);
+            }
+            FOut::store(out, row, FOut::from_words(w));
+        }
+        __syncthreads();
+    }
+}
+// Variables the first pass binds: all of them unless that leaves fewer than 2^9 rows of a table for which more warps are
+// wanted (eight of them share a row at most); at most 14, so that a block's WH stays a few KB.
+inline int dot_rows_vars(int log_n, int m) {
+    int k = log_n - 9 > 9 ? log_n - 9 : 9;
+    if (k > 14) k = 14;
+    return m < k ? m : k;
+}
+template <class FIn, class FOut>
+inline void launch_dot_rows(const uint64_t* in, uint64_t* out, const uint64_t* r, int lvl, int k, size_t n_out, cudaStream_t st) {
+    // eight warps an SM sub-core until the rows alone give them, as long as a warp keeps an iteration
+    int parts_log = 0;
+    while (parts_log < 3 && (n_out << parts_log) < 4096 && parts_log < k - 6) parts_log++;
+    const size_t blocks = (n_out << parts_log) / 8;   // a table of 2^9 elements or more has at least one block's worth
+    const size_t cap = (size_t)sm_count() * 8;
+    MB_KERNEL_ON("partial_eval_rows", st);
+    dot_rows_kernel<FIn, FOut><<<(unsigned)(blocks < cap ? blocks : cap), 256, sizeof(uint64_t) * ((size_t)2 << (k - 6)), st>>>(
+        in, out, r, lvl, k, parts_log, n_out);
+}
+
 template <class FIn, class FOut>
 inline void launch_dot(const uint64_t* in, uint64_t* out, const uint64_t* r, int lvl, int k, size_t n_out, cudaStream_t st) {
     int grid = grid_for(n_out, 256, 4);
@@ -139,7 +248,11 @@ inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, 
                         cudaStream_t st) {
     if (log_n < 0 || log_n > 40 || m < 0 || m > log_n || !d_in || !d_out || (m > 0 && !d_r)) return MB_ERR_ARG;
     if (m == 0) return MB_OK;
-    int passes = (m + K_MAX - 1) / K_MAX;
+    // dot_rows_kernel reads pairs of elements, and eight warps of 64 elements or more make a block
+    int first_vars = 0;
+    if constexpr (FIn::NW == 1 && FOut::NW == 2)
+        if (m >= 6 && log_n >= 9 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) first_vars = dot_rows_vars(log_n, m);
+    int passes = first_vars ? 1 + (m - first_vars + K_MAX - 1) / K_MAX : (m + K_MAX - 1) / K_MAX;
     if (passes > 1 && !d_tmp) return MB_ERR_ARG;
     // ping-pong so that the last pass lands in d_out
     uint64_t* bufs[2] = {d_out, d_tmp};
@@ -148,12 +261,15 @@ inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, 
     int lvl = 0, left = m, cur_log = log_n;
     bool first = true;
     while (left > 0) {
-        int k = left < K_MAX ? left : K_MAX;
+        int k = first && first_vars ? first_vars : left < K_MAX ? left : K_MAX;
         size_t n_out = (size_t)1 << (cur_log - k);
         uint64_t* dst = bufs[which];
         bool done = false;
         if constexpr (FIn::NW == 1 && FOut::NW == 2) {
-            if (first && n_out >= 256) {
+            if (first && first_vars) {
+                launch_dot_rows<FIn, FOut>(src, dst, d_r, lvl, k, n_out, st);
+                done = true;
+            } else if (first && n_out >= 256) {
                 launch_dot<FIn, FOut>(src, dst, d_r, lvl, k, n_out, st);
                 done = true;
             }
