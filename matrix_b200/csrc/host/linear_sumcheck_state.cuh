@@ -79,7 +79,7 @@ public:
         if (d == 2 && num_vars > 0 && aligned16(d_tables)) {
             pair_.reset(new typename PairOf<typename Ext::T>::type);
             const size_t words = n_ * (base_field ? 1 : 2);
-            return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0);
+            return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0, true);
         }
         products_ = Product::handles(d) && aligned16(d_tables) && num_vars > 0;
         if (products_ && num_vars <= Product::limit(d)) {

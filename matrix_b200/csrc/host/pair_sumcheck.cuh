@@ -90,8 +90,11 @@ public:
         pool_free(counter_);
     }
     // a, b: instance 0's device tables of 2^n elements (never written), instances inst_stride words apart; base: base
-    // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. Queues the first pass.
-    int init(const uint64_t* a, const uint64_t* b, size_t inst_stride, int K, int n, bool base, const uint64_t* eq_pt, int eq_vars) {
+    // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. together: b follows a in one allocation
+    // (addresses alone do not say so: two allocations may touch). Queues the first pass.
+    int init(const uint64_t* a, const uint64_t* b, size_t inst_stride, int K, int n, bool base, const uint64_t* eq_pt, int eq_vars,
+             bool together = false) {
+        together_ = together;
         a_ = a; b_ = b; stride_ = inst_stride; K_ = K; n_ = n; base_ = base;
         pt_.resize(eq_vars);
         for (int i = 0; i < eq_vars; i++) pt_[i] = H::canon(E2{eq_pt[2 * i], eq_pt[2 * i + 1]});
@@ -317,7 +320,7 @@ private:
         const size_t w = tn_ * (base_ ? 1 : 2);
         if (2 * w * K_ > PinnedPool::WORDS) return MB_ERR_UNSUPPORTED;
         pending_ = true;
-        if (K_ == 1 && b_ == a_ + w) {
+        if (together_) {
             MB_CUDA(cudaMemcpyAsync(pin_, a_, 16 * w, cudaMemcpyDeviceToHost, MB_STREAM));
             return MB_OK;
         }
@@ -459,7 +462,7 @@ private:
     const uint64_t *a_ = nullptr, *b_ = nullptr;
     size_t stride_ = 0;
     int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0;
-    bool base_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
+    bool base_ = false, together_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;
     std::vector<E2> pt_, r_, scale_, m_, w_, ta_, tb_;

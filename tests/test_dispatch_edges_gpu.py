@@ -1,0 +1,118 @@
+"""The sizes at which a prover changes kernels: tables that go to the host, several rounds per pass, one round per pass,
+uneven last blocks; hashing layers around the switch between lanes and threads; column chunks of the tensor-core commit.
+Bit equality with the CPU oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from matrix_b200.ffi import DeviceBuffer, load_agl, load_gl
+from matrix_b200.inputs import AGL_Q, GL_P, field_elems, splitmix64
+from oracle import pyoracle
+
+from .test_agl_sumcheck_prover_gpu import _prove, _state, _transcript
+from .test_ajtai_gpu import KEY
+from .test_basefold_gpu import test_commit_open_matches_oracle as basefold_matches_oracle
+from .test_batched_gpu import test_whole_proof_inside_the_library as batched_matches_oracle
+from .test_monolith_gpu import test_commit_open_with_monolith_trees as monolith_basefold_matches_oracle
+from .test_sumcheck_gpu import test_whole_proof_matches_oracle as gl_sumcheck_matches_oracle
+
+pytestmark = pytest.mark.gpu
+
+# one table: host up to 2^8, then four rounds a pass; two: host up to 2^10 (base) or 2^9, blocks of 4, 3, 2 rounds; three:
+# passes from 2^9 to 2^16, a round a pass above; four: to 2^13
+ROUNDS = [(1, 8), (1, 9), (1, 13), (1, 17), (2, 1), (2, 9), (2, 10), (2, 11), (2, 18), (2, 19), (3, 8), (3, 9), (3, 14), (3, 15),
+          (3, 16), (3, 17), (3, 18), (4, 8), (4, 10), (4, 13), (4, 14), (4, 16)]
+
+
+@pytest.fixture(scope="module")
+def gl():
+    lib = load_gl()
+    assert lib.goldilocks_cuda_init() == 0
+    assert lib.monolith_cuda_init() == 0
+    return lib
+
+
+@pytest.mark.parametrize("d,nv", ROUNDS)
+@pytest.mark.parametrize("base", [True, False])
+def test_sumcheck_rounds_agl(d, nv, base):
+    lib = load_agl()
+    raw = splitmix64(900 + 100 * d + nv, (d << nv) * (1 if base else 2))   # words at or above q among them
+    raw[:3] = [AGL_Q, 2**64 - 1, AGL_Q - 1][:len(raw[:3])]
+    want = pyoracle.agl_sumcheck_prove(raw, d, nv, base, b"edges")
+    h = _transcript(lib, b"edges")
+    got = _prove(lib, raw, d, nv, base, h)
+    for g, w in zip(got + (_state(lib, h),), want):
+        assert np.array_equal(g, np.array(w, dtype=np.uint64))
+    lib.agl_transcript_destroy(h)
+
+
+@pytest.mark.parametrize("d,nv", ROUNDS)
+@pytest.mark.parametrize("base", [True, False])
+def test_sumcheck_rounds_gl(gl, d, nv, base):
+    gl_sumcheck_matches_oracle(gl, nv, d, base)
+
+
+@pytest.mark.parametrize("K,nv", [(1, 9), (2, 9), (3, 10), (4, 12), (7, 13), (64, 4), (64, 11), (1, 18), (5, 17)])
+def test_batched_rounds(K, nv):
+    batched_matches_oracle(K, nv, 0)
+
+
+@pytest.mark.parametrize("nv,lr,nq", [(2, 2, 1), (2, 3, 2), (5, 2, 3), (8, 3, 7), (9, 0, 4), (11, 1, 8), (12, 2, 8), (14, 1, 8), (15, 2, 8)])
+def test_basefold_sizes(gl, nv, lr, nq):
+    basefold_matches_oracle(gl, nv, lr, nq)
+    monolith_basefold_matches_oracle(gl, nv, lr, nq)
+
+
+def test_poseidon2_with_a_missed_carry(gl, oracle):
+    """The throughput form adds without the rare carry and borrow repairs and redoes a permutation that needed one. The
+    first round constant makes lane 0 of this state 2^48 before its S-box, whose square is a power of two that does;
+    the extreme residues come along."""
+    states = field_elems(77, 8 * 64)
+    states[0] = (2**48 - 0xdd5743e7f2a5a5d9) % GL_P
+    states[1:8] = 0
+    states[8:16] = GL_P - 1
+    states[16:24] = 2**32 - 1
+    d_in, d_out = DeviceBuffer.from_numpy(gl, states), DeviceBuffer(gl, states.nbytes)
+    assert gl.poseidon2_hash_batch_ffi(d_in.ptr, d_out.ptr, 64) == 0
+    got = d_out.to_numpy().reshape(64, 8)
+    for k in range(64):
+        s = (ctypes.c_uint64 * 8)(*[int(x) for x in states[8 * k:8 * k + 8]])
+        oracle.gl_poseidon2_permute(s)
+        assert list(got[k]) == list(s), k
+
+
+@pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15)])
+def test_partial_evaluation_rows(oracle, gl, log_n, m):
+    for lib, mod, fn, ofn in ((load_agl(), AGL_Q, load_agl().agl_partial_eval_ext2_from_base_ffi, oracle.oracle_agl_partial_eval_ext2_from_base),
+                              (gl, GL_P, gl.partial_eval_ext2_from_gl_ffi, oracle.oracle_gl_partial_eval_ext2_from_base)):
+        data, r = field_elems(40 + log_n, 1 << log_n, mod), field_elems(41 + m, 2 * m, mod)
+        d_in, d_r, d_out = DeviceBuffer.from_numpy(lib, data), DeviceBuffer.from_numpy(lib, r), DeviceBuffer(lib, 8 << log_n)
+        assert fn(d_in.ptr, d_out.ptr, d_r.ptr, log_n, m) == 0
+        exp = np.zeros(2 << (log_n - m), dtype=np.uint64)
+        ofn(data.ctypes.data, exp.ctypes.data, r.ctypes.data, log_n, m)
+        assert np.array_equal(d_out.to_numpy()[:len(exp)], exp)
+
+
+@pytest.mark.parametrize("n,planes", [(3, 2), (8, 1), (9, 4), (49 * 8, 3), (49 * 8 + 1, 2), (1999, 4), (25088, 1), (25089, 3)])
+def test_tensor_core_commit_chunks(n, planes):
+    """One wave of chunks, its last column, the first of the next; stages on both digit groups, odd counts of stages."""
+    lib = load_agl()
+    rng = np.random.default_rng(n + planes)
+    dig = rng.integers(-127, 128, size=planes * n * 64, dtype=np.int8)
+    dig[:64], dig[-64:] = 127, -127
+    d_k, d_z, d_t = DeviceBuffer.from_numpy(lib, KEY), DeviceBuffer.from_numpy(lib, dig), DeviceBuffer(lib, lib.ajtai_tc_matrix_bytes(n))
+    d_a, d_b, d_s = (DeviceBuffer(lib, planes * 42 * 64 * 8) for _ in range(3))
+    assert lib.ajtai_materialize_tc_ffi(d_k.ptr, d_t.ptr, n, 0) == 0
+    assert lib.ajtai_commit_s8_tiled_ffi(d_t.ptr, d_z.ptr, n, planes, d_a.ptr) == 0
+    assert lib.ajtai_commit_s8_ffi(d_k.ptr, d_z.ptr, n, planes, 0, d_b.ptr) == 0
+    if n < 500:
+        want = pyoracle.ajtai_commit(KEY, dig, 1, n, planes)
+    else:   # the scalar kernel, which has its own comparison with the oracle
+        assert lib.ajtai_commit_s8_scalar_ffi(d_k.ptr, d_z.ptr, n, planes, 0, d_s.ptr) == 0
+        want = d_s.to_numpy()
+    assert np.array_equal(d_a.to_numpy(), want) and np.array_equal(d_b.to_numpy(), want)
+    dig[(planes * n - 1) * 64 + 63] = -128   # the last digit of the last pair
+    d_z = DeviceBuffer.from_numpy(lib, dig)
+    assert lib.ajtai_commit_s8_tiled_ffi(d_t.ptr, d_z.ptr, n, planes, d_a.ptr) == -3
+    assert lib.ajtai_commit_s8_ffi(d_k.ptr, d_z.ptr, n, planes, 0, d_b.ptr) == -3
