@@ -312,20 +312,18 @@ def run_batched(args):
     kernels = prof_report(lib)
     elems = 2 * K * (1 << nv)  # field elements of the 2K witness tables (eq is derived, not counted)
     peak, peak_kind = measured_peaks()
-    # algorithmic bytes of the dominant pass (fold of round 0 fused with message 1): read 8 B, write 8 B per element
+    # algorithmic bytes of the passes: the base tables once for the first block of rounds and once for its fold, then every
+    # folded table (16 B an element, a quarter of the one before) written once and read once
     roofline = None
-    if "batched_fold_message" in kernels:
-        cnt, kms = kernels["batched_fold_message"]
-        # per step and rank: round 0 fold reads 2K*m*8 + eq m*16, writes (2K+1)*m/2*16; later rounds halve: read S, write S/2
-        first = 2 * K * m * 8 + m * 16 + (2 * K + 1) * (m // 2) * 16
-        later = sum((2 * K + 1) * (m >> r) * 16 * 1.5 for r in range(1, n_loc - 1))
-        total_bytes = (first + later) * psteps
+    if "pair_pass" in kernels:
+        cnt, kms = kernels["pair_pass"]
+        total_bytes = (2 * 2 * K * m * 8 + 2 * sum(2 * K * (m >> (2 * r)) * 16 for r in range(1, n_loc // 2 + 1))) * psteps
         ach = total_bytes / (kms * 1e-3) / 1e9
-        roofline = {"kernel": "batched_fold_message", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+        roofline = {"kernel": "pair_pass", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                     "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "launches": cnt,
                     "avg_launch_ms": kms / cnt,
                     "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % psteps,
-                    "note": "per rank; all rounds' fold+message launches together"}
+                    "note": "per rank; all passes together (two or more rounds each, taken as two); bound by the integer pipes"}
     kernel_ms = sum(x for _, x in kernels.values()) / psteps
     how = {"mailbox": "round loop inside the library; host mailbox in POSIX shared memory",
            "nccl": "Python round loop; NCCL all-gather", "shm": "Python round loop; mailbox file in /dev/shm"}[args.exchange]
@@ -1334,10 +1332,10 @@ def run_basefold(args):
     leaves_folded = sum((cw_len >> (i + 2)) for i in range(nv - 1)) // world
     nodes_per_step = leaves_commit + sum(max((cw_len >> (i + 2)) - 1, 0) for i in range(nv - 1)) // world
     roofline = None
-    hash_ms = sum(kernels.get(k, (0, 0))[1] for k in ("hash_leaves", "compress_layer", "tree_tail", "compress_layer_coop",
-                                                       "hash_leaves_coop"))
+    prefix = "" if args.hash == "poseidon2" else "monolith_"
+    hash_ms = sum(kernels.get(k, (0, 0))[1] for k in (prefix + "hash_leaves", prefix + "compress_layer", "tree_up"))
     perms_per_s = (leaves_commit + leaves_folded + nodes_per_step) * prof_steps / (hash_ms * 1e-3) if hash_ms else 0.0
-    inst_per_perm = 15550.0 if args.hash == "poseidon2" else 6900.0  # thread instructions per permutation (ncu)
+    inst_per_perm = 5442.0 if args.hash == "poseidon2" else 2715.0  # thread instructions per permutation (ncu)
     sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
     if dom is not None:
         cnt, ms = kernels[dom]
@@ -1371,8 +1369,8 @@ def run_basefold(args):
                                   "achieved_warp_inst_per_s": perms_per_s * inst_per_perm / 32.0,
                                   "peak_warp_inst_per_s": 148 * 4 * sm_hz,
                                   "frac": perms_per_s * inst_per_perm / 32.0 / (148 * 4 * sm_hz),
-                                  "note": "integer additions, logic and multiply-adds share one 16-lane datapath per "
-                                          "scheduler: 0.57 of the issue slots is the measured ceiling for this mix"}}
+                                  "note": "two 16-lane pipes per scheduler take a warp instruction every two cycles each, wide "
+                                          "multiply-adds two or three of those: a mix with many of them cannot fill the slots"}}
     line = {
         "metric": METRIC if args.hash == "poseidon2" else METRIC.replace("Poseidon2 Merkle", "Monolith Merkle"),
         "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

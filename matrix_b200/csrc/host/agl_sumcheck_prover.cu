@@ -34,13 +34,6 @@ static Ext2 aext2_mul_host(Ext2 a, Ext2 b) {
 static Ext2 aext2_add_host(Ext2 a, Ext2 b) {
     return Ext2{agl::canon(agl::add(a.c0, b.c0)), agl::canon(agl::add(a.c1, b.c1))};
 }
-static Ext2 aext2_sub_host(Ext2 a, Ext2 b) {
-    return Ext2{agl::canon(agl::sub(a.c0, b.c0)), agl::canon(agl::sub(a.c1, b.c1))};
-}
-static Ext2 aext2_inv_host(Ext2 a) {
-    agl::E2 r = agl::e2_canon(agl::e2_inv(agl::E2{a.c0, a.c1}));
-    return Ext2{r.c0, r.c1};
-}
 static Ext2 challenge_ext2(AglTranscript& t) {
     uint64_t w[2];
     t.challenge_vector(L_CHALLENGE, sizeof(L_CHALLENGE) - 1, w, 2);  // label once, two squeezes (transcript.rs:120-125)

@@ -447,24 +447,5 @@ __global__ void fold_lift_kernel(const uint64_t* __restrict__ in, uint64_t* __re
     }
 }
 
-// Sum `nblocks` block partials of NV words each into out[0..NV): one block.
-template <int BLOCKDIM, class AddFn, class CanonFn>
-__global__ void reduce_partials_kernel(const uint64_t* __restrict__ partial, int nblocks, int nv,
-                                       uint64_t* __restrict__ out) {
-    __shared__ uint64_t sm[BLOCKDIM];
-    for (int k = 0; k < nv; k++) {
-        uint64_t s = 0;
-        for (int b = threadIdx.x; b < nblocks; b += BLOCKDIM) s = AddFn()(s, partial[(size_t)b * nv + k]);
-        sm[threadIdx.x] = s;
-        __syncthreads();
-        for (int off = BLOCKDIM / 2; off > 0; off >>= 1) {
-            if (threadIdx.x < off) sm[threadIdx.x] = AddFn()(sm[threadIdx.x], sm[threadIdx.x + off]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[k] = CanonFn()(sm[0]);
-        __syncthreads();
-    }
-}
-
 }  // namespace sc
 }  // namespace mb
