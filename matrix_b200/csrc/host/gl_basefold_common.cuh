@@ -458,6 +458,16 @@ inline std::atomic<int> g_merkle_hash{0};
 // ---- BasefoldCommitment -----------------------------------------------------------------
 class BasefoldCommitment {
 public:
+    // The caller's evaluations when they came from the host: kept as long as the commitment, because a hole freed between a
+    // commitment and its opening makes the memory pool remap its blocks (2^24: 40 to 80 ms every few calls instead of 30).
+    DevBuf d_host_evals;
+    // A commitment and its opening: evaluations three times, the codeword with its tree, every folded codeword and tree
+    // (6 words per codeword element), and some for the small pieces.
+    static void reserve(int nv, int lr) {
+        if (nv < 1 || lr < 0 || nv + lr > 32) return;
+        const size_t n = (size_t)1 << nv, cw = (size_t)1 << (nv + lr);
+        pool_reserve(sizeof(uint64_t) * (3 * n + 11 * cw + ((size_t)1 << 18)));
+    }
     // commit_device (basefold.rs:382-414): interpolate, encode, Merkle tree.
     int commit_device(const uint64_t* d_evals, int nv, int lr) {
         if (nv < 1 || lr < 0 || nv + lr > 32 || !d_evals) return MB_ERR_ARG;

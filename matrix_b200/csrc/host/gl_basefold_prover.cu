@@ -181,6 +181,7 @@ const uint64_t* basefold_table_level_ptr(const void* table, int level) {
 
 int basefold_commit_device(const uint64_t* d_evals, int num_vars, int log_rate, void** commitment, uint64_t* h_root) {
     if (!commitment) return MB_ERR_ARG;
+    BasefoldCommitment::reserve(num_vars, log_rate);
     auto* c = new BasefoldCommitment;
     int rc = c->commit_device(d_evals, num_vars, log_rate);
     if (rc != MB_OK) { delete c; return rc; }
@@ -189,12 +190,17 @@ int basefold_commit_device(const uint64_t* d_evals, int num_vars, int log_rate, 
     return MB_OK;
 }
 int basefold_commit_host(const uint64_t* h_evals, int num_vars, int log_rate, void** commitment, uint64_t* h_root) {
-    if (num_vars < 1 || num_vars > 32 || !h_evals) return MB_ERR_ARG;
-    mbhost::DevBuf ev;
-    int rc = ev.alloc((size_t)1 << num_vars);
-    if (rc != MB_OK) return rc;
-    MB_CUDA(cudaMemcpyAsync(ev.p, h_evals, sizeof(uint64_t) << num_vars, cudaMemcpyHostToDevice, MB_STREAM));
-    return basefold_commit_device(ev.p, num_vars, log_rate, commitment, h_root);
+    if (num_vars < 1 || num_vars > 32 || !h_evals || !commitment) return MB_ERR_ARG;
+    BasefoldCommitment::reserve(num_vars, log_rate);
+    auto* c = new BasefoldCommitment;
+    int rc = c->d_host_evals.alloc((size_t)1 << num_vars);
+    if (rc == MB_OK && cudaMemcpyAsync(c->d_host_evals.p, h_evals, sizeof(uint64_t) << num_vars, cudaMemcpyHostToDevice, MB_STREAM) != cudaSuccess)
+        rc = MB_ERR_CUDA;
+    if (rc == MB_OK) rc = c->commit_device(c->d_host_evals.p, num_vars, log_rate);
+    if (rc != MB_OK) { delete c; return rc; }
+    if (h_root) std::memcpy(h_root, c->root, 32);
+    *commitment = c;
+    return MB_OK;
 }
 int basefold_commitment_destroy(void* commitment) { delete static_cast<BasefoldCommitment*>(commitment); return MB_OK; }
 // Device pointers of the commitment's parts (owned by the commitment).
