@@ -179,7 +179,10 @@ public:
         s2 = H::sub(H::add(s0, s1), cross);
         return MB_OK;
     }
+    // Stands on its own: the round's sums need not have been asked for.
     int fold(E2 r) {
+        int rc = wait();   // the rounds may be the host's by now
+        if (rc != MB_OK) return rc;
         const int round = round_++;
         r_[round] = r;
         if (round < (int)pt_.size()) {
@@ -192,6 +195,7 @@ public:
             block_++;
             return pass();
         }
+        if (m_.empty()) combine();
         const int half = side_ / 2;   // rows, then columns
         for (int i = 0; i < half; i++)
             for (int j = 0; j < side_; j++) at(i, j) = H::fold(at(2 * i, j), at(2 * i + 1, j), r);
