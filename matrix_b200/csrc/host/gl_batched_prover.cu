@@ -49,16 +49,14 @@ public:
         int rc = pair_.init(d_a, d_b, (size_t)1 << n_loc, K, n_loc, true, h_point_low, n_loc);
         return rc == MB_OK ? finish_call() : rc;
     }
-    // Local share of the per-instance claims sum_x eq a_k b_k (K extension elements).
+    // Local share of the per-instance claims sum_x eq a_k b_k (K extension elements), whatever round the state is in: they
+    // are read off the first pass, which the folds overwrite, so the first fold keeps them.
     int claims(uint64_t* h_out) {
-        std::vector<E2> c(K_);
-        if (round_ != 0) return MB_ERR_ARG;
-        int rc = pair_.claims(c.data());
+        int rc = keep_claims();
         if (rc != MB_OK) return rc;
         for (int k = 0; k < K_; k++) {
-            c[k] = H::mul(c[k], shard_);
-            h_out[2 * k] = c[k].c0;
-            h_out[2 * k + 1] = c[k].c1;
+            h_out[2 * k] = claims_[k].c0;
+            h_out[2 * k + 1] = claims_[k].c1;
         }
         return MB_OK;
     }
@@ -94,8 +92,10 @@ public:
     }
     int fold(Ext2 ch) {
         if (alphas_.empty() || round_ >= n_loc_) return MB_ERR_ARG;
+        int rc = round_ == 0 ? keep_claims() : MB_OK;
+        if (rc != MB_OK) return rc;
         round_++;
-        int rc = pair_.fold(H::canon(E2{ch.c0, ch.c1}));
+        rc = pair_.fold(H::canon(E2{ch.c0, ch.c1}));
         return rc == MB_OK ? finish_call() : rc;
     }
     // After n_loc folds: eq (with the shard's factor), a_k, b_k: (2K + 1) extension elements; scaled: alpha^k a_k.
@@ -114,6 +114,15 @@ public:
     }
 
 private:
+    int keep_claims() {
+        if (!claims_.empty()) return MB_OK;
+        std::vector<E2> c(K_);
+        int rc = pair_.claims(c.data());
+        if (rc != MB_OK) return rc;
+        for (E2& v : c) v = H::mul(v, shard_);
+        claims_.swap(c);
+        return MB_OK;
+    }
     int finish_call() {
         if (threads_) MB_CUDA(cudaStreamSynchronize(MB_STREAM));
         return MB_OK;
@@ -121,7 +130,7 @@ private:
     int K_ = 0, n_loc_ = 0, round_ = 0;
     bool threads_ = false;
     E2 shard_{1, 0};
-    std::vector<E2> alphas_;
+    std::vector<E2> alphas_, claims_;
     Pair pair_;
 };
 

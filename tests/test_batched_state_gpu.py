@@ -1,5 +1,5 @@
-"""The batched sumcheck's state handle driven call by call: a fold without the round's message. Messages, claims and
-finals against the oracle's proof, whose challenges the handle is given."""
+"""The batched sumcheck's state handle driven call by call: a fold without the round's message, claims asked for late. Messages,
+claims and finals against the oracle's proof, whose challenges the handle is given."""
 import numpy as np
 import pytest
 
@@ -56,4 +56,20 @@ def test_fold_without_message(lib, K, nv, asked):
         if {"none": False, "last": rnd == nv - 1, "even": rnd % 2 == 0, "odd": rnd % 2 == 1, "thirds": rnd % 3 == 1}[asked]:
             d.check_message(rnd)
         d.fold(rnd)
+    d.check_finals()
+
+
+@pytest.mark.parametrize("K,nv", [(1, 1), (1, 9), (16, 12), (3, 17)])
+@pytest.mark.parametrize("asked_at", ["after the first fold", "after the last fold", "before and after"])
+def test_claims_after_a_fold(lib, K, nv, asked_at):
+    d = Driven(lib, K, nv)
+    want = d.proof["claims"].reshape(-1)
+    if asked_at == "before and after":
+        assert np.array_equal(d.shard.claims(), want)
+    d.shard.set_alpha(d.alpha)
+    for rnd in range(nv):
+        d.fold(rnd)
+        if rnd == 0 and asked_at != "after the last fold":
+            assert np.array_equal(d.shard.claims(), want)
+    assert np.array_equal(d.shard.claims(), want)
     d.check_finals()
