@@ -20,11 +20,13 @@ constexpr uint64_t GL_EPS = 0xFFFFFFFFULL;   // 2^64 mod p
 // carry by + EPS (the wrapped value is below hi_lo EPS < 2^64 - 2^33).
 static inline uint64_t gl_red(u128 x) {
 #if defined(__x86_64__)
-    // seven micro-operations: hi_lo (2^32 - 1) is one multiplication, the borrow (once in 2^32 random words) a jump
+    // seven micro-operations: hi_lo (2^32 - 1) is one multiplication, the borrow (once in 2^32 random words) a jump.
+    // Early-clobber operands: the constant is read after they are written, so one that the compiler knows to hold the same
+    // value must not share its register (here and in agl_red).
     uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64), t;
     asm("mov %k[hi], %k[t]\n\timul %[eps], %[t]\n\tshr $32, %[hi]\n\tsub %[hi], %[lo]\n\tjb 2f\n1:\tadd %[t], %[lo]\n\t"
         "sbb %k[t], %k[t]\n\tadd %[t], %[lo]\n\t.subsection 1\n2:\tsub %[eps], %[lo]\n\tjmp 1b\n\t.previous"
-        : [lo] "+r"(lo), [hi] "+r"(hi), [t] "=&r"(t) : [eps] "r"(GL_EPS) : "cc");
+        : [lo] "+&r"(lo), [hi] "+&r"(hi), [t] "=&r"(t) : [eps] "r"(GL_EPS) : "cc");
     return lo;
 #else
     const uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64);
@@ -66,7 +68,7 @@ static inline uint64_t agl_red(u128 x) {
     uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64), a = hi;
     asm("mul %[c]\n\tadd %%rax, %[lo]\n\tadc $0, %%rdx\n\tmov %%rdx, %%rax\n\tmul %[c]\n\tadd %%rax, %[lo]\n\tadc $0, %%rdx\n\t"
         "imul %[c], %%rdx\n\tadd %%rdx, %[lo]\n\tjc 2f\n1:\n\t.subsection 1\n2:\tadd %[c], %[lo]\n\tjmp 1b\n\t.previous"
-        : [lo] "+r"(lo), "+a"(a), "=&d"(hi) : [c] "r"(AGL_C) : "cc");
+        : [lo] "+&r"(lo), "+&a"(a), "=&d"(hi) : [c] "r"(AGL_C) : "cc");
     return lo;
 #else
     x = (u128)(uint64_t)(x >> 64) * AGL_C + (uint64_t)x;

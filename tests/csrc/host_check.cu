@@ -77,6 +77,15 @@ void hc_hf_e2(int agl_field, const uint64_t* a, const uint64_t* b, uint64_t* o) 
         o[4] = gl_sub(a[0], b[0]); o[5] = gl_sub(a[1], b[1]);
     }
 }
+// the reductions with one word known to the compiler: o = red(C : x), red(x : C) and red(C : C) for C = 2^64 mod p
+void hc_hf_red_constant(int agl_field, uint64_t x, uint64_t* o) {
+    using namespace mbhost::hf;
+    if (agl_field) {
+        o[0] = agl_red(((u128)AGL_C << 64) | x); o[1] = agl_red(((u128)x << 64) | AGL_C); o[2] = agl_red(((u128)AGL_C << 64) | AGL_C);
+    } else {
+        o[0] = gl_red(((u128)GL_EPS << 64) | x); o[1] = gl_red(((u128)x << 64) | GL_EPS); o[2] = gl_red(((u128)GL_EPS << 64) | GL_EPS);
+    }
+}
 void hc_aglm_circulant12(const int64_t* x, int64_t* out) { mbhost::hf::circulant12(x, out); }
 uint64_t hc_p2host_red(uint64_t lo, uint64_t hi) { return mbhost::p2host::red(((unsigned __int128)hi << 64) | lo); }
 uint64_t hc_aglm_reduce_wide(uint64_t lo, uint64_t hi) { return mbhost::aglm::reduce_wide(((unsigned __int128)hi << 64) | lo); }

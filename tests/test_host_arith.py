@@ -138,6 +138,18 @@ def test_host_form_extension_arithmetic(hostcheck):
             assert (o[4], o[5]) == ((a0 - b0) % q, (a1 - b1) % q)
 
 
+def test_host_reductions_of_known_words(hostcheck):
+    """A high or low word that the compiler knows, equal to the constant the reduction multiplies by: the assembly must
+    not be given one register for both."""
+    rnd = random.Random(29)
+    for agl_field, q in ((0, P), (1, 2**64 - 2**32 - 31)):
+        c = 2**64 - q
+        for x in [0, 1, c - 1, c, c + 1, q - 1, q, 2**64 - 1] + [rnd.randrange(2**64) for _ in range(200)]:
+            o = (u64 * 3)()
+            hostcheck.hc_hf_red_constant(agl_field, u64(x), o)
+            assert [w % q for w in o] == [((c << 64) + x) % q, ((x << 64) + c) % q, ((c << 64) + c) % q], (agl_field, x)
+
+
 def test_transcript_matches_oracle(hostcheck, oracle):
     # Random scripts of absorbs and squeezes against the oracle's transcript.
     class T(ctypes.Structure):
