@@ -196,12 +196,18 @@ dot_rows_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, con
         __syncthreads();
     }
 }
-// Variables the first pass binds: all of them unless that leaves fewer than 2^9 rows of a table for which more warps are
-// wanted (eight of them share a row at most); at most 14, so that a block's WH stays a few KB.
+// Variables the first pass binds by rows: all of them unless that leaves fewer than 2^9 rows of a table for which more warps
+// are wanted (eight of them share a row at most); at most 14, so that a block's WH stays a few KB. 0: not by rows. A row costs
+// the chip about 0.6 ns at its end (five shuffles of two words, two products) whatever its length, so many short rows are
+// left to dot_levels_kernel and the passes behind it. Measured, Goldilocks, us by passes of four / by rows: 2^24 elements, m = 6
+// (2^18 rows) 65 / 222, m = 9 70 / 78, m = 10 (2^14 rows) 70 / 70, m = 11 72 / 65; 2^21, m = 7 30 / 41, m = 9 (2^12 rows)
+// 35 / 30; 2^19, m = 7 (2^12 rows) 27 / 26 (almost-Goldilocks 27 / 29), m = 8 28 / 27: rows of 2^10 elements and more, at most
+// 2^12 rows of 2^8 or 2^9, at most 2^11 shorter ones.
 inline int dot_rows_vars(int log_n, int m) {
     int k = log_n - 9 > 9 ? log_n - 9 : 9;
     if (k > 14) k = 14;
-    return m < k ? m : k;
+    if (m < k) k = m;
+    return k >= 10 || log_n - k <= (k >= 8 ? 12 : 11) ? k : 0;
 }
 template <class FIn, class FOut>
 inline void launch_dot_rows(const uint64_t* in, uint64_t* out, const uint64_t* r, int lvl, int k, size_t n_out, cudaStream_t st) {

@@ -94,6 +94,28 @@ def test_partial_evaluation_rows(oracle, gl, log_n, m):
         assert np.array_equal(d_out.to_numpy()[:len(exp)], exp)
 
 
+# rows of 2^10 elements, at most 2^12 of 2^8 or 2^9, or at most 2^11 shorter ones go by rows; many short rows took up to four times as
+# long that way (2^24, m = 6)
+@pytest.mark.parametrize("log_n,m,rows", [(8, 6, False), (9, 6, True), (17, 6, True), (18, 6, False), (18, 7, True), (19, 7, False),
+                                          (20, 8, True), (21, 8, False), (21, 9, True), (22, 9, False), (22, 10, True)])
+def test_partial_evaluation_route(oracle, gl, log_n, m, rows):
+    for lib, mod, fn, ofn in ((load_agl(), AGL_Q, load_agl().agl_partial_eval_ext2_from_base_ffi, oracle.oracle_agl_partial_eval_ext2_from_base),
+                              (gl, GL_P, gl.partial_eval_ext2_from_gl_ffi, oracle.oracle_gl_partial_eval_ext2_from_base)):
+        data, r = field_elems(60 + log_n, 1 << log_n, mod), field_elems(61 + m, 2 * m, mod)
+        d_in, d_r, d_out = DeviceBuffer.from_numpy(lib, data), DeviceBuffer.from_numpy(lib, r), DeviceBuffer(lib, 8 << log_n)
+        buf = ctypes.create_string_buffer(4096)
+        lib.mb_prof_enable(1)
+        lib.mb_prof_reset()
+        rc = fn(d_in.ptr, d_out.ptr, d_r.ptr, log_n, m)
+        lib.mb_prof_report(buf, len(buf))
+        lib.mb_prof_enable(0)
+        assert rc == 0
+        assert ("partial_eval_rows" in buf.value.decode()) == rows
+        exp = np.zeros(2 << (log_n - m), dtype=np.uint64)
+        ofn(data.ctypes.data, exp.ctypes.data, r.ctypes.data, log_n, m)
+        assert np.array_equal(d_out.to_numpy()[:len(exp)], exp)
+
+
 @pytest.mark.parametrize("n,planes", [(3, 2), (8, 1), (9, 4), (49 * 8, 3), (49 * 8 + 1, 2), (1999, 4), (25088, 1), (25089, 3)])
 def test_tensor_core_commit_chunks(n, planes):
     """One wave of chunks, its last column, the first of the next; stages on both digit groups, odd counts of stages."""
