@@ -30,6 +30,21 @@ inline int threads_for(size_t items, int num_blocks) {
         default: return MB_ERR_ARG;       \
     }
 
+// The kernel for a grid of num_blocks blocks (sumcheck_kernels.cuh, blocks_resident).
+template <class F, int D>
+auto round_message_for(int num_blocks) {
+    if constexpr (D == 8)
+        if (num_blocks > sm_count()) return round_message_kernel<F, D, 2>;
+    return round_message_kernel<F, D, blocks_resident(D)>;
+}
+template <class FIn, class FOut, int D>
+auto fold_message_for(int num_blocks) {
+    if constexpr (D == 8) return fold_message_kernel<FIn, FOut, D, 2>;
+    if constexpr (D == 7)
+        if (num_blocks > sm_count()) return fold_message_kernel<FIn, FOut, D, 2>;
+    return fold_message_kernel<FIn, FOut, D, blocks_resident(D)>;
+}
+
 // Writes num_blocks * (d+1) partial sums; the caller adds them up (as the
 // reference's GpuSumcheckState does on the host,
 // goldilocks-cuda-rs/src/sumcheck_prover.rs:109-121).
@@ -46,8 +61,8 @@ int launch_round_message(const uint64_t* d_polys, uint64_t* d_partial, int d, si
     const int bound = d == 2 ? 512 : 256;
     if (threads > bound) threads = bound;
     MB_KERNEL_ON("sumcheck_round_message", st);
-    MB_DISPATCH_D(d, (round_message_kernel<F, D><<<num_blocks, threads, 0, st>>>(d_polys, stride, half, d_partial,
-                                                                                     d_counter, d_final)));
+    MB_DISPATCH_D(d, (round_message_for<F, D>(num_blocks)<<<num_blocks, threads, 0, st>>>(d_polys, stride, half, d_partial,
+                                                                                          d_counter, d_final)));
     return finish_async();
 }
 
@@ -75,7 +90,7 @@ int launch_fold_message(const uint64_t* d_in, uint64_t* d_out, typename FOut::T 
     if (!aligned16(d_in) || !aligned16(d_out) || ((stride_in * FIn::NW) & 1) || ((stride_out * FOut::NW) & 1))
         return MB_ERR_ARG;
     MB_KERNEL_ON("sumcheck_fold_message", st);
-    MB_DISPATCH_D(d, (fold_message_kernel<FIn, FOut, D><<<num_blocks, BLOCK, 0, st>>>(
+    MB_DISPATCH_D(d, (fold_message_for<FIn, FOut, D>(num_blocks)<<<num_blocks, BLOCK, 0, st>>>(
                          d_in, d_out, r, d_r, stride_in, stride_out, quarter, d_partial, d_counter, d_final)));
     return finish_async();
 }

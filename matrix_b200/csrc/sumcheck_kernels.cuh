@@ -297,10 +297,17 @@ __device__ __forceinline__ void store_partials(typename F::T (&acc)[D + 1], uint
     if (threadIdx.x == 0) *counter = 0;
 }
 
+// Blocks per SM that the two kernels below keep registers for (RES). The exact sums of three and four tables want two. With
+// seven and eight tables one block takes all 255 registers, which is faster while the grid has at most a block per SM; two
+// blocks at 128, with some spills, are where it has more, and for the fold of eight tables, which spills either way. Measured,
+// Goldilocks extension tables of 2^20, us at RES = 1 / 2: round message of eight, 148 blocks 231 / 340, 592 blocks 287 / 247;
+// fold and message of seven (base tables) 119 / 147 and 161 / 133, of eight (extension) 315 / 283 and 349 / 214.
+constexpr int blocks_resident(int d) { return d == 3 || d == 4 ? 2 : 1; }
+
 // ---- round message ----------------------------------------------------------
 // partial[(blockIdx.x * (D+1) + c) * NW ...] = this block's share of P(c).
-template <class F, int D>
-__global__ void __launch_bounds__(D == 2 ? 512 : 256, D == 3 || D == 4 ? 2 : 1)   // exact sums in registers for D = 2, 3, 4
+template <class F, int D, int RES>
+__global__ void __launch_bounds__(D == 2 ? 512 : 256, RES)   // exact sums in registers for D = 2, 3, 4
 round_message_kernel(const uint64_t* __restrict__ polys, size_t stride, size_t half, uint64_t* __restrict__ partial,
                      unsigned int* counter, uint64_t* final_out) {
     using T = typename F::T;
@@ -379,8 +386,8 @@ struct FoldOp<GlExt2, GlExt2> {
     }
 };
 
-template <class FIn, class FOut, int D>
-__global__ void __launch_bounds__(BLOCK, D == 3 || D == 4 ? 2 : 1)
+template <class FIn, class FOut, int D, int RES>
+__global__ void __launch_bounds__(BLOCK, RES)
 fold_message_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, typename FOut::T r_val,
                     const uint64_t* __restrict__ r_ptr, size_t stride_in, size_t stride_out, size_t quarter,
                     uint64_t* __restrict__ partial, unsigned int* counter, uint64_t* final_out) {

@@ -53,6 +53,28 @@ def test_sumcheck_rounds_gl(gl, d, nv, base):
     gl_sumcheck_matches_oracle(gl, nv, d, base)
 
 
+@pytest.mark.parametrize("d", [6, 7, 8])
+@pytest.mark.parametrize("blocks", [1, 148, 149, 600])   # a block per SM, and more
+def test_many_tables(gl, oracle, d, blocks):
+    n = 1 << 15
+    tabs, r = field_elems(950 + d, 2 * n * d), [2**63 + 11, 5]
+    d_in, d_out, d_part = DeviceBuffer.from_numpy(gl, tabs), DeviceBuffer(gl, tabs.nbytes), DeviceBuffer(gl, blocks * (d + 1) * 16)
+
+    def totals():
+        return [sum(int(x) for x in col) % GL_P for col in d_part.to_numpy().reshape(blocks, -1).T]
+
+    want, folded = np.zeros(2 * (d + 1), dtype=np.uint64), tabs.copy()
+    oracle.oracle_gl_round_message_ext2(tabs.ctypes.data, d, n, n // 2, want.ctypes.data)
+    assert gl.sumcheck_round_message_ext2_ffi(d_in.ptr, d_part.ptr, d, n, n // 2, blocks) == 0
+    assert totals() == [int(x) for x in want]
+    oracle.oracle_gl_fold_ext2(tabs.ctypes.data, folded.ctypes.data, *r, d, n, n // 2)
+    oracle.oracle_gl_round_message_ext2(folded.ctypes.data, d, n, n // 4, want.ctypes.data)
+    assert gl.sumcheck_fold_round_ext2_ffi(d_in.ptr, d_out.ptr, *r, d, n, n // 4, d_part.ptr, blocks) == 0
+    assert totals() == [int(x) for x in want]
+    got = d_out.to_numpy().reshape(d, 2 * n)[:, :n]
+    assert np.array_equal(got, folded.reshape(d, 2 * n)[:, :n])
+
+
 @pytest.mark.parametrize("K,nv", [(1, 9), (2, 9), (3, 10), (4, 12), (7, 13), (64, 4), (64, 11), (1, 18), (5, 17)])
 def test_batched_rounds(K, nv):
     batched_matches_oracle(K, nv, 0)
