@@ -60,7 +60,9 @@ public:
         }
         return MB_OK;
     }
+    // Counts until the first fold, which combines the instances; later calls change nothing.
     int set_alpha(Ext2 alpha) {
+        if (round_ > 0) return MB_OK;
         alphas_.resize(K_);
         E2 p{1, 0};
         const E2 a = H::canon(E2{alpha.c0, alpha.c1});

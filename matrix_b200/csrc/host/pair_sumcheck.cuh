@@ -124,9 +124,11 @@ public:
         r_.resize(n);
         return pass();
     }
-    // The instances' factors (K = 1: not needed). sums() and fold() may be called from then on.
+    // The instances' factors (K = 1: not needed). sums() and fold() may be called from then on; before the first fold the
+    // factors may be replaced.
     int set_scale(const E2* s) {
         scale_.assign(s, s + K_);
+        m_.clear();
         return MB_OK;
     }
     // sum_x w(x) a_k(x) b_k(x) of every instance, before the first fold

@@ -1,4 +1,5 @@
-"""The batched sumcheck's state handle driven call by call: a fold without the round's message, claims asked for late. Messages,
+"""The batched sumcheck's state handle driven call by call: a fold without the round's message, claims asked for late,
+alpha set again. Messages,
 claims and finals against the oracle's proof, whose challenges the handle is given."""
 import numpy as np
 import pytest
@@ -72,4 +73,19 @@ def test_claims_after_a_fold(lib, K, nv, asked_at):
         if rnd == 0 and asked_at != "after the last fold":
             assert np.array_equal(d.shard.claims(), want)
     assert np.array_equal(d.shard.claims(), want)
+    d.check_finals()
+
+
+@pytest.mark.parametrize("K,nv", [(2, 1), (1, 9), (16, 6), (16, 12), (3, 17)])
+def test_alpha_set_again(lib, K, nv):
+    """Before the first fold the last value counts, also when a message has been formed with another one; after it the call
+    changes nothing."""
+    d = Driven(lib, K, nv)
+    d.shard.set_alpha((12345, 678))
+    d.shard.round_message()
+    d.shard.set_alpha(d.alpha)
+    for rnd in range(nv):
+        d.check_message(rnd)
+        d.fold(rnd)
+        d.shard.set_alpha((999 + rnd, 5))
     d.check_finals()
