@@ -77,17 +77,6 @@ inline void pool_free(void* p) {
     if (p) cudaFreeAsync(p, MB_STREAM);
 }
 
-// Makes the pool hold `bytes` in one piece before a sequence of allocations that takes about that much: pieces cut from
-// one free block join again when they are freed, while a large request that fits no free block makes the pool remap its
-// memory (10 ms to 1 s). Only a hint: nothing happens where there is not enough memory, nor for more than 32 GB, which
-// the caller may want to split otherwise.
-inline void pool_reserve(size_t bytes) {
-    if (bytes > (size_t)32 << 30) return;
-    void* p = nullptr;
-    if (pool_alloc(&p, bytes) == cudaSuccess) pool_free(p);
-    else cudaGetLastError();
-}
-
 // Small pinned host landing zone, one per host thread, for results that are
 // read back every round (round polynomials, roots).
 inline uint64_t* pinned_scratch() {

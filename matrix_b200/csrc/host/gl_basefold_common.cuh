@@ -458,27 +458,26 @@ inline std::atomic<int> g_merkle_hash{0};
 // ---- BasefoldCommitment -----------------------------------------------------------------
 class BasefoldCommitment {
 public:
-    // The caller's evaluations when they came from the host: kept as long as the commitment, because a hole freed between a
-    // commitment and its opening makes the memory pool remap its blocks (2^24: 40 to 80 ms every few calls instead of 30).
-    DevBuf d_host_evals;
-    // A commitment and its opening: evaluations three times, the codeword with its tree, every folded codeword and tree
-    // (6 words per codeword element), and some for the small pieces.
-    static void reserve(int nv, int lr) {
-        if (nv < 1 || lr < 0 || nv + lr > 32) return;
-        const size_t n = (size_t)1 << nv, cw = (size_t)1 << (nv + lr);
-        pool_reserve(sizeof(uint64_t) * (3 * n + 11 * cw + ((size_t)1 << 18)));
-    }
-    // commit_device (basefold.rs:382-414): interpolate, encode, Merkle tree.
-    int commit_device(const uint64_t* d_evals, int nv, int lr) {
-        if (nv < 1 || lr < 0 || nv + lr > 32 || !d_evals) return MB_ERR_ARG;
+    // What the commitment keeps. Before anything that is given back once it is made (uploaded evaluations, scratch): those
+    // leave no hole between it and what an opening takes. A large request that fits no free block makes the memory pool remap
+    // its memory; with the scratch first, 2^24 from host memory took 30 ms or 40 ms to 1 s by turns.
+    int allocate(int nv, int lr) {
+        if (nv < 1 || lr < 0 || nv + lr > 32) return MB_ERR_ARG;
         num_vars = nv; log_rate = lr;
+        const size_t cw_len = (size_t)1 << (nv + lr);
+        int rc = d_bh_evals.alloc((size_t)1 << nv);
+        if (rc == MB_OK) rc = d_codeword.alloc(cw_len);
+        if (rc == MB_OK) rc = d_tree.alloc(4 * (cw_len - 1));
+        return rc;
+    }
+    // commit_device (basefold.rs:382-414): interpolate, encode, Merkle tree. After allocate.
+    int commit_device(const uint64_t* d_evals) {
+        if (!d_evals) return MB_ERR_ARG;
+        const int nv = num_vars, lr = log_rate;
         hash = g_merkle_hash.load();
         size_t n = (size_t)1 << nv, cw_len = (size_t)1 << (nv + lr);
         DevBuf work;
         int rc = work.alloc(n);
-        if (rc == MB_OK) rc = d_bh_evals.alloc(n);
-        if (rc == MB_OK) rc = d_codeword.alloc(cw_len);
-        if (rc == MB_OK) rc = d_tree.alloc(4 * (cw_len - 1));
         if (rc != MB_OK) return rc;
         rc = bf::bit_reverse_async(d_evals, d_bh_evals.p, nv, MB_STREAM);
         if (rc == MB_OK) rc = bf::evals_to_codeword_async(d_evals, work.p, d_codeword.p, nv, lr, MB_STREAM);

@@ -140,6 +140,26 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     return MB_OK;
 }
 
+// Evaluations on the device, or in host memory.
+static int commit(const uint64_t* d_evals, const uint64_t* h_evals, int nv, int lr, void** commitment, uint64_t* h_root) {
+    if (!commitment || (!d_evals && !h_evals)) return MB_ERR_ARG;
+    auto c = std::make_unique<BasefoldCommitment>();
+    int rc = c->allocate(nv, lr);
+    if (rc != MB_OK) return rc;
+    DevBuf uploaded;
+    if (h_evals) {
+        rc = uploaded.alloc((size_t)1 << nv);
+        if (rc != MB_OK) return rc;
+        MB_CUDA(cudaMemcpyAsync(uploaded.p, h_evals, sizeof(uint64_t) << nv, cudaMemcpyHostToDevice, MB_STREAM));
+        d_evals = uploaded.p;
+    }
+    rc = c->commit_device(d_evals);
+    if (rc != MB_OK) return rc;
+    if (h_root) std::memcpy(h_root, c->root, 32);
+    *commitment = c.release();
+    return MB_OK;
+}
+
 }  // namespace mbhost
 
 // ---- C-ABI of the host layer -----------------------------------------------------------
@@ -180,27 +200,10 @@ const uint64_t* basefold_table_level_ptr(const void* table, int level) {
 }
 
 int basefold_commit_device(const uint64_t* d_evals, int num_vars, int log_rate, void** commitment, uint64_t* h_root) {
-    if (!commitment) return MB_ERR_ARG;
-    BasefoldCommitment::reserve(num_vars, log_rate);
-    auto* c = new BasefoldCommitment;
-    int rc = c->commit_device(d_evals, num_vars, log_rate);
-    if (rc != MB_OK) { delete c; return rc; }
-    if (h_root) std::memcpy(h_root, c->root, 32);
-    *commitment = c;
-    return MB_OK;
+    return mbhost::commit(d_evals, nullptr, num_vars, log_rate, commitment, h_root);
 }
 int basefold_commit_host(const uint64_t* h_evals, int num_vars, int log_rate, void** commitment, uint64_t* h_root) {
-    if (num_vars < 1 || num_vars > 32 || !h_evals || !commitment) return MB_ERR_ARG;
-    BasefoldCommitment::reserve(num_vars, log_rate);
-    auto* c = new BasefoldCommitment;
-    int rc = c->d_host_evals.alloc((size_t)1 << num_vars);
-    if (rc == MB_OK && cudaMemcpyAsync(c->d_host_evals.p, h_evals, sizeof(uint64_t) << num_vars, cudaMemcpyHostToDevice, MB_STREAM) != cudaSuccess)
-        rc = MB_ERR_CUDA;
-    if (rc == MB_OK) rc = c->commit_device(c->d_host_evals.p, num_vars, log_rate);
-    if (rc != MB_OK) { delete c; return rc; }
-    if (h_root) std::memcpy(h_root, c->root, 32);
-    *commitment = c;
-    return MB_OK;
+    return mbhost::commit(nullptr, h_evals, num_vars, log_rate, commitment, h_root);
 }
 int basefold_commitment_destroy(void* commitment) { delete static_cast<BasefoldCommitment*>(commitment); return MB_OK; }
 // Device pointers of the commitment's parts (owned by the commitment).

@@ -359,3 +359,35 @@ def test_reference_call_sequence_through_dropin_entry_points(lib, oracle):
     got = np.array([x for o in oracles for x in o] + [int(x) for r in roots for x in r] + [int(x) for x in d_fin.to_numpy()],
                    dtype=np.uint64)
     assert np.array_equal(got, exp[2:2 + len(got)])
+
+
+@pytest.mark.parametrize("source", ["device", "host"])
+def test_held_commitments_take_no_more_than_they_keep(lib, source):
+    """A commitment may never be opened: nothing is set aside for that. It keeps the evaluations and the codeword with its
+    tree, n + 5 2^(nv + lr) words, and needs n more (2 n from host memory) while it is made."""
+    from matrix_b200.ffi import load_agl
+    nv, lr, count = 20, 1, 6
+    evals = field_elems(31, 1 << nv)
+    d_evals = DeviceBuffer.from_numpy(lib, evals)
+
+    def used():
+        free, total = ctypes.c_size_t(), ctypes.c_size_t()
+        assert lib.cuda_mem_get_info(ctypes.byref(free), ctypes.byref(total)) == 0
+        return total.value - free.value
+
+    lib.mb_stream_sync()
+    assert load_agl().cuda_pool_trim(0) == 0   # the memory pool of both libraries
+    before, handles = used(), []
+    for _ in range(count):
+        h = ctypes.c_void_p()
+        if source == "device":
+            assert lib.basefold_commit_device(d_evals.ptr, nv, lr, ctypes.byref(h), None) == 0
+        else:
+            assert lib.basefold_commit_host(evals.ctypes.data, nv, lr, ctypes.byref(h), None) == 0
+        handles.append(h)
+    grown = used() - before
+    for h in handles:
+        lib.basefold_commitment_destroy(h)
+    kept = 8 * ((1 << nv) + (5 << (nv + lr)))
+    # two arrays of evaluations at a time for the work, and the pool's own granularity
+    assert grown <= count * kept + 2 * (8 << nv) + (48 << 20), (grown >> 20, count * kept >> 20)
