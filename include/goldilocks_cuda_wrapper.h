@@ -344,14 +344,15 @@ int basefold_prove_sharded_host(const uint64_t* h_evals_shard, int num_vars, int
  * S = sum_k alpha^k sum_x eq(t, x) a_k(x) b_k(x). d_a, d_b: [K][2^n_loc] base-field
  * slices of this shard; h_point_low: n_loc (c0, c1) pairs; h_eq_scale: eq of the
  * sharded (top) coordinates at this shard's index, (1, 0) for a single shard.
- * claims: K local shares of the per-instance sums; round_message: local share of
- * m(0..3) (4 extension elements); fold binds the low variable on the challenge;
- * finals (after n_loc folds): eq, alpha^k a_k (K), b_k (K). The caller adds the
- * shards' shares and runs the transcript (matrix_b200/sharded.py).
- * Threads: create returns with the handle's tables complete, and a handle may then
- * be used from any host thread, one call at a time. Work is queued on the calling
- * thread's stream; claims, round_message and finals wait for it, fold does not, so
- * pass a handle to another thread only after one of the waiting calls. */
+ * claims: K local shares of the per-instance sums, in any round; set_alpha: before the
+ * first message, may be repeated until the first fold (later calls change nothing);
+ * round_message: local share of m(0..3) (4 extension elements); fold binds the low
+ * variable on the challenge, with or without the round's message asked for; finals
+ * (after n_loc folds): eq, alpha^k a_k (K), b_k (K). The caller adds the shards' shares
+ * and runs the transcript (matrix_b200/sharded.py). d_a and d_b are read by create and
+ * by folds until the tables are folded: they stay as they are until finals.
+ * Threads: every call returns with the work it queued complete, so a handle may be used
+ * from any host thread, one call at a time. */
 int gl_batched_state_create(const uint64_t* d_a, const uint64_t* d_b, const uint64_t* h_point_low,
                             const uint64_t* h_eq_scale, int K, int n_loc, void** state);
 int gl_batched_state_destroy(void* state);

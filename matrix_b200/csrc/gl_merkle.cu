@@ -59,7 +59,7 @@ int mb_merkle_layer_variant(const uint64_t* d_input, uint64_t* d_output, int n, 
     if (n < 1 || !d_input || !d_output) return MB_ERR_ARG;
     if (variant == 1) {
         MB_KERNEL("compress_layer_coop");
-        compress_layer_coop_kernel<HashPoseidon2><<<grid_for((size_t)n * 8, 256, 8), 256, 0, MB_STREAM>>>(d_input, d_output, (size_t)n);
+        compress_layer_coop_kernel<<<grid_for((size_t)n * 8, 256, 8), 256, 0, MB_STREAM>>>(d_input, d_output, (size_t)n);
     } else {
         MB_KERNEL("compress_layer");
         compress_layer_kernel<HashPoseidon2><<<grid_for((size_t)n, BLOCK, 16), BLOCK, 0, MB_STREAM>>>(d_input, d_output, (size_t)n, 1);

@@ -14,12 +14,11 @@
 //    after a fold only reads (d+1) extension elements back.
 // Base / Ext are the field traits of sumcheck_kernels.cuh (GlBase, GlExt2) or
 // agl_traits.cuh (AglBase, AglExt2).
-//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh), and so do one, three or four tables that
-//    are small (product_sumcheck.cuh); other sizes and counts take a round per pass:
-//  * once a table is down to host_tail(d) elements the live tables are read back and the remaining rounds run on
-//    the host: a round on the device costs a launch and a synchronisation (about 20 us) whatever its size, the
-//    same round on a few hundred elements takes a host core less (about 7 ns per extension product). The field
-//    arithmetic is exact, so the messages are the same words.
+//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh), and so does one table, and three or four
+//    that are small (product_sumcheck.cuh); larger ones, and five and more, take a round per pass;
+//  * five and more tables that are down to HOST_TAIL elements are read back and the remaining rounds run on the host: a
+//    round on the device costs a launch and a synchronisation whatever its size. The field arithmetic is exact, so the
+//    messages are the same words.
 #pragma once
 #include <memory>
 #include <vector>
@@ -54,9 +53,10 @@ template <class T> struct PairOf;
 template <> struct PairOf<gl::E2> { using type = PairSumcheck<pr::GlF, PairGl>; using product = ProductSumcheck<pr::GlF, PairGl>; };
 template <> struct PairOf<agl::E2> { using type = PairSumcheck<pr::AglF, PairAgl>; using product = ProductSumcheck<pr::AglF, PairAgl>; };
 
-// Live elements per table at which the rounds move to the host: a host round costs live / 2 x (d^2 - 1 + d)
-// extension products, about 9 us at 512 elements of two tables and 10 us at 256 elements of three.
-inline size_t host_tail(int d) { return d <= 2 ? 512 : 256; }
+// Live elements per table at which the rounds of five and more tables move to the host. A host round on them costs half of
+// that times d^2 + d - 1 extension products of about 7 ns: 26 us with five tables at 256 elements, and half as much the
+// round after, where a round on the device takes about 20 us each.
+constexpr size_t HOST_TAIL = 256;
 
 template <class Base, class Ext>
 class LinearSumcheckState {
@@ -76,12 +76,13 @@ public:
         round_ = 0;
         cur_ = nullptr;
         host_mode_ = false;
-        if (d == 2 && num_vars > 0 && aligned16(d_tables)) {
+        if (num_vars > 0 && !aligned16(d_tables)) return MB_ERR_ARG;   // every kernel reads pairs of words
+        if (d == 2 && num_vars > 0) {
             pair_.reset(new typename PairOf<typename Ext::T>::type);
             const size_t words = n_ * (base_field ? 1 : 2);
             return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0, true);
         }
-        products_ = Product::handles(d) && aligned16(d_tables) && num_vars > 0;
+        products_ = Product::handles(d) && num_vars > 0;
         if (products_ && num_vars <= Product::limit(d)) {
             product_.reset(new Product);
             return product_->init(d_tables, n_ * (base_field ? 1 : 2), d, num_vars, base_field, nullptr);
@@ -178,7 +179,7 @@ public:
             int rc = take_tables();
             if (rc != MB_OK) return rc;
         }
-        if (!host_mode_ && round_ >= 1 && live <= host_tail(d_)) {
+        if (!host_mode_ && round_ >= 1 && live <= HOST_TAIL) {
             int rc = to_host(live);
             if (rc != MB_OK) return rc;
         }

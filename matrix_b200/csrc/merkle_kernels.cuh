@@ -168,19 +168,18 @@ monolith_permute_batch_kernel(const uint64_t* __restrict__ in, uint64_t* __restr
 }
 
 // ---- latency-oriented variants: several lanes per permutation ---------------------------
-// Node k of the output layer is handled by LANES consecutive threads: thread l < 8 loads word l of the 64-byte input
-// pair and threads 0..3 store the digest.
-template <class H>
-__global__ void __launch_bounds__(256)
+// One layer, eight lanes per permutation (mb_merkle_layer_variant only; the trees use tree_up_coop_kernel): node k is handled by
+// eight consecutive threads, each loads a word of the 64-byte input pair and threads 0..3 store the digest.
+static __global__ void __launch_bounds__(256)
 compress_layer_coop_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
-    const int l = threadIdx.x & (H::LANES - 1);
-    const size_t groups = ((size_t)gridDim.x * blockDim.x) / H::LANES;
+    const int l = threadIdx.x & 7;
+    const size_t groups = ((size_t)gridDim.x * blockDim.x) / 8;
     const size_t rounds = (n + groups - 1) / groups;  // every lane of a warp runs the same trip count
-    size_t k = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / H::LANES;
+    size_t k = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 8;
     for (size_t it = 0; it < rounds; it++, k += groups) {
         const bool live = k < n;
-        uint64_t x = (live && l < 8) ? in[8 * k + l] : 0;
-        x = H::coop(x, l);
+        uint64_t x = live ? in[8 * k + l] : 0;
+        x = HashPoseidon2::coop(x, l);
         if (live && l < 4) out[4 * k + l] = gl::canon(x);
     }
 }

@@ -92,28 +92,9 @@ struct GlExt2 {
     static __device__ __forceinline__ uint64_t reduce_acc(const gl::Acc& s) { return gl::acc_reduce(s); }
 };
 
-// Exact sums of products for a field: A holds sum x_k y_k without any reduction; at most LAZY_MAX products
-// may be added before reduce(). Specialised per field (almost-Goldilocks in agl_traits.cuh).
-template <class F>
-struct Lazy;
-constexpr int LAZY_MAX = 64;
-template <>
-struct Lazy<GlBase> {
-    using A = gl::Acc;
-    static __device__ __forceinline__ A zero() { return gl::acc_zero(); }
-    static __device__ __forceinline__ void mul(A& s, uint64_t x, uint64_t y) { gl::acc_mul(s, x, y); }
-    static __device__ __forceinline__ uint64_t reduce(const A& s) { return gl::acc_reduce(s); }
-};
-template <>
-struct Lazy<GlExt2> {
-    using A = gl::E2Acc;
-    static __device__ __forceinline__ A zero() { return gl::e2acc_zero(); }
-    static __device__ __forceinline__ void mul(A& s, gl::E2 x, gl::E2 y) { gl::e2acc_mul(s, x, y); }
-    static __device__ __forceinline__ gl::E2 reduce(const A& s) { return gl::e2acc_reduce(s); }
-};
-
-// The same with the non-residue multiplied into the second factor first, for kernels that keep several sums in registers:
-// two sums per extension element instead of three, and any number of products.
+// Exact sums of products for a field: A holds sum x_k y_k without any reduction, any number of products. The non-residue is
+// multiplied into the second factor first, so an extension element takes two sums. Specialised per field (almost-Goldilocks in
+// agl_traits.cuh).
 template <class F>
 struct NarrowLazy;
 struct NarrowSum {
