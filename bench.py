@@ -1069,29 +1069,19 @@ def part_sumcheck(lib, args, peak, peak_kind):
     step()
     lib.mb_prof_enable(0)
     kernels = prof_report(lib)
-    alg_bytes = d * n * 48.0   # round 0 reads 8 B per element, the first fold reads 8 and writes 8, later rounds halve
-    # The dominant kernel alone, through the per-round entry point the reference's state object would call: the fold
-    # of round 0 fused with the message of round 1 over the full tables (8 B read and 8 B written per element),
-    # timed by the library's CUDA events around the launch.
-    d_o = DeviceBuffer(lib, d * n * 16)
-    nblk = 592
-    d_pp = DeviceBuffer(lib, nblk * (d + 1) * 2 * 8)
-    big_reps = 5
-    lib.mb_prof_reset(); lib.mb_prof_enable(1)
-    for _ in range(big_reps):
-        assert lib.sumcheck_fold_round_mixed_ffi(d_t.ptr, d_o.ptr, 0x1234567, 0x7654321, d, n, n // 4, d_pp.ptr, nblk) == 0
-    lib.mb_prof_enable(0)
-    big_ms = sum(x for _, x in prof_report(lib).values()) / big_reps
-    big_bytes = d * n * 16.0
-    ach = big_bytes / (big_ms * 1e-3) / 1e9
+    # The passes' algorithmic bytes, blocks of rounds taken as two (they are two or more): the base tables once for the sums
+    # of the first block and once for its fold, then every folded table (16 B an element, a quarter of the one before)
+    # written once and read once.
+    alg_bytes = 2.0 * d * n * 8 + 2.0 * sum(d * (n >> (2 * r)) * 16 for r in range(1, nv // 2 + 1))
+    cnt, pass_ms = kernels["pair_pass"]
+    ach = alg_bytes / (pass_ms * 1e-3) / 1e9
     whole = alg_bytes / (ms * 1e-3) / 1e9
     out = {"metric": "field-elems/s: sumcheck of f*g over 2^%d points, Goldilocks" % nv, "value": d * n / (ms * 1e-3), "unit": UNIT,
            "ms": ms, "config": {"workload": "sumcheck nv=%d d=2" % nv},
-           "roofline": {"kernel": "sumcheck_fold_message (fold of round 0 + message of round 1, 2^%d elements per table)" % nv,
-                        "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": None,
-                        "peak_kind": peak_kind, "avg_launch_ms": big_ms, "launches": big_reps,
-                        "timed_in": "a separate pass of %d launches through sumcheck_fold_round_mixed_ffi with CUDA events "
-                                    "around each (not the timed region)" % big_reps,
+           "roofline": {"kernel": "pair_pass (all passes of a proof)", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+                        "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "avg_launch_ms": pass_ms / cnt, "launches": cnt,
+                        "timed_in": "a proof of its own with CUDA events around every launch (not the timed region)",
+                        "note": "two or more rounds per pass; the products of the sums bound it (integer pipes), not HBM",
                         "whole_proof": {"achieved": whole, "frac": whole / peak,
                                         "note": "%d rounds with the host transcript between them against the %.2f GB the passes "
                                                 "must move; the last rounds are latency bound" % (nv, alg_bytes / 1e9)}},
@@ -1320,9 +1310,11 @@ def run_basefold(args):
     value = n * args.steps / (ms_total * 1e-3)
     e2e_value = n * args.steps / (ms_e2e * 1e-3)
 
-    # Roofline of the dominant kernel by device time. Algorithmic bytes per unit:
-    #   hash_leaves     base pair 16 B in + 32 B digest out (commit tree); extension pair 32 B + 32 B (folded trees)
-    #   compress_layer  64 B in + 32 B out per node
+    # Roofline of the dominant kernel by device time. Algorithmic bytes per unit, layers of more than 4096 nodes (smaller ones
+    # are tree_up's):
+    #   hash_leaves     commitment: base pair 16 B in, digest 32 B out (times the codeword's equal blocks); folded codeword: its
+    #                   source 32 B (base, first round) or 64 B, table 32 B in, codeword 32 B and digest 32 B out
+    #   compress_layer  64 B in, 32 B out per node (times the blocks in the commitment's tree)
     # Units per launch come from this rank's share of the work (1 / world of every tree before the gather).
     peak, peak_kind = measured_peaks()
     total_kernel_ms = sum(ms for _, ms in kernels.values()) or 1.0
@@ -1332,31 +1324,42 @@ def run_basefold(args):
     leaves_folded = sum((cw_len >> (i + 2)) for i in range(nv - 1)) // world
     nodes_per_step = leaves_commit + sum(max((cw_len >> (i + 2)) - 1, 0) for i in range(nv - 1)) // world
     roofline = None
-    prefix = "" if args.hash == "poseidon2" else "monolith_"
-    hash_ms = sum(kernels.get(k, (0, 0))[1] for k in (prefix + "hash_leaves", prefix + "compress_layer", "tree_up"))
+    small = 1 << 12
+    copies = 1 << lr if world == 1 else 1
+    big_commit_leaves = leaves_commit if leaves_commit > small else 0
+    big_folded = [cw_len >> (i + 2) for i in range(nv - 1) if (cw_len >> (i + 2)) // world > small]   # whole codewords
+    leaf_bytes = big_commit_leaves * (16 + 32 * copies) + sum(m * (128 if i == 0 else 160) for i, m in enumerate(big_folded)) // world
+
+    def big_nodes(leaves):
+        return sum(leaves >> k for k in range(1, 40) if leaves >> k > small)
+    node_bytes = big_nodes(leaves_commit) * (64 + 32 * copies) + sum(big_nodes(m // world) for m in big_folded) * 96
+    hash_ms = sum(kernels.get(k, (0, 0))[1] for k in ("hash_leaves", "compress_layer", "tree_up"))
     perms_per_s = (leaves_commit + leaves_folded + nodes_per_step) * prof_steps / (hash_ms * 1e-3) if hash_ms else 0.0
-    inst_per_perm = 5442.0 if args.hash == "poseidon2" else 2715.0  # thread instructions per permutation (ncu)
+    inst_per_perm = 10870.0 if args.hash == "poseidon2" else 5615.0  # of a permutation's thread (profiles/poseidon2_permute_batch_ncu.md)
     sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
     if dom is not None:
         cnt, ms = kernels[dom]
         if dom == "hash_leaves":
-            total_bytes = (leaves_commit * 48 + leaves_folded * 64) * prof_steps
+            total_bytes = leaf_bytes * prof_steps
         elif dom == "compress_layer":
-            total_bytes = 96 * nodes_per_step * prof_steps
+            total_bytes = node_bytes * prof_steps
         else:
             total_bytes = None
         if total_bytes is not None:
             achieved = total_bytes / (ms * 1e-3) / 1e9
             # DRAM bytes per launch, scaled from an ncu capture of the 2^22 case by the units hashed (reads equal the
-            # algorithmic reads; most digest writes are still in L2 when a kernel ends): 65.06 B per node,
-            # 20.44 B per base leaf pair, extension leaf pairs taken as 32 B read + the same write share.
-            if dom == "compress_layer":
-                traffic = 65.06 * nodes_per_step * prof_steps / cnt
+            # algorithmic reads; many digest writes are still in L2 when a kernel ends): 65 B per node, 53.6 B per base leaf
+            # pair of the commitment, 104.3 B per folded leaf of the first round, 119.5 B of the later ones.
+            if args.hash != "poseidon2":
+                traffic = None
+            elif dom == "compress_layer":
+                traffic = 65.0 * (big_nodes(leaves_commit) + sum(big_nodes(m // world) for m in big_folded)) * prof_steps / cnt
             else:
-                traffic = (20.44 * leaves_commit + 36.4 * leaves_folded) * prof_steps / cnt
+                traffic = (53.6 * big_commit_leaves
+                           + sum((104.3 if i == 0 else 119.5) * m for i, m in enumerate(big_folded)) / world) * prof_steps / cnt
             roofline = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                        "traffic_note": "bytes per launch (average), scaled from the ncu capture in profiles/",
+                        "traffic_note": "bytes per launch (average), scaled from the capture in profiles/bench_basefold_launches.md",
                         "launches": cnt, "avg_launch_ms": ms / cnt, "share_of_kernel_time": ms / total_kernel_ms,
                         "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % prof_steps,
                         "note": ("Poseidon2 hashing: ~520 modular multiplications per 32-byte digest, bound by the "
@@ -1370,7 +1373,7 @@ def run_basefold(args):
                                   "peak_warp_inst_per_s": 148 * 4 * sm_hz,
                                   "frac": perms_per_s * inst_per_perm / 32.0 / (148 * 4 * sm_hz),
                                   "note": "two 16-lane pipes per scheduler take a warp instruction every two cycles each, wide "
-                                          "multiply-adds two or three of those: a mix with many of them cannot fill the slots"}}
+                                          "products two of those: a mix with many of them cannot fill the slots"}}
     line = {
         "metric": METRIC if args.hash == "poseidon2" else METRIC.replace("Poseidon2 Merkle", "Monolith Merkle"),
         "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

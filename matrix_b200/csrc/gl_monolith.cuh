@@ -14,7 +14,7 @@
 // with the halves moved into the weights, which all become powers of two: M -1 8 1 2 -4 1 (negacyclic), A 16 16 8,
 // B -8 -1 -1 (negacyclic). That is 84 additions and shift-additions a limb where the circulant on 32-bit halves took
 // 288 multiply-adds with 64-bit results, which cost the multiply pipe two to three times as much each
-// (2^19 compressions: 96 -> 61 us). Values are loose in [0, 2^64) between layers; words 0..3 are made canonical before the
+// (2^18 compressions: 96 -> 61 us). Values are loose in [0, 2^64) between layers; words 0..3 are made canonical before the
 // bars (the S-box acts on the canonical bit pattern), and the caller canonicalises what it stores.
 #pragma once
 #include "gl_field.cuh"
