@@ -258,7 +258,7 @@ public:
         MB_CUDA(cudaMemsetAsync(counter_.p, 0, 8 * counter_.words, MB_STREAM));
         {
             MB_KERNEL_ON("open_eq_tables", MB_STREAM);
-            pr::eq_tables_kernel<pr::GlF><<<nt, pr::BLK, 0, MB_STREAM>>>(set, tabs_.p + words, tabs_.p);
+            pr::eq_tables_kernel<pr::GlF><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, tabs_.p + words, tabs_.p);
         }
         return pass();
     }

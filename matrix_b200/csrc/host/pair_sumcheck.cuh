@@ -14,6 +14,7 @@
 #include <vector>
 #include "../common.cuh"
 #include "../pair_kernels.cuh"
+#include "../pair_mma_kernels.cuh"
 #include "host_field.hpp"
 #include "pinned_pool.hpp"
 
@@ -103,16 +104,19 @@ public:
         if (base && ((size_t)K << n) <= 1024 && n > t) t = n;
         for (int v = n; v > t;) {
             const size_t size = (size_t)K << v;
-            const bool first = v == n;
-            int g = size <= (1u << 17) ? 4 : size <= (first && base && eq_vars == 0 ? 1u << 21 : 1u << 19) ? 3 : 2;
+            const bool first = v == n, words = base && blocks_.size() <= 1;   // a pass over words of the base field
+            const int fb = first ? 0 : blocks_.back().rounds;
+            const bool mma = size >= MMA_MIN && v >= pr::mma_min_vars(fb > 0, words) && (first || pr::mma_folds(fb, words));
+            int g = mma ? (first && base ? 4 : 3) : size <= (1u << 17) ? 4 : size <= (first && base && eq_vars == 0 ? 1u << 21 : 1u << 19) ? 3 : 2;
             while (g > 1 && ((size_t)K << (2 * g)) > 1024) g--;
             if (g > v - t) g = v - t;
-            blocks_.push_back(Block{n - v, g, 0, 0, 0, 63, 0});
+            blocks_.push_back(Block{n - v, g, 0, 0, 0, 63, 0, mma});
             v -= g;
         }
         tail_first_ = n - (n > t ? t : n);
         pin_ = PinnedPool::take();
         if (!pin_) return MB_ERR_CUDA;
+        pin_[ERROR_WORD] = 0;
         if (!blocks_.empty()) {
             cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;   // a wave: four blocks of at most 64 registers fit an SM
             MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 4 * 256 * (size_t)cap_ * K));
@@ -217,11 +221,14 @@ public:
     E2 eq_coord(int round) const { return pt_[round]; }
 
 private:
+    static constexpr size_t ERROR_WORD = PinnedPool::WORDS - 2;
+    static constexpr size_t MMA_MIN = (size_t)1 << 14;
     struct Block {
         int first, rounds;
         size_t wl, wh;      // word offsets of the eq tables
         int lo, row_shift;
         size_t row_mask;
+        bool mma;           // on the tensor cores
     };
     // eq tables of the passes: over the variables above a block, those of WL first
     int tables() {
@@ -239,7 +246,8 @@ private:
         for (Block& b : blocks_) {
             const int above = ne - b.first - b.rounds;
             if (above <= 0) continue;
-            b.lo = above < pr::ROW_BITS ? above : pr::ROW_BITS;
+            const int most = b.mma ? pr::MMA_ROW_BITS : pr::ROW_BITS;
+            b.lo = above < most ? above : most;
             b.wl = table(b.first + b.rounds, b.lo);
             b.wh = table(b.first + b.rounds + b.lo, above - b.lo);
             if (above > b.lo) {
@@ -250,11 +258,11 @@ private:
         if (!nt) return MB_OK;
         MB_CUDA(pool_alloc((void**)&tabs_, sizeof(uint64_t) * (words + 2 * (size_t)ne)));
         uint64_t* d_pt = tabs_ + words;
-        uint64_t* h = pin_ + PinnedPool::WORDS - 2 * (size_t)ne;   // the end of the block: no pass writes there
+        uint64_t* h = pin_ + ERROR_WORD - 2 * (size_t)ne;   // the end of the block: no pass writes there
         for (int i = 0; i < ne; i++) { h[2 * i] = pt_[i].c0; h[2 * i + 1] = pt_[i].c1; }
         MB_CUDA(cudaMemcpyAsync(d_pt, h, 16 * (size_t)ne, cudaMemcpyHostToDevice, MB_STREAM));
         MB_KERNEL("pair_eq_tables");
-        pr::eq_tables_kernel<F><<<nt, pr::BLK, 0, MB_STREAM>>>(set, d_pt, tabs_);
+        pr::eq_tables_kernel<F><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, d_pt, tabs_);
         return finish_async();
     }
     // The pass before block block_ (or, after the last one, before the host tables): folds the challenges of the block
@@ -290,9 +298,12 @@ private:
             p.wl = tabs_ + b.wl; p.wh = tabs_ + b.wh;
         }
         p.partial = partial_; p.counter = counter_; p.sums = pin_;
-        const size_t tiles = (((size_t)1 << p.v) + pr::BLK - 1) / pr::BLK;
-        const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);
-        {
+        if (!last && blocks_[block_].mma) {
+            int rc = launch_mma(gb, weighted, p, fw);
+            if (rc != MB_OK) return rc;
+        } else {
+            const size_t tiles = (((size_t)1 << p.v) + pr::BLK - 1) / pr::BLK;
+            const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);
             MB_KERNEL("pair_pass");
             if (fb) base_ ? launch<true, true>(gb, weighted, grid, p, fw) : launch<true, false>(gb, weighted, grid, p, fw);
             else base_ ? launch<false, true>(gb, weighted, grid, p, fw) : launch<false, false>(gb, weighted, grid, p, fw);
@@ -322,6 +333,32 @@ private:
             default: launch_w<FOLD, BASE, 4>(weighted, grid, p, fw); break;
         }
     }
+    template <bool FOLD, bool BASE, bool WEIGHTED>
+    static int launch_mma_as(dim3 grid, uint32_t smem, const pr::PairMmaArgs& p, const pr::FoldWeights<F>& fw) {
+        const auto k = pr::pair_mma_kernel<F, FOLD, BASE, WEIGHTED>;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return MB_ERR_CUDA;
+        k<<<grid, pr::MMA_BLK, smem, MB_STREAM>>>(p, fw);
+        return MB_OK;
+    }
+    // one block an SM, shared out over the instances
+    int launch_mma(int gb, bool weighted, const pr::PairArgs& q, const pr::FoldWeights<F>& fw) {
+        pr::PairMmaArgs p{};
+        p.fb = q.fb; p.a = q.a; p.b = q.b; p.in_stride = q.in_stride; p.out = q.out; p.v = q.v; p.g = gb;
+        p.lo = q.lo; p.row_shift = q.row_shift; p.row_mask = q.row_mask; p.wl = q.wl; p.wh = q.wh;
+        p.partial = q.partial; p.counter = q.counter; p.sums = q.sums; p.error = pin_ + ERROR_WORD;
+        const size_t tile = q.fb ? pr::MMA_FOLD_TILE : pr::MMA_RAW_ROWS * (base_ ? 16 : 8), tiles = ((size_t)1 << q.v) / tile;
+        const size_t most = sm_count() / K_ > 1 ? sm_count() / K_ : 1;
+        const dim3 grid(tiles < most ? (unsigned)tiles : (unsigned)most, K_);
+        MB_KERNEL("pair_mma");
+        if (q.fb) {
+            const uint32_t smem = pr::mma_fold_smem(base_ ? 4 - q.fb : 3 - q.fb);
+            if (weighted) return base_ ? launch_mma_as<true, true, true>(grid, smem, p, fw) : launch_mma_as<true, false, true>(grid, smem, p, fw);
+            return base_ ? launch_mma_as<true, true, false>(grid, smem, p, fw) : launch_mma_as<true, false, false>(grid, smem, p, fw);
+        }
+        const uint32_t smem = pr::mma_raw_smem(base_, weighted);
+        if (weighted) return base_ ? launch_mma_as<false, true, true>(grid, smem, p, fw) : launch_mma_as<false, false, true>(grid, smem, p, fw);
+        return base_ ? launch_mma_as<false, true, false>(grid, smem, p, fw) : launch_mma_as<false, false, false>(grid, smem, p, fw);
+    }
     int copy_tables() {
         const size_t w = tn_ * (base_ ? 1 : 2);
         if (2 * w * K_ > PinnedPool::WORDS) return MB_ERR_UNSUPPORTED;
@@ -340,6 +377,7 @@ private:
         if (!pending_) return MB_OK;
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
         pending_ = false;
+        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;   // a wait of a pass on the tensor cores ran out
         if (block_ < blocks_.size()) return MB_OK;
         host_ = true;
         const size_t nw = base_ ? 1 : 2;

@@ -68,26 +68,46 @@ constexpr int MAX_TABLES = 48;
 struct TableSet {
     TableDesc d[MAX_TABLES];
 };
+// A block forms the products over each seven variables of its table (a tree of six products a thread) and then its share
+// of the entries from them, so a table of 2^14 takes two barriers on 64 SMs and not fourteen doublings on one.
+constexpr int EQ_PART = 7, EQ_PARTS = 4;      // tables of up to 28 variables
+inline unsigned eq_table_chunks(const TableSet& set, int nt) {   // blocks a table
+    int bits = 0;
+    for (int i = 0; i < nt; i++) bits = set.d[i].bits > bits ? set.d[i].bits : bits;
+    return bits <= 8 ? 1u : bits >= 14 ? 64u : 1u << (bits - 8);
+}
 template <class F>
 __global__ void __launch_bounds__(BLK)
 eq_tables_kernel(const __grid_constant__ TableSet set, const uint64_t* __restrict__ pt, uint64_t* __restrict__ tabs) {
     using E2 = typename F::E2;
+    __shared__ E2 part[EQ_PARTS][1 << EQ_PART];
     const TableDesc d = set.d[blockIdx.x];
-    uint64_t* out = tabs + d.off;
-    if (threadIdx.x == 0) store2(out, 1, 0);
-    __syncthreads();
-    for (int b = 0; b < d.bits; b++) {
-        const E2 rb = load2<E2>(pt + 2 * (d.first + b));
-        const size_t half = (size_t)1 << b;
-        for (size_t j = threadIdx.x; j < half; j += BLK) {
-            const E2 a = load2<E2>(out + 4 * j), ar = F::mul(a, rb), s = F::sub(a, ar);
-            store2(out + 4 * j, F::canon(s.c0), F::canon(s.c1));
-            store2(out + 4 * (j + half), F::canon(ar.c0), F::canon(ar.c1));
+    const size_t n = (size_t)1 << d.bits, first = (size_t)blockIdx.y * BLK;
+    if (first >= n) return;
+    const int parts = d.bits > 0 ? (d.bits + EQ_PART - 1) / EQ_PART : 1;
+    for (int i = threadIdx.x; i < parts << EQ_PART; i += BLK) {
+        const int p = i >> EQ_PART, j = i & ((1 << EQ_PART) - 1), nb = d.bits - EQ_PART * p;
+        if (nb < EQ_PART && j >= (1 << nb)) continue;
+        E2 f[EQ_PART];
+#pragma unroll
+        for (int b = 0; b < EQ_PART; b++) {
+            f[b] = E2{1, 0};
+            if (b < nb) {
+                const E2 r = load2<E2>(pt + 2 * (d.first + EQ_PART * p + b));
+                f[b] = (j >> b) & 1 ? r : F::sub(f[b], r);
+            }
         }
-        __syncthreads();
+        part[p][j] = F::mul(F::mul(F::mul(f[0], f[1]), F::mul(f[2], f[3])), F::mul(F::mul(f[4], f[5]), f[6]));
     }
-    for (size_t j = threadIdx.x; j < ((size_t)1 << d.bits); j += BLK)
-        store2(out + 4 * j + 2, F::canon(F::times_w(out[4 * j + 1])), 0);
+    __syncthreads();
+    uint64_t* out = tabs + d.off;
+    for (size_t j = first + threadIdx.x; j < n; j += (size_t)gridDim.y * BLK) {
+        E2 x = part[0][j & ((1 << EQ_PART) - 1)];
+        for (int p = 1; p < parts; p++) x = F::mul(x, part[p][(j >> (EQ_PART * p)) & ((1 << EQ_PART) - 1)]);
+        const uint64_t c0 = F::canon(x.c0), c1 = F::canon(x.c1);
+        store2(out + 4 * j, c0, c1);
+        store2(out + 4 * j + 2, F::canon(F::times_w(c1)), 0);
+    }
 }
 template <class F>
 __device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
