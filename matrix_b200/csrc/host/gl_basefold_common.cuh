@@ -15,7 +15,7 @@
 #include "host_tree_top.hpp"
 #include "gl_transcript.hpp"
 #include "pair_sumcheck.cuh"
-#include "pinned_pool.hpp"
+#include "scratch_pool.hpp"
 
 namespace mb {
 namespace bf {
@@ -165,8 +165,7 @@ struct OpenPassArgs {
     uint64_t* out;           // 2^v folded elements, or null
     int fb, v, rounds;       // challenges to fold; variables left after that; rounds of the next block
     const uint64_t *wl, *wh; // eq over the s variables: the low 8 (or fewer), and the others
-    uint64_t* partial;       // [2^rounds][2 gridDim.x][2]
-    unsigned* counter;       // [2^rounds][GROUPS + 1]
+    uint64_t* acc;           // [2^rounds][pr::grid_words(1)]
     uint64_t* sums;          // pinned: [2^rounds][2]
 };
 template <bool FOLD, bool BASE>
@@ -220,7 +219,7 @@ open_pass_kernel(const OpenPassArgs a, const __grid_constant__ pr::FoldWeights<p
     if (ns > pr::BLK) x = gl::E2{gl::acc_reduce_wide(s0), gl::acc_reduce_wide(s1)};
     if (sb > 0 && (size_t)t < ns) x = F::fma(pr::load_weight<F>(a.wl + 4 * t), x, gl::E2{0, 0});
     gl::E2 total[1] = {x};
-    if (!pr::grid_sum<F, 1>(total, 0, sm, a.partial + 4 * (size_t)gridDim.x * m, a.counter + (pr::GROUPS + 1) * m)) return;
+    if (!pr::grid_sum<F, 1>(total, 0, sm, a.acc + pr::grid_words(1) * m)) return;
     if (t == 0) pr::store2(a.sums + 2 * m, sm[0].c0, sm[0].c1);
 }
 
@@ -228,10 +227,11 @@ class OpenSumcheck {
 public:
     using H = PairHost<pr::GlF, PairGl>;
     using E2 = gl::E2;
-    // bh: 2^nv bit-reversed evaluations on the device; point: nv (c0, c1) pairs; pinned: 32 words for the passes' sums
-    // and 2 nv for the point's upload. Queues the first pass.
-    int init(const uint64_t* bh, int nv, const uint64_t* point, uint64_t* sums, uint64_t* upload) {
-        nv_ = nv; in_ = bh; sums_ = sums;
+    // bh: 2^nv bit-reversed evaluations on the device; point: nv (c0, c1) pairs; sums: 32 words of pinned memory for the
+    // passes' sums; acc: the scratch block's device words. Queues the first pass.
+    int init(const uint64_t* bh, int nv, const uint64_t* point, uint64_t* sums, uint64_t* acc) {
+        if (nv > pr::MAX_POINT) return MB_ERR_UNSUPPORTED;
+        nv_ = nv; in_ = bh; sums_ = sums; acc_ = acc;
         pt_.resize(nv);
         r_.resize(nv);
         for (int i = 0; i < nv; i++) pt_[i] = H::canon(E2{point[2 * i], point[2 * i + 1]});
@@ -249,16 +249,12 @@ public:
             stages_.push_back(s);
             at += s.rounds;
         }
-        int rc = tabs_.alloc(words + 2 * (size_t)nv);
-        if (rc == MB_OK) rc = partial_.alloc(4 * (size_t)GX * 16);
-        if (rc == MB_OK) rc = counter_.alloc((16 * (pr::GROUPS + 1) + 1) / 2);
+        int rc = tabs_.alloc(words);
         if (rc != MB_OK) return rc;
-        for (int i = 0; i < nv; i++) { upload[2 * i] = pt_[nv - 1 - i].c0; upload[2 * i + 1] = pt_[nv - 1 - i].c1; }
-        MB_CUDA(cudaMemcpyAsync(tabs_.p + words, upload, 16 * (size_t)nv, cudaMemcpyHostToDevice, MB_STREAM));
-        MB_CUDA(cudaMemsetAsync(counter_.p, 0, 8 * counter_.words, MB_STREAM));
+        for (int i = 0; i < nv; i++) { set.pt[2 * i] = pt_[nv - 1 - i].c0; set.pt[2 * i + 1] = pt_[nv - 1 - i].c1; }
         {
             MB_KERNEL_ON("open_eq_tables", MB_STREAM);
-            pr::eq_tables_kernel<pr::GlF><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, tabs_.p + words, tabs_.p);
+            pr::eq_tables_kernel<pr::GlF><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, tabs_.p);
         }
         return pass();
     }
@@ -313,7 +309,7 @@ private:
         OpenPassArgs a;
         a.fb = fb; a.v = nv_ - st.first; a.rounds = st.rounds;
         a.wl = tabs_.p + st.wl; a.wh = tabs_.p + st.wh;
-        a.partial = partial_.p; a.counter = reinterpret_cast<unsigned*>(counter_.p); a.sums = sums_;
+        a.acc = acc_; a.sums = sums_;
         a.in = in_; a.out = nullptr;
         if (fb && stage_ + 1 < stages_.size()) {
             DevBuf& t = tables_[stage_ & 1];
@@ -342,11 +338,11 @@ private:
     int nv_ = 0, round_ = 0;
     size_t stage_ = 0;
     const uint64_t* in_ = nullptr;
-    uint64_t* sums_ = nullptr;
+    uint64_t *sums_ = nullptr, *acc_ = nullptr;
     E2 scale_{1, 0};
     std::vector<Stage> stages_;
     std::vector<E2> pt_, r_, g_;
-    DevBuf tabs_, partial_, counter_, tables_[2];
+    DevBuf tabs_, tables_[2];
 };
 
 // Query phase: every value pair and authentication path of every query in
@@ -495,16 +491,15 @@ public:
 };
 
 // ---- host hashing of tree tops: host_tree_top.hpp -------------------------------------------
-// A pinned block for the length of a scope (nothing may still be writing it when the scope ends).
-struct PinnedBlock {
-    uint64_t* p = PinnedPool::take();
-    PinnedBlock() = default;
-    PinnedBlock(const PinnedBlock&) = delete;
-    PinnedBlock& operator=(const PinnedBlock&) = delete;
-    ~PinnedBlock() {
-        if (!p) return;
-        cudaStreamSynchronize(MB_STREAM);
-        PinnedPool::give(p);
+// A scratch block for the length of a scope (nothing may still be writing it when the scope ends).
+struct ScopedScratch {
+    ScratchBlock b = ScratchPool::take();
+    uint64_t* p = b.host;
+    ScopedScratch() = default;
+    ScopedScratch(const ScopedScratch&) = delete;
+    ScopedScratch& operator=(const ScopedScratch&) = delete;
+    ~ScopedScratch() {
+        if (b) ScratchPool::give(b, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);
     }
 };
 

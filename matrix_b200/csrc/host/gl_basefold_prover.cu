@@ -35,16 +35,15 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     uint64_t* p_final = p_roots + (size_t)(nv - 1) * 4;
     uint64_t* p_queries = p_final + ((size_t)2 << lr);
 
-    t.observe_hash(cm.root);
-    for (int i = 0; i < nv; i++) t.observe_ext2(Ext2{point[2 * i], point[2 * i + 1]});
-
-    PinnedBlock pin;   // sums of the inner sumcheck (32 words), a tree's last device layer (from word 64)
-    uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv + 2 * (size_t)nv);   // host-hashed tree tops on their way up
+    ScopedScratch pin;   // sums of the inner sumcheck (32 words), a tree's last device layer (from word 64)
+    uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv);   // host-hashed tree tops on their way up
     if (!pin.p || !top_staging) return MB_ERR_CUDA;
     uint64_t* nodes = pin.p + 64;
     OpenSumcheck sc;
-    int rc = sc.init(cm.d_bh_evals.p, nv, point, pin.p, top_staging + 4 * (HOST_TOP - 1) * (size_t)nv);
+    int rc = sc.init(cm.d_bh_evals.p, nv, point, pin.p, pin.b.dev);
     if (rc != MB_OK) return rc;
+    t.observe_hash(cm.root);   // while the first pass runs
+    for (int i = 0; i < nv; i++) t.observe_ext2(Ext2{point[2 * i], point[2 * i + 1]});
     MB_CUDA(cudaStreamSynchronize(MB_STREAM));
     // oracle 0 and the claimed value eval = p(0) + p(1) = 2 c0 + c1 + c2
     sc.oracle(p_oracles);

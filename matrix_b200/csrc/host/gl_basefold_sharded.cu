@@ -222,7 +222,7 @@ int prove_sharded(const uint64_t* d_evals, int nv, int lr, const uint64_t* point
     uint64_t* p_queries = p_final + ((size_t)2 << lr);
 
     std::vector<uint64_t> h_mine, h_all;
-    PinnedBlock pin;
+    ScopedScratch pin;
     uint64_t* h_small = pin.p;   // words 0..5 oracle, 6..9 subtree root, from 16 the subtree's last device layer
     uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv);
     if (!h_small || !top_staging) return MB_ERR_CUDA;

@@ -16,7 +16,7 @@
 #include "../pair_kernels.cuh"
 #include "../pair_mma_kernels.cuh"
 #include "host_field.hpp"
-#include "pinned_pool.hpp"
+#include "scratch_pool.hpp"
 
 namespace mbhost {
 
@@ -80,15 +80,13 @@ public:
     using H = PairHost<F, O>;
     using E2 = typename F::E2;
     ~PairSumcheck() {
-        if (pin_) {
-            cudaStreamSynchronize(MB_STREAM);   // nothing may still be writing the block
-            PinnedPool::give(pin_);
+        if (scratch_) {   // nothing may still be writing it
+            const bool clean = cudaStreamSynchronize(MB_STREAM) == cudaSuccess;
+            ScratchPool::give(scratch_, clean && pin_[ERROR_WORD] == 0);
         }
         pool_free(t0_);
         pool_free(t1_);
         pool_free(tabs_);
-        pool_free(partial_);
-        pool_free(counter_);
     }
     // a, b: instance 0's device tables of 2^n elements (never written), instances inst_stride words apart; base: base
     // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. together: b follows a in one allocation
@@ -114,19 +112,18 @@ public:
             v -= g;
         }
         tail_first_ = n - (n > t ? t : n);
-        pin_ = PinnedPool::take();
-        if (!pin_) return MB_ERR_CUDA;
+        scratch_ = ScratchPool::take();
+        if (!scratch_) return MB_ERR_CUDA;
+        pin_ = scratch_.host;
         pin_[ERROR_WORD] = 0;
-        if (!blocks_.empty()) {
-            cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;   // a wave: four blocks of at most 64 registers fit an SM
-            MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * 4 * 256 * (size_t)cap_ * K));
-            MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned) * (pr::GROUPS + 1) * K));
-            MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * (pr::GROUPS + 1) * K, MB_STREAM));
-            int rc = tables();
-            if (rc != MB_OK) return rc;
-        }
         r_.resize(n);
-        return pass();
+        cap_ = sm_count() * 4 / K > 1 ? sm_count() * 4 / K : 1;   // a wave: four blocks of at most 64 registers fit an SM
+        int rc = tables();
+        if (rc == MB_OK) rc = pass();
+        // what the later passes fold into, allocated while the first one runs
+        for (size_t i = 1; rc == MB_OK && i < blocks_.size() && i <= 2; i++)
+            MB_CUDA(pool_alloc((void**)(i == 1 ? &t0_ : &t1_), sizeof(uint64_t) * ((size_t)4 << (n - blocks_[i].first)) * K));
+        return rc;
     }
     // The instances' factors (K = 1: not needed). sums() and fold() may be called from then on; before the first fold the
     // factors may be replaced.
@@ -221,7 +218,7 @@ public:
     E2 eq_coord(int round) const { return pt_[round]; }
 
 private:
-    static constexpr size_t ERROR_WORD = PinnedPool::WORDS - 2;
+    static constexpr size_t ERROR_WORD = ScratchPool::WORDS - 2;
     static constexpr size_t MMA_MIN = (size_t)1 << 14;
     struct Block {
         int first, rounds;
@@ -256,13 +253,11 @@ private:
             }
         }
         if (!nt) return MB_OK;
-        MB_CUDA(pool_alloc((void**)&tabs_, sizeof(uint64_t) * (words + 2 * (size_t)ne)));
-        uint64_t* d_pt = tabs_ + words;
-        uint64_t* h = pin_ + ERROR_WORD - 2 * (size_t)ne;   // the end of the block: no pass writes there
-        for (int i = 0; i < ne; i++) { h[2 * i] = pt_[i].c0; h[2 * i + 1] = pt_[i].c1; }
-        MB_CUDA(cudaMemcpyAsync(d_pt, h, 16 * (size_t)ne, cudaMemcpyHostToDevice, MB_STREAM));
+        if (ne > pr::MAX_POINT) return MB_ERR_UNSUPPORTED;
+        MB_CUDA(pool_alloc((void**)&tabs_, sizeof(uint64_t) * words));
+        for (int i = 0; i < ne; i++) { set.pt[2 * i] = pt_[i].c0; set.pt[2 * i + 1] = pt_[i].c1; }
         MB_KERNEL("pair_eq_tables");
-        pr::eq_tables_kernel<F><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, d_pt, tabs_);
+        pr::eq_tables_kernel<F><<<dim3(nt, pr::eq_table_chunks(set, nt)), pr::BLK, 0, MB_STREAM>>>(set, tabs_);
         return finish_async();
     }
     // The pass before block block_ (or, after the last one, before the host tables): folds the challenges of the block
@@ -284,9 +279,7 @@ private:
             tn_ = (size_t)1 << p.v;
             if (fb == 0) return copy_tables();   // everything on the host
         } else if (fb) {
-            uint64_t*& t = flip_ ? t1_ : t0_;
-            if (!t) MB_CUDA(pool_alloc((void**)&t, sizeof(uint64_t) * ((size_t)4 << p.v) * K_));
-            p.out = t;
+            p.out = flip_ ? t1_ : t0_;
             flip_ = !flip_;
         }
         const int gb = last ? 0 : blocks_[block_].rounds;
@@ -297,7 +290,7 @@ private:
             p.lo = b.lo; p.row_shift = b.row_shift; p.row_mask = b.row_mask;
             p.wl = tabs_ + b.wl; p.wh = tabs_ + b.wh;
         }
-        p.partial = partial_; p.counter = counter_; p.sums = pin_;
+        p.acc = scratch_.dev; p.sums = pin_;
         if (!last && blocks_[block_].mma) {
             int rc = launch_mma(gb, weighted, p, fw);
             if (rc != MB_OK) return rc;
@@ -345,7 +338,7 @@ private:
         pr::PairMmaArgs p{};
         p.fb = q.fb; p.a = q.a; p.b = q.b; p.in_stride = q.in_stride; p.out = q.out; p.v = q.v; p.g = gb;
         p.lo = q.lo; p.row_shift = q.row_shift; p.row_mask = q.row_mask; p.wl = q.wl; p.wh = q.wh;
-        p.partial = q.partial; p.counter = q.counter; p.sums = q.sums; p.error = pin_ + ERROR_WORD;
+        p.acc = q.acc; p.sums = q.sums; p.error = pin_ + ERROR_WORD;
         const size_t tile = q.fb ? pr::MMA_FOLD_TILE : pr::MMA_RAW_ROWS * (base_ ? 16 : 8), tiles = ((size_t)1 << q.v) / tile;
         const size_t most = sm_count() / K_ > 1 ? sm_count() / K_ : 1;
         const dim3 grid(tiles < most ? (unsigned)tiles : (unsigned)most, K_);
@@ -361,7 +354,7 @@ private:
     }
     int copy_tables() {
         const size_t w = tn_ * (base_ ? 1 : 2);
-        if (2 * w * K_ > PinnedPool::WORDS) return MB_ERR_UNSUPPORTED;
+        if (2 * w * K_ > ScratchPool::WORDS) return MB_ERR_UNSUPPORTED;
         pending_ = true;
         if (together_) {
             MB_CUDA(cudaMemcpyAsync(pin_, a_, 16 * w, cudaMemcpyDeviceToHost, MB_STREAM));
@@ -513,8 +506,8 @@ private:
     int side_ = 0, width_ = 0;
     size_t tn_ = 0, live_ = 0;
     E2 eq_scale_{1, 0};
-    uint64_t *pin_ = nullptr, *t0_ = nullptr, *t1_ = nullptr, *tabs_ = nullptr, *partial_ = nullptr;
-    unsigned* counter_ = nullptr;
+    ScratchBlock scratch_;
+    uint64_t *pin_ = nullptr, *t0_ = nullptr, *t1_ = nullptr, *tabs_ = nullptr;
 };
 
 }  // namespace mbhost

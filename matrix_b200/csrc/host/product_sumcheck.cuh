@@ -24,14 +24,9 @@ public:
     static bool handles(int d) { return d == 1 || d == 3 || d == 4; }
     static int limit(int d) { return d == 1 ? 40 : d == 3 ? 16 : 13; }
     ~ProductSumcheck() {
-        if (pin_) {
-            cudaStreamSynchronize(MB_STREAM);   // nothing may still be writing the block
-            PinnedPool::give(pin_);
-        }
+        if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);   // nothing may still be writing it
         pool_free(t0_);
         pool_free(t1_);
-        pool_free(partial_);
-        pool_free(counter_);
     }
     // d device tables of 2^vars elements, `stride` words apart (never written); r: a challenge they have still to be
     // folded on, or null. Queues the first pass.
@@ -52,14 +47,10 @@ public:
             v -= g;
         }
         tail_vars_ = v;
-        pin_ = PinnedPool::take();
-        if (!pin_) return MB_ERR_CUDA;
-        if (block_ < blocks_.size()) {
-            cap_ = sm_count() * (d == 1 ? 8 : 4);
-            MB_CUDA(pool_alloc((void**)&partial_, sizeof(uint64_t) * (d == 1 ? 64 : 2048) * (size_t)cap_));
-            MB_CUDA(pool_alloc((void**)&counter_, sizeof(unsigned) * (pr::GROUPS + 1)));
-            MB_CUDA(cudaMemsetAsync(counter_, 0, sizeof(unsigned) * (pr::GROUPS + 1), MB_STREAM));
-        }
+        scratch_ = ScratchPool::take();
+        if (!scratch_) return MB_ERR_CUDA;
+        pin_ = scratch_.host;
+        cap_ = sm_count() * (d == 1 ? 8 : 4);
         return pass();
     }
     // Every round that is left is the host's: tables() has them.
@@ -142,7 +133,7 @@ private:
         p.fb = fb;
         p.in = in_; p.stride = stride_;
         p.v = n_ - (last ? n_ - tail_vars_ : blocks_[block_].first);
-        p.partial = partial_; p.counter = counter_; p.sums = pin_;
+        p.acc = scratch_.dev; p.sums = pin_;
         loaded_ = false;
         if (last) {
             p.out = pin_;
@@ -217,8 +208,8 @@ private:
     std::vector<Block> blocks_;
     size_t block_ = 0;
     std::vector<E2> r_, t_;
-    uint64_t *pin_ = nullptr, *t0_ = nullptr, *t1_ = nullptr, *partial_ = nullptr;
-    unsigned* counter_ = nullptr;
+    ScratchBlock scratch_;
+    uint64_t *pin_ = nullptr, *t0_ = nullptr, *t1_ = nullptr;
 };
 
 }  // namespace mbhost

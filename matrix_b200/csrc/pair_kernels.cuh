@@ -65,8 +65,10 @@ struct TableDesc {
     size_t off;   // words
 };
 constexpr int MAX_TABLES = 48;
+constexpr int MAX_POINT = 40;
 struct TableSet {
     TableDesc d[MAX_TABLES];
+    uint64_t pt[2 * MAX_POINT];   // the point's coordinates, (c0, c1)
 };
 // A block forms the products over each seven variables of its table (a tree of six products a thread) and then its share
 // of the entries from them, so a table of 2^14 takes two barriers on 64 SMs and not fourteen doublings on one.
@@ -78,7 +80,7 @@ inline unsigned eq_table_chunks(const TableSet& set, int nt) {   // blocks a tab
 }
 template <class F>
 __global__ void __launch_bounds__(BLK)
-eq_tables_kernel(const __grid_constant__ TableSet set, const uint64_t* __restrict__ pt, uint64_t* __restrict__ tabs) {
+eq_tables_kernel(const __grid_constant__ TableSet set, uint64_t* __restrict__ tabs) {
     using E2 = typename F::E2;
     __shared__ E2 part[EQ_PARTS][1 << EQ_PART];
     const TableDesc d = set.d[blockIdx.x];
@@ -93,7 +95,8 @@ eq_tables_kernel(const __grid_constant__ TableSet set, const uint64_t* __restric
         for (int b = 0; b < EQ_PART; b++) {
             f[b] = E2{1, 0};
             if (b < nb) {
-                const E2 r = load2<E2>(pt + 2 * (d.first + EQ_PART * p + b));
+                const int c = 2 * (d.first + EQ_PART * p + b);
+                const E2 r{set.pt[c], set.pt[c + 1]};
                 f[b] = (j >> b) & 1 ? r : F::sub(f[b], r);
             }
         }
@@ -115,81 +118,84 @@ __device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
     return typename F::Pre{a.x, a.y, p[2]};
 }
 
+// Sums over the blocks of a grid, in a scratch area of grid_words(entries) words a sum that is zero between kernels: word 0
+// counts the blocks that are through, from word 8 on there are four words an entry, the sums of the low and high halves
+// of the blocks' canonical words (exact for 2^32 blocks). A block adds its entries with atomics that nobody waits for, so
+// the one that finishes last reads each sum once, whatever the grid. (With rows of partial sums it read them all: 148
+// rows of 256 entries, 600 KB, took it 7 us; in two levels a fence and a ticket more.)
+constexpr int ACC_FIRST = 8;
+__host__ __device__ constexpr size_t grid_words(size_t entries) { return ACC_FIRST + 4 * entries; }
+__device__ __forceinline__ void grid_add(uint64_t* acc, int entry, uint64_t c0, uint64_t c1) {
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(acc + ACC_FIRST + 4 * (size_t)entry);
+    atomicAdd(p, (unsigned long long)gl::lo32(c0));
+    atomicAdd(p + 1, (unsigned long long)gl::hi32(c0));
+    if (c1 != 0) {
+        atomicAdd(p + 2, (unsigned long long)gl::lo32(c1));
+        atomicAdd(p + 3, (unsigned long long)gl::hi32(c1));
+    }
+}
+template <class F>
+__device__ __forceinline__ uint64_t grid_value(uint64_t lo, uint64_t hi) {
+    const unsigned __int128 x = ((unsigned __int128)hi << 32) + lo;
+    return F::canon(F::red(gl::Acc{(uint32_t)x, (uint32_t)(x >> 32), (uint32_t)(x >> 64), (uint32_t)(x >> 96), 0}));
+}
+// after every thread's grid_add: true in the block that is through last (uniform over the block's `threads`)
+__device__ __forceinline__ bool grid_last(uint64_t* acc, bool* flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) *flag = atomicAdd(reinterpret_cast<unsigned*>(acc), 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!*flag) return false;
+    __threadfence();
+    if (threadIdx.x == 0) *reinterpret_cast<unsigned*>(acc) = 0;
+    return true;
+}
+// the sum of an entry, which is zero afterwards
+template <class F>
+__device__ __forceinline__ typename F::E2 grid_take(uint64_t* acc, int entry) {
+    ulonglong2* p = reinterpret_cast<ulonglong2*>(acc + ACC_FIRST + 4 * (size_t)entry);
+    const ulonglong2 a = __ldcg(p), b = __ldcg(p + 1);
+    p[0] = p[1] = make_ulonglong2(0, 0);
+    return typename F::E2{grid_value<F>(a.x, a.y), grid_value<F>(b.x, b.y)};
+}
+
 // Sums the threads' V values by t mod 2^bits over the block and then over the gridDim.x blocks of blockIdx.y; true in
 // the block that finishes last, with the sums (canonical) in sm[0 .. V 2^bits), value j of t at j 2^bits + t.
-// partial: 2 gridDim.x * V 2^bits elements of this blockIdx.y; counters: GROUPS + 1 of this blockIdx.y, zero before and after.
-// A block that reads hundreds of rows one after another waits for L2 each time (512 rows: 70 us), so beyond sixteen rows
-// a thread they are summed in groups of about sqrt(gridDim.x) by each group's last block, then the groups by the last
-// of those; up to sixteen (their loads overlap) one level is faster by a fence and an atomic.
-constexpr int GROUPS = 64;
+// acc: grid_words(V 2^bits) words of this blockIdx.y.
 template <class F, int V>
-__device__ __forceinline__ bool grid_sum(typename F::E2 (&v)[V], int bits, typename F::E2* sm, uint64_t* partial, unsigned* counters) {
+__device__ __forceinline__ bool grid_sum(typename F::E2 (&v)[V], int bits, typename F::E2* sm, uint64_t* acc) {
     using E2 = typename F::E2;
     __shared__ bool last;
     const int t = threadIdx.x, n = 1 << bits;
-    const auto block_sum = [&]() {
-        E2 x[V];
+    E2 x[V];
 #pragma unroll
-        for (int j = 0; j < V; j++) {
+    for (int j = 0; j < V; j++) {
+        __syncthreads();
+        sm[t] = v[j];
+        __syncthreads();
+        for (int s = BLK / 2; s >= n; s >>= 1) {
+            if (t < s) sm[t] = F::add(sm[t], sm[t + s]);
             __syncthreads();
-            sm[t] = v[j];
-            __syncthreads();
-            for (int s = BLK / 2; s >= n; s >>= 1) {
-                if (t < s) sm[t] = F::add(sm[t], sm[t + s]);
-                __syncthreads();
-            }
-            x[j] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
         }
-        __syncthreads();
-        if (t < n) {
-#pragma unroll
-            for (int j = 0; j < V; j++) sm[j * n + t] = x[j];
-        }
-        __syncthreads();
-    };
-    // writes sm to row `row`, takes a ticket of `counter`; true in the block that takes the last of `of`
-    const auto publish = [&](size_t row, unsigned* counter, unsigned of) {
-        if (t < n) {
-#pragma unroll
-            for (int j = 0; j < V; j++) store2(partial + 2 * ((row * V + j) * n + t), sm[j * n + t].c0, sm[j * n + t].c1);
-            __threadfence();
-        }
-        __syncthreads();
-        if (t == 0) {
-            last = atomicAdd(counter, 1u) == of - 1;
-            if (last) *counter = 0;
-        }
-        __syncthreads();
-        return last;
-    };
-    const auto rows_sum = [&](size_t first, unsigned count) {
-        __threadfence();
-#pragma unroll
-        for (int j = 0; j < V; j++) v[j] = E2{0, 0};
-#pragma unroll 8
-        for (unsigned b = t >> bits; b < count; b += BLK >> bits) {
-#pragma unroll
-            for (int j = 0; j < V; j++) {
-                const uint64_t* p = partial + 2 * (((first + b) * V + j) * n + (t & (n - 1)));
-                v[j] = F::add(v[j], E2{__ldcg(p), __ldcg(p + 1)});
-            }
-        }
-        block_sum();
-    };
-    block_sum();
-    if (gridDim.x == 1) return true;
-    unsigned per = 16 * (BLK >> bits);   // rows per group
-    if (gridDim.x > per) {
-        per = 8;
-        while (per * per < gridDim.x || (gridDim.x + per - 1) / per > GROUPS) per += 8;
+        x[j] = E2{F::canon(sm[t].c0), F::canon(sm[t].c1)};
     }
-    const unsigned groups = (gridDim.x + per - 1) / per, g = blockIdx.x / per;
-    const unsigned members = (g + 1) * per <= gridDim.x ? per : gridDim.x - g * per;
-    if (!publish(blockIdx.x, counters + 1 + g, members)) return false;
-    rows_sum((size_t)g * per, members);
-    if (groups == 1) return true;
-    if (!publish(gridDim.x + g, counters, groups)) return false;
-    rows_sum(gridDim.x, groups);
+    if (gridDim.x > 1) {
+        if (t < n) {
+#pragma unroll
+            for (int j = 0; j < V; j++) grid_add(acc, j * n + t, x[j].c0, x[j].c1);
+        }
+        if (!grid_last(acc, &last)) return false;
+        if (t < n) {
+#pragma unroll
+            for (int j = 0; j < V; j++) x[j] = grid_take<F>(acc, j * n + t);
+        }
+    }
+    __syncthreads();
+    if (t < n) {
+#pragma unroll
+        for (int j = 0; j < V; j++) sm[j * n + t] = x[j];
+    }
+    __syncthreads();
     return true;
 }
 
@@ -204,8 +210,7 @@ struct PairArgs {
     int row_shift;            // log2 of the elements between two entries of WH (63: WH is a single 1)
     size_t row_mask;
     const uint64_t *wl, *wh;
-    uint64_t* partial;        // [instance][2 gridDim.x][4^B][2]
-    unsigned* counter;        // [instance][GROUPS + 1]
+    uint64_t* acc;            // [instance][grid_words(4^B)]
     uint64_t* sums;           // pinned: [instance][4^B][2]
 };
 template <class F>
@@ -344,7 +349,7 @@ pair_pass_kernel(const PairArgs a, const __grid_constant__ FoldWeights<F> fw) {
     }
     if constexpr (GB > 0) {
         if constexpr (!WEIGHTED) sum[0] = E2{F::redw(s0), F::redw(s1)};
-        if (!grid_sum<F, 1>(sum, 2 * GB, sa, a.partial + ((size_t)(4 * gridDim.x) << (2 * GB)) * k, a.counter + (GROUPS + 1) * k)) return;
+        if (!grid_sum<F, 1>(sum, 2 * GB, sa, a.acc + grid_words(E) * k)) return;
         if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), sa[t].c0, sa[t].c1);
     }
 }

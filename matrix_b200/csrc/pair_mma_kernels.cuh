@@ -9,7 +9,7 @@
 // A product of extension elements on the integer pipes takes four chains of 24 cycles a warp (64 x 64 into a 160-bit sum);
 // here 256 rows' worth of them costs the tensor pipe 64 cycles an SM, so what is left is the traffic, the weights (a is
 // multiplied by WL before it becomes an operand) and the reductions after a fold (about 30 instructions a component).
-// Sixteen instances of 2^22 under a weight: first pass 740 -> 289 us, the pass that folds it 672 -> 242 us.
+// Sixteen instances of 2^22 under a weight: first pass 740 -> 268 us, the pass that folds it 672 -> 240 us.
 //
 // One block an SM: sixteen warps that copy, weigh and reduce, and one that issues the MMAs. They meet at mbarriers only, so a
 // warp may be two tiles ahead of another. Copies to shared memory run two or more tiles ahead (cp.async into the swizzled
@@ -45,8 +45,7 @@ struct PairMmaArgs {
     int row_shift;            // log2 of the elements between two entries of WH (63: WH is a single 1)
     size_t row_mask;
     const uint64_t *wl, *wh;
-    uint64_t* partial;        // [instance][gridDim.x][4^g][2]
-    unsigned* counter;        // [instance][GROUPS + 1]
+    uint64_t* acc;            // [instance][grid_words(4^g)]
     uint64_t* sums;           // pinned: [instance][4^g][2]
     uint64_t* error;          // pinned, set to 1 when a wait ran out
 };
@@ -137,14 +136,8 @@ __device__ __forceinline__ typename F::E2 gather_sums(uint32_t tmem, uint64_t* r
 // w(y) x for an element of the base field (BASE) or the extension
 template <class F, bool BASE>
 __device__ __forceinline__ typename F::E2 weigh(const typename F::Pre& w, uint64_t c0, uint64_t c1) {
-    gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
-    gl::acc_mul(s0, w.c0, c0);
-    gl::acc_mul(s1, w.c1, c0);
-    if constexpr (!BASE) {
-        gl::acc_mul(s0, w.c1w, c1);
-        gl::acc_mul(s1, w.c0, c1);
-    }
-    return typename F::E2{F::red(s0), F::red(s1)};
+    if constexpr (BASE) return typename F::E2{MmaField<F>::mul(w.c0, c0), MmaField<F>::mul(w.c1, c0)};
+    else return F::fma(w, typename F::E2{c0, c1}, typename F::E2{0, 0});
 }
 
 constexpr int MMA_FOLD_STAGES = 3;
@@ -220,8 +213,11 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
             }
         }
     };
-    const auto weight = [&](size_t x) {   // of element x
-        return load_weight<F>(a.wl + 4 * ((x >> a.g) & (((size_t)1 << a.lo) - 1)));
+    const auto weight = [&](size_t x) {   // of element x; W c1 only where it is used
+        const uint64_t* p = a.wl + 4 * ((x >> a.g) & (((size_t)1 << a.lo) - 1));
+        if constexpr (FOLD || !BASE) return load_weight<F>(p);
+        const E2 w = load2<E2>(p);
+        return typename F::Pre{w.c0, w.c1, 0};
     };
     constexpr uint32_t idesc_s = tc::idesc_u8(N, true);
 
@@ -398,36 +394,10 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
     // ---- over the blocks ----
     const int E = 1 << (2 * a.g);
     if (gridDim.x > 1) {
-        uint64_t* partial = a.partial + (size_t)2 * E * gridDim.x * k;
-        unsigned* counter = a.counter + (GROUPS + 1) * k;
-        if (t < E) {
-            store2(partial + 2 * ((size_t)blockIdx.x * E + t), F::canon(sum.c0), F::canon(sum.c1));
-            __threadfence();
-        }
-        __syncthreads();
-        if (t == 0) {
-            last_sm = atomicAdd(counter, 1u) == gridDim.x - 1;
-            if (last_sm) *counter = 0;
-        }
-        __syncthreads();
-        if (!last_sm) return;
-        __threadfence();
-        E2* s2 = reinterpret_cast<E2*>(sm);
-        sum = E2{0, 0};
-        if (t < MMA_WORKERS) {
-#pragma unroll 16
-            for (unsigned b = t >> (2 * a.g); b < gridDim.x; b += MMA_WORKERS >> (2 * a.g)) {
-                const ulonglong2 p = __ldcg(reinterpret_cast<const ulonglong2*>(partial + 2 * ((size_t)b * E + (t & (E - 1)))));
-                sum = F::add(sum, E2{p.x, p.y});
-            }
-            s2[t] = sum;
-        }
-        __syncthreads();
-        for (int s = MMA_WORKERS / 2; s >= E; s >>= 1) {
-            if (t < s) s2[t] = F::add(s2[t], s2[t + s]);
-            __syncthreads();
-        }
-        if (t < E) sum = s2[t];
+        uint64_t* acc = a.acc + grid_words(E) * k;
+        if (t < E) grid_add(acc, t, F::canon(sum.c0), F::canon(sum.c1));
+        if (!grid_last(acc, &last_sm)) return;
+        if (t < E) sum = grid_take<F>(acc, t);
     }
     if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), F::canon(sum.c0), F::canon(sum.c1));
 }

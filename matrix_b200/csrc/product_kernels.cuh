@@ -25,8 +25,7 @@ struct ProductArgs {
     size_t stride;        // words from one table to the next
     uint64_t* out;        // [D][2^v][2] folded tables, or null
     int v;                // variables left after the fold, at least 6
-    uint64_t* partial;    // [2 gridDim.x][2^(D B)][2]
-    unsigned* counter;    // [GROUPS + 1]
+    uint64_t* acc;        // grid_words(2^(D B))
     uint64_t* sums;       // pinned: [2^(D B)][2]
 };
 
@@ -49,7 +48,7 @@ product_pass_kernel(const ProductArgs a, const __grid_constant__ FoldWeights<F> 
             if constexpr (GB > 0) sum[0] = F::add(sum[0], f);
         }
         if constexpr (GB > 0)
-            if (grid_sum<F, 1>(sum, GB, sm, a.partial, a.counter) && t < E) store2(a.sums + 2 * t, sm[t].c0, sm[t].c1);
+            if (grid_sum<F, 1>(sum, GB, sm, a.acc) && t < E) store2(a.sums + 2 * t, sm[t].c0, sm[t].c1);
         return;
     }
     __shared__ E2 s[D][PTILE];
@@ -94,7 +93,7 @@ product_pass_kernel(const ProductArgs a, const __grid_constant__ FoldWeights<F> 
         E2 sum[PER];
 #pragma unroll
         for (int p = 0; p < PER; p++) sum[p] = E2{F::redw(s0[p]), F::redw(s1[p])};
-        if (grid_sum<F, PER>(sum, BITS, sm, a.partial, a.counter) && t < (1 << BITS)) {
+        if (grid_sum<F, PER>(sum, BITS, sm, a.acc) && t < (1 << BITS)) {
 #pragma unroll
             for (int p = 0; p < PER; p++) store2(a.sums + 2 * (size_t)(t * PER + p), sm[(p << BITS) + t].c0, sm[(p << BITS) + t].c1);
         }
