@@ -2,14 +2,16 @@
 // (product_kernels.cuh). The object plans the blocks of rounds, queues the passes, runs the rounds of a block on the
 // sums they return, and hands over the folded tables once they are small enough for the host.
 //
-//   rounds per block   one table: 4. Three tables: 3 up to 2^14 elements, then 2. Four tables: 2. Each is where the
-//                      pass's products cost about what the launch and the synchronisation of a round more do.
-//   limit(d)           the largest tables (log2) this is for: with three tables two rounds at 2^17 take 15 us of
-//                      products against two launches; with four tables the same holds at 2^14; one table has no products.
+//   rounds per block   one table: 4. Three tables: 3 up to 2^14 elements, then 2, on the tensor cores
+//                      (product_mma_kernels.cuh). Four tables: 2. Each is where the pass's products cost about what the
+//                      launch and the synchronisation of a round more do.
+//   limit(d)           the largest tables (log2) this is for: with four tables two rounds at 2^14 take as long as two
+//                      launches more; one table has no products, three have them on the tensor cores.
 //   host tables        at most 2^8 elements, 2^7 where a pass can end there: the rest of a proof on them takes a core 10 to 20 us.
 #pragma once
 #include <vector>
 #include "../product_kernels.cuh"
+#include "../product_mma_kernels.cuh"
 #include "pair_sumcheck.cuh"
 
 namespace mbhost {
@@ -22,9 +24,9 @@ public:
     using H = PairHost<F, O>;
     using E2 = typename F::E2;
     static bool handles(int d) { return d == 1 || d == 3 || d == 4; }
-    static int limit(int d) { return d == 1 ? 40 : d == 3 ? 16 : 13; }
+    static int limit(int d) { return d == 4 ? 13 : 40; }
     ~ProductSumcheck() {
-        if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);   // nothing may still be writing it
+        if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess && pin_[ERROR_WORD] == 0);   // nothing may still be writing it
         pool_free(t0_);
         pool_free(t1_);
     }
@@ -35,7 +37,7 @@ public:
         r_.resize(vars);
         if (r) {
             r_[0] = *r;
-            blocks_.push_back(Block{0, 1});
+            blocks_.push_back(Block{0, 1, false});
             block_ = 1;
             round_ = 1;
         }
@@ -43,14 +45,17 @@ public:
         while (v > 8) {
             int g = d == 1 ? 4 : d == 3 && v <= 14 ? 3 : 2;
             if (g > v - (d == 1 ? 8 : 7)) g = v - (d == 1 ? 8 : 7);
-            blocks_.push_back(Block{n_ - v, g});
+            const int fb = blocks_.empty() ? 0 : blocks_.back().rounds;
+            const bool mma = d == 3 && v > MMA_ABOVE && (fb == 0 || pr::tri_folds(fb, base && blocks_.size() == 1));
+            blocks_.push_back(Block{n_ - v, g, mma});
             v -= g;
         }
         tail_vars_ = v;
         scratch_ = ScratchPool::take();
         if (!scratch_) return MB_ERR_CUDA;
         pin_ = scratch_.host;
-        cap_ = sm_count() * (d == 1 ? 8 : 4);
+        pin_[ERROR_WORD] = 0;
+        cap_ = sm_count() * (d == 1 ? 8 : 2);
         return pass();
     }
     // Every round that is left is the host's: tables() has them.
@@ -58,6 +63,7 @@ public:
     // [d][2^tail] elements, canonical
     int tables(std::vector<E2>& tab, size_t& stride) {
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;
         stride = (size_t)1 << tail_vars_;
         tab.resize(d_ * stride);
         const int nw = base_ ? 1 : 2;
@@ -120,7 +126,12 @@ public:
     }
 
 private:
-    struct Block { int first, rounds; };
+    static constexpr size_t ERROR_WORD = ScratchPool::WORDS - 2;
+    static constexpr int MMA_ABOVE = 14;
+    struct Block {
+        int first, rounds;
+        bool mma;   // three tables, two rounds: tri_mma_kernel
+    };
     int pass() {
         const int from = block_ > 0 ? blocks_[block_ - 1].first : 0, fb = block_ > 0 ? blocks_[block_ - 1].rounds : 0;
         const bool last = at_tail();
@@ -144,10 +155,15 @@ private:
             p.out = t;
             flip_ = !flip_;
         }
-        const size_t tiles = ((size_t)1 << p.v) / (d_ == 1 ? pr::BLK : pr::PTILE);
-        const unsigned grid = last ? (tiles ? (unsigned)tiles : 1u) : tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_;
-        const int gb = last ? 0 : blocks_[block_].rounds;
-        {
+        if (!last && blocks_[block_].mma) {
+            int rc = launch_mma(p, fw);
+            if (rc != MB_OK) return rc;
+        } else {
+            const size_t tiles = ((size_t)1 << p.v) / (d_ == 1 ? pr::BLK : pr::PTILE);
+            const int gb = last ? 0 : blocks_[block_].rounds;
+            // 2^9 sums: half as many blocks as SMs, or their atomics take longer than the products (2^14 elements: 30 -> 27 us)
+            const size_t most = gb * d_ >= 9 ? cap_ / 4 : cap_;
+            const unsigned grid = last ? (tiles ? (unsigned)tiles : 1u) : (unsigned)(tiles < most ? tiles : most);
             MB_KERNEL("product_pass");
             if (d_ == 1) launch_d<1>(gb, fb > 0, grid, p, fw);
             else if (d_ == 3) launch_d<3>(gb, fb > 0, grid, p, fw);
@@ -161,6 +177,25 @@ private:
             }
         }
         return finish_async();
+    }
+    template <bool FOLD, bool BASE>
+    static int launch_mma_as(unsigned grid, const pr::TriArgs& p, const pr::FoldWeights<F>& fw) {
+        constexpr uint32_t smem = FOLD ? pr::TRI_FOLD_SMEM : pr::TRI_RAW_SMEM;
+        const auto k = pr::tri_mma_kernel<F, FOLD, BASE>;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return MB_ERR_CUDA;
+        k<<<grid, pr::TRI_BLK, smem, MB_STREAM>>>(p, fw);
+        return MB_OK;
+    }
+    int launch_mma(const pr::ProductArgs& q, const pr::FoldWeights<F>& fw) const {
+        pr::TriArgs p{};
+        p.fb = q.fb; p.in = q.in; p.stride = q.stride; p.out = q.out; p.v = q.v;
+        p.acc = q.acc; p.sums = q.sums; p.error = pin_ + ERROR_WORD;
+        const size_t tiles = ((size_t)1 << q.v) / (4 * pr::TRI_Y), least = (tiles + pr::TRI_MOST - 1) / pr::TRI_MOST;
+        const size_t sms = (size_t)sm_count() > least ? (size_t)sm_count() : least;
+        const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
+        MB_KERNEL("product_mma");
+        if (q.fb) return base_ ? launch_mma_as<true, true>(grid, p, fw) : launch_mma_as<true, false>(grid, p, fw);
+        return base_ ? launch_mma_as<false, true>(grid, p, fw) : launch_mma_as<false, false>(grid, p, fw);
     }
     template <int D, int GB>
     void launch(bool fold, unsigned grid, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
@@ -193,12 +228,35 @@ private:
     int load() {
         if (loaded_) return MB_OK;
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;
         const int g = blocks_[block_].rounds;
         side_ = 1 << g;
         t_.resize((size_t)1 << (g * d_));
-        for (size_t j = 0; j < t_.size(); j++) t_[j] = E2{pin_[2 * j], pin_[2 * j + 1]};
+        if (blocks_[block_].mma) expand();
+        else for (size_t j = 0; j < t_.size(); j++) t_[j] = E2{pin_[2 * j], pin_[2 * j + 1]};
         loaded_ = true;
         return MB_OK;
+    }
+
+    // The rounds only use f g as a polynomial: with its values q0, q1 and leading coefficient q2 in a variable, entries
+    // (0, 0) = q0, (1, 1) = q1, (0, 1) = q0 + q1 - q2 and (1, 0) = 0 of the two tables give the same one.
+    void expand() {
+        const auto q = [&](int p, int k) { return E2{pin_[2 * (4 * p + k)], pin_[2 * (4 * p + k) + 1]}; };
+        for (int i = 0; i < 4; i++)
+            for (int j = 0; j < 4; j++)
+                for (int k = 0; k < 4; k++) {
+                    const int first = 2 * (i & 1) + (j & 1), second = 2 * (i >> 1) + (j >> 1);   // of table f and g, in each variable
+                    const auto in_first = [&](int p1) {
+                        if (first == 0) return q(3 * p1, k);
+                        if (first == 3) return q(3 * p1 + 1, k);
+                        return H::sub(H::add(q(3 * p1, k), q(3 * p1 + 1, k)), q(3 * p1 + 2, k));
+                    };
+                    E2& t = t_[(4 * i + j) * 4 + k];
+                    if (first == 2 || second == 2) t = E2{0, 0};
+                    else if (second == 0) t = in_first(0);
+                    else if (second == 3) t = in_first(1);
+                    else t = H::sub(H::add(in_first(0), in_first(1)), in_first(2));
+                }
     }
 
     const uint64_t* in_ = nullptr;

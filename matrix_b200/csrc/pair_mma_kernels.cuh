@@ -54,6 +54,7 @@ template <class F> struct MmaField;
 template <> struct MmaField<GlF> {
     static __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) { return gl::mul(a, b); }
     static __device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return gl::add(a, b); }
+    static __device__ __forceinline__ uint64_t sub_c(uint64_t a, uint64_t b) { return gl::sub_c(a, b); }   // b canonical
     static __device__ __forceinline__ uint64_t red128(uint64_t lo, uint64_t hi) { return gl::reduce128(lo, hi); }
     // lo + hi 2^64 for hi < 2^18
     static __device__ __forceinline__ uint64_t red_small(uint64_t lo, uint32_t hi) {
@@ -65,6 +66,7 @@ template <> struct MmaField<GlF> {
 template <> struct MmaField<AglF> {
     static __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) { return agl::mul(a, b); }
     static __device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return agl::add(a, b); }
+    static __device__ __forceinline__ uint64_t sub_c(uint64_t a, uint64_t b) { return agl::sub_c(a, b); }   // b canonical
     static __device__ __forceinline__ uint64_t red128(uint64_t lo, uint64_t hi) { return agl::reduce128(lo, hi); }
     static __device__ __forceinline__ uint64_t red_small(uint64_t lo, uint32_t hi) {
         uint32_t c;
@@ -91,6 +93,52 @@ __device__ __forceinline__ uint64_t bytes_value_wide(const uint32_t* s) {
     return MmaField<F>::red128((uint64_t)x, (uint64_t)(x >> 64));
 }
 
+// w(y) x for an element of the base field (BASE) or the extension
+template <class F, bool BASE>
+__device__ __forceinline__ typename F::E2 weigh(const typename F::Pre& w, uint64_t c0, uint64_t c1) {
+    if constexpr (BASE) return typename F::E2{MmaField<F>::mul(w.c0, c0), MmaField<F>::mul(w.c1, c0)};
+    else return F::fma(w, typename F::E2{c0, c1}, typename F::E2{0, 0});
+}
+
+// The fold's operand of weights, K-major, by the first `workers` threads: row (sub, component, byte) holds that byte of the
+// factor of each input byte, and zero outside the sub-th of the 2^le elements in 128 bytes of input.
+template <class F, bool BASE>
+__device__ __forceinline__ void fold_operand(uint8_t* cst, int le, const FoldWeights<F>& fw, uint32_t workers) {
+    const uint32_t t = threadIdx.x, words = 16u >> le;   // words of one element
+    for (uint32_t x = t; x < (16u << le) * 8; x += workers) *reinterpret_cast<uint4*>(cst + 16 * x) = make_uint4(0, 0, 0, 0);
+    tc::named_sync(workers);
+    for (uint32_t x = t; x < words * 16; x += workers) {
+        const uint32_t comp = x & 1, i = (x >> 1) & 7, w = x >> 4;
+        uint64_t f;
+        if constexpr (BASE) {
+            f = comp ? fw.w[w].c1 : fw.w[w].c0;
+        } else {
+            const typename F::Pre& e = fw.w[w >> 1];
+            f = comp ? ((w & 1) ? e.c0 : e.c1) : ((w & 1) ? e.c1w : e.c0);
+        }
+        f = F::canon(MmaField<F>::mul(f, 1ULL << (8 * i)));
+        for (uint32_t sub = 0; sub < (1u << le); sub++) {
+            const uint32_t col = sub * 8 * words + 8 * w + i;
+            for (uint32_t byte = 0; byte < 8; byte++) {
+                const uint32_t row = sub * 16 + comp * 8 + byte;
+                cst[tc::swz(row, col >> 4) + (col & 15)] = (uint8_t)(f >> (8 * byte));
+            }
+        }
+    }
+}
+// one group of eight columns of the accumulators: byte products of two words, by the lane's byte of the other operand; the
+// sum over its eight lanes, loose, in each of them
+template <class F>
+__device__ __forceinline__ uint64_t gather_word(uint32_t addr, uint64_t scale) {
+    using M = MmaField<F>;
+    uint32_t s[8];
+    tc::ld8(addr, s);
+    uint64_t v = M::mul(bytes_value_wide<F>(s), scale);
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) v = M::add(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+
 // Sums of the block's rows of 4^g byte products: what the accumulators hold, put together by byte of b (eight lanes), byte
 // of a (eight columns), component and diagonal block (rows hold more elements than 2^g when the block is shorter).
 // r_sm: 16 x 32 words. Threads below 4^g get the entry M[t >> g][t mod 2^g].
@@ -106,11 +154,7 @@ __device__ __forceinline__ typename F::E2 gather_sums(uint32_t tmem, uint64_t* r
 #pragma unroll
     for (int x = 0; x < GROUPS_A / 4; x++) {
         const int ga = part * (GROUPS_A / 4) + x;
-        uint32_t s[8];
-        tc::ld8(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(8 * ga), s);
-        uint64_t v = M::mul(bytes_value_wide<F>(s), scale);
-#pragma unroll
-        for (int off = 1; off < 8; off <<= 1) v = M::add(v, __shfl_xor_sync(0xffffffffu, v, off));
+        const uint64_t v = gather_word<F>(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(8 * ga), scale);
         if ((lane & 7) == 0) r_sm[(4 * q + (lane >> 3)) * 32 + ga] = v;
     }
     tc::fence_before();
@@ -131,13 +175,6 @@ __device__ __forceinline__ typename F::E2 gather_sums(uint32_t tmem, uint64_t* r
         }
     }
     return e;
-}
-
-// w(y) x for an element of the base field (BASE) or the extension
-template <class F, bool BASE>
-__device__ __forceinline__ typename F::E2 weigh(const typename F::Pre& w, uint64_t c0, uint64_t c1) {
-    if constexpr (BASE) return typename F::E2{MmaField<F>::mul(w.c0, c0), MmaField<F>::mul(w.c1, c0)};
-    else return F::fma(w, typename F::E2{c0, c1}, typename F::E2{0, 0});
 }
 
 constexpr int MMA_FOLD_STAGES = 3;
@@ -306,28 +343,7 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
         };
         if (t < MMA_WORKERS) {
             for (int i = 0; i < 3; i++) load(i);
-            // row (sub, component, k): byte k of the factor of each input byte, zero outside the sub-th element's bytes
-            for (uint32_t x = t; x < (16u << le) * 8; x += MMA_WORKERS) *reinterpret_cast<uint4*>(sm + cst + 16 * x) = make_uint4(0, 0, 0, 0);
-            tc::named_sync(MMA_WORKERS);
-            const uint32_t words = 16u >> le;   // of one element
-            for (uint32_t x = t; x < words * 16; x += MMA_WORKERS) {
-                const uint32_t comp = x & 1, i = (x >> 1) & 7, w = x >> 4;
-                uint64_t f;
-                if constexpr (BASE) {
-                    f = comp ? fw.w[w].c1 : fw.w[w].c0;
-                } else {
-                    const typename F::Pre& e = fw.w[w >> 1];
-                    f = comp ? ((w & 1) ? e.c0 : e.c1) : ((w & 1) ? e.c1w : e.c0);
-                }
-                f = F::canon(MmaField<F>::mul(f, 1ULL << (8 * i)));
-                for (uint32_t sub = 0; sub < epr; sub++) {
-                    const uint32_t col = sub * 8 * words + 8 * w + i;
-                    for (uint32_t byte = 0; byte < 8; byte++) {
-                        const uint32_t row = sub * 16 + comp * 8 + byte;
-                        sm[cst + tc::swz(row, col >> 4) + (col & 15)] = (uint8_t)(f >> (8 * byte));
-                    }
-                }
-            }
+            fold_operand<F, BASE>(sm + cst, le, fw, MMA_WORKERS);
             tc::copy_wait<1>();   // tiles 0 and 1
             tc::fence_operands();
         }

@@ -51,8 +51,8 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// barrier of the first `threads` threads of a block
-__device__ __forceinline__ void named_sync(uint32_t threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+// barrier of `threads` threads of a block, id from 1
+__device__ __forceinline__ void named_sync(uint32_t threads, uint32_t id = 1) { asm volatile("bar.sync %1, %0;" ::"r"(threads), "r"(id) : "memory"); }
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // bounded: false after about a million polls
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {

@@ -19,9 +19,9 @@ from .test_sumcheck_gpu import test_whole_proof_matches_oracle as gl_sumcheck_ma
 
 pytestmark = pytest.mark.gpu
 
-# one table: host up to 2^8, then four rounds a pass; two: host up to 2^10 (base) or 2^9, blocks of 4, 3, 2 rounds; three:
-# passes from 2^9 to 2^16, a round a pass above; four: to 2^13
-ROUNDS = [(1, 8), (1, 9), (1, 13), (1, 17), (2, 1), (2, 9), (2, 10), (2, 11), (2, 18), (2, 19), (3, 8), (3, 9), (3, 14), (3, 15),
+# one table: host up to 2^8, then four rounds a pass; two: host up to 2^10 (base) or 2^9, blocks of 4 and 3 rounds, on the
+# tensor cores from 2^14; three: passes from 2^9, on the tensor cores from 2^15; four: to 2^13
+ROUNDS = [(2, 13), (2, 14), (2, 15), (2, 16), (3, 19), (1, 8), (1, 9), (1, 13), (1, 17), (2, 1), (2, 9), (2, 10), (2, 11), (2, 18), (2, 19), (3, 8), (3, 9), (3, 14), (3, 15),
           (3, 16), (3, 17), (3, 18), (4, 8), (4, 10), (4, 13), (4, 14), (4, 16)]
 
 
@@ -75,7 +75,8 @@ def test_many_tables(gl, oracle, d, blocks):
     assert np.array_equal(got, folded.reshape(d, 2 * n)[:, :n])
 
 
-@pytest.mark.parametrize("K,nv", [(1, 9), (2, 9), (3, 10), (4, 12), (7, 13), (64, 4), (64, 11), (1, 18), (5, 17)])
+@pytest.mark.parametrize("K,nv", [(1, 9), (2, 9), (3, 10), (4, 12), (7, 13), (64, 4), (64, 11), (1, 18), (5, 17),
+                                  (1, 13), (1, 14), (1, 20), (3, 13), (16, 11), (16, 14), (64, 8), (64, 10)])
 def test_batched_rounds(K, nv):
     batched_matches_oracle(K, nv, 0)
 
