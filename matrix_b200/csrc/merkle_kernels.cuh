@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "gl_poseidon2.cuh"
 #include "gl_monolith.cuh"
+#include "poseidon2_tiles.cuh"
 
 namespace mb {
 namespace mk {
@@ -254,9 +255,93 @@ permute_batch_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out
     }
 }
 
+// The throughput kernels above for Poseidon2 in tiles of 128 (poseidon2_tiles.cuh): node or leaf k < n of a layer, from f as in
+// TreeSource, written `copies` times. Every tile runs as many turns as the longest, for the order in tensor memory.
+template <TreeSource SRC>
+static __global__ void __launch_bounds__(P2_BLK, 1)
+poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n, size_t copies) {
+    extern __shared__ __align__(128) uint8_t p2_sm[];
+    __shared__ __align__(8) uint64_t done[P2_TILES], free[P2_TILES];
+    __shared__ uint32_t tmem_sm;
+    __shared__ int failed;
+    const int t = threadIdx.x, g = t / P2_TILE;
+    p2_operands(p2_sm);
+    if (t == 0) {
+        failed = 0;
+        for (int i = 0; i < P2_TILES; i++) {
+            tc::mbar_init(&done[i], 1);
+            tc::mbar_init(&free[i], P2_TILE / 32);
+        }
+        tc::mbar_init_fence();
+    }
+    if (t < 32) tc::tmem_alloc(&tmem_sm, 512);
+    tc::fence_operands();
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    P2Tile tile;
+    tile.row = t % P2_TILE;
+    tile.tmem = tmem_sm + 256 * (g & 1) + ((tile.row & ~31u) << 16);
+    tile.consts = tc::smem_u32(p2_sm);
+    tile.rows = p2_sm + P2_CONST + g * P2_TILE * 64;
+    tile.done = tc::smem_u32(&done[g]);
+    tile.free = tc::smem_u32(&free[g]);
+    tile.before = tc::smem_u32(&free[(g + P2_TILES - 2) % P2_TILES]);
+    tile.id = 1 + g;
+    tile.use = g < 2 ? -1 : 0;   // the first two find their halves empty
+    tile.failed = &failed;
+    const uint64_t r1w = gl::mul_small(f.r.c1, 7);
+    const size_t step = (size_t)gridDim.x * P2_BLK, turns = (n + step - 1) / step;
+    size_t k = (size_t)blockIdx.x * P2_BLK + t;
+    for (size_t i = 0; i < turns; i++, k += step) {
+        const bool live = k < n;
+        if ((SRC == FOLD_BASE || SRC == FOLD_EXT) && live) {
+            gl::e2_store(f.out + 4 * k, folded_element<SRC == FOLD_BASE>(f, 2 * k, r1w));
+            gl::e2_store(f.out + 4 * k + 2, folded_element<SRC == FOLD_BASE>(f, 2 * k + 1, r1w));
+        }
+        const auto load = [&](uint64_t* s) {
+            constexpr int WORDS = SRC == NODES ? 8 : SRC == LEAF_BASE ? 2 : 4;
+            const uint64_t* in = (SRC == FOLD_BASE || SRC == FOLD_EXT ? f.out : f.in) + WORDS * k;   // this thread's own stores
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                ulonglong2 v = make_ulonglong2(0, 0);
+                if (j < WORDS && live) v = *reinterpret_cast<const ulonglong2*>(in + j);
+                s[j] = v.x;
+                s[j + 1] = v.y;
+            }
+        };
+        uint64_t s[8];
+        load(s);
+        if (!p2_permute_tile(tile, s)) {
+            load(s);
+            gl::poseidon2_permute(s);
+        }
+        if (live)
+            for (size_t c = 0; c < copies; c++) store_digest(dst + 4 * (c * n + k), s);
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (t < 32) tc::tmem_free(tmem_sm, 512);
+}
+// Layers of this many permutations and more go in tiles: 2^20 take 503 us a thread each and 474 in tiles, 2^19 250 to 259 and 246
+// to 266 (five turns of every tile, the last of them a tenth full).
+constexpr size_t P2_TILES_FROM = (size_t)1 << 20;
+template <TreeSource SRC>
+inline void launch_poseidon2_tiles(const FoldSource& f, uint64_t* dst, size_t n, size_t copies, cudaStream_t st) {
+    cudaFuncSetAttribute(poseidon2_tiles_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM);
+    poseidon2_tiles_kernel<SRC><<<sm_count(), P2_BLK, P2_SMEM, st>>>(f, dst, n, copies);
+}
+template <class H> constexpr bool in_tiles(size_t) { return false; }
+template <> constexpr bool in_tiles<HashPoseidon2>(size_t n) { return n >= P2_TILES_FROM; }
+
 template <class H>
 inline void launch_compress_layer(const uint64_t* in, uint64_t* out, size_t n, size_t copies, cudaStream_t st) {
     MB_KERNEL_ON(H::layer_name(), st);
+    if (in_tiles<H>(n)) {
+        FoldSource f{};
+        f.in = in;
+        return launch_poseidon2_tiles<NODES>(f, out, n, copies, st);
+    }
     compress_layer_kernel<H><<<grid_for(n, BLOCK, 16), BLOCK, 0, st>>>(in, out, n, copies);
 }
 
@@ -332,6 +417,7 @@ inline int build_tree(const uint64_t* d_codeword, uint64_t* d_tree, size_t num_l
     FoldSource f{};
     f.in = d_codeword;
     return build_from_leaves<H, EXT2 ? LEAF_EXT : LEAF_BASE>(f, d_tree, num_leaves, 1, st, root_out, stop, [&] {
+        if (in_tiles<H>(num_leaves)) return launch_poseidon2_tiles<EXT2 ? LEAF_EXT : LEAF_BASE>(f, d_tree, num_leaves, 1, st);
         hash_leaves_kernel<H, EXT2><<<grid_for(num_leaves, BLOCK, 16), BLOCK, 0, st>>>(d_codeword, d_tree, num_leaves, 1);
     });
 }
@@ -340,6 +426,7 @@ inline int build_tree(const uint64_t* d_codeword, uint64_t* d_tree, size_t num_l
 template <class H, bool MIXED>
 inline int fold_tree(const FoldSource& f, uint64_t* d_tree, size_t num_leaves, cudaStream_t st, uint64_t* root_out, size_t stop) {
     return build_from_leaves<H, MIXED ? FOLD_BASE : FOLD_EXT>(f, d_tree, num_leaves, 1, st, root_out, stop, [&] {
+        if (in_tiles<H>(num_leaves)) return launch_poseidon2_tiles<MIXED ? FOLD_BASE : FOLD_EXT>(f, d_tree, num_leaves, 1, st);
         fold_leaves_kernel<H, MIXED><<<grid_for(num_leaves, BLOCK, 16), BLOCK, 0, st>>>(f, d_tree, num_leaves);
     });
 }
@@ -359,6 +446,7 @@ inline int build_tree_periodic(const uint64_t* d_codeword, uint64_t* d_tree, siz
     FoldSource f{};
     f.in = d_codeword;
     int rc = build_from_leaves<H, LEAF_BASE>(f, d_tree, uniq, copies, st, nullptr, 1, [&] {
+        if (in_tiles<H>(uniq)) return launch_poseidon2_tiles<LEAF_BASE>(f, d_tree, uniq, copies, st);
         hash_leaves_kernel<H, false><<<grid_for(uniq, BLOCK, 16), BLOCK, 0, st>>>(d_codeword, d_tree, uniq, copies);
     });
     if (rc != MB_OK) return rc;
