@@ -15,8 +15,9 @@
 // the CPU prover's (heterogeneous arities stay on that path, as in the reference).
 //
 // Device side (same_point_kernels.cuh): the eq polynomials stay factored, and one pass over a table serves up to four
-// rounds (six for the packed witness): it returns 2^B eq-weighted sums per leaf, on which the host runs the messages
-// and folds of B rounds, and the next pass folds the B challenges at once. The first pass is queued before the header of
+// rounds (six for the packed witness): it returns the 3^B values of the rounds' polynomial over all leaves, on which the host
+// runs the messages and folds of B rounds, and the next pass folds the B challenges at once. (With 2^B sums per leaf returned
+// the host's rounds over 42 leaves took 200 of 686 us.) The first pass is queued before the header of
 // the transcript (every claim point, label by label), which the host absorbs while the device works: after the pass
 // that header is the longest part of a proof. The reference launches a message and a fold kernel per round over eq and f
 // tables; with one fused pass per round over both tables, arity 22 and 42 binary leaves took 7.4 ms and 11 GB.
@@ -24,6 +25,7 @@
 #include "../same_point_kernels.cuh"
 #include "agl_transcript.hpp"
 #include "host_field.hpp"
+#include "scratch_pool.hpp"
 
 using namespace mb;
 using namespace mb::sc;
@@ -79,31 +81,6 @@ E2 mul(E2 a, E2 b) {   // canonical words in and out, on the host core's multipl
 }
 E2 add(E2 a, E2 b) { return E2{hf::agl_add(a.c0, b.c0), hf::agl_add(a.c1, b.c1)}; }
 E2 sub(E2 a, E2 b) { return E2{hf::agl_sub(a.c0, b.c0), hf::agl_sub(a.c1, b.c1)}; }
-// sum of products, reduced once
-struct Dot {
-    struct Wide {
-        hf::u128 s = 0;
-        uint64_t top = 0;
-        void mac(uint64_t x, uint64_t y) {
-            const hf::u128 p = (hf::u128)x * y;
-            s += p;
-            top += s < p;
-        }
-        // 2^128 = 63 2^32 + 992 (mod q)
-        uint64_t red() const { return hf::agl_red((hf::u128)top * (63ULL * (1ULL << 32) + 992ULL) + hf::agl_red(s)); }
-    };
-    Wide p00, p11, p01;
-    void mac(E2 a, E2 b) {
-        p00.mac(a.c0, b.c0);
-        p11.mac(a.c1, b.c1);
-        p01.mac(a.c0, b.c1);
-        p01.mac(a.c1, b.c0);
-    }
-    E2 value() const {
-        return E2{hf::agl_canon(hf::agl_red((hf::u128)p11.red() * 3 + p00.red())), hf::agl_canon(p01.red())};
-    }
-};
-
 // A block of rounds from variable `first` on, and what the pass before it reads.
 enum Source { FROM_WITNESS, FROM_WORD_SUMS, FROM_WORDS, FROM_TABLE };
 struct Stage {
@@ -113,10 +90,10 @@ struct Stage {
 };
 
 struct Buffers {
-    uint64_t *pts = nullptr, *tabs = nullptr, *partial = nullptr, *g6 = nullptr, *t0 = nullptr, *t1 = nullptr;
+    uint64_t *pts = nullptr, *tabs = nullptr, *partial = nullptr, *g6 = nullptr, *t0 = nullptr, *t1 = nullptr, *scale = nullptr;
     unsigned* counter = nullptr;
     ~Buffers() {
-        pool_free(pts); pool_free(tabs); pool_free(partial); pool_free(g6); pool_free(t0); pool_free(t1); pool_free(counter);
+        pool_free(pts); pool_free(scale); pool_free(tabs); pool_free(partial); pool_free(g6); pool_free(t0); pool_free(t1); pool_free(counter);
     }
 };
 
@@ -141,6 +118,9 @@ uint64_t* pinned_words(size_t words) {
 
 class SamePointDevice {
 public:
+    ~SamePointDevice() {
+        if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);
+    }
     // Stages of the proof, eq tables of all passes, and the first pass, all queued; the sums of the first stage are in
     // sums() after a stream synchronisation. claims_only: nothing after the first pass will be asked for.
     int init(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool claims_only) {
@@ -188,6 +168,11 @@ public:
         MB_CUDA(pool_alloc((void**)&b_.tabs, sizeof(uint64_t) * leaf_words_ * M));
         MB_CUDA(pool_alloc((void**)&b_.partial, sizeof(uint64_t) * 2 * 64 * (size_t)cap * M));
         MB_CUDA(pool_alloc((void**)&b_.counter, sizeof(unsigned) * M));
+        if (!claims_only) {
+            MB_CUDA(pool_alloc((void**)&b_.scale, sizeof(uint64_t) * 2 * (size_t)M));
+            scratch_ = ScratchPool::take();
+            if (!scratch_) return MB_ERR_CUDA;
+        }
         if (inside) MB_CUDA(pool_alloc((void**)&b_.g6, sizeof(uint64_t) * 2 * 64 * (size_t)M));
         // staging: the points go up from page-locked memory, the sums come back behind them
         const size_t pt_words = 2 * (size_t)arity * M;
@@ -217,6 +202,12 @@ public:
         }
         return finish_async();
     }
+    // The polynomial of the first stage's rounds, once alpha is known.
+    int first_share(E2 alpha) {
+        MB_KERNEL("same_point_share");
+        sp::first_share_kernel<<<M_, sp::BLK, 0, MB_STREAM>>>(h_sums_, stages_[0].rounds, b_.pts, k_, alpha, b_.scale, scratch_.dev, scratch_.host);
+        return finish_async();
+    }
     // The pass before stage i: folds the challenges r[0 .. count) that bind the variables the pass consumes (all six of
     // a word for the first extension table, those of the stage before otherwise) and queues the sums of stage i.
     int fold(size_t i, const E2* r, int count) {
@@ -227,7 +218,13 @@ public:
         if (s.source == FROM_WORD_SUMS) a.v = s.rounds;   // the other variables are summed already
         a.t_bits = a.v < 8 ? a.v : 8;
         a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = s.wl; a.wh_off = s.wh;
-        a.partial = b_.partial; a.counter = b_.counter; a.out = h_sums_;
+        a.partial = b_.partial; a.counter = b_.counter;
+        a.out = i == 0 || i + 1 == stages_.size() ? h_sums_ : nullptr;   // for the first share; for the reveals
+        if (i > 0) {
+            a.pts = b_.pts; a.arity = k_; a.first = s.first; a.bound = stages_[i - 1].rounds;
+            a.scale = b_.scale; a.acc = scratch_.dev; a.u = scratch_.host;
+            for (int j = 0; j < a.bound; j++) a.r[j] = r[count - a.bound + j];
+        }
         const size_t iters = (size_t)1 << (a.v - a.t_bits);
         const int half = (max_blocks_ + 1) / 2, gx = iters < (size_t)half ? (int)iters : half;
         const dim3 grid(gx, M_);
@@ -271,7 +268,8 @@ public:
         return finish_async();
     }
     const std::vector<Stage>& stages() const { return stages_; }
-    const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the stage queued last
+    const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the first stage, then of the last
+    const uint64_t* values() const { return scratch_.host; }   // [3^rounds][2] of the stage queued last
 
 private:
     // out[x] = prod_k (x_k ? r_k : 1 - r_k)
@@ -290,6 +288,7 @@ private:
     uint64_t *h_sums_ = nullptr, *cur_ = nullptr;
     bool flip_ = false;
     std::vector<Stage> stages_;
+    ScratchBlock scratch_;
     Buffers b_;
 };
 
@@ -332,100 +331,62 @@ int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_
     if (rc != MB_OK) return rc;
     header(t, M, arity, h_pts, h_vals);
     const E2 alpha = challenge(t, SP_LABEL(L_ALPHA));
-    // scale_i = alpha^i eq(r_i[0 .. j), R[0 .. j))
-    std::vector<E2> scale(M);
-    E2 pw{1, 0};
-    for (int i = 0; i < M; i++) { scale[i] = pw; pw = mul(pw, alpha); }
-
-    std::vector<E2> R(arity), g((size_t)M << sp::MAX_B), up(M), down(M);
-    // suffix eq tables of the block's variables, per leaf: 2^(rounds - 1 - j) entries for round j, back to back
-    std::vector<E2> suffix((size_t)M << sp::MAX_B);
-    bool label_absorbed = false;
+    std::vector<E2> R(arity), u(sp::SHARE);
     for (size_t si = 0; si < dev.stages().size(); si++) {
         const Stage st = dev.stages()[si];
         if (si > 0) {
             // the challenges that the pass consumes: all of a word's for the first extension table
             const int from = st.source == FROM_WORDS ? 0 : dev.stages()[si - 1].first;
             rc = dev.fold(si, R.data() + from, st.first - from);
-            if (rc != MB_OK) return rc;
+        } else {
+            rc = dev.first_share(alpha);
         }
-        if (si > 0) {   // while the pass runs
-            t.begin_append(SP_LABEL(L_MSG));
-            label_absorbed = true;
-        }
-        const int B = st.rounds, size = 1 << B;
-        for (int i = 0; i < M; i++) {
-            // tables for rounds B - 1, B - 2, ..: each from the one before by its lowest variable
-            E2* w = suffix.data() + ((size_t)i << B);
-            w[0] = E2{1, 0};
-            int at = 0;
-            for (int j = B - 2; j >= 0; j--) {
-                const E2 rj = ld(h_pts + 2 * ((size_t)i * arity + st.first + j + 1));
-                const int n = 1 << (B - 2 - j);
-                for (int y = 0; y < n; y++) {
-                    const E2 hi = mul(w[at + y], rj);
-                    w[at + n + 2 * y + 1] = hi;
-                    w[at + n + 2 * y] = sub(w[at + y], hi);
-                }
-                at += n;
-            }
-        }
+        if (rc != MB_OK) return rc;
+        t.begin_append(SP_LABEL(L_MSG));   // while the pass runs
         MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        for (size_t x = 0; x < (size_t)M * size; x++) g[x] = E2{dev.sums()[2 * x], dev.sums()[2 * x + 1]};
-        for (int j = 0; j < B; j++) {
-            const int round = st.first + j, half = size >> (j + 1);
-            // T_i(c) = scale_i ((1 - r)(1 - c) + r c) (A + c (B - A)) with A, B the weighted even and odd sums;
-            // with u = scale (1 - r), v = scale r: T(0) = u A, T(1) = v B, T(2) = (2 v - u)(2 B - A)
-            Dot m0, m1, m2;
-            for (int i = 0; i < M; i++) {
-                const E2* w = suffix.data() + ((size_t)i << B) + (half - 1);
-                const E2* gi = g.data() + (size_t)i * size;
-                E2 a = gi[0], b = gi[1];
-                if (half > 1) {
-                    Dot da, db;
-                    for (int y = 0; y < half; y++) { da.mac(w[y], gi[2 * y]); db.mac(w[y], gi[2 * y + 1]); }
-                    a = da.value();
-                    b = db.value();
-                }
-                up[i] = mul(scale[i], ld(h_pts + 2 * ((size_t)i * arity + round)));
-                down[i] = sub(scale[i], up[i]);
-                m0.mac(down[i], a);
-                m1.mac(up[i], b);
-                m2.mac(sub(add(up[i], up[i]), down[i]), sub(add(b, b), a));
+        int size = 1;
+        for (int j = 0; j < st.rounds; j++) size *= 3;
+        for (int x = 0; x < size; x++) u[x] = E2{dev.values()[2 * x], dev.values()[2 * x + 1]};
+        for (int j = 0; j < st.rounds; j++) {
+            // q0 (1 - c) + q1 c + q2 (c^2 - c): the sums over the later variables at 0 and 1
+            const int round = st.first + j, rest = size / 3, later = st.rounds - j - 1;
+            E2 q[3] = {E2{0, 0}, E2{0, 0}, E2{0, 0}};
+            for (int m = 0; m < (1 << later); m++) {
+                int at = 0, digit = 1;
+                for (int b = 0; b < later; b++, digit *= 3) at += ((m >> b) & 1) * digit;
+                for (int p = 0; p < 3; p++) q[p] = add(q[p], u[3 * at + p]);
             }
-            const E2 msg[3] = {m0.value(), m1.value(), m2.value()};
+            const E2 q12 = add(q[1], q[2]), msg[3] = {q[0], q[1], sub(add(q12, q12), q[0])};
             for (int c = 0; c < 3; c++) {
-                if (c > 0 || !label_absorbed) t.begin_append(SP_LABEL(L_MSG));
+                if (c > 0 || j > 0) t.begin_append(SP_LABEL(L_MSG));
                 t.finish_append_ext2(msg[c].c0, msg[c].c1);
                 h_round_msgs[((size_t)round * 3 + c) * 2] = msg[c].c0;
                 h_round_msgs[((size_t)round * 3 + c) * 2 + 1] = msg[c].c1;
             }
-            label_absorbed = false;
             const E2 r = challenge(t, SP_LABEL(L_CH));
             R[round] = r;
             if (h_challenges) { h_challenges[2 * round] = r.c0; h_challenges[2 * round + 1] = r.c1; }
-            const bool last = si + 1 == dev.stages().size();
-            for (int i = 0; i < M; i++) {
-                scale[i] = add(down[i], mul(r, sub(up[i], down[i])));
-                if (j + 1 == B && !last) continue;   // the next pass folds
-                E2* gi = g.data() + (size_t)i * size;
-                for (int y = 0; y < half; y++) gi[y] = add(gi[2 * y], mul(r, sub(gi[2 * y + 1], gi[2 * y])));
-            }
+            const E2 rr = sub(mul(r, r), r);
+            for (int y = 0; y < rest; y++)
+                u[y] = add(add(u[3 * y], mul(r, sub(u[3 * y + 1], u[3 * y]))), mul(rr, u[3 * y + 2]));
+            size = rest;
         }
-        if (si + 1 == dev.stages().size())
-            for (int i = 0; i < M; i++) {   // nothing is left to sum over: the folded sums are the reveals f_i(R)
-                h_f_evals[2 * i] = g[(size_t)i * size].c0;
-                h_f_evals[2 * i + 1] = g[(size_t)i * size].c1;
-            }
     }
-    Dot fin;
+    // nothing is left to sum over: the last stage's sums, folded, are the reveals f_i(R), and what is left of the polynomial is
+    // sum_i alpha^i eq(r_i, R) f_i(R)
+    const Stage end = dev.stages().back();
     for (int i = 0; i < M; i++) {
-        t.append_ext2(SP_LABEL(L_FEVAL), h_f_evals[2 * i], h_f_evals[2 * i + 1]);
-        fin.mac(scale[i], E2{h_f_evals[2 * i], h_f_evals[2 * i + 1]});   // scale_i = alpha^i eq(r_i, R)
+        E2 g[1 << sp::MAX_B];
+        for (int m = 0; m < (1 << end.rounds); m++) g[m] = ld(dev.sums() + 2 * (((size_t)i << end.rounds) + m));
+        for (int j = 0; j < end.rounds; j++)
+            for (int m = 0; m < (1 << (end.rounds - j - 1)); m++)
+                g[m] = add(g[2 * m], mul(R[end.first + j], sub(g[2 * m + 1], g[2 * m])));
+        h_f_evals[2 * i] = g[0].c0;
+        h_f_evals[2 * i + 1] = g[0].c1;
+        t.append_ext2(SP_LABEL(L_FEVAL), g[0].c0, g[0].c1);
     }
-    const E2 v = fin.value();
-    h_final_eval[0] = v.c0;
-    h_final_eval[1] = v.c1;
+    h_final_eval[0] = u[0].c0;
+    h_final_eval[1] = u[0].c1;
     return MB_OK;
 }
 

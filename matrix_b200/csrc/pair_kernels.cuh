@@ -139,11 +139,11 @@ __device__ __forceinline__ uint64_t grid_value(uint64_t lo, uint64_t hi) {
     const unsigned __int128 x = ((unsigned __int128)hi << 32) + lo;
     return F::canon(F::red(gl::Acc{(uint32_t)x, (uint32_t)(x >> 32), (uint32_t)(x >> 64), (uint32_t)(x >> 96), 0}));
 }
-// after every thread's grid_add: true in the block that is through last (uniform over the block's `threads`)
-__device__ __forceinline__ bool grid_last(uint64_t* acc, bool* flag) {
+// after every thread's grid_add: true in the block that is through last of the `of` that add (uniform over the block)
+__device__ __forceinline__ bool grid_last(uint64_t* acc, bool* flag, unsigned of) {
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) *flag = atomicAdd(reinterpret_cast<unsigned*>(acc), 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) *flag = atomicAdd(reinterpret_cast<unsigned*>(acc), 1u) == of - 1;
     __syncthreads();
     if (!*flag) return false;
     __threadfence();
@@ -184,7 +184,7 @@ __device__ __forceinline__ bool grid_sum(typename F::E2 (&v)[V], int bits, typen
 #pragma unroll
             for (int j = 0; j < V; j++) grid_add(acc, j * n + t, x[j].c0, x[j].c1);
         }
-        if (!grid_last(acc, &last)) return false;
+        if (!grid_last(acc, &last, gridDim.x)) return false;
         if (t < n) {
 #pragma unroll
             for (int j = 0; j < V; j++) x[j] = grid_take<F>(acc, j * n + t);

@@ -14,10 +14,15 @@
 // additions (bits_pass), and the first extension table, 1/64 of the witness, comes from eight table look-ups per
 // word (fold_pass with SRC 1 or 2).
 //
+// The B rounds' polynomial over all leaves, sum_i scale_i prod_j eq(r_ij, c_j) G_i(c), has degree two in each variable, so
+// 3^B values (at 0, 1 and infinity) hold it: the block that finishes a leaf's G multiplies it out and adds it to the others'
+// (leaf_share), and the host runs the rounds on at most 81 elements, whatever the number of leaves.
+//
 // Arity 22, 42 binary leaves: what the proof reads from DRAM is the 22 MB of bits; the largest table is 44 MB.
 // bits_pass is bound by the integer pipe (18 instructions per word and warp), the other passes by launch latency.
 #pragma once
 #include "agl_traits.cuh"
+#include "pair_kernels.cuh"
 
 namespace mb {
 namespace sp {
@@ -111,6 +116,56 @@ __device__ __forceinline__ bool leaf_sum(E2 v, int bits, E2* sm, uint64_t* parti
     block_sum(x);
     if (t == 0) *counter = 0;
     return true;
+}
+
+// ---- the rounds' polynomial over the leaves -----------------------------------------------------------
+constexpr int SHARE = 81;      // 3^MAX_B
+// Leaf share of the values at {0, 1, inf}^B, variable 0 the lowest digit, from the leaf's 2^B sums g (shared memory), added to the
+// other leaves'; the block that adds the last one writes them to u (pinned) and leaves acc zero. r: the leaf's
+// coordinates of the B variables; acc: pr::grid_words(SHARE).
+__device__ __forceinline__ void leaf_share(const E2* g, int B, const uint64_t* r, E2 scale, unsigned leaves, uint64_t* acc, uint64_t* u) {
+    __shared__ E2 f[3 * MAX_B], buf[2][SHARE];
+    __shared__ bool last;
+    const int t = threadIdx.x;
+    if (t < 3 * B) {   // c^0 .. : 1 - r at 0, r at 1, 2 r - 1 the coefficient of c^2 with g(1) - g(0)
+        const E2 x = agl::e2_load(r + 2 * (t / 3)), one{1, 0};
+        E2 v = t % 3 == 0 ? agl::e2_sub(one, x) : t % 3 == 1 ? x : agl::e2_sub(agl::e2_add(x, x), one);
+        if (t < 3) v = agl::e2_mul_lazy(v, scale);
+        f[t] = v;
+    }
+    __syncthreads();
+    int low = 1, high = 1 << (B - 1);
+    for (int j = 0; j < B; j++, low *= 3, high /= 2) {
+        const E2* in = j == 0 ? g : buf[(j - 1) & 1];
+        if (t < 3 * low * high) {
+            const int l = t % low, p = (t / low) % 3, h = t / (3 * low);
+            const E2 g0 = in[l + low * 2 * h], g1 = in[l + low * (2 * h + 1)];
+            buf[j & 1][t] = agl::e2_mul_lazy(f[3 * j + p], p == 0 ? g0 : p == 1 ? g1 : agl::e2_sub(g1, g0));
+        }
+        __syncthreads();
+    }
+    if (t < low) {
+        const E2 v = agl::e2_canon(buf[(B - 1) & 1][t]);
+        pr::grid_add(acc, t, v.c0, v.c1);
+    }
+    if (!pr::grid_last(acc, &last, leaves)) return;
+    if (t < low) agl::e2_store(u + 2 * t, pr::grid_take<pr::AglF>(acc, t));
+}
+// The same for the sums of the first pass, which is queued before alpha is known: leaf i's scale is alpha^i.
+static __global__ void __launch_bounds__(BLK)
+first_share_kernel(const uint64_t* __restrict__ sums, int B, const uint64_t* __restrict__ pts, int arity, E2 alpha,
+                   uint64_t* __restrict__ scale, uint64_t* acc, uint64_t* u) {
+    __shared__ E2 g[1 << MAX_B];
+    const int leaf = blockIdx.x, t = threadIdx.x;
+    if (t < (1 << B)) g[t] = agl::e2_load(sums + 2 * (((size_t)leaf << B) + t));
+    E2 s{1, 0}, p = alpha;
+    for (int e = leaf; e > 0; e >>= 1) {
+        if (e & 1) s = agl::e2_mul_lazy(s, p);
+        if (e > 1) p = agl::e2_mul_lazy(p, p);
+    }
+    if (t == 0) agl::e2_store(scale + 2 * (size_t)leaf, agl::e2_canon(s));
+    __syncthreads();
+    leaf_share(g, B, pts + 2 * (size_t)arity * leaf, s, gridDim.x, acc, u);
 }
 
 // ---- pass over the packed words ----------------------------------------------------------------------
@@ -210,7 +265,12 @@ struct FoldArgs {
     size_t leaf_words, wl_off, wh_off;   // over variables next .. t_bits and t_bits .. v of the folded table
     uint64_t* partial;              // [leaf][gridDim.x][2^next][2]
     unsigned* counter;
-    uint64_t* out;                  // pinned: [leaf][2^next][2]
+    uint64_t* out;                  // pinned: [leaf][2^next][2], or null
+    // the rounds' polynomial (u null: not yet, alpha is not known): scale_i takes in `bound` variables from first - bound on
+    const uint64_t* pts;
+    int arity, first, bound;        // first: the variable the stage starts at
+    uint64_t *scale, *acc, *u;      // [leaf][2]; pr::grid_words(SHARE); pinned: [3^next][2]
+    E2 r[MAX_B];                    // their challenges
 };
 struct FoldWeights {
     E2Pre w[1 << MAX_B];            // eq of the challenges, index bit k: challenge k
@@ -284,7 +344,24 @@ fold_pass_kernel(const FoldArgs a, const __grid_constant__ W fw) {
     if (a.next < a.t_bits && t < (1 << a.t_bits))
         single = agl::e2_fma_pre(load_weight(tabs + a.wl_off + 4 * (t >> a.next)), single, E2{0, 0});
     if (!leaf_sum(single, a.next, sm, a.partial + ((size_t)(2 * gridDim.x) << a.next) * leaf, a.counter + leaf)) return;
-    if (t < (1 << a.next)) agl::e2_store(a.out + 2 * (((size_t)leaf << a.next) + t), sm[t]);
+    if (a.out != nullptr && t < (1 << a.next)) agl::e2_store(a.out + 2 * (((size_t)leaf << a.next) + t), sm[t]);
+    if (a.u == nullptr) return;
+    __shared__ E2 f[MAX_B];
+    const uint64_t* pts = a.pts + 2 * ((size_t)a.arity * leaf + a.first);
+    if (t < MAX_B) {   // eq(r, R) = 1 - r - R + 2 r R
+        E2 v{1, 0};
+        if (t < a.bound) {
+            const E2 x = agl::e2_load(pts + 2 * (t - a.bound)), xr = agl::e2_mul_lazy(x, a.r[t]);
+            v = agl::e2_add(agl::e2_sub(agl::e2_sub(v, x), a.r[t]), agl::e2_add(xr, xr));
+        }
+        f[t] = v;
+    }
+    __syncthreads();
+    const E2 scale = agl::e2_canon(agl::e2_mul_lazy(agl::e2_mul_lazy(agl::e2_mul_lazy(f[0], f[1]), agl::e2_mul_lazy(f[2], f[3])),
+                                                    agl::e2_load(a.scale + 2 * (size_t)leaf)));
+    __syncthreads();
+    if (t == 0) agl::e2_store(a.scale + 2 * (size_t)leaf, scale);
+    leaf_share(sm, a.next, pts, scale, gridDim.y, a.acc, a.u);
 }
 
 }  // namespace sp
