@@ -7,12 +7,14 @@
 // about N (1 + 2^-4) instead of about 3 N.
 //  * The first pass over a base-field table (the large one) is an inner product with the eq vector of the variables it
 //    binds, as exact 160-bit sums (two multiply-accumulate chains per element instead of a reduced fold per level):
-//    six or more variables by warps that stream whole rows (dot_rows_kernel), fewer with the 2^K weights in shared
+//    six or more variables by warps that stream whole rows (dot_rows_kernel), of tables of 2^22 elements and more on the
+//    tensor cores (peval_mma_kernels.cuh), fewer with the 2^K weights in shared
 //    memory (dot_levels_kernel: a block stages 4096 consecutive elements with coalesced 16-byte loads; each thread
 //    then reads its run of 2^K from a padded layout without bank conflicts).
 //  * Other passes (extension tables, what the first left) fold a run of 2^K
 //    consecutive elements through K variables in registers.
 #pragma once
+#include "peval_mma_kernels.cuh"
 #include "sumcheck_kernels.cuh"
 
 namespace mb {
@@ -256,8 +258,13 @@ inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, 
     if (m == 0) return MB_OK;
     // dot_rows_kernel reads pairs of elements, and eight warps of 64 elements or more make a block
     int first_vars = 0;
+    bool mma = false;
     if constexpr (FIn::NW == 1 && FOut::NW == 2)
-        if (m >= 6 && log_n >= 9 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) first_vars = dot_rows_vars(log_n, m);
+        if (m >= 6 && log_n >= 9 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) {
+            first_vars = dot_mma_vars(log_n, m);
+            mma = first_vars > 0;
+            if (!mma) first_vars = dot_rows_vars(log_n, m);
+        }
     int passes = first_vars ? 1 + (m - first_vars + K_MAX - 1) / K_MAX : (m + K_MAX - 1) / K_MAX;
     if (passes > 1 && !d_tmp) return MB_ERR_ARG;
     // ping-pong so that the last pass lands in d_out
@@ -272,7 +279,11 @@ inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, 
         uint64_t* dst = bufs[which];
         bool done = false;
         if constexpr (FIn::NW == 1 && FOut::NW == 2) {
-            if (first && first_vars) {
+            if (first && mma) {
+                int rc = launch_dot_mma<FOut>(src, dst, d_r, k, n_out, st);
+                if (rc != MB_OK) return rc;
+                done = true;
+            } else if (first && first_vars) {
                 launch_dot_rows<FIn, FOut>(src, dst, d_r, lvl, k, n_out, st);
                 done = true;
             } else if (first && n_out >= 256) {

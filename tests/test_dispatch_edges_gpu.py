@@ -105,7 +105,8 @@ def test_poseidon2_with_a_missed_carry(gl, oracle):
         assert list(got[k]) == list(s), k
 
 
-@pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15)])
+@pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
+                                     (22, 6), (22, 9), (24, 10), (24, 13)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):
     for lib, mod, fn, ofn in ((load_agl(), AGL_Q, load_agl().agl_partial_eval_ext2_from_base_ffi, oracle.oracle_agl_partial_eval_ext2_from_base),
                               (gl, GL_P, gl.partial_eval_ext2_from_gl_ffi, oracle.oracle_gl_partial_eval_ext2_from_base)):
