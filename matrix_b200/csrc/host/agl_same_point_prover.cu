@@ -15,9 +15,9 @@
 // the CPU prover's (heterogeneous arities stay on that path, as in the reference).
 //
 // Device side (same_point_kernels.cuh): the eq polynomials stay factored, and one pass over a table serves up to four
-// rounds (six for the packed witness): it returns the 3^B values of the rounds' polynomial over all leaves, on which the host
-// runs the messages and folds of B rounds, and the next pass folds the B challenges at once. (With 2^B sums per leaf returned
-// the host's rounds over 42 leaves took 200 of 686 us.) The first pass is queued before the header of
+// rounds (six for the packed witness): it returns the 3^B values of the rounds' polynomial over all leaves, or 2^B eq-weighted
+// sums per leaf where there are few, on which the host runs the messages and folds of B rounds, and the next pass folds the B
+// challenges at once. The first pass is queued before the header of
 // the transcript (every claim point, label by label), which the host absorbs while the device works: after the pass
 // that header is the longest part of a proof. The reference launches a message and a fold kernel per round over eq and f
 // tables; with one fused pass per round over both tables, arity 22 and 42 binary leaves took 7.4 ms and 11 GB.
@@ -81,6 +81,31 @@ E2 mul(E2 a, E2 b) {   // canonical words in and out, on the host core's multipl
 }
 E2 add(E2 a, E2 b) { return E2{hf::agl_add(a.c0, b.c0), hf::agl_add(a.c1, b.c1)}; }
 E2 sub(E2 a, E2 b) { return E2{hf::agl_sub(a.c0, b.c0), hf::agl_sub(a.c1, b.c1)}; }
+// sum of products, reduced once
+struct Dot {
+    struct Wide {
+        hf::u128 s = 0;
+        uint64_t top = 0;
+        void mac(uint64_t x, uint64_t y) {
+            const hf::u128 p = (hf::u128)x * y;
+            s += p;
+            top += s < p;
+        }
+        // 2^128 = 63 2^32 + 992 (mod q)
+        uint64_t red() const { return hf::agl_red((hf::u128)top * (63ULL * (1ULL << 32) + 992ULL) + hf::agl_red(s)); }
+    };
+    Wide p00, p11, p01;
+    void mac(E2 a, E2 b) {
+        p00.mac(a.c0, b.c0);
+        p11.mac(a.c1, b.c1);
+        p01.mac(a.c0, b.c1);
+        p01.mac(a.c1, b.c0);
+    }
+    E2 value() const {
+        return E2{hf::agl_canon(hf::agl_red((hf::u128)p11.red() * 3 + p00.red())), hf::agl_canon(p01.red())};
+    }
+};
+
 // A block of rounds from variable `first` on, and what the pass before it reads.
 enum Source { FROM_WITNESS, FROM_WORD_SUMS, FROM_WORDS, FROM_TABLE };
 struct Stage {
@@ -122,9 +147,10 @@ public:
         if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);
     }
     // Stages of the proof, eq tables of all passes, and the first pass, all queued; the sums of the first stage are in
-    // sums() after a stream synchronisation. claims_only: nothing after the first pass will be asked for.
-    int init(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool claims_only) {
-        M_ = M; k_ = arity; kind_ = kind; w0_ = d_w0; w1_ = d_w1;
+    // sums() after a stream synchronisation. claims_only: nothing after the first pass will be asked for; share: later stages
+    // return the values of their rounds' polynomial, else each leaf's sums.
+    int init(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool claims_only, bool share) {
+        M_ = M; share_ = share; k_ = arity; kind_ = kind; w0_ = d_w0; w1_ = d_w1;
         const int inside = kind == 2 ? 0 : (arity < sp::BITS ? arity : sp::BITS);
         words_ = arity >= 6 ? (size_t)1 << (arity - 6) : 1;
         if (inside) {
@@ -168,7 +194,7 @@ public:
         MB_CUDA(pool_alloc((void**)&b_.tabs, sizeof(uint64_t) * leaf_words_ * M));
         MB_CUDA(pool_alloc((void**)&b_.partial, sizeof(uint64_t) * 2 * 64 * (size_t)cap * M));
         MB_CUDA(pool_alloc((void**)&b_.counter, sizeof(unsigned) * M));
-        if (!claims_only) {
+        if (share_) {
             MB_CUDA(pool_alloc((void**)&b_.scale, sizeof(uint64_t) * 2 * (size_t)M));
             scratch_ = ScratchPool::take();
             if (!scratch_) return MB_ERR_CUDA;
@@ -219,8 +245,8 @@ public:
         a.t_bits = a.v < 8 ? a.v : 8;
         a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = s.wl; a.wh_off = s.wh;
         a.partial = b_.partial; a.counter = b_.counter;
-        a.out = i == 0 || i + 1 == stages_.size() ? h_sums_ : nullptr;   // for the first share; for the reveals
-        if (i > 0) {
+        a.out = !share_ || i == 0 || i + 1 == stages_.size() ? h_sums_ : nullptr;   // for the first share; for the reveals
+        if (share_ && i > 0) {
             a.pts = b_.pts; a.arity = k_; a.first = s.first; a.bound = stages_[i - 1].rounds;
             a.scale = b_.scale; a.acc = scratch_.dev; a.u = scratch_.host;
             for (int j = 0; j < a.bound; j++) a.r[j] = r[count - a.bound + j];
@@ -268,7 +294,7 @@ public:
         return finish_async();
     }
     const std::vector<Stage>& stages() const { return stages_; }
-    const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the first stage, then of the last
+    const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the stage queued last; share: of the first or the last
     const uint64_t* values() const { return scratch_.host; }   // [3^rounds][2] of the stage queued last
 
 private:
@@ -286,7 +312,7 @@ private:
     size_t words_ = 1, leaf_words_ = 0;
     const uint64_t *w0_ = nullptr, *w1_ = nullptr;
     uint64_t *h_sums_ = nullptr, *cur_ = nullptr;
-    bool flip_ = false;
+    bool flip_ = false, share_ = false;
     std::vector<Stage> stages_;
     ScratchBlock scratch_;
     Buffers b_;
@@ -300,7 +326,7 @@ int same_point_claims(int M, int arity, const uint64_t* h_pts, int kind, const u
     if (M < 1 || M > 4096 || arity < 1 || arity > 32 || !h_pts || !d_w0 || kind < 0 || kind > 2 || (kind == 1 && !d_w1) || !h_vals)
         return MB_ERR_ARG;
     SamePointDevice dev;
-    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, true);
+    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, true, false);
     if (rc != MB_OK) return rc;
     MB_CUDA(cudaStreamSynchronize(MB_STREAM));
     const int b = dev.stages()[0].rounds;
@@ -316,24 +342,119 @@ int same_point_claims(int M, int arity, const uint64_t* h_pts, int kind, const u
     return MB_OK;
 }
 
-// kind 0: d_w0 = packed bits [M][words]; 1: d_w0 / d_w1 = +1 / -1 masks [M][words]; 2: d_w0 = extension tables
-// [M][2^arity][2]. words = max(1, 2^(arity - 6)).
-int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_vals, int kind, const uint64_t* d_w0,
-                     const uint64_t* d_w1, AglTranscript& t, uint64_t* h_round_msgs, uint64_t* h_challenges, uint64_t* h_f_evals,
-                     uint64_t* h_final_eval) {
-    if (M < 1 || M > 4096 || arity < 1 || arity > 32 || !h_pts || !h_vals || !d_w0 || kind < 0 || kind > 2 || (kind == 1 && !d_w1) ||
-        !h_round_msgs || !h_f_evals || !h_final_eval)
-        return MB_ERR_ARG;
-    // the first pass does not depend on alpha: it is queued first, and the header of the transcript (every claim
-    // point, label by label) is absorbed while the device works
-    SamePointDevice dev;
-    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, false);
-    if (rc != MB_OK) return rc;
-    header(t, M, arity, h_pts, h_vals);
-    const E2 alpha = challenge(t, SP_LABEL(L_ALPHA));
+// Leaves from which their shares are added up on the device: that takes about 25 us more for the first stage and 8 for each of the
+// others, the host's sums 0.2 us a leaf and round (4 leaves of arity 8: 99 us by leaf, 136 by share; 20 of arity 12 219 and 240; 7 of
+// arity 18 195 and 237; 42 of arity 22 688 and 554).
+constexpr int SHARE_FROM = 24;
+
+namespace {
+// The rounds on the 2^B sums of each leaf.
+int rounds_by_leaf(SamePointDevice& dev, int M, int arity, const uint64_t* h_pts, E2 alpha, AglTranscript& t, uint64_t* h_round_msgs,
+                   uint64_t* h_challenges, uint64_t* h_f_evals, uint64_t* h_final_eval) {
+    // scale_i = alpha^i eq(r_i[0 .. j), R[0 .. j))
+    std::vector<E2> scale(M);
+    E2 pw{1, 0};
+    for (int i = 0; i < M; i++) { scale[i] = pw; pw = mul(pw, alpha); }
+
+    std::vector<E2> R(arity), g((size_t)M << sp::MAX_B), up(M), down(M);
+    // suffix eq tables of the block's variables, per leaf: 2^(rounds - 1 - j) entries for round j, back to back
+    std::vector<E2> suffix((size_t)M << sp::MAX_B);
+    bool label_absorbed = false;
+    for (size_t si = 0; si < dev.stages().size(); si++) {
+        const Stage st = dev.stages()[si];
+        if (si > 0) {
+            // the challenges that the pass consumes: all of a word's for the first extension table
+            const int from = st.source == FROM_WORDS ? 0 : dev.stages()[si - 1].first;
+            int rc = dev.fold(si, R.data() + from, st.first - from);
+            if (rc != MB_OK) return rc;
+        }
+        if (si > 0) {   // while the pass runs
+            t.begin_append(SP_LABEL(L_MSG));
+            label_absorbed = true;
+        }
+        const int B = st.rounds, size = 1 << B;
+        for (int i = 0; i < M; i++) {
+            // tables for rounds B - 1, B - 2, ..: each from the one before by its lowest variable
+            E2* w = suffix.data() + ((size_t)i << B);
+            w[0] = E2{1, 0};
+            int at = 0;
+            for (int j = B - 2; j >= 0; j--) {
+                const E2 rj = ld(h_pts + 2 * ((size_t)i * arity + st.first + j + 1));
+                const int n = 1 << (B - 2 - j);
+                for (int y = 0; y < n; y++) {
+                    const E2 hi = mul(w[at + y], rj);
+                    w[at + n + 2 * y + 1] = hi;
+                    w[at + n + 2 * y] = sub(w[at + y], hi);
+                }
+                at += n;
+            }
+        }
+        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        for (size_t x = 0; x < (size_t)M * size; x++) g[x] = E2{dev.sums()[2 * x], dev.sums()[2 * x + 1]};
+        for (int j = 0; j < B; j++) {
+            const int round = st.first + j, half = size >> (j + 1);
+            // T_i(c) = scale_i ((1 - r)(1 - c) + r c) (A + c (B - A)) with A, B the weighted even and odd sums;
+            // with u = scale (1 - r), v = scale r: T(0) = u A, T(1) = v B, T(2) = (2 v - u)(2 B - A)
+            Dot m0, m1, m2;
+            for (int i = 0; i < M; i++) {
+                const E2* w = suffix.data() + ((size_t)i << B) + (half - 1);
+                const E2* gi = g.data() + (size_t)i * size;
+                E2 a = gi[0], b = gi[1];
+                if (half > 1) {
+                    Dot da, db;
+                    for (int y = 0; y < half; y++) { da.mac(w[y], gi[2 * y]); db.mac(w[y], gi[2 * y + 1]); }
+                    a = da.value();
+                    b = db.value();
+                }
+                up[i] = mul(scale[i], ld(h_pts + 2 * ((size_t)i * arity + round)));
+                down[i] = sub(scale[i], up[i]);
+                m0.mac(down[i], a);
+                m1.mac(up[i], b);
+                m2.mac(sub(add(up[i], up[i]), down[i]), sub(add(b, b), a));
+            }
+            const E2 msg[3] = {m0.value(), m1.value(), m2.value()};
+            for (int c = 0; c < 3; c++) {
+                if (c > 0 || !label_absorbed) t.begin_append(SP_LABEL(L_MSG));
+                t.finish_append_ext2(msg[c].c0, msg[c].c1);
+                h_round_msgs[((size_t)round * 3 + c) * 2] = msg[c].c0;
+                h_round_msgs[((size_t)round * 3 + c) * 2 + 1] = msg[c].c1;
+            }
+            label_absorbed = false;
+            const E2 r = challenge(t, SP_LABEL(L_CH));
+            R[round] = r;
+            if (h_challenges) { h_challenges[2 * round] = r.c0; h_challenges[2 * round + 1] = r.c1; }
+            const bool last = si + 1 == dev.stages().size();
+            for (int i = 0; i < M; i++) {
+                scale[i] = add(down[i], mul(r, sub(up[i], down[i])));
+                if (j + 1 == B && !last) continue;   // the next pass folds
+                E2* gi = g.data() + (size_t)i * size;
+                for (int y = 0; y < half; y++) gi[y] = add(gi[2 * y], mul(r, sub(gi[2 * y + 1], gi[2 * y])));
+            }
+        }
+        if (si + 1 == dev.stages().size())
+            for (int i = 0; i < M; i++) {   // nothing is left to sum over: the folded sums are the reveals f_i(R)
+                h_f_evals[2 * i] = g[(size_t)i * size].c0;
+                h_f_evals[2 * i + 1] = g[(size_t)i * size].c1;
+            }
+    }
+    Dot fin;
+    for (int i = 0; i < M; i++) {
+        t.append_ext2(SP_LABEL(L_FEVAL), h_f_evals[2 * i], h_f_evals[2 * i + 1]);
+        fin.mac(scale[i], E2{h_f_evals[2 * i], h_f_evals[2 * i + 1]});   // scale_i = alpha^i eq(r_i, R)
+    }
+    const E2 v = fin.value();
+    h_final_eval[0] = v.c0;
+    h_final_eval[1] = v.c1;
+    return MB_OK;
+}
+
+// The rounds on the values of their polynomial over all leaves.
+int rounds_by_share(SamePointDevice& dev, int M, int arity, E2 alpha, AglTranscript& t, uint64_t* h_round_msgs, uint64_t* h_challenges,
+                    uint64_t* h_f_evals, uint64_t* h_final_eval) {
     std::vector<E2> R(arity), u(sp::SHARE);
     for (size_t si = 0; si < dev.stages().size(); si++) {
         const Stage st = dev.stages()[si];
+        int rc;
         if (si > 0) {
             // the challenges that the pass consumes: all of a word's for the first extension table
             const int from = st.source == FROM_WORDS ? 0 : dev.stages()[si - 1].first;
@@ -388,6 +509,27 @@ int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_
     h_final_eval[0] = u[0].c0;
     h_final_eval[1] = u[0].c1;
     return MB_OK;
+}
+
+}  // namespace
+
+// kind 0: d_w0 = packed bits [M][words]; 1: d_w0 / d_w1 = +1 / -1 masks [M][words]; 2: d_w0 = extension tables
+// [M][2^arity][2]. words = max(1, 2^(arity - 6)).
+int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_vals, int kind, const uint64_t* d_w0,
+                     const uint64_t* d_w1, AglTranscript& t, uint64_t* h_round_msgs, uint64_t* h_challenges, uint64_t* h_f_evals,
+                     uint64_t* h_final_eval) {
+    if (M < 1 || M > 4096 || arity < 1 || arity > 32 || !h_pts || !h_vals || !d_w0 || kind < 0 || kind > 2 || (kind == 1 && !d_w1) ||
+        !h_round_msgs || !h_f_evals || !h_final_eval)
+        return MB_ERR_ARG;
+    // the first pass does not depend on alpha: it is queued first, and the header of the transcript (every claim
+    // point, label by label) is absorbed while the device works
+    SamePointDevice dev;
+    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, false, M >= SHARE_FROM);
+    if (rc != MB_OK) return rc;
+    header(t, M, arity, h_pts, h_vals);
+    const E2 alpha = challenge(t, SP_LABEL(L_ALPHA));
+    return M < SHARE_FROM ? rounds_by_leaf(dev, M, arity, h_pts, alpha, t, h_round_msgs, h_challenges, h_f_evals, h_final_eval)
+                          : rounds_by_share(dev, M, arity, alpha, t, h_round_msgs, h_challenges, h_f_evals, h_final_eval);
 }
 
 // verify_same_point for instances of any arity <= num_vars: pts are concatenated (arity[i] pairs each).

@@ -19,7 +19,7 @@ struct ScratchBlock {
 class ScratchPool {
 public:
     static constexpr size_t WORDS = 8192;       // host: 64 KB
-    static constexpr size_t DEV_WORDS = 5120;   // device: 40 KB
+    static constexpr size_t DEV_WORDS = 33280;  // device: 260 KB (64 instances of sixteen sums in eight copies)
     static constexpr size_t MAX_KEPT = 32;
     static ScratchBlock take() {
         ScratchBlock b;

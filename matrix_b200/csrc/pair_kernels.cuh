@@ -122,11 +122,14 @@ __device__ __forceinline__ typename F::Pre load_weight(const uint64_t* p) {
 // counts the blocks that are through, from word 8 on there are four words an entry, the sums of the low and high halves
 // of the blocks' canonical words (exact for 2^32 blocks). A block adds its entries with atomics that nobody waits for, so
 // the one that finishes last reads each sum once, whatever the grid. (With rows of partial sums it read them all: 148
-// rows of 256 entries, 600 KB, took it 7 us; in two levels a fence and a ticket more.)
+// rows of 256 entries, 600 KB, took it 7 us; in two levels a fence and a ticket more.) Where there are few sums, blocks add to one
+// of several copies: 1184 blocks on the same sixteen sums waited 20 us for one another.
 constexpr int ACC_FIRST = 8;
-__host__ __device__ constexpr size_t grid_words(size_t entries) { return ACC_FIRST + 4 * entries; }
-__device__ __forceinline__ void grid_add(uint64_t* acc, int entry, uint64_t c0, uint64_t c1) {
-    unsigned long long* p = reinterpret_cast<unsigned long long*>(acc + ACC_FIRST + 4 * (size_t)entry);
+__host__ __device__ constexpr int grid_copies(int entries) { return entries >= 128 ? 1 : entries <= 8 ? 16 : 128 / entries; }
+__host__ __device__ constexpr size_t grid_words(int entries) { return ACC_FIRST + 4 * (size_t)entries * grid_copies(entries); }
+__device__ __forceinline__ void grid_add(uint64_t* acc, int entries, unsigned block, int entry, uint64_t c0, uint64_t c1) {
+    const size_t at = (size_t)(block % grid_copies(entries)) * entries + entry;
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(acc + ACC_FIRST + 4 * at);
     atomicAdd(p, (unsigned long long)gl::lo32(c0));
     atomicAdd(p + 1, (unsigned long long)gl::hi32(c0));
     if (c1 != 0) {
@@ -152,10 +155,15 @@ __device__ __forceinline__ bool grid_last(uint64_t* acc, bool* flag, unsigned of
 }
 // the sum of an entry, which is zero afterwards
 template <class F>
-__device__ __forceinline__ typename F::E2 grid_take(uint64_t* acc, int entry) {
+__device__ __forceinline__ typename F::E2 grid_take(uint64_t* acc, int entries, int entry) {
+    ulonglong2 a = make_ulonglong2(0, 0), b = a;
     ulonglong2* p = reinterpret_cast<ulonglong2*>(acc + ACC_FIRST + 4 * (size_t)entry);
-    const ulonglong2 a = __ldcg(p), b = __ldcg(p + 1);
-    p[0] = p[1] = make_ulonglong2(0, 0);
+#pragma unroll 4
+    for (int c = 0; c < grid_copies(entries); c++, p += 2 * entries) {
+        const ulonglong2 x = __ldcg(p), y = __ldcg(p + 1);
+        p[0] = p[1] = make_ulonglong2(0, 0);
+        a.x += x.x; a.y += x.y; b.x += y.x; b.y += y.y;
+    }
     return typename F::E2{grid_value<F>(a.x, a.y), grid_value<F>(b.x, b.y)};
 }
 
@@ -182,12 +190,12 @@ __device__ __forceinline__ bool grid_sum(typename F::E2 (&v)[V], int bits, typen
     if (gridDim.x > 1) {
         if (t < n) {
 #pragma unroll
-            for (int j = 0; j < V; j++) grid_add(acc, j * n + t, x[j].c0, x[j].c1);
+            for (int j = 0; j < V; j++) grid_add(acc, V * n, blockIdx.x, j * n + t, x[j].c0, x[j].c1);
         }
         if (!grid_last(acc, &last, gridDim.x)) return false;
         if (t < n) {
 #pragma unroll
-            for (int j = 0; j < V; j++) x[j] = grid_take<F>(acc, j * n + t);
+            for (int j = 0; j < V; j++) x[j] = grid_take<F>(acc, V * n, j * n + t);
         }
     }
     __syncthreads();

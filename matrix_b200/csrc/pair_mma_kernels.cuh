@@ -411,9 +411,9 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
     const int E = 1 << (2 * a.g);
     if (gridDim.x > 1) {
         uint64_t* acc = a.acc + grid_words(E) * k;
-        if (t < E) grid_add(acc, t, F::canon(sum.c0), F::canon(sum.c1));
+        if (t < E) grid_add(acc, E, blockIdx.x, t, F::canon(sum.c0), F::canon(sum.c1));
         if (!grid_last(acc, &last_sm, gridDim.x)) return;
-        if (t < E) sum = grid_take<F>(acc, t);
+        if (t < E) sum = grid_take<F>(acc, E, t);
     }
     if (t < E) store2(a.sums + 2 * ((size_t)k * E + t), F::canon(sum.c0), F::canon(sum.c1));
 }

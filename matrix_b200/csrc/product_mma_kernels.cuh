@@ -277,9 +277,9 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
         else sum = E2{F::canon(MmaField<F>::add(r[0], F::times_w(r[19]))), F::canon(MmaField<F>::add(r[1], r[18]))};
     }
     if (gridDim.x > 1) {
-        if (t < TRI_ENTRIES) grid_add(a.acc, t, sum.c0, sum.c1);
+        if (t < TRI_ENTRIES) grid_add(a.acc, TRI_ENTRIES, blockIdx.x, t, sum.c0, sum.c1);
         if (!grid_last(a.acc, &last_sm, gridDim.x)) return;
-        if (t < TRI_ENTRIES) sum = grid_take<F>(a.acc, t);
+        if (t < TRI_ENTRIES) sum = grid_take<F>(a.acc, TRI_ENTRIES, t);
     }
     if (t < TRI_ENTRIES) store2(a.sums + 2 * t, sum.c0, sum.c1);
 }

@@ -122,8 +122,8 @@ __device__ __forceinline__ bool leaf_sum(E2 v, int bits, E2* sm, uint64_t* parti
 constexpr int SHARE = 81;      // 3^MAX_B
 // Leaf share of the values at {0, 1, inf}^B, variable 0 the lowest digit, from the leaf's 2^B sums g (shared memory), added to the
 // other leaves'; the block that adds the last one writes them to u (pinned) and leaves acc zero. r: the leaf's
-// coordinates of the B variables; acc: pr::grid_words(SHARE).
-__device__ __forceinline__ void leaf_share(const E2* g, int B, const uint64_t* r, E2 scale, unsigned leaves, uint64_t* acc, uint64_t* u) {
+// coordinates of the B variables; acc: pr::grid_words(3^B).
+__device__ __forceinline__ void leaf_share(const E2* g, int B, const uint64_t* r, E2 scale, unsigned leaf, unsigned leaves, uint64_t* acc, uint64_t* u) {
     __shared__ E2 f[3 * MAX_B], buf[2][SHARE];
     __shared__ bool last;
     const int t = threadIdx.x;
@@ -146,10 +146,10 @@ __device__ __forceinline__ void leaf_share(const E2* g, int B, const uint64_t* r
     }
     if (t < low) {
         const E2 v = agl::e2_canon(buf[(B - 1) & 1][t]);
-        pr::grid_add(acc, t, v.c0, v.c1);
+        pr::grid_add(acc, low, leaf, t, v.c0, v.c1);
     }
     if (!pr::grid_last(acc, &last, leaves)) return;
-    if (t < low) agl::e2_store(u + 2 * t, pr::grid_take<pr::AglF>(acc, t));
+    if (t < low) agl::e2_store(u + 2 * t, pr::grid_take<pr::AglF>(acc, low, t));
 }
 // The same for the sums of the first pass, which is queued before alpha is known: leaf i's scale is alpha^i.
 static __global__ void __launch_bounds__(BLK)
@@ -165,7 +165,7 @@ first_share_kernel(const uint64_t* __restrict__ sums, int B, const uint64_t* __r
     }
     if (t == 0) agl::e2_store(scale + 2 * (size_t)leaf, agl::e2_canon(s));
     __syncthreads();
-    leaf_share(g, B, pts + 2 * (size_t)arity * leaf, s, gridDim.x, acc, u);
+    leaf_share(g, B, pts + 2 * (size_t)arity * leaf, s, leaf, gridDim.x, acc, u);
 }
 
 // ---- pass over the packed words ----------------------------------------------------------------------
@@ -269,7 +269,7 @@ struct FoldArgs {
     // the rounds' polynomial (u null: not yet, alpha is not known): scale_i takes in `bound` variables from first - bound on
     const uint64_t* pts;
     int arity, first, bound;        // first: the variable the stage starts at
-    uint64_t *scale, *acc, *u;      // [leaf][2]; pr::grid_words(SHARE); pinned: [3^next][2]
+    uint64_t *scale, *acc, *u;      // [leaf][2]; pr::grid_words(3^next); pinned: [3^next][2]
     E2 r[MAX_B];                    // their challenges
 };
 struct FoldWeights {
@@ -361,7 +361,7 @@ fold_pass_kernel(const FoldArgs a, const __grid_constant__ W fw) {
                                                     agl::e2_load(a.scale + 2 * (size_t)leaf)));
     __syncthreads();
     if (t == 0) agl::e2_store(a.scale + 2 * (size_t)leaf, scale);
-    leaf_share(sm, a.next, pts, scale, gridDim.y, a.acc, a.u);
+    leaf_share(sm, a.next, pts, scale, leaf, gridDim.y, a.acc, a.u);
 }
 
 }  // namespace sp
