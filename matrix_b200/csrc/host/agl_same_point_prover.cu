@@ -275,8 +275,8 @@ public:
             for (int j = 1 << count; j < 64; j++) w.w[j] = E2{0, 0};
             MB_KERNEL("same_point_words");
             constexpr int lut = 8 * 256 * 16;
-            if (kind_ == 1) sp::fold_pass_kernel<0, 2, sp::WordWeights><<<grid, sp::BLK, lut, MB_STREAM>>>(a, w);
-            else sp::fold_pass_kernel<0, 1, sp::WordWeights><<<grid, sp::BLK, lut, MB_STREAM>>>(a, w);
+            if (kind_ == 1) launch<0, 2>(a.u != nullptr, grid, lut, a, w);
+            else launch<0, 1>(a.u != nullptr, grid, lut, a, w);
             return finish_async();
         }
         sp::FoldWeights w;
@@ -285,11 +285,11 @@ public:
         for (int j = 0; j < (1 << count); j++) w.w[j] = agl::e2_pre(e[j]);
         MB_KERNEL("same_point_fold");
         switch (count) {
-            case 0: sp::fold_pass_kernel<0, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
-            case 1: sp::fold_pass_kernel<1, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
-            case 2: sp::fold_pass_kernel<2, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
-            case 3: sp::fold_pass_kernel<3, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
-            default: sp::fold_pass_kernel<4, 0, sp::FoldWeights><<<grid, sp::BLK, 0, MB_STREAM>>>(a, w); break;
+            case 0: launch<0, 0>(a.u != nullptr, grid, 0, a, w); break;
+            case 1: launch<1, 0>(a.u != nullptr, grid, 0, a, w); break;
+            case 2: launch<2, 0>(a.u != nullptr, grid, 0, a, w); break;
+            case 3: launch<3, 0>(a.u != nullptr, grid, 0, a, w); break;
+            default: launch<4, 0>(a.u != nullptr, grid, 0, a, w); break;
         }
         return finish_async();
     }
@@ -298,6 +298,11 @@ public:
     const uint64_t* values() const { return scratch_.host; }   // [3^rounds][2] of the stage queued last
 
 private:
+    template <int B, int SRC, class W>
+    static void launch(bool share, dim3 grid, size_t smem, const sp::FoldArgs& a, const W& w) {
+        if (share) sp::fold_pass_kernel<B, SRC, true, W><<<grid, sp::BLK, smem, MB_STREAM>>>(a, w);
+        else sp::fold_pass_kernel<B, SRC, false, W><<<grid, sp::BLK, smem, MB_STREAM>>>(a, w);
+    }
     // out[x] = prod_k (x_k ? r_k : 1 - r_k)
     static void eq_vector(const E2* r, int n, E2* out) {
         out[0] = E2{1, 0};
@@ -342,10 +347,10 @@ int same_point_claims(int M, int arity, const uint64_t* h_pts, int kind, const u
     return MB_OK;
 }
 
-// Leaves from which their shares are added up on the device: that takes about 25 us more for the first stage and 8 for each of the
-// others, the host's sums 0.2 us a leaf and round (4 leaves of arity 8: 99 us by leaf, 136 by share; 20 of arity 12 219 and 240; 7 of
-// arity 18 195 and 237; 42 of arity 22 688 and 554).
-constexpr int SHARE_FROM = 24;
+// Leaves times rounds from which the shares are added up on the device: that takes 60 to 90 us a proof, the host's sums 0.2 us a
+// leaf and round. By leaf / by share, us: 4 leaves of arity 8 99 / 136, 7 of arity 18 195 / 237, 30 of arity 12 267 / 284, 50 of
+// arity 9 301 / 283, 30 of arity 21 497 / 430, 42 of arity 22 688 / 554.
+constexpr int SHARE_FROM = 440;
 
 namespace {
 // The rounds on the 2^B sums of each leaf.
@@ -523,12 +528,13 @@ int same_point_prove(int M, int arity, const uint64_t* h_pts, const uint64_t* h_
         return MB_ERR_ARG;
     // the first pass does not depend on alpha: it is queued first, and the header of the transcript (every claim
     // point, label by label) is absorbed while the device works
+    const bool share = M * arity >= SHARE_FROM;
     SamePointDevice dev;
-    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, false, M >= SHARE_FROM);
+    int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, false, share);
     if (rc != MB_OK) return rc;
     header(t, M, arity, h_pts, h_vals);
     const E2 alpha = challenge(t, SP_LABEL(L_ALPHA));
-    return M < SHARE_FROM ? rounds_by_leaf(dev, M, arity, h_pts, alpha, t, h_round_msgs, h_challenges, h_f_evals, h_final_eval)
+    return !share ? rounds_by_leaf(dev, M, arity, h_pts, alpha, t, h_round_msgs, h_challenges, h_f_evals, h_final_eval)
                           : rounds_by_share(dev, M, arity, alpha, t, h_round_msgs, h_challenges, h_f_evals, h_final_eval);
 }
 

@@ -266,7 +266,7 @@ struct FoldArgs {
     uint64_t* partial;              // [leaf][gridDim.x][2^next][2]
     unsigned* counter;
     uint64_t* out;                  // pinned: [leaf][2^next][2], or null
-    // the rounds' polynomial (u null: not yet, alpha is not known): scale_i takes in `bound` variables from first - bound on
+    // SHARE_OUT: the rounds' polynomial; scale_i takes in `bound` variables from first - bound on
     const uint64_t* pts;
     int arity, first, bound;        // first: the variable the stage starts at
     uint64_t *scale, *acc, *u;      // [leaf][2]; pr::grid_words(3^next); pinned: [3^next][2]
@@ -283,7 +283,8 @@ __device__ __forceinline__ void add_entry(gl::Acc& c0, gl::Acc& c1, ulonglong2 e
     gl::acc_add(c0, e.x);
     gl::acc_add(c1, e.y);
 }
-template <int B, int SRC, class W>
+// SHARE_OUT: the leaf's share of the rounds' polynomial too (the code and its shared memory cost the other form 3 us a pass)
+template <int B, int SRC, bool SHARE_OUT, class W>
 __global__ void __launch_bounds__(BLK)
 fold_pass_kernel(const FoldArgs a, const __grid_constant__ W fw) {
     extern __shared__ ulonglong2 lut[];   // SRC > 0: [8][256]
@@ -345,23 +346,24 @@ fold_pass_kernel(const FoldArgs a, const __grid_constant__ W fw) {
         single = agl::e2_fma_pre(load_weight(tabs + a.wl_off + 4 * (t >> a.next)), single, E2{0, 0});
     if (!leaf_sum(single, a.next, sm, a.partial + ((size_t)(2 * gridDim.x) << a.next) * leaf, a.counter + leaf)) return;
     if (a.out != nullptr && t < (1 << a.next)) agl::e2_store(a.out + 2 * (((size_t)leaf << a.next) + t), sm[t]);
-    if (a.u == nullptr) return;
-    __shared__ E2 f[MAX_B];
-    const uint64_t* pts = a.pts + 2 * ((size_t)a.arity * leaf + a.first);
-    if (t < MAX_B) {   // eq(r, R) = 1 - r - R + 2 r R
-        E2 v{1, 0};
-        if (t < a.bound) {
-            const E2 x = agl::e2_load(pts + 2 * (t - a.bound)), xr = agl::e2_mul_lazy(x, a.r[t]);
-            v = agl::e2_add(agl::e2_sub(agl::e2_sub(v, x), a.r[t]), agl::e2_add(xr, xr));
+    if constexpr (SHARE_OUT) {
+        __shared__ E2 f[MAX_B];
+        const uint64_t* pts = a.pts + 2 * ((size_t)a.arity * leaf + a.first);
+        if (t < MAX_B) {   // eq(r, R) = 1 - r - R + 2 r R
+            E2 v{1, 0};
+            if (t < a.bound) {
+                const E2 x = agl::e2_load(pts + 2 * (t - a.bound)), xr = agl::e2_mul_lazy(x, a.r[t]);
+                v = agl::e2_add(agl::e2_sub(agl::e2_sub(v, x), a.r[t]), agl::e2_add(xr, xr));
+            }
+            f[t] = v;
         }
-        f[t] = v;
+        __syncthreads();
+        const E2 scale = agl::e2_canon(agl::e2_mul_lazy(agl::e2_mul_lazy(agl::e2_mul_lazy(f[0], f[1]), agl::e2_mul_lazy(f[2], f[3])),
+                                                        agl::e2_load(a.scale + 2 * (size_t)leaf)));
+        __syncthreads();
+        if (t == 0) agl::e2_store(a.scale + 2 * (size_t)leaf, scale);
+        leaf_share(sm, a.next, pts, scale, leaf, gridDim.y, a.acc, a.u);
     }
-    __syncthreads();
-    const E2 scale = agl::e2_canon(agl::e2_mul_lazy(agl::e2_mul_lazy(agl::e2_mul_lazy(f[0], f[1]), agl::e2_mul_lazy(f[2], f[3])),
-                                                    agl::e2_load(a.scale + 2 * (size_t)leaf)));
-    __syncthreads();
-    if (t == 0) agl::e2_store(a.scale + 2 * (size_t)leaf, scale);
-    leaf_share(sm, a.next, pts, scale, leaf, gridDim.y, a.acc, a.u);
 }
 
 }  // namespace sp

@@ -105,6 +105,23 @@ def test_poseidon2_with_a_missed_carry(gl, oracle):
         assert list(got[k]) == list(s), k
 
 
+@pytest.mark.parametrize("leaves,ext", [((1 << 20) - 2**19, False), (1 << 20, False), (1 << 20, True), (1 << 21, False)])
+def test_poseidon2_tiles(gl, oracle, leaves, ext):
+    """Layers of 2^20 permutations and more go in tiles (the smaller tree has none, the largest one with two such layers):
+    words at the ends of their range, and leaves whose reduction needs the exact form, among them."""
+    width = 4 if ext else 2
+    cw = field_elems(78, leaves * width).reshape(leaves, width)
+    cw[3], cw[130] = GL_P - 1, 2**32 - 1
+    for k in (5, 127, 128, leaves - 1):
+        cw[k] = 0
+        cw[k, 0] = (2**48 - 0xdd5743e7f2a5a5d9) % GL_P
+    d_cw, d_t = DeviceBuffer.from_numpy(gl, cw.reshape(-1)), DeviceBuffer(gl, 32 * (2 * leaves - 1))
+    assert (gl.poseidon2_merkle_tree_ext2_ffi if ext else gl.poseidon2_merkle_tree_gl_ffi)(d_cw.ptr, d_t.ptr, leaves) == 0
+    exp = np.zeros(4 * (2 * leaves - 1), dtype=np.uint64)
+    oracle.oracle_bf_merkle_tree(cw.ctypes.data, leaves, int(ext), exp.ctypes.data)
+    assert np.array_equal(d_t.to_numpy(), exp)
+
+
 @pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
                                      (22, 6), (22, 9), (24, 10), (24, 13)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):

@@ -76,7 +76,8 @@ def lib_verify(lib, instances, n, proof, label):
 
 
 @pytest.mark.parametrize("kind,arity,leaves", [(0, 1, 1), (0, 4, 2), (0, 6, 3), (0, 7, 1), (0, 11, 5), (0, 16, 4), (0, 13, 42),
-                                               (1, 6, 2), (1, 9, 3), (1, 14, 4), (2, 1, 2), (2, 5, 3), (2, 12, 2), (2, 15, 6)])
+                                               (1, 6, 2), (1, 9, 3), (1, 14, 4), (2, 1, 2), (2, 5, 3), (2, 12, 2), (2, 15, 6),
+                                               (0, 11, 39), (0, 11, 40), (1, 10, 44), (2, 8, 55), (0, 1, 440)])
 def test_gpu_proof_equals_the_cpu_prover(lib, kind, arity, leaves):
     insts = [random_instance(300 + 17 * i, kind, arity) for i in range(leaves)]
     exp = pyoracle.agl_same_point_prove(insts, arity, b"sp-gpu")
