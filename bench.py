@@ -313,17 +313,18 @@ def run_batched(args):
     elems = 2 * K * (1 << nv)  # field elements of the 2K witness tables (eq is derived, not counted)
     peak, peak_kind = measured_peaks()
     # algorithmic bytes of the passes: the base tables once for the first block of rounds and once for its fold, then every
-    # folded table (16 B an element, a quarter of the one before) written once and read once
+    # folded table (16 B an element, an eighth of the one before) written once and read once
     roofline = None
-    if "pair_pass" in kernels:
-        cnt, kms = kernels["pair_pass"]
-        total_bytes = (2 * 2 * K * m * 8 + 2 * sum(2 * K * (m >> (2 * r)) * 16 for r in range(1, n_loc // 2 + 1))) * psteps
+    cnt, kms = pass_times(kernels)
+    if cnt:
+        total_bytes = (2 * 2 * K * m * 8 + 2 * sum(2 * K * (m >> (3 * r)) * 16 for r in range(1, n_loc // 3 + 1))) * psteps
         ach = total_bytes / (kms * 1e-3) / 1e9
-        roofline = {"kernel": "pair_pass", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+        roofline = {"kernel": "pair_mma + pair_pass", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                     "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "launches": cnt,
                     "avg_launch_ms": kms / cnt,
                     "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % psteps,
-                    "note": "per rank; all passes together (two or more rounds each, taken as two); bound by the integer pipes"}
+                    "note": "per rank; all passes together (three rounds each); fold and sums on the tensor cores, the large passes "
+                            "bound by HBM and the weights' products"}
     kernel_ms = sum(x for _, x in kernels.values()) / psteps
     how = {"mailbox": "round loop inside the library; host mailbox in POSIX shared memory",
            "nccl": "Python round loop; NCCL all-gather", "shm": "Python round loop; mailbox file in /dev/shm"}[args.exchange]
@@ -903,6 +904,12 @@ def basefold_config(nv, hash_name, world):
     return cfg
 
 
+def pass_times(kernels):
+    """Launches and milliseconds of the passes over two tables, on the tensor cores and below their sizes."""
+    both = [kernels[k] for k in ("pair_mma", "pair_pass") if k in kernels]
+    return sum(c for c, _ in both), sum(ms for _, ms in both)
+
+
 def prof_report(lib):
     need = lib.mb_prof_report(None, 0)
     buf = ctypes.create_string_buffer(need + 16)
@@ -1069,19 +1076,18 @@ def part_sumcheck(lib, args, peak, peak_kind):
     step()
     lib.mb_prof_enable(0)
     kernels = prof_report(lib)
-    # The passes' algorithmic bytes, blocks of rounds taken as two (they are two or more): the base tables once for the sums
-    # of the first block and once for its fold, then every folded table (16 B an element, a quarter of the one before)
-    # written once and read once.
-    alg_bytes = 2.0 * d * n * 8 + 2.0 * sum(d * (n >> (2 * r)) * 16 for r in range(1, nv // 2 + 1))
-    cnt, pass_ms = kernels["pair_pass"]
+    # The passes' algorithmic bytes: the base tables once for the sums of the first block of four rounds and once for its fold,
+    # then every folded table (16 B an element, a sixteenth, then an eighth of the one before) written once and read once.
+    alg_bytes = 2.0 * d * n * 8 + 2.0 * sum(d * (n >> (3 * r + 1)) * 16 for r in range(1, nv // 3))
+    cnt, pass_ms = pass_times(kernels)
     ach = alg_bytes / (pass_ms * 1e-3) / 1e9
     whole = alg_bytes / (ms * 1e-3) / 1e9
     out = {"metric": "field-elems/s: sumcheck of f*g over 2^%d points, Goldilocks" % nv, "value": d * n / (ms * 1e-3), "unit": UNIT,
            "ms": ms, "config": {"workload": "sumcheck nv=%d d=2" % nv},
-           "roofline": {"kernel": "pair_pass (all passes of a proof)", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+           "roofline": {"kernel": "pair_mma + pair_pass (all passes of a proof)", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                         "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "avg_launch_ms": pass_ms / cnt, "launches": cnt,
                         "timed_in": "a proof of its own with CUDA events around every launch (not the timed region)",
-                        "note": "two or more rounds per pass; the products of the sums bound it (integer pipes), not HBM",
+                        "note": "three or four rounds per pass, fold and sums on the tensor cores; latency bound after the first two",
                         "whole_proof": {"achieved": whole, "frac": whole / peak,
                                         "note": "%d rounds with the host transcript between them against the %.2f GB the passes "
                                                 "must move; the last rounds are latency bound" % (nv, alg_bytes / 1e9)}},
@@ -1335,7 +1341,9 @@ def run_basefold(args):
     node_bytes = big_nodes(leaves_commit) * (64 + 32 * copies) + sum(big_nodes(m // world) for m in big_folded) * 96
     hash_ms = sum(kernels.get(k, (0, 0))[1] for k in ("hash_leaves", "compress_layer", "tree_up"))
     perms_per_s = (leaves_commit + leaves_folded + nodes_per_step) * prof_steps / (hash_ms * 1e-3) if hash_ms else 0.0
-    inst_per_perm = 10870.0 if args.hash == "poseidon2" else 5615.0  # of a permutation's thread (profiles/poseidon2_permute_batch_ncu.md)
+    # of a permutation's thread: Poseidon2 10870 a thread each (profiles/poseidon2_permute_batch_ncu.md), 9700 in tiles, where nine
+    # tenths of the permutations are at 2^24
+    inst_per_perm = 9800.0 if args.hash == "poseidon2" else 5615.0
     sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
     if dom is not None:
         cnt, ms = kernels[dom]

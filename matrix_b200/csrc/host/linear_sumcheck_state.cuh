@@ -38,14 +38,14 @@ using namespace mb::sc;
 // made canonical when they come to the host), through the host forms of host_field.hpp.
 template <class T> struct HostExt;
 template <class T, class F> struct HostExtOps {
-    static T add(T a, T b) { return T{F::add(a.c0, b.c0), F::add(a.c1, b.c1)}; }
-    static T sub(T a, T b) { return T{F::sub(a.c0, b.c0), F::sub(a.c1, b.c1)}; }
-    static T mul(T a, T b) {
+    static MB_HOT T add(T a, T b) { return T{F::add(a.c0, b.c0), F::add(a.c1, b.c1)}; }
+    static MB_HOT T sub(T a, T b) { return T{F::sub(a.c0, b.c0), F::sub(a.c1, b.c1)}; }
+    static MB_HOT T mul(T a, T b) {
         T r;
         hf::e2_mul<F>(a.c0, a.c1, b.c0, b.c1, r.c0, r.c1);
         return r;
     }
-    static T canon(T a) { return T{F::canon(a.c0), F::canon(a.c1)}; }
+    static MB_HOT T canon(T a) { return T{F::canon(a.c0), F::canon(a.c1)}; }
 };
 template <> struct HostExt<gl::E2> : HostExtOps<gl::E2, hf::GlE2Ops> {};
 template <> struct HostExt<agl::E2> : HostExtOps<agl::E2, hf::AglE2Ops> {};
