@@ -14,8 +14,8 @@
 //    after a fold only reads (d+1) extension elements back.
 // Base / Ext are the field traits of sumcheck_kernels.cuh (GlBase, GlExt2) or
 // agl_traits.cuh (AglBase, AglExt2).
-//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh), and so does one table, and three or four
-//    that are small (product_sumcheck.cuh); larger ones, and five and more, take a round per pass;
+//  * a product of two tables runs several rounds per pass (pair_sumcheck.cuh), and so do one table and three, and four
+//    that are small (product_sumcheck.cuh); four larger ones, and five and more, take a round per pass;
 //  * five and more tables that are down to HOST_TAIL elements are read back and the remaining rounds run on the host: a
 //    round on the device costs a launch and a synchronisation whatever its size. The field arithmetic is exact, so the
 //    messages are the same words.

@@ -1,12 +1,15 @@
-// Host side of the several-rounds-per-pass sumcheck over products of two tables (pair_kernels.cuh):
+// Host side of the several-rounds-per-pass sumcheck over products of two tables (pair_kernels.cuh, pair_mma_kernels.cuh):
 //     sum_x w(x) sum_k s_k a_k(x) b_k(x),   w = 1 or eq(t, x) on the first eq_vars variables,
 // for K instances whose factors s_k may be chosen after the first pass (powers of a challenge). The object plans the
 // blocks of rounds, queues the passes and runs the rounds of a block on the matrices they return; the last rounds, on
 // tables of at most 512 elements together, run on the host altogether. The caller owns the transcript.
 //
-//   rounds per block  4 while a pass has at most 2^17 elements, 3 up to 2^19 (2^21 of the base field), then 2: a round more
-//                     doubles the products per element (2^B), which pays while a launch and a synchronisation (about
-//                     12 us) cost more than they do; bounded too by what the host then has to fold, K 4^B entries.
+//   tensor cores      passes over 2^14 elements and more, three rounds each, four on words of the base field: their products
+//                     cost next to nothing there (a pass that folds words to 2^16 elements takes 15 us, 26 without; 2^11 and fewer
+//                     elements a table are less than a tile).
+//   rounds per block  otherwise 4 while a pass has at most 2^17 elements, 3 up to 2^19 (2^21 of the base field), then 2: a round
+//                     more doubles the products per element (2^B), which pays while a launch and a synchronisation (about
+//                     12 us) cost more than they do. In every case bounded by what the host then has to fold, K 4^B entries.
 //   host tables       2^t elements per table with K 2^t <= 512: the rest of a proof on them takes a core about as long
 //                     as one more pass and its synchronisation.
 //   all on the host   base-field tables of at most 2^10 elements: the copy and the rounds (35 us) cost less than two passes.

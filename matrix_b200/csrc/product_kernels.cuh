@@ -5,8 +5,8 @@
 // folding and evaluating the round polynomials only combine entries, so the host runs the B rounds on T. A round of
 // its own costs a launch, a synchronisation and two reductions whatever its size (about 20 us); T takes 2^((D-1) B)
 // products per element instead of the few of a round polynomial, so it is for tables that leave the chip idle: at 2^16
-// elements of three tables 2^20 products, 8 us, replace two rounds. Larger tables take a round per pass
-// (sumcheck_kernels.cuh).
+// elements of three tables 2^20 products, 8 us, replace two rounds. Three tables of 2^15 elements and more go to the tensor cores
+// (product_mma_kernels.cuh), four of 2^14 and more take a round per pass (sumcheck_kernels.cuh).
 //
 // One table: the sums by x mod 2^B are a thread's own, its elements lie a multiple of 256 apart. Otherwise a block takes
 // tiles of 64 folded elements per table in shared memory; thread t owns entry t mod 2^(D B) (two
