@@ -10,9 +10,6 @@ namespace mbhost {
 namespace hf {
 
 typedef unsigned __int128 u128;
-// Arithmetic of the inner loops: always inlined, whatever else the translation unit holds (left to the compiler's budget, host
-// rounds of four tables took 119 us where they take 99).
-#define MB_HOT inline __attribute__((always_inline))
 
 // ---- Goldilocks --------------------------------------------------------------------
 constexpr uint64_t GL_P = 0xFFFFFFFF00000001ULL;
@@ -21,7 +18,7 @@ constexpr uint64_t GL_EPS = 0xFFFFFFFFULL;   // 2^64 mod p
 // x mod p as a loose 64-bit residue, for any 128-bit x: with 2^64 = 2^32 - 1 and 2^96 = -1 (mod p),
 // x = lo - hi_hi + hi_lo (2^32 - 1). A borrow is repaired by - EPS (the wrapped value is above 2^64 - 2^32), a
 // carry by + EPS (the wrapped value is below hi_lo EPS < 2^64 - 2^33).
-static MB_HOT uint64_t gl_red(u128 x) {
+static inline uint64_t gl_red(u128 x) {
 #if defined(__x86_64__)
     // seven micro-operations: hi_lo (2^32 - 1) is one multiplication, the borrow (once in 2^32 random words) a jump.
     // Early-clobber operands: the constant is read after they are written, so one that the compiler knows to hold the same
@@ -41,31 +38,31 @@ static MB_HOT uint64_t gl_red(u128 x) {
     return r;
 #endif
 }
-static MB_HOT uint64_t gl_canon(uint64_t x) { return x >= GL_P ? x - GL_P : x; }
+static inline uint64_t gl_canon(uint64_t x) { return x >= GL_P ? x - GL_P : x; }
 // canonical in, canonical out
-static MB_HOT uint64_t gl_add(uint64_t a, uint64_t b) {
+static inline uint64_t gl_add(uint64_t a, uint64_t b) {
     const uint64_t s = a + b, w = s - GL_P;
     return ((s < a) | (s >= GL_P)) ? w : s;
 }
-static MB_HOT uint64_t gl_sub(uint64_t a, uint64_t b) {
+static inline uint64_t gl_sub(uint64_t a, uint64_t b) {
     const uint64_t d = a - b;
     return a < b ? d + GL_P : d;
 }
-static MB_HOT uint64_t gl_mul(uint64_t a, uint64_t b) { return gl_canon(gl_red((u128)a * b)); }
+static inline uint64_t gl_mul(uint64_t a, uint64_t b) { return gl_canon(gl_red((u128)a * b)); }
 
 // ---- almost-Goldilocks ---------------------------------------------------------------
 constexpr uint64_t AGL_P = 0xFFFFFFFEFFFFFFE1ULL;
 constexpr uint64_t AGL_C = 0x000000010000001FULL;   // 2^64 mod q
 
 // lo + hi c for a high word below 2^31, loose result: one carry repair (the wrapped sum is below hi c).
-static MB_HOT uint64_t agl_red_small(u128 x) {
+static inline uint64_t agl_red_small(u128 x) {
     const uint64_t lo = (uint64_t)x, t = (uint64_t)(x >> 64) * AGL_C;
     uint64_t r = lo + t;
     r += (0 - (uint64_t)(r < t)) & AGL_C;
     return r;
 }
 // Any 128-bit value: two folds of the high word (2^64 = c) bring it below 2^34 and then below 8.
-static MB_HOT uint64_t agl_red(u128 x) {
+static inline uint64_t agl_red(u128 x) {
 #if defined(__x86_64__)
     // the same two folds in registers; the last carry (h 2^64 for h below 8 leaves a word near 2^64 only once in 2^28) a jump
     uint64_t lo = (uint64_t)x, hi = (uint64_t)(x >> 64), a = hi;
@@ -79,12 +76,12 @@ static MB_HOT uint64_t agl_red(u128 x) {
     return agl_red_small(x);
 #endif
 }
-static MB_HOT uint64_t agl_canon(uint64_t x) { return x >= AGL_P ? x - AGL_P : x; }
-static MB_HOT uint64_t agl_add(uint64_t a, uint64_t b) {
+static inline uint64_t agl_canon(uint64_t x) { return x >= AGL_P ? x - AGL_P : x; }
+static inline uint64_t agl_add(uint64_t a, uint64_t b) {
     const uint64_t s = a + b, w = s - AGL_P;
     return ((s < a) | (s >= AGL_P)) ? w : s;
 }
-static MB_HOT uint64_t agl_sub(uint64_t a, uint64_t b) {
+static inline uint64_t agl_sub(uint64_t a, uint64_t b) {
     const uint64_t d = a - b;
     return a < b ? d + AGL_P : d;
 }
@@ -94,20 +91,20 @@ static MB_HOT uint64_t agl_sub(uint64_t a, uint64_t b) {
 // (times W) can be added to a product without overflow.
 struct GlE2Ops {
     static constexpr uint64_t W = 7;
-    static MB_HOT uint64_t add(uint64_t a, uint64_t b) { return gl_add(a, b); }
-    static MB_HOT uint64_t sub(uint64_t a, uint64_t b) { return gl_sub(a, b); }
-    static MB_HOT uint64_t red(u128 x) { return gl_red(x); }
-    static MB_HOT uint64_t canon(uint64_t x) { return gl_canon(x); }
+    static uint64_t add(uint64_t a, uint64_t b) { return gl_add(a, b); }
+    static uint64_t sub(uint64_t a, uint64_t b) { return gl_sub(a, b); }
+    static uint64_t red(u128 x) { return gl_red(x); }
+    static uint64_t canon(uint64_t x) { return gl_canon(x); }
 };
 struct AglE2Ops {
     static constexpr uint64_t W = 3;
-    static MB_HOT uint64_t add(uint64_t a, uint64_t b) { return agl_add(a, b); }
-    static MB_HOT uint64_t sub(uint64_t a, uint64_t b) { return agl_sub(a, b); }
-    static MB_HOT uint64_t red(u128 x) { return agl_red(x); }
-    static MB_HOT uint64_t canon(uint64_t x) { return agl_canon(x); }
+    static uint64_t add(uint64_t a, uint64_t b) { return agl_add(a, b); }
+    static uint64_t sub(uint64_t a, uint64_t b) { return agl_sub(a, b); }
+    static uint64_t red(u128 x) { return agl_red(x); }
+    static uint64_t canon(uint64_t x) { return agl_canon(x); }
 };
 template <class F>
-static MB_HOT void e2_mul(uint64_t a0, uint64_t a1, uint64_t b0, uint64_t b1, uint64_t& c0, uint64_t& c1) {
+static inline void e2_mul(uint64_t a0, uint64_t a1, uint64_t b0, uint64_t b1, uint64_t& c0, uint64_t& c1) {
     const uint64_t t11 = F::red((u128)a1 * b1), t10 = F::red((u128)a1 * b0);
     c0 = F::canon(F::red((u128)a0 * b0 + (u128)t11 * F::W));
     c1 = F::canon(F::red((u128)a0 * b1 + t10));

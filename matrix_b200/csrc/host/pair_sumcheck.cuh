@@ -35,20 +35,20 @@ struct PairAgl : hf::AglE2Ops {
 template <class F, class O>
 struct PairHost {
     using E2 = typename F::E2;
-    static MB_HOT E2 mul(E2 a, E2 b) {
+    static E2 mul(E2 a, E2 b) {
         E2 r;
         hf::e2_mul<O>(a.c0, a.c1, b.c0, b.c1, r.c0, r.c1);
         return r;
     }
-    static MB_HOT E2 add(E2 a, E2 b) { return E2{O::add(a.c0, b.c0), O::add(a.c1, b.c1)}; }
-    static MB_HOT E2 sub(E2 a, E2 b) { return E2{O::sub(a.c0, b.c0), O::sub(a.c1, b.c1)}; }
-    static MB_HOT E2 fold(E2 a, E2 b, E2 r) { return add(a, mul(r, sub(b, a))); }
-    static MB_HOT E2 canon(E2 a) { return E2{O::canon(a.c0), O::canon(a.c1)}; }
+    static E2 add(E2 a, E2 b) { return E2{O::add(a.c0, b.c0), O::add(a.c1, b.c1)}; }
+    static E2 sub(E2 a, E2 b) { return E2{O::sub(a.c0, b.c0), O::sub(a.c1, b.c1)}; }
+    static E2 fold(E2 a, E2 b, E2 r) { return add(a, mul(r, sub(b, a))); }
+    static E2 canon(E2 a) { return E2{O::canon(a.c0), O::canon(a.c1)}; }
     // sum of products, reduced once
     struct Wide {
         hf::u128 s = 0;
         uint64_t top = 0;
-        MB_HOT void mac(uint64_t x, uint64_t y) {
+        void mac(uint64_t x, uint64_t y) {
             const hf::u128 p = (hf::u128)x * y;
             s += p;
             top += s < p;
@@ -57,7 +57,7 @@ struct PairHost {
     };
     struct Dot {
         Wide p00, p11, p01;
-        MB_HOT void mac(E2 a, E2 b) {
+        void mac(E2 a, E2 b) {
             p00.mac(a.c0, b.c0);
             p11.mac(a.c1, b.c1);
             p01.mac(a.c0, b.c1);
