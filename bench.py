@@ -1370,7 +1370,8 @@ def run_basefold(args):
                         "traffic_note": "bytes per launch (average), scaled from the capture in profiles/bench_basefold_launches.md",
                         "launches": cnt, "avg_launch_ms": ms / cnt, "share_of_kernel_time": ms / total_kernel_ms,
                         "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % prof_steps,
-                        "note": ("Poseidon2 hashing: ~520 modular multiplications per 32-byte digest, bound by the "
+                        "note": ("Poseidon2 hashing: ~380 modular multiplications per 32-byte digest and thread, the internal "
+                                 "rounds' linear algebra on the tensor cores (520 below 2^20 nodes a layer), bound by the "
                                  "integer pipes, not HBM; permutations/s is the meaningful rate") if args.hash == "poseidon2"
                         else "Monolith hashing: bound by the integer pipes, not HBM; permutations/s is the meaningful rate",
                         "permutations_per_s": perms_per_s,
