@@ -15,15 +15,15 @@ namespace p2host {
 
 using hf::u128;
 constexpr uint64_t EPS = hf::GL_EPS;
-static inline uint64_t red(u128 x) { return hf::gl_red(x); }   // any 128-bit value, loose result
-static inline uint64_t mul(uint64_t a, uint64_t b) { return red((u128)a * b); }
-static inline uint64_t sbox7(uint64_t x) {
+static MB_HOT uint64_t red(u128 x) { return hf::gl_red(x); }   // any 128-bit value, loose result
+static MB_HOT uint64_t mul(uint64_t a, uint64_t b) { return red((u128)a * b); }
+static MB_HOT uint64_t sbox7(uint64_t x) {
     const uint64_t x2 = mul(x, x), x4 = mul(x2, x2), x3 = mul(x2, x);
     return mul(x4, x3);
 }
 
 // y = M4 x for M4 = [2 3 1 1; 1 2 3 1; 1 1 2 3; 3 1 1 2], as 128-bit sums (inputs below 2^64: outputs below 7 2^64).
-static inline void mat4(const uint64_t* x, u128* y) {
+static MB_HOT void mat4(const uint64_t* x, u128* y) {
     const u128 t01 = (u128)x[0] + x[1], t23 = (u128)x[2] + x[3];
     const u128 t0123 = t01 + t23;
     const u128 t01123 = t0123 + x[1], t01233 = t0123 + x[3];
@@ -34,7 +34,7 @@ static inline void mat4(const uint64_t* x, u128* y) {
 }
 
 // s <- [[2 M4, M4], [M4, 2 M4]] s + rc (rc may be null): sums stay below 22 2^64.
-static inline void external_linear(uint64_t* s, const uint64_t* rc) {
+static MB_HOT void external_linear(uint64_t* s, const uint64_t* rc) {
     u128 a[4], b[4];
     mat4(s, a);
     mat4(s + 4, b);
@@ -91,19 +91,19 @@ static inline void permute_portable(uint64_t* s) {
     "sbb %k[t], %k[t]\n\tadd %[t], %[lo]\n\t.subsection 1\n2:\tsub %[eps], %[lo]\n\tjmp 1b\n\t.previous"
 namespace bmi2 {
 // a b, a b + c and a b + c + d mod p, loose ((2^64 - 1)^2 + 2 (2^64 - 1) < 2^128)
-static inline uint64_t mul(uint64_t a, uint64_t b) {
+static MB_HOT uint64_t mul(uint64_t a, uint64_t b) {
     uint64_t lo, hi, t;
     asm("mulx %[b], %[lo], %[hi]\n\t" MB_P2_RED
         : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t) : [eps] "r"(EPS), "d"(a), [b] "rm"(b) : "cc");
     return lo;
 }
-static inline uint64_t mul_add(uint64_t a, uint64_t b, uint64_t c) {
+static MB_HOT uint64_t mul_add(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t lo, hi, t;
     asm("mulx %[b], %[lo], %[hi]\n\tadd %[c], %[lo]\n\tadc $0, %[hi]\n\t" MB_P2_RED
         : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t) : [eps] "r"(EPS), "d"(a), [b] "rm"(b), [c] "r"(c) : "cc");
     return lo;
 }
-static inline uint64_t mul_add2(uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+static MB_HOT uint64_t mul_add2(uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
     uint64_t lo, hi, t;
     asm("mulx %[b], %[lo], %[hi]\n\tadd %[c], %[lo]\n\tadc $0, %[hi]\n\tadd %[d], %[lo]\n\tadc $0, %[hi]\n\t" MB_P2_RED
         : [lo] "=&r"(lo), [hi] "=&r"(hi), [t] "=&r"(t)
@@ -111,23 +111,23 @@ static inline uint64_t mul_add2(uint64_t a, uint64_t b, uint64_t c, uint64_t d) 
     return lo;
 }
 // hi 2^64 + lo mod p, loose, for hi < 2^32 (the wrapped sum is below hi EPS, so the repair cannot carry)
-static inline uint64_t red_small(uint64_t lo, uint64_t hi) {
+static MB_HOT uint64_t red_small(uint64_t lo, uint64_t hi) {
     uint64_t u = (hi << 32) - hi;
     asm("add %[u], %[lo]\n\tsbb %k[u], %k[u]\n\tadd %[u], %[lo]" : [lo] "+r"(lo), [u] "+r"(u) : : "cc");
     return lo;
 }
-static inline uint64_t red_small(u128 x) { return red_small((uint64_t)x, (uint64_t)(x >> 64)); }
-static inline uint64_t sbox7(uint64_t x) {
+static MB_HOT uint64_t red_small(u128 x) { return red_small((uint64_t)x, (uint64_t)(x >> 64)); }
+static MB_HOT uint64_t sbox7(uint64_t x) {
     const uint64_t x2 = mul(x, x), x4 = mul(x2, x2), x3 = mul(x2, x);
     return mul(x4, x3);
 }
-static inline void full_round(uint64_t* s, const uint64_t* rc) {   // rc: the next round's constants
+static MB_HOT void full_round(uint64_t* s, const uint64_t* rc) {   // rc: the next round's constants
     s[0] = sbox7(s[0]); s[1] = sbox7(s[1]); s[2] = sbox7(s[2]); s[3] = sbox7(s[3]);   // unrolled by hand
     s[4] = sbox7(s[4]); s[5] = sbox7(s[5]); s[6] = sbox7(s[6]); s[7] = sbox7(s[7]);
     u128 a[4], b[4];
     mat4(s, a);
     mat4(s + 4, b);
-    const auto out = [&](int i) {
+    const auto out = [&](int i) __attribute__((always_inline)) {
         const u128 sum = a[i] + b[i];
         s[i] = red_small(a[i] + sum + rc[i]);
         s[i + 4] = red_small(b[i] + sum + rc[i + 4]);
@@ -151,7 +151,7 @@ static inline void permute(uint64_t* st) {
         x = mul_add2(x4, w3, rest, r < 21 ? rc_int[r + 1] : 0);
         const uint64_t all = red_small((u128)mul(x3, x4) + rest);
         uint64_t lo = 0, hi = 0;
-        const auto lane = [&](int i) {
+        const auto lane = [&](int i) __attribute__((always_inline)) {
             const uint64_t v = s[i] = mul_add(s[i], diag[i], all);
             asm("add %[v], %[lo]\n\tadc $0, %[hi]" : [lo] "+r"(lo), [hi] "+r"(hi) : [v] "r"(v) : "cc");
         };

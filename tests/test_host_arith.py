@@ -4,6 +4,7 @@ import ctypes
 import random
 
 import numpy as np
+import pytest
 
 from .conftest import GL_P
 
@@ -309,3 +310,19 @@ def test_ext5_oracle_and_host_forms(hostcheck, oracle):
             assert pyoracle.e5_op("pow", a, e=e) == want
             hostcheck.hc_e5_pow(u5(*a), u64(e), O)
             assert list(O) == want
+
+
+def test_host_permutation_is_inlined_in_every_unit():
+    """Goldilocks arithmetic has no out-of-line copies in the library, and every translation unit compiled the host permutation to
+    the same size: left to the inlining budget, one that grew called its helpers, 1.2 % of every proof and verification."""
+    import os
+    import platform
+    import re
+    import subprocess
+    from matrix_b200.build import LIB
+    if platform.machine() != "x86_64":
+        pytest.skip("the permutation in assembly is for x86-64")
+    names = subprocess.run(["nm", "-S", "-C", os.path.join(LIB, "libgoldilocks_cuda_wrapper.so")], capture_output=True, text=True, check=True).stdout
+    sizes = re.findall(r"^\w+ (\w+) \w mbhost::p2host::bmi2::permute\(", names, re.M)
+    assert len(sizes) >= 4 and len(set(sizes)) == 1, sizes
+    assert re.findall(r"mbhost::(?:hf::(?:gl_\w+|GlE2Ops::\w+)|p2host::(?:bmi2::)?(?:red\w*|mul\w*|sbox7|mat4|full_round|external_linear))\(", names) == []
