@@ -85,7 +85,7 @@ public:
     ~PairSumcheck() {
         if (scratch_) {   // nothing may still be writing it
             const bool clean = cudaStreamSynchronize(MB_STREAM) == cudaSuccess;
-            ScratchPool::give(scratch_, clean && pin_[ERROR_WORD] == 0);
+            ScratchPool::give(scratch_, clean && bad_ == MB_OK && pin_[ERROR_WORD] == 0);
         }
         pool_free(t0_);
         pool_free(t1_);
@@ -125,8 +125,9 @@ public:
         if (rc == MB_OK) rc = pass();
         // what the later passes fold into, allocated while the first one runs
         for (size_t i = 1; rc == MB_OK && i < blocks_.size() && i <= 2; i++)
-            MB_CUDA(pool_alloc((void**)(i == 1 ? &t0_ : &t1_), sizeof(uint64_t) * ((size_t)4 << (n - blocks_[i].first)) * K));
-        return rc;
+            if (pool_alloc((void**)(i == 1 ? &t0_ : &t1_), sizeof(uint64_t) * ((size_t)4 << (n - blocks_[i].first)) * K) != cudaSuccess)
+                rc = MB_ERR_CUDA;
+        return failed(rc);
     }
     // The instances' factors (K = 1: not needed). sums() and fold() may be called from then on; before the first fold the
     // factors may be replaced.
@@ -199,7 +200,7 @@ public:
         const Block& bl = blocks_[block_];
         if (round + 1 == bl.first + bl.rounds) {
             block_++;
-            return pass();
+            return failed(pass());
         }
         if (m_.empty()) combine();
         const int half = side_ / 2;   // rows, then columns
@@ -368,12 +369,17 @@ private:
                 MB_CUDA(cudaMemcpyAsync(pin_ + (2 * k + s) * w, (s ? b_ : a_) + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
         return MB_OK;
     }
+    // A pass that could not be queued or did not finish leaves nothing to go on from: every later call returns its error too.
+    int failed(int rc) {
+        if (rc != MB_OK) bad_ = rc;
+        return rc;
+    }
     // Results of the pass queued last.
     int wait() {
-        if (!pending_) return MB_OK;
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        if (bad_ != MB_OK || !pending_) return bad_;
+        if (cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
         pending_ = false;
-        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;   // a wait of a pass on the tensor cores ran out
+        if (pin_[ERROR_WORD] != 0) return failed(MB_ERR_CUDA);   // a wait of a pass on the tensor cores ran out
         if (block_ < blocks_.size()) return MB_OK;
         host_ = true;
         const size_t nw = base_ ? 1 : 2;
@@ -501,7 +507,7 @@ private:
 
     const uint64_t *a_ = nullptr, *b_ = nullptr;
     size_t stride_ = 0;
-    int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0;
+    int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0, bad_ = MB_OK;
     bool base_ = false, together_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;

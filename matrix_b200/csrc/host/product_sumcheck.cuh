@@ -26,7 +26,10 @@ public:
     static bool handles(int d) { return d == 1 || d == 3 || d == 4; }
     static int limit(int d) { return d == 4 ? 13 : 40; }
     ~ProductSumcheck() {
-        if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess && pin_[ERROR_WORD] == 0);   // nothing may still be writing it
+        if (scratch_) {   // nothing may still be writing it
+            const bool clean = cudaStreamSynchronize(MB_STREAM) == cudaSuccess;
+            ScratchPool::give(scratch_, clean && bad_ == MB_OK && pin_[ERROR_WORD] == 0);
+        }
         pool_free(t0_);
         pool_free(t1_);
     }
@@ -56,14 +59,14 @@ public:
         pin_ = scratch_.host;
         pin_[ERROR_WORD] = 0;
         cap_ = sm_count() * (d == 1 ? 8 : 2);
-        return pass();
+        return failed(pass());
     }
     // Every round that is left is the host's: tables() has them.
     bool at_tail() const { return block_ == blocks_.size(); }
     // [d][2^tail] elements, canonical
     int tables(std::vector<E2>& tab, size_t& stride) {
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;
+        int rc = wait();
+        if (rc != MB_OK) return rc;
         stride = (size_t)1 << tail_vars_;
         tab.resize(d_ * stride);
         const int nw = base_ ? 1 : 2;
@@ -109,7 +112,7 @@ public:
         const Block& bl = blocks_[block_];
         if (round + 1 == bl.first + bl.rounds) {
             block_++;
-            return pass();
+            return failed(pass());
         }
         // one axis after the other: the last one is halved and moved to the front
         const int half = side_ / 2;
@@ -224,11 +227,21 @@ private:
             MB_CUDA(cudaMemcpyAsync(pin_ + w * k, in_ + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
         return MB_OK;
     }
+    // As PairSumcheck: after a failure every later call fails.
+    int failed(int rc) {
+        if (rc != MB_OK) bad_ = rc;
+        return rc;
+    }
+    int wait() {
+        if (bad_ != MB_OK) return bad_;
+        if (cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
+        return failed(pin_[ERROR_WORD] != 0 ? MB_ERR_CUDA : MB_OK);
+    }
     // The sums of the current block.
     int load() {
-        if (loaded_) return MB_OK;
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
-        if (pin_[ERROR_WORD] != 0) return MB_ERR_CUDA;
+        if (bad_ == MB_OK && loaded_) return MB_OK;
+        int rc = wait();
+        if (rc != MB_OK) return rc;
         const int g = blocks_[block_].rounds;
         side_ = 1 << g;
         t_.resize((size_t)1 << (g * d_));
@@ -261,7 +274,7 @@ private:
 
     const uint64_t* in_ = nullptr;
     size_t stride_ = 0;
-    int d_ = 0, n_ = 0, cap_ = 1, round_ = 0, side_ = 0, tail_vars_ = 0;
+    int d_ = 0, n_ = 0, cap_ = 1, round_ = 0, side_ = 0, tail_vars_ = 0, bad_ = MB_OK;
     bool base_ = false, flip_ = false, loaded_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;
