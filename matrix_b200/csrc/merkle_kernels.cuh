@@ -319,6 +319,7 @@ poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n,
         if (live)
             for (size_t c = 0; c < copies; c++) store_digest(dst + 4 * (c * n + k), s);
     }
+    tile.issued.drain();
     tc::fence_before();
     __syncthreads();
     if (t < 32) tc::tmem_free(tmem_sm, 512);

@@ -14,7 +14,8 @@
 // One block an SM: sixteen warps that copy, weigh and reduce, and one that issues the MMAs. They meet at mbarriers only, so a
 // warp may be two tiles ahead of another. Copies to shared memory run two or more tiles ahead (cp.async into the swizzled
 // operand layout), the fold's MMAs two tiles ahead of the warps that reduce them. Every wait is bounded; a thread whose wait
-// ran out goes on without waiting or touching buffers (the block's barriers count every warp), and the block sets *a.error.
+// ran out goes on without waiting or touching buffers (the block's barriers count every warp), and the block sets *a.error
+// (tcgen05.cuh).
 #pragma once
 #include "pair_kernels.cuh"
 #include "tcgen05.cuh"
@@ -311,6 +312,7 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
                 take_sums(i);
             }
         } else if (lane == 0) {
+            tc::Issued issued;
             for (int i = 0; i < count && !failed; i++) {
                 wait(full, i);
                 if (failed) break;
@@ -321,12 +323,13 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
                 for (int ks = 0; ks < MMA_RAW_ROWS / 32; ks++)
                     tc::mma_i8(tmem, tc::desc_sw128(st + 4096 * ks, MMA_HALF), tc::desc_sw128(opa + 4096 * ks, MMA_HALF), idesc_s,
                                !(start && ks == 0));
-                tc::commit(tc::smem_u32(&summed[i & 1]));
+                issued.commit_to(tc::smem_u32(&summed[i & 1]), i >> 1);
             }
+            issued.drain();
         }
     } else {
         const int le = BASE ? 4 - a.fb : 3 - a.fb;                 // log2 of the folded elements in 128 bytes of input
-        const uint32_t epr = 1u << le, stage = mma_fold_stage(le);
+        const uint32_t stage = mma_fold_stage(le);
         const uint32_t ops = MMA_FOLD_STAGES * stage, cst = ops + 16384;   // sums' operands [buffer][b, a]; weights of the fold
         constexpr uint32_t fold_cols = 128;                        // two buffers of 64 columns above the sums
         const uint32_t idesc_f = tc::idesc_u8(16 << le, false);
@@ -377,13 +380,14 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
                 take_sums(i);
             }
         } else if (lane == 0) {
+            tc::Issued issued;
             const auto issue_fold = [&](int i) {
                 const uint32_t st = sm32 + (uint32_t)(i % MMA_FOLD_STAGES) * stage;
                 for (uint32_t q = 0; q < (4u >> le); q++)
                     for (uint32_t ks = 0; ks < 4; ks++)
                         tc::mma_i8(tmem + fold_cols + (i & 1) * 64 + q * (16u << le), tc::desc_sw128(st + q * 16384 + ks * 32, 0),
                                    tc::desc_sw128(sm32 + cst + ks * 32, 0), idesc_f, ks > 0);
-                tc::commit(tc::smem_u32(&folded[i & 1]));
+                issued.commit_to(tc::smem_u32(&folded[i & 1]), i >> 1);
             };
             tc::fence_after();
             for (int i = 0; i < 2 && i < count; i++) issue_fold(i);
@@ -393,9 +397,10 @@ pair_mma_kernel(const PairMmaArgs a, const __grid_constant__ FoldWeights<F> fw) 
                 tc::fence_after();
                 const uint32_t op = sm32 + ops + (i & 1) * 8192;
                 tc::mma_i8(tmem, tc::desc_sw128(op, 4096), tc::desc_sw128(op + 4096, 4096), idesc_s, !starts(i));
-                tc::commit(tc::smem_u32(&summed[i & 1]));
+                issued.commit_to(tc::smem_u32(&summed[i & 1]), i >> 1);
                 if (i + 2 < count) issue_fold(i + 2);
             }
+            issued.drain();
         }
     }
     tc::copy_wait<0>();

@@ -141,6 +141,7 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
     tc::fence_after();
     const uint32_t tmem = tmem_sm;
     bool failed = false;
+    tc::Issued issued;   // thread 0's
     for (int s = 0; s < total; s++) {
         const int tile = s / steps, step = s % steps;
         tc::copy_wait<DM_STAGES - 2>();
@@ -154,8 +155,8 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
             for (int q = 0; q < 8; q++)
                 tc::mma_i8(tmem + 16 * (tile & 1), tc::desc_sw128(st + (q >> 2) * 16384 + (q & 3) * 32, 0),
                            tc::desc_sw128(sm32 + cst + (2 * step + (q >> 2)) * 2048 + (q & 3) * 32, 0), tc::idesc_u8(16, false), step > 0 || q > 0);
-            tc::commit(tc::smem_u32(&used[s % DM_STAGES]));
-            if (step + 1 == steps) tc::commit(tc::smem_u32(&summed));
+            issued.commit_to(tc::smem_u32(&used[s % DM_STAGES]), s / DM_STAGES);
+            if (step + 1 == steps) issued.commit_to(tc::smem_u32(&summed), tile);
         }
         // the stage before this one is free for the one after the next
         if (s > 0 && !failed && !tc::mbar_wait(tc::smem_u32(&used[(s - 1) % DM_STAGES]), (uint32_t)(((s - 1) / DM_STAGES) & 1))) failed = true;
@@ -193,6 +194,7 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
         }
     }
     tc::copy_wait<0>();
+    issued.drain();
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::tmem_free(tmem, 32);

@@ -129,6 +129,7 @@ struct P2Tile {
     uint32_t id;          // named barrier
     int use;              // phase of `before` to wait for next, or negative
     uint32_t turn = 0;    // phases of `done`
+    tc::Issued issued;    // row 0's MMAs, one commit a turn of `done`
     volatile int* failed; // the block's: a wait ran out
     __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
         if (!*failed && !tc::mbar_wait(bar, parity)) *failed = 1;
@@ -161,7 +162,7 @@ __device__ __forceinline__ void p2_internal_rounds(P2Tile& t, uint64_t* s, gl::p
 #pragma unroll
         for (int ks = 0; ks < 2; ks++)
             tc::mma_i8(z, p2_desc(ops + 4096 * ks, 128), p2_desc(t.consts + P2_Z + ks * 32 * P2_N, P2_N), tc::idesc_u8(P2_N, false), ks > 0);
-        tc::commit(t.done);
+        t.issued.commit_to(t.done, t.turn);
     }
     t.finish();
 #pragma unroll 1
@@ -188,7 +189,7 @@ __device__ __forceinline__ void p2_internal_rounds(P2Tile& t, uint64_t* s, gl::p
             if (b < 5)
                 tc::mma_i8(z + 32 * (b + 1), rows, p2_desc(t.consts + P2_Y, 144), tc::idesc_u8(0, false) | ((uint32_t)(18 - 4 * b) << 17), true);
             tc::mma_i8(z + P2_X, rows, p2_desc(t.consts + P2_O + b * 64 * 32, 64), tc::idesc_u8(64, false), true);
-            tc::commit(t.done);
+            t.issued.commit_to(t.done, t.turn);
         }
         t.finish();
     }

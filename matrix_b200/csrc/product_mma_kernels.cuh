@@ -129,12 +129,13 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
             }
         }
     };
+    tc::Issued issued;
     const auto issue_sums = [&](int i, uint32_t h, uint32_t op) {   // the issuing thread
         constexpr uint32_t idesc = tc::idesc_u8(N, true);
 #pragma unroll
         for (int ks = 0; ks < TRI_Y / 32; ks++)
             tc::mma_i8(tmem, tc::desc_sw128(h + 4096 * ks, TRI_P / 2), tc::desc_sw128(op + 4096 * ks, TRI_P / 2), idesc, !(i == 0 && ks == 0));
-        tc::commit(tc::smem_u32(&summed[i % GROUPS]));
+        issued.commit_to(tc::smem_u32(&summed[i % GROUPS]), i / GROUPS);
     };
     const int group = t / GROUP, gt = t % GROUP, gw = gt >> 5;   // a worker's group, its thread and warp in it
 
@@ -173,6 +174,7 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
                 const uint32_t off = sm32 + g * TRI_RAW_GROUP;
                 issue_sums(i, off + (turn & 1) * TRI_TILE + 2 * TRI_FG, off + 2 * TRI_TILE);
             }
+            issued.drain();
         }
     } else {
         const int le = BASE ? 4 - a.fb : 3 - a.fb;                 // log2 of the folded elements in 128 bytes of input: 1 or 2
@@ -234,7 +236,7 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
                     for (uint32_t ks = 0; ks < 4; ks++)
                         tc::mma_i8(tmem + fold_cols + g * 128 + q * (16u << le), tc::desc_sw128(st + q * 16384 + ks * 32, 0),
                                    tc::desc_sw128(sm32 + cst + ks * 32, 0), idesc_f, ks > 0);
-                tc::commit(tc::smem_u32(&folded[g]));
+                issued.commit_to(tc::smem_u32(&folded[g]), i / GROUPS);
             };
             tc::fence_after();
             for (int i = 0; i < GROUPS && i < count; i++) issue_fold(i);
@@ -246,6 +248,7 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
                 if (i + GROUPS < count) issue_fold(i + GROUPS);
                 issue_sums(i, buf + 2 * TRI_FG, buf + TRI_TILE);
             }
+            issued.drain();
         }
     }
     tc::copy_wait<0>();

@@ -5,6 +5,10 @@
 //   K-major    row = row of M or N, its 128 bytes = K; the next 32 of K are 32 bytes on;
 //   MN-major   row = index of K, its 128 bytes = M or N; the next 32 of K are 32 rows (4096 bytes) on; a second 128 of N
 //              lies `lead` bytes on.
+// Waits are bounded. Where one runs out a kernel goes on to its end without waiting again, so that every barrier is met; the thread that
+// issues MMAs waits (Issued::drain) for those in flight before tensor memory is freed. A kernel whose results are a block's own
+// then forms them again from memory (rows of a partial evaluation, hashes). One whose results are sums over all blocks cannot: it sets
+// an error word for the host, which fails the proof and discards the scratch.
 // Measured: an MMA of M = 128, K = 32 takes the pipe 59 cycles up to N = 64, 64 at N = 128, 128 at N = 256, whichever
 // layout its operands have.
 #pragma once
@@ -54,9 +58,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // barrier of `threads` threads of a block, id from 1
 __device__ __forceinline__ void named_sync(uint32_t threads, uint32_t id = 1) { asm volatile("bar.sync %1, %0;" ::"r"(threads), "r"(id) : "memory"); }
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-// bounded: false after about a million polls
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (int it = 0; it < (1 << 20); it++) {
+// bounded: false after `polls` polls. MB_TC_POLLS: 0 in a test build, where every wait of a kernel but Issued::drain runs out at once.
+#ifndef MB_TC_POLLS
+#define MB_TC_POLLS (1 << 20)
+#endif
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int polls = MB_TC_POLLS) {
+    for (int it = 0; it < polls; it++) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
@@ -64,6 +71,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
+// What a thread has issued: the last barrier that it committed its MMAs to. drain: every MMA before that is done, or a million polls are.
+struct Issued {
+    uint32_t bar = ~0u, parity = 0;
+    __device__ __forceinline__ void commit_to(uint32_t b, uint32_t phase) {
+        commit(b);
+        bar = b;
+        parity = phase & 1;
+    }
+    __device__ __forceinline__ void drain() const {
+        if (bar != ~0u) mbar_wait(bar, parity, 1 << 20);
+    }
+};
 // eight or sixteen columns from addr of the calling thread's lane; complete on return
 __device__ __forceinline__ void ld8(uint32_t addr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
