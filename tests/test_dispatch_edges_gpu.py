@@ -123,7 +123,7 @@ def test_poseidon2_tiles(gl, oracle, leaves, ext):
 
 
 @pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
-                                     (22, 6), (22, 9), (24, 10), (24, 13)])
+                                     (22, 6), (22, 7), (22, 9), (24, 10), (24, 11), (24, 13), (25, 11), (25, 12)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):
     for lib, mod, fn, ofn in ((load_agl(), AGL_Q, load_agl().agl_partial_eval_ext2_from_base_ffi, oracle.oracle_agl_partial_eval_ext2_from_base),
                               (gl, GL_P, gl.partial_eval_ext2_from_gl_ffi, oracle.oracle_gl_partial_eval_ext2_from_base)):
