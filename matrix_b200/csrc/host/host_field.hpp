@@ -12,7 +12,7 @@ namespace hf {
 typedef unsigned __int128 u128;
 // Goldilocks arithmetic is inlined whatever else a translation unit holds: left to the compiler's budget for the unit, one that
 // grew made calls inside the transcript's permutation and the rounds on host tables (two tables of 2^10 words 145.1 -> 146.4 us
-// a proof, 141.8 this way; verifying 2^18 points 174.9, 171.0 this way). The almost-Goldilocks forms are left to the compiler:
+// a proof, 141.8 this way; verifying 2^18 points 173.3 -> 175.1, 171.1 this way). The almost-Goldilocks forms are left to the compiler:
 // forced, same-point proofs take 2 to 4 % longer.
 #define MB_HOT inline __attribute__((always_inline))
 

@@ -7,9 +7,9 @@
 //   tensor cores      passes over 2^14 elements and more, three rounds each, four on words of the base field: their products
 //                     cost next to nothing there (a pass that folds words to 2^16 elements takes 15 us, 26 without; 2^11 and fewer
 //                     elements a table are less than a tile).
-//   rounds per block  otherwise 4 while a pass has at most 2^17 elements, 3 up to 2^19 (2^21 of the base field), then 2: a round
-//                     more doubles the products per element (2^B), which pays while a launch and a synchronisation (about
-//                     12 us) cost more than they do. In every case bounded by what the host then has to fold, K 4^B entries.
+//   rounds per block  otherwise 4: a round more doubles the products per element (2^B), which pays while a launch and a
+//                     synchronisation (about 12 us) cost more than they do, and with at most 64 instances these passes have at
+//                     most 2^17 elements. In every case bounded by what the host then has to fold, K 4^B entries.
 //   host tables       2^t elements per table with K 2^t <= 512: the rest of a proof on them takes a core about as long
 //                     as one more pass and its synchronisation.
 //   all on the host   base-field tables of at most 2^10 elements: the copy and the rounds (35 us) cost less than two passes.
@@ -108,7 +108,7 @@ public:
             const bool first = v == n, words = base && blocks_.size() <= 1;   // a pass over words of the base field
             const int fb = first ? 0 : blocks_.back().rounds;
             const bool mma = size >= MMA_MIN && v >= pr::mma_min_vars(fb > 0, words) && (first || pr::mma_folds(fb, words));
-            int g = mma ? (first && base ? 4 : 3) : size <= (1u << 17) ? 4 : size <= (first && base && eq_vars == 0 ? 1u << 21 : 1u << 19) ? 3 : 2;
+            int g = mma ? (first && base ? 4 : 3) : 4;
             while (g > 1 && ((size_t)K << (2 * g)) > 1024) g--;
             if (g > v - t) g = v - t;
             blocks_.push_back(Block{n - v, g, 0, 0, 0, 63, 0, mma});

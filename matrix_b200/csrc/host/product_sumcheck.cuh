@@ -1,5 +1,5 @@
-// Host side of the several-rounds-per-pass sumcheck over products of one, three or four small tables
-// (product_kernels.cuh). The object plans the blocks of rounds, queues the passes, runs the rounds of a block on the
+// Host side of the several-rounds-per-pass sumcheck over products of one table, three, or four small ones
+// (product_kernels.cuh, product_mma_kernels.cuh). The object plans the blocks of rounds, queues the passes, runs the rounds of a block on the
 // sums they return, and hands over the folded tables once they are small enough for the host.
 //
 //   rounds per block   one table: 4. Three tables: 3 up to 2^14 elements, then 2, on the tensor cores
@@ -34,7 +34,7 @@ public:
         pool_free(t1_);
     }
     // d device tables of 2^vars elements, `stride` words apart (never written); r: a challenge they have still to be
-    // folded on, or null. Queues the first pass.
+    // folded on (four tables that were too large before it), or null. Queues the first pass.
     int init(const uint64_t* in, size_t stride, int d, int vars, bool base, const E2* r) {
         in_ = in; stride_ = stride; d_ = d; n_ = vars; base_ = base;
         r_.resize(vars);
@@ -48,9 +48,7 @@ public:
         while (v > 8) {
             int g = d == 1 ? 4 : d == 3 && v <= 14 ? 3 : 2;
             if (g > v - (d == 1 ? 8 : 7)) g = v - (d == 1 ? 8 : 7);
-            const int fb = blocks_.empty() ? 0 : blocks_.back().rounds;
-            const bool mma = d == 3 && v > MMA_ABOVE && (fb == 0 || pr::tri_folds(fb, base && blocks_.size() == 1));
-            blocks_.push_back(Block{n_ - v, g, mma});
+            blocks_.push_back(Block{n_ - v, g, d == 3 && v > MMA_ABOVE});
             v -= g;
         }
         tail_vars_ = v;
@@ -191,7 +189,7 @@ private:
     }
     int launch_mma(const pr::ProductArgs& q, const pr::FoldWeights<F>& fw) const {
         pr::TriArgs p{};
-        p.fb = q.fb; p.in = q.in; p.stride = q.stride; p.out = q.out; p.v = q.v;
+        p.in = q.in; p.stride = q.stride; p.out = q.out; p.v = q.v;
         p.acc = q.acc; p.sums = q.sums; p.error = pin_ + ERROR_WORD;
         const size_t tiles = ((size_t)1 << q.v) / (4 * pr::TRI_Y), least = (tiles + pr::TRI_MOST - 1) / pr::TRI_MOST;
         const size_t sms = (size_t)sm_count() > least ? (size_t)sm_count() : least;

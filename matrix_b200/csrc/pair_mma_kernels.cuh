@@ -33,7 +33,8 @@ constexpr uint32_t MMA_HALF = MMA_RAW_ROWS * 128;
 
 // log2 of the fewest elements after the fold; input bytes of a folded element from 32 to 128
 constexpr int mma_min_vars(bool fold, bool base) { return fold ? 8 : base ? 11 : 10; }
-constexpr bool mma_folds(int fb, bool base) { return base ? fb >= 2 && fb <= 4 : fb >= 1 && fb <= 3; }
+// (a block of one round is a proof's last: no pass folds one challenge)
+constexpr bool mma_folds(int fb, bool base) { return fb >= 2 && fb <= (base ? 4 : 3); }
 
 struct PairMmaArgs {
     int fb;                   // challenges to fold (0: none)

@@ -202,7 +202,9 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
 
 // Variables to bind this way: six and more, at most twelve, of a table of 2^22 elements where a block has its rows to itself (2^21:
 // no gain), of 2^24 where a cluster shares them (2^22 elements in rows of 2^10: 41 by rows, 52 here, on 32 blocks). Rows of 2^13 would
-// need clusters of eight, which leave a part of each GPC idle (2^24: 72 by rows, 84 here). 0: not this way.
+// need clusters of eight, which leave a part of each GPC idle (2^24: 72 by rows, 84 here); twelve variables and a short pass for the rest
+// are faster than by rows in one: 2^24 elements, m = 13 61 / 50, m = 14 62 / 50, m = 16 (by rows in two passes) 67 / 54; 2^26, m = 14 169 /
+// 127. 0: not this way.
 inline int dot_mma_vars(int log_n, int m) {
     const int k = m < DM_MAX ? m : DM_MAX;
     return k >= DM_MIN && log_n >= (k < DM_SLICE ? 22 : 24) && log_n - k >= 7 ? k : 0;

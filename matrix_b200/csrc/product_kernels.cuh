@@ -1,11 +1,11 @@
-// Several rounds of a sumcheck over a product of one, three or four tables per pass, for tables that are small.
+// Several rounds of a sumcheck over a product of one table, or of three or four small ones, per pass.
 //
 // For sum_x prod_k t_k(x) the next B rounds need nothing of the tables but the 2^(D B) sums
 //     T[i_1 .. i_D] = sum_y prod_k t_k(i_k + 2^B y):
 // folding and evaluating the round polynomials only combine entries, so the host runs the B rounds on T. A round of
 // its own costs a launch, a synchronisation and two reductions whatever its size (about 20 us); T takes 2^((D-1) B)
-// products per element instead of the few of a round polynomial, so it is for tables that leave the chip idle: at 2^16
-// elements of three tables 2^20 products, 8 us, replace two rounds. Three tables of 2^15 elements and more go to the tensor cores
+// products per element instead of the few of a round polynomial, so it is for tables that leave the chip idle: at 2^14
+// elements of three tables 2^20 products, 8 us, replace three rounds. Three tables of 2^15 elements and more go to the tensor cores
 // (product_mma_kernels.cuh), four of 2^14 and more take a round per pass (sumcheck_kernels.cuh).
 //
 // One table: the sums by x mod 2^B are a thread's own, its elements lie a multiple of 256 apart. Otherwise a block takes

@@ -24,11 +24,9 @@ constexpr int TRI_ENTRIES = 36;            // T[p][k] at 4 p + k, p = 3 p(second
 constexpr uint32_t TRI_TMEM = 512;
 constexpr int TRI_Y = 64;                  // y of a tile
 constexpr int TRI_MOST = 32768 / TRI_Y;    // tiles a block: the 32-bit sums of 2^15 rows
-constexpr bool tri_folds(int fb, bool base) { return base ? fb == 2 : fb == 1 || fb == 2; }
 
 struct TriArgs {
-    int fb;               // challenges to fold (0: none)
-    const uint64_t* in;   // three tables of 2^(v + fb) elements
+    const uint64_t* in;   // three tables of 2^v elements, or 2^(v + 2) where there are challenges to fold: the two of the pass before
     size_t stride;        // words from one table to the next
     uint64_t* out;        // [3][2^v][2] folded tables, or null
     int v;                // variables left after the fold, at least 8
@@ -177,10 +175,10 @@ tri_mma_kernel(const TriArgs a, const __grid_constant__ FoldWeights<F> fw) {
             issued.drain();
         }
     } else {
-        const int le = BASE ? 4 - a.fb : 3 - a.fb;                 // log2 of the folded elements in 128 bytes of input: 1 or 2
-        const uint32_t rows = 256u >> le, units = 8 * rows;        // of a table
+        constexpr int le = BASE ? 2 : 1;                           // log2 of the folded elements in 128 bytes of input
+        constexpr uint32_t rows = 256u >> le, units = 8 * rows;    // of a table
         constexpr uint32_t cst = GROUPS * TRI_FOLD_GROUP, fold_cols = 256;   // 128 columns a group
-        const uint32_t idesc_f = tc::idesc_u8(16 << le, false);
+        constexpr uint32_t idesc_f = tc::idesc_u8(16 << le, false);
         const auto load = [&](int turn) {
             const int i = group + GROUPS * turn;
             if (i < count && !failed) {
