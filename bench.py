@@ -1341,9 +1341,9 @@ def run_basefold(args):
     node_bytes = big_nodes(leaves_commit) * (64 + 32 * copies) + sum(big_nodes(m // world) for m in big_folded) * 96
     hash_ms = sum(kernels.get(k, (0, 0))[1] for k in ("hash_leaves", "compress_layer", "tree_up"))
     perms_per_s = (leaves_commit + leaves_folded + nodes_per_step) * prof_steps / (hash_ms * 1e-3) if hash_ms else 0.0
-    # of a permutation's thread: Poseidon2 10870 a thread each (profiles/poseidon2_permute_batch_ncu.md), 9700 in tiles, where nine
-    # tenths of the permutations are at 2^24
-    inst_per_perm = 9800.0 if args.hash == "poseidon2" else 5615.0
+    # of a permutation's thread: Poseidon2 10870 a thread each (profiles/poseidon2_permute_batch_ncu.md), 8640 to 9630 in tiles, where
+    # 85 % of the permutations are at 2^24 (profiles/bench_basefold_launches.md)
+    inst_per_perm = 9090.0 if args.hash == "poseidon2" else 5615.0
     sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
     if dom is not None:
         cnt, ms = kernels[dom]
@@ -1356,15 +1356,15 @@ def run_basefold(args):
         if total_bytes is not None:
             achieved = total_bytes / (ms * 1e-3) / 1e9
             # DRAM bytes per launch, scaled from an ncu capture of the 2^22 case by the units hashed (reads equal the
-            # algorithmic reads; many digest writes are still in L2 when a kernel ends): 65 B per node, 53.6 B per base leaf
-            # pair of the commitment, 104.3 B per folded leaf of the first round, 119.5 B of the later ones.
+            # algorithmic reads; many digest writes are still in L2 when a kernel ends): 66 B per node, 51.7 B per base leaf
+            # pair of the commitment, 104.1 B per folded leaf of the first round, 123.2 B of the later ones.
             if args.hash != "poseidon2":
                 traffic = None
             elif dom == "compress_layer":
-                traffic = 65.0 * (big_nodes(leaves_commit) + sum(big_nodes(m // world) for m in big_folded)) * prof_steps / cnt
+                traffic = 66.0 * (big_nodes(leaves_commit) + sum(big_nodes(m // world) for m in big_folded)) * prof_steps / cnt
             else:
-                traffic = (53.6 * big_commit_leaves
-                           + sum((104.3 if i == 0 else 119.5) * m for i, m in enumerate(big_folded)) / world) * prof_steps / cnt
+                traffic = (51.7 * big_commit_leaves
+                           + sum((104.1 if i == 0 else 123.2) * m for i, m in enumerate(big_folded)) / world) * prof_steps / cnt
             roofline = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                         "traffic_note": "bytes per launch (average), scaled from the capture in profiles/bench_basefold_launches.md",
