@@ -165,29 +165,36 @@ GLF void poseidon2_permute(uint64_t* s) {
 
 #ifdef __CUDACC__
 // ---- one permutation per thread, throughput form ---------------------------------------
-// Bound by the two integer pipes (68 % and 77 % busy in ncu: 2080 wide products of four cycles, the rest carry additions
-// of two). Against the exact form:
+// Bound by the integer pipes: 1436 to 2080 wide products (four cycles of the one pipe) and about as many carry additions (two of the
+// other), which overlap to about 1.4. Against the exact form:
 //   * the last repair of a reduction is left out. It is needed when a 64-bit word comes out below a 33-bit subtrahend (or
-//     a sum of eight words has a high word within 64 of 2^32): about once in 2^31 products. The borrows are collected
-//     in `missed` (one operation instead of three per product), and the caller runs the exact form on the same input
-//     when any was seen (one permutation in four million);
-//   * the linear layers are sums of whole words in 96 bits, three carry additions each, sharing the partial sums of M4,
-//     instead of 128 multiply-adds by small constants (6 cycles each).
-// 25.3 k -> 17.7 k cycles per warp of permutations (1.47e9 -> 2.1e9 permutations/s on the whole GPU).
+//     a sum of eight words has a high word within 64 of 2^32): about once in 2^31 products. Missed tells, and the caller runs the
+//     exact form on the same input (one permutation in a hundred thousand, by the words that only look like it);
+//   * the sums of the internal layer are sums of whole words in 96 bits, three carry additions each; the external layers are on
+//     the FP64 pipe.
+// Exact form 25.3 k cycles per warp of permutations, carries counted and external layers in 96 bits 17.5 k, now 16.8 k (2^19
+// permutations: 253 -> 241 us; tiles, which leave out the internal layers' products, 203 us).
 namespace p2t {
-// Repairs left out so far: borrows are counted downwards, carries upwards, apart, so that they cannot cancel.
+// Repairs left out so far. A borrow left as it is shows in the word it leaves: at least 2^64 - 2^38. So the largest high word
+// tells of them all (and of one right word in 2^26); a maximum goes to the other pipe than a carry kept in a register, and
+// the same holds for an addition to which its own carry is added at once: 27.1 -> 23.4 cycles a product. Carries left
+// out are counted.
 struct Missed {
-    uint32_t borrows, carries;
+    uint32_t top, carries;
+    __device__ __forceinline__ bool any() const { return top >= 0xFFFFFFC0u || carries != 0; }
 };
+// reduce_limbs without the repair; z4 2^128 = -z4 2^32 for z4 < 32
+__device__ __forceinline__ uint64_t reduce(uint32_t z0, uint32_t z1, uint32_t z2, uint32_t z3, uint32_t z4, Missed& missed) {
+    uint32_t A, B0, B1, r0, r1;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %3, %4;\n\taddc.u32 %0, t, 0;\n\taddc.cc.u32 %1, %4, %5;\n\taddc.u32 %2, %6, 0;\n\t}"
+        : "=&r"(A), "=&r"(B0), "=r"(B1) : "r"(z1), "r"(z2), "r"(z3), "r"(z4));
+    asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, %4, %5;" : "=&r"(r0), "=r"(r1) : "r"(z0), "r"(B0), "r"(A), "r"(B1));
+    missed.top = max(missed.top, r1);
+    return pack64(r0, r1);
+}
 __device__ __forceinline__ uint64_t reduce(unsigned __int128 f, Missed& missed) {
     const uint64_t lo = (uint64_t)f, hi = (uint64_t)(f >> 64);
-    uint32_t A, c, B0, B1, r0, r1;   // reduce_limbs without the repair
-    asm("add.cc.u32 %0, %4, %5;\n\taddc.u32 %1, 0, 0;\n\taddc.cc.u32 %2, %5, %6;\n\taddc.u32 %3, 0, 0;"
-        : "=&r"(A), "=&r"(c), "=&r"(B0), "=r"(B1) : "r"(hi32(lo)), "r"(lo32(hi)), "r"(hi32(hi)));
-    A += c;
-    asm("sub.cc.u32 %0, %3, %4;\n\tsubc.cc.u32 %1, %5, %6;\n\tsubc.u32 %2, %2, 0;"
-        : "=&r"(r0), "=r"(r1), "+r"(missed.borrows) : "r"(lo32(lo)), "r"(B0), "r"(A), "r"(B1));
-    return pack64(r0, r1);
+    return reduce(lo32(lo), hi32(lo), lo32(hi), hi32(hi), 0, missed);
 }
 __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b, Missed& missed) { return reduce((unsigned __int128)a * b, missed); }
 __device__ __forceinline__ uint64_t mul_add(uint64_t a, uint64_t b, uint64_t c, Missed& missed) {
@@ -213,42 +220,68 @@ __device__ __forceinline__ Sum sum(Sum x, uint64_t y) {
         : "=&r"(r.a), "=&r"(r.b), "=r"(r.c) : "r"(x.a), "r"(x.b), "r"(x.c), "r"(lo32(y)), "r"(hi32(y)));
     return r;
 }
-__device__ __forceinline__ Sum sum(Sum x, Sum y) {
-    Sum r;
-    asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
-        : "=&r"(r.a), "=&r"(r.b), "=r"(r.c) : "r"(x.a), "r"(x.b), "r"(x.c), "r"(y.a), "r"(y.b), "r"(y.c));
-    return r;
-}
-// (b:a) + c EPS for c < 64; a carry out of b + c and a borrow of (b:a) - c are not repaired
+// (b:a) + c EPS for c < 64; a carry out of b + c and a borrow of (b + c : a) - c are not repaired
 __device__ __forceinline__ uint64_t reduce(Sum x, Missed& missed) {
     uint32_t r0, r1;
-    asm("add.cc.u32 %1, %5, %6;\n\taddc.u32 %2, %2, 0;\n\tsub.cc.u32 %0, %4, %6;\n\tsubc.cc.u32 %1, %1, 0;\n\t"
-        "subc.u32 %3, %3, 0;"
-        : "=&r"(r0), "=&r"(r1), "+r"(missed.carries), "+r"(missed.borrows) : "r"(x.a), "r"(x.b), "r"(x.c));
+    asm("add.cc.u32 %1, %4, %5;\n\taddc.u32 %2, %2, 0;\n\tsub.cc.u32 %0, %3, %5;\n\tsubc.u32 %1, %1, 0;"
+        : "=&r"(r0), "=&r"(r1), "+r"(missed.carries) : "r"(x.a), "r"(x.b), "r"(x.c));
+    missed.top = max(missed.top, r1);
     return pack64(r0, r1);
 }
-template <bool HAS_RC>
+// The external layer on the FP64 pipe, which the integer work leaves idle: the 32-bit halves of the words are whole numbers in
+// doubles (2^52 + x is the word 0x43300000 in front of x), their weighted sums (row sum 21) stay below 2^37, so every
+// operation is exact, and 2^52 + sum carries the sum in its mantissa again. What is left to the integer pipes are the two
+// words of each sum: 84 operations of the FP64 pipe take the place of 160 carry additions. A round with its S-boxes:
+// 1286 -> 1064 cycles a warp and scheduler (990 with the shorter reduction).
+constexpr uint32_t FP_ONE = 0x43300000u;   // high word of 2^52
+__device__ __forceinline__ double whole(uint32_t x) { return __hiloint2double((int)FP_ONE, (int)x); }
+// The constants' halves in front of round r (8: none) with what makes words of the sums: 2^52 on the low sum L, 2^52 + 2^32 - FP_ONE on
+// the high one H, so that FP_ONE in the high word of the first meets its complement in the low word of the second.
+struct RoundConstants {
+    double half[9][8][2];
+};
+constexpr RoundConstants round_constants() {
+    constexpr uint64_t rc[8][8] = GLP2_RC_EXT_INIT;
+    RoundConstants c{};
+    for (int r = 0; r < 9; r++)
+        for (int i = 0; i < 8; i++) {
+            c.half[r][i][0] = 4503599627370496.0 + (double)(r < 8 ? rc[r][i] & 0xFFFFFFFFu : 0);
+            c.half[r][i][1] = 4503599627370496.0 + (double)(r < 8 ? rc[r][i] >> 32 : 0) + (4294967296.0 - (double)FP_ONE);
+        }
+    return c;
+}
+static __constant__ RoundConstants d_round_constants = round_constants();
 __device__ __forceinline__ void external_linear(uint64_t* s, int next_round, Missed& missed) {
-    Sum y[8];
+    double y[2][8];
 #pragma unroll
-    for (int h = 0; h < 8; h += 4) {   // M4 on each half
-        const Sum t01 = sum(s[h], s[h + 1]), t23 = sum(s[h + 2], s[h + 3]), t = sum(t01, t23);
-        const Sum t1 = sum(t, s[h + 1]), t3 = sum(t, s[h + 3]);
-        y[h] = sum(t1, t01);
-        y[h + 1] = sum(sum(t1, s[h + 2]), s[h + 2]);
-        y[h + 2] = sum(t3, t23);
-        y[h + 3] = sum(sum(t3, s[h]), s[h]);
+    for (int h = 0; h < 2; h++) {
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = __dadd_rn(whole(h ? hi32(s[i]) : lo32(s[i])), -4503599627370496.0);
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {   // M4 on each half
+            const double t01 = __dadd_rn(v[q], v[q + 1]), t23 = __dadd_rn(v[q + 2], v[q + 3]), t = __dadd_rn(t01, t23);
+            const double t1 = __dadd_rn(t, v[q + 1]), t3 = __dadd_rn(t, v[q + 3]);
+            y[h][q] = __dadd_rn(t1, t01);
+            y[h][q + 1] = __fma_rn(2.0, v[q + 2], t1);
+            y[h][q + 2] = __dadd_rn(t3, t23);
+            y[h][q + 3] = __fma_rn(2.0, v[q], t3);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const double a = y[h][i], b = y[h][i + 4];
+            y[h][i] = __dadd_rn(__fma_rn(2.0, a, b), d_round_constants.half[next_round][i][h]);
+            y[h][i + 4] = __dadd_rn(__fma_rn(2.0, b, a), d_round_constants.half[next_round][i + 4][h]);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const Sum c = sum(y[i], y[i + 4]);
-        Sum a = sum(y[i], c), b = sum(y[i + 4], c);
-        if (HAS_RC) {
-            a = sum(a, p2_rc_ext(next_round, i));
-            b = sum(b, p2_rc_ext(next_round, i + 4));
-        }
-        s[i] = reduce(a, missed);
-        s[i + 4] = reduce(b, missed);
+    for (int i = 0; i < 8; i++) {
+        Sum x;
+        x.a = (uint32_t)__double2loint(y[0][i]);
+        asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;"
+            : "=&r"(x.b), "=r"(x.c)
+            : "r"((uint32_t)__double2hiint(y[0][i])), "r"((uint32_t)__double2loint(y[1][i])), "r"((uint32_t)__double2hiint(y[1][i])), "n"(0u - FP_ONE - 1));
+        s[i] = reduce(x, missed);
     }
 }
 }  // namespace p2t
@@ -262,13 +295,9 @@ __device__ __forceinline__ bool poseidon2_permute_throughput(uint64_t* s) {
     for (int r = 0; r < 4; r++) {
 #pragma unroll
         for (int i = 0; i < 8; i++) s[i] = p2t::sbox7(s[i], missed);
-        if (r < 3) {
-            p2t::external_linear<true>(s, r + 1, missed);
-        } else {
-            p2t::external_linear<false>(s, 0, missed);
-            s[0] = add_c(s[0], p2_rc_int(0));
-        }
+        p2t::external_linear(s, r < 3 ? r + 1 : 8, missed);
     }
+    s[0] = add_c(s[0], p2_rc_int(0));
 #pragma unroll 1
     for (int r = 0; r < 22; r++) {
         s[0] = p2t::sbox7(s[0], missed);
@@ -286,10 +315,9 @@ __device__ __forceinline__ bool poseidon2_permute_throughput(uint64_t* s) {
     for (int r = 4; r < 8; r++) {
 #pragma unroll
         for (int i = 0; i < 8; i++) s[i] = p2t::sbox7(s[i], missed);
-        if (r < 7) p2t::external_linear<true>(s, r + 1, missed);
-        else p2t::external_linear<false>(s, 0, missed);
+        p2t::external_linear(s, r + 1, missed);
     }
-    return (missed.borrows | missed.carries) == 0;
+    return !missed.any();
 }
 
 // ---- one permutation spread over 8 lanes ----------------------------------------

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "gl_poseidon2.cuh"
 #include "gl_monolith.cuh"
+#include "poseidon2_linear.cuh"
 #include "poseidon2_tiles.cuh"
 
 namespace mb {
@@ -33,7 +34,7 @@ constexpr int BLOCK = 128;
 // coop(x, l): the permutation spread over LANES lanes, lane l holding word l. COOP_NODES: layers of at most this many
 // nodes take the spread form.
 struct HashPoseidon2 {
-    static constexpr int WIDTH = 8, LANES = 8, MIN_BLOCKS = 8;
+    static constexpr int WIDTH = 8, LANES = 8, MIN_BLOCKS = 6;
     static constexpr size_t COOP_NODES = (size_t)1 << 12;
     static __device__ __forceinline__ uint64_t coop(uint64_t x, int l) { return gl::poseidon2_permute_coop8(x, l); }
     template <class Load>
@@ -256,22 +257,19 @@ permute_batch_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out
 }
 
 // The throughput kernels above for Poseidon2 in tiles of 128 (poseidon2_tiles.cuh): node or leaf k < n of a layer, from f as in
-// TreeSource, written `copies` times. Every tile runs as many turns as the longest, for the order in tensor memory.
+// TreeSource, written `copies` times.
 template <TreeSource SRC>
 static __global__ void __launch_bounds__(P2_BLK, 1)
 poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n, size_t copies) {
     extern __shared__ __align__(128) uint8_t p2_sm[];
-    __shared__ __align__(8) uint64_t done[P2_TILES], free[P2_TILES];
+    __shared__ __align__(8) uint64_t done[P2_TILES];
     __shared__ uint32_t tmem_sm;
     __shared__ int failed;
     const int t = threadIdx.x, g = t / P2_TILE;
     p2_operands(p2_sm);
     if (t == 0) {
         failed = 0;
-        for (int i = 0; i < P2_TILES; i++) {
-            tc::mbar_init(&done[i], 1);
-            tc::mbar_init(&free[i], P2_TILE / 32);
-        }
+        for (int i = 0; i < P2_TILES; i++) tc::mbar_init(&done[i], 1);
         tc::mbar_init_fence();
     }
     if (t < 32) tc::tmem_alloc(&tmem_sm, 512);
@@ -281,19 +279,16 @@ poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n,
     tc::fence_after();
     P2Tile tile;
     tile.row = t % P2_TILE;
-    tile.tmem = tmem_sm + 256 * (g & 1) + ((tile.row & ~31u) << 16);
+    tile.tmem = tmem_sm + P2_NA * g + ((tile.row & ~31u) << 16);
     tile.consts = tc::smem_u32(p2_sm);
-    tile.rows = p2_sm + P2_CONST + g * P2_TILE * 64;
+    tile.rows = p2_sm + P2_ROWS + g * P2_TILE * 16 * P2_UNITS;
     tile.done = tc::smem_u32(&done[g]);
-    tile.free = tc::smem_u32(&free[g]);
-    tile.before = tc::smem_u32(&free[(g + P2_TILES - 2) % P2_TILES]);
     tile.id = 1 + g;
-    tile.use = g < 2 ? -1 : 0;   // the first two find their halves empty
     tile.failed = &failed;
     const uint64_t r1w = gl::mul_small(f.r.c1, 7);
-    const size_t step = (size_t)gridDim.x * P2_BLK, turns = (n + step - 1) / step;
-    size_t k = (size_t)blockIdx.x * P2_BLK + t;
-    for (size_t i = 0; i < turns; i++, k += step) {
+    // a layer's tiles go to all SMs before a second one to any
+    const size_t step = (size_t)gridDim.x * P2_BLK;
+    for (size_t k = ((size_t)g * gridDim.x + blockIdx.x) * P2_TILE + tile.row; k - tile.row < n; k += step) {
         const bool live = k < n;
         if ((SRC == FOLD_BASE || SRC == FOLD_EXT) && live) {
             gl::e2_store(f.out + 4 * k, folded_element<SRC == FOLD_BASE>(f, 2 * k, r1w));
@@ -324,13 +319,13 @@ poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n,
     __syncthreads();
     if (t < 32) tc::tmem_free(tmem_sm, 512);
 }
-// Layers of this many permutations and more go in tiles: 2^20 take 503 us a thread each and 474 in tiles, 2^19 250 to 259 and 246
-// to 266 (five turns of every tile, the last of them a tenth full).
-constexpr size_t P2_TILES_FROM = (size_t)1 << 20;
+// Layers of this many permutations and more go in tiles (us, a thread each and in tiles): 2^15 25 and 25, 2^16 42 and 35, 2^17 75 and 57,
+// 2^18 134 and 117, 2^19 245 and 203, 2^20 487 and 383. One tile an SM takes 20 us whatever their number (2^13 and 2^14: a thread each 19).
+constexpr size_t P2_TILES_FROM = (size_t)1 << 16;
 template <TreeSource SRC>
 inline void launch_poseidon2_tiles(const FoldSource& f, uint64_t* dst, size_t n, size_t copies, cudaStream_t st) {
     cudaFuncSetAttribute(poseidon2_tiles_kernel<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2_SMEM);
-    poseidon2_tiles_kernel<SRC><<<sm_count(), P2_BLK, P2_SMEM, st>>>(f, dst, n, copies);
+    poseidon2_tiles_kernel<SRC><<<grid_for(n, P2_TILE, 1), P2_BLK, P2_SMEM, st>>>(f, dst, n, copies);
 }
 template <class H> constexpr bool in_tiles(size_t) { return false; }
 template <> constexpr bool in_tiles<HashPoseidon2>(size_t n) { return n >= P2_TILES_FROM; }

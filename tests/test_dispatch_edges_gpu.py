@@ -122,6 +122,12 @@ def test_poseidon2_tiles(gl, oracle, leaves, ext):
     assert np.array_equal(d_t.to_numpy(), exp)
 
 
+# a layer of 2^15 permutations goes a thread each, 2^16 take three or four tiles an SM, 2^17 a second turn of some
+@pytest.mark.parametrize("leaves,ext", [(1 << 15, True), (1 << 16, False), (1 << 16, True), (1 << 17, False)])
+def test_poseidon2_tiles_of_few_turns(gl, oracle, leaves, ext):
+    test_poseidon2_tiles(gl, oracle, leaves, ext)
+
+
 @pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
                                      (22, 6), (22, 7), (22, 9), (24, 10), (24, 11), (24, 13), (25, 11), (25, 12)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):
