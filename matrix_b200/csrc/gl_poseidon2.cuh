@@ -204,6 +204,20 @@ __device__ __forceinline__ uint64_t sbox7(uint64_t x, Missed& missed) {
     const uint64_t x2 = mul(x, x, missed), x4 = mul(x2, x2, missed), x3 = mul(x2, x, missed);
     return mul(x4, x3, missed);
 }
+// For code that waits for single results: a product less (the cross one doubled) takes 9 cycles off an S-box; where many run at a time,
+// the shifts cost more than the product.
+__device__ __forceinline__ uint64_t sqr(uint64_t a, Missed& missed) {
+    const uint32_t a0 = lo32(a), a1 = hi32(a);
+    const uint64_t e = (uint64_t)a0 * a0, f = (uint64_t)a1 * a1, o = (uint64_t)a0 * a1;
+    uint32_t z1 = hi32(e), z2 = lo32(f), z3 = hi32(f);
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(z1), "+r"(z2), "+r"(z3) : "r"(lo32(o) << 1), "r"((uint32_t)(o >> 31)), "r"(hi32(o) >> 31));
+    return reduce(lo32(e), z1, z2, z3, 0, missed);
+}
+__device__ __forceinline__ uint64_t sbox7_soon(uint64_t x, Missed& missed) {
+    const uint64_t x2 = sqr(x, missed), x4 = sqr(x2, missed), x3 = mul(x2, x, missed);
+    return mul(x4, x3, missed);
+}
 // sums of words: 96 bits
 struct Sum {
     uint32_t a, b, c;
@@ -323,78 +337,88 @@ __device__ __forceinline__ bool poseidon2_permute_throughput(uint64_t* s) {
 // ---- one permutation spread over 8 lanes ----------------------------------------
 // Layers near the top of a Merkle tree (and a transcript) have too few
 // permutations to fill the machine; what matters there is the latency of one
-// permutation. Eight consecutive lanes of a warp hold one state word each: the
+// permutation: the length of the chain of dependent instructions, 56 cycles for a product with its reduction, 24 for a
+// shuffle. Eight consecutive lanes of a warp hold one state word each: the
 // S-boxes of an external round run in parallel, the linear layers exchange
-// halves with warp shuffles, and in the internal rounds lane 0 runs the S-box
-// while the sum is formed by a three-step butterfly. Per-lane constants come
+// words with warp shuffles. Per-lane constants come
 // from global copies of the tables (a divergent index into __constant__ memory
 // would serialise). All 32 lanes of the warp must call; `lane8` = lane & 7.
 static __device__ const uint64_t g_p2_rc_ext[8][8] = GLP2_RC_EXT_INIT;
 static __device__ const uint64_t g_p2_diag[8] = GLP2_DIAG_INIT;
 
-__device__ __forceinline__ uint64_t p2_coop_external(uint64_t x, const uint32_t (&w)[8], uint64_t rc) {
-    uint64_t L = lo32(rc), H = hi32(rc);
-    const uint32_t xl = lo32(x), xh = hi32(x);
+// y = M x + rc over limbs of 22 bits (sums of weight 21 stay in 32), which butterflies of a lane's half and a shuffle across form: 208 cycles,
+// 292 with every word sent to every lane and multiplied there.
+__device__ __forceinline__ uint64_t p2_coop_external(uint64_t x, int lane8, uint64_t rc, p2t::Missed& missed) {
+    const uint32_t limb[3] = {lo32(x) & 0x3FFFFFu, (uint32_t)(x >> 22) & 0x3FFFFFu, hi32(x) >> 12};
+    const int next = (lane8 & 4) | ((lane8 + 1) & 3);
+    uint32_t o[3];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        L = madwide(__shfl_sync(0xffffffffu, xl, j, 8), w[j], L);
-        H = madwide(__shfl_sync(0xffffffffu, xh, j, 8), w[j], H);
+    for (int k = 0; k < 3; k++) {
+        const uint32_t l = limb[k], r = __shfl_sync(0xffffffffu, l, next, 8);
+        uint32_t t = l + __shfl_xor_sync(0xffffffffu, l, 1, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 2, 8);
+        const uint32_t y = t + l + 2 * r;   // M4 is circulant: first row 2 3 1 1
+        o[k] = 2 * y + __shfl_xor_sync(0xffffffffu, y, 4, 8);
     }
-    return reduce_limb_sums(L, H);
+    const uint64_t L = madwide(o[1], 1u << 22, (uint64_t)o[0]) + lo32(rc), H = madwide(o[2], 1u << 12, (uint64_t)hi32(rc));
+    p2t::Sum s;
+    s.a = lo32(L);
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;" : "=&r"(s.b), "=r"(s.c) : "r"(hi32(L)), "r"(lo32(H)), "r"(hi32(H)));
+    return p2t::reduce(s, missed);
+}
+
+// The exact form for the whole warp, a permutation a thread: what the form below falls back to.
+static __device__ __noinline__ uint64_t poseidon2_permute_gathered(uint64_t x, int lane8) {
+    uint64_t s[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) s[j] = pack64(__shfl_sync(0xffffffffu, lo32(x), j, 8), __shfl_sync(0xffffffffu, hi32(x), j, 8));
+    poseidon2_permute(s);
+#pragma unroll
+    for (int j = 0; j < 8; j++) x = j == lane8 ? s[j] : x;
+    return x;
 }
 
 __device__ __forceinline__ uint64_t poseidon2_permute_coop8(uint64_t x, int lane8) {
-    // row lane8 of M = [[2 M4, M4], [M4, 2 M4]]
-    uint32_t w[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        int d = ((j & 3) - (lane8 & 3)) & 3;  // M4 is circulant: first row 2 3 1 1
-        uint32_t m4 = d == 0 ? 2u : (d == 1 ? 3u : 1u);
-        w[j] = ((j >> 2) == (lane8 >> 2)) ? 2u * m4 : m4;
-    }
-    const uint64_t diag = g_p2_diag[lane8];
+    const uint64_t in = x;
+    p2t::Missed missed{0, 0};
     x = add_c(x, g_p2_rc_ext[0][lane8]);
 #pragma unroll 1
     for (int r = 0; r < 4; r++) {
-        x = sbox7(x);
-        x = p2_coop_external(x, w, r < 3 ? g_p2_rc_ext[r + 1][lane8] : (lane8 == 0 ? p2_rc_int(0) : 0));
+        x = p2t::sbox7_soon(x, missed);
+        x = p2_coop_external(x, lane8, r < 3 ? g_p2_rc_ext[r + 1][lane8] : 0, missed);
     }
-    // Internal rounds: x_0 <- sbox(x_0), then x_i <- diag_i x_i + sum_j x_j. What matters here is the length of
-    // the dependent chain, so everything that does not need the S-box output runs beside it: the products
-    // diag_i x_i of the other lanes and the sum of their x_i (a three-step butterfly) are formed from the round's
-    // inputs while the S-box chain (three multiplications deep) is in flight; afterwards lane 0's value is
-    // broadcast, added to the partial sum, and one 128-bit add and reduction finish every lane. All lanes execute
-    // the S-box arithmetic (only lane 0 keeps it), which keeps the warp converged so that the two chains interleave.
+    // Internal rounds: y = (word 0 + constant)^7, words <- diag words + (y + the sum Q of words 1 .. 7). Every lane has the S-box
+    // input s and forms y itself, so that no shuffle is on the chain from one S-box to the next:
+    //     s <- (diag_0 + 1) y + Q + constant      four products deep
+    // and Q, which needs the words one round late only, is formed beside the S-box: a three-step butterfly over limbs of
+    // 22 bits (sums of eight stay in 32).
     const bool lane0 = lane8 == 0;
+    const uint64_t diag = g_p2_diag[lane8], first = p2_diag(0) + 1;
+    uint64_t s = add_c(pack64(__shfl_sync(0xffffffffu, lo32(x), 0, 8), __shfl_sync(0xffffffffu, hi32(x), 0, 8)), p2_rc_int(0));
 #pragma unroll 1
     for (int r = 0; r < 22; r++) {
-        const uint64_t t = sbox7(x);
-        // beside the S-box: the other lanes' products and their partial sum
-        uint64_t ylo = x * diag, yhi = umulhi(x, diag);
-        uint64_t UL = lane0 ? 0 : lo32(x), UH = lane0 ? 0 : hi32(x);
+        const uint64_t y = p2t::sbox7_soon(s, missed);
+        const uint64_t v = lane0 ? 0 : x;
+        uint32_t l0 = lo32(v) & 0x3FFFFFu, l1 = (uint32_t)(v >> 22) & 0x3FFFFFu, l2 = hi32(v) >> 12;
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) {
-            UL += __shfl_xor_sync(0xffffffffu, UL, off, 8);
-            UH += __shfl_xor_sync(0xffffffffu, UH, off, 8);
+            l0 += __shfl_xor_sync(0xffffffffu, l0, off, 8);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, off, 8);
+            l2 += __shfl_xor_sync(0xffffffffu, l2, off, 8);
         }
-        // after the S-box: its output to every lane, the full sum, lane 0's own product
-        const uint32_t tl = __shfl_sync(0xffffffffu, lo32(t), 0, 8), th = __shfl_sync(0xffffffffu, hi32(t), 0, 8);
-        // lane 0's own product needs the S-box output; formed on every lane (no branch) beside the sum
-        const uint64_t zlo = t * diag, zhi = umulhi(t, diag);
-        uint64_t sum = reduce_limb_sums(UL + tl, UH + th);
-        sum = add_c(sum, (lane0 && r < 21) ? p2_rc_int(r + 1) : 0);
-        ylo = lane0 ? zlo : ylo;
-        yhi = lane0 ? zhi : yhi;
-        uint32_t carry;
-        const uint64_t l2 = add_carry(ylo, sum, carry);
-        x = reduce128(l2, yhi + carry);
+        const uint64_t q = reduce_limb_sums(madwide(l1, 1u << 22, l0), (uint64_t)l2 << 12);
+        const unsigned __int128 beside = (unsigned __int128)x * diag + q;
+        const uint64_t qc = r < 21 ? add_c(q, p2_rc_int(r + 1)) : q;
+        s = p2t::mul_add(y, first, qc, missed);
+        x = p2t::reduce(beside + y, missed);   // below 2^128: diag < p
     }
-    x = add_c(x, g_p2_rc_ext[4][lane8]);
+    x = add_c(lane0 ? s : x, g_p2_rc_ext[4][lane8]);
 #pragma unroll 1
     for (int r = 4; r < 8; r++) {
-        x = sbox7(x);
-        x = p2_coop_external(x, w, r < 7 ? g_p2_rc_ext[r + 1][lane8] : 0);
+        x = p2t::sbox7_soon(x, missed);
+        x = p2_coop_external(x, lane8, r < 7 ? g_p2_rc_ext[r + 1][lane8] : 0, missed);
     }
+    if (__any_sync(0xffffffffu, missed.any())) return poseidon2_permute_gathered(in, lane8);
     return x;
 }
 #endif

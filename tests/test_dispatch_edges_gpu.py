@@ -128,6 +128,22 @@ def test_poseidon2_tiles_of_few_turns(gl, oracle, leaves, ext):
     test_poseidon2_tiles(gl, oracle, leaves, ext)
 
 
+@pytest.mark.parametrize("log_leaves", range(13))
+@pytest.mark.parametrize("ext", [False, True])
+def test_small_poseidon2_trees(gl, oracle, log_leaves, ext):
+    """Eight lanes a permutation and a warp a permutation, by the number of levels left: every split of levels into launches, with
+    leaves whose first product needs the exact form (2^96) in the lowest layer."""
+    leaves, width = 1 << log_leaves, 4 if ext else 2
+    cw = field_elems(91 + log_leaves, leaves * width).reshape(leaves, width)
+    for k in {0, leaves // 3, leaves - 1}:
+        cw[k, 0] = (2**48 - 0xdd5743e7f2a5a5d9) % GL_P
+    d_cw, d_t = DeviceBuffer.from_numpy(gl, cw.reshape(-1)), DeviceBuffer(gl, 32 * (2 * leaves - 1))
+    assert (gl.poseidon2_merkle_tree_ext2_ffi if ext else gl.poseidon2_merkle_tree_gl_ffi)(d_cw.ptr, d_t.ptr, leaves) == 0
+    exp = np.zeros(4 * (2 * leaves - 1), dtype=np.uint64)
+    oracle.oracle_bf_merkle_tree(cw.ctypes.data, leaves, int(ext), exp.ctypes.data)
+    assert np.array_equal(d_t.to_numpy(), exp)
+
+
 @pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
                                      (22, 6), (22, 7), (22, 9), (24, 10), (24, 11), (24, 13), (25, 11), (25, 12)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):
