@@ -17,7 +17,7 @@
 // (2^18 compressions: 96 -> 61 us). Values are loose in [0, 2^64) between layers; words 0..3 are made canonical before the
 // bars (the S-box acts on the canonical bit pattern), and the caller canonicalises what it stores.
 #pragma once
-#include "gl_field.cuh"
+#include "gl_fast.cuh"
 
 namespace gl {
 
@@ -56,14 +56,13 @@ GLF uint64_t mono_rc(int round, int i) {
 #endif
 }
 
-// The byte S-box on four bytes at once: y = rotl8(x ^ (rotl8(~x,1) & rotl8(x,2) & rotl8(x,3)), 1).
+// The byte S-box on four bytes at once: y = rotl8(x ^ (rotl8(~x,1) & rotl8(x,2) & rotl8(x,3)), 1). A rotation is two shifts and one choice by
+// a mask.
+GLF uint32_t mono_pick(uint32_t a, uint32_t b, uint32_t mask) { return (a & mask) | (b & ~mask); }
 GLF uint32_t mono_bar32(uint32_t x) {
-    uint32_t nx = ~x;
-    uint32_t l1 = ((nx & 0x80808080u) >> 7) | ((nx & 0x7F7F7F7Fu) << 1);
-    uint32_t l2 = ((x & 0xC0C0C0C0u) >> 6) | ((x & 0x3F3F3F3Fu) << 2);
-    uint32_t l3 = ((x & 0xE0E0E0E0u) >> 5) | ((x & 0x1F1F1F1Fu) << 3);
-    uint32_t t = x ^ (l1 & l2 & l3);
-    return ((t & 0x80808080u) >> 7) | ((t & 0x7F7F7F7Fu) << 1);
+    const uint32_t l1 = mono_pick(x << 1, x >> 7, 0xFEFEFEFEu), l2 = mono_pick(x << 2, x >> 6, 0xFCFCFCFCu), l3 = mono_pick(x << 3, x >> 5, 0xF8F8F8F8u);
+    const uint32_t t = x ^ (~l1 & l2 & l3);
+    return mono_pick(t << 1, t >> 7, 0xFEFEFEFEu);
 }
 GLF uint64_t mono_bar(uint64_t x) { return pack64(mono_bar32(lo32(x)), mono_bar32(hi32(x))); }
 
@@ -150,6 +149,96 @@ GLF void monolith_permute(uint64_t* s) {
 }
 
 #ifdef __CUDACC__
+// ---- one permutation per thread, throughput form ---------------------------------------
+// The linear layers on the FP64 pipe (halves of 32 bits: sums below 2^40), 192 of its operations a layer where the integer pipes took three
+// limbs of 84 additions, their masks and their sums. As in Poseidon2's throughput form the rare repairs are left out and told of; the
+// caller runs the exact form then. 7.4 k -> 6.2 k cycles a warp of permutations and scheduler (2^21 nodes: 428 -> 360 us), issue slots
+// 0.68, the carry pipe 0.6 and the FP64 pipe 0.42 busy.
+namespace monot {
+using namespace fast;
+struct RoundConstants {
+    double half[MONO_ROUNDS + 1][MONO_W][2];
+};
+constexpr RoundConstants round_constants() {
+    constexpr uint64_t rc[MONO_ROUNDS + 1][MONO_W] = GLMONO_RC_INIT;
+    RoundConstants c{};
+    for (int r = 0; r <= MONO_ROUNDS; r++)
+        for (int i = 0; i < MONO_W; i++) {
+            c.half[r][i][0] = LOW_HALF + (double)(rc[r][i] & 0xFFFFFFFFu);
+            c.half[r][i][1] = HIGH_HALF + (double)(rc[r][i] >> 32);
+        }
+    return c;
+}
+static __constant__ RoundConstants d_round_constants = round_constants();
+
+// o = circulant times the words x: mono_circulant's split, the differences x_j - x_(j+6) straight from 2^52 + x.
+__device__ __forceinline__ void circulant(const uint32_t (&x)[MONO_W], double (&o)[MONO_W]) {
+    double p[6], m[6], u[3], v[3], A[3], B[3], M[6];
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+        const double a = whole(x[j]), b = whole(x[j + 6]);
+        m[j] = __dsub_rn(a, b);
+        p[j] = __dadd_rn(__dadd_rn(a, -2 * TWO_52), b);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        u[j] = __dadd_rn(p[j], p[j + 3]);
+        v[j] = __dsub_rn(p[j], p[j + 3]);
+    }
+    const double sum16 = __dmul_rn(__dadd_rn(__dadd_rn(u[0], u[1]), u[2]), 16.0);
+#pragma unroll
+    for (int i = 0; i < 3; i++) A[i] = __fma_rn(u[(i + 2) % 3], -8.0, sum16);
+    B[0] = __dsub_rn(__fma_rn(v[0], -8.0, -v[1]), v[2]);
+    B[1] = __dsub_rn(__fma_rn(v[1], -8.0, v[0]), v[2]);
+    B[2] = __dadd_rn(__fma_rn(v[2], -8.0, v[0]), v[1]);
+    const auto row = [](double a, double b, double c, double by8, double by2, double by4, double two, double four) {
+        return __fma_rn(by4, four, __fma_rn(by2, two, __fma_rn(by8, 8.0, __dadd_rn(__dadd_rn(a, b), c))));
+    };
+    M[0] = row(m[2], m[5], -m[0], m[1], m[3], m[4], 2.0, -4.0);
+    M[1] = row(m[3], -m[0], -m[1], m[2], m[4], m[5], 2.0, -4.0);
+    M[2] = row(m[4], -m[1], -m[2], m[3], m[5], m[0], 2.0, 4.0);
+    M[3] = row(m[5], -m[2], -m[3], m[4], m[0], m[1], -2.0, 4.0);
+    M[4] = row(-m[0], -m[3], -m[4], m[5], m[1], m[2], -2.0, 4.0);
+    M[5] = row(-m[1], -m[4], -m[5], -m[0], m[2], m[3], -2.0, 4.0);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const double lo = __dadd_rn(A[i], B[i]), hi = __dsub_rn(A[i], B[i]);
+        o[i] = __dadd_rn(lo, M[i]);
+        o[i + 6] = __dsub_rn(lo, M[i]);
+        o[i + 3] = __dadd_rn(hi, M[i + 3]);
+        o[i + 9] = __dsub_rn(hi, M[i + 3]);
+    }
+}
+__device__ __forceinline__ void concrete(uint64_t* s, int round, Missed& missed) {
+    uint32_t x[MONO_W];
+    double l[MONO_W], h[MONO_W];
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) x[j] = lo32(s[j]);
+    circulant(x, l);
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) x[j] = hi32(s[j]);
+    circulant(x, h);
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++)
+        s[j] = from_halves(__dadd_rn(l[j], d_round_constants.half[round][j][0]), __dadd_rn(h[j], d_round_constants.half[round][j][1]), missed);
+}
+}  // namespace monot
+
+// In place; loose in, loose out. False: the state is not the permutation's (run the exact form on the input again).
+__device__ __forceinline__ bool monolith_permute_throughput(uint64_t* s) {
+    fast::Missed missed{0, 0};
+    monot::concrete(s, 0, missed);
+#pragma unroll 1
+    for (int r = 1; r <= MONO_ROUNDS; r++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[i] = mono_bar(canon(s[i]));
+#pragma unroll
+        for (int i = MONO_W - 1; i >= 1; i--) s[i] = fast::mul_add(s[i - 1], s[i - 1], s[i], missed);
+        monot::concrete(s, r, missed);
+    }
+    return !missed.any();
+}
+
 // ---- one permutation spread over 16 lanes ----------------------------------------
 // For layers too small to fill the machine, where the latency of a permutation is what counts: lane i < 12 holds word i.
 // A linear layer is twelve shuffles of each half against the lane's row of the circulant (two chains of twelve

@@ -6,7 +6,7 @@
 // constants (cuda/poseidon2.cuh:50-94). State words are loose residues in
 // [0, 2^64); callers canonicalise what they write out.
 #pragma once
-#include "gl_field.cuh"
+#include "gl_fast.cuh"
 
 namespace gl {
 
@@ -175,53 +175,16 @@ GLF void poseidon2_permute(uint64_t* s) {
 // Exact form 25.3 k cycles per warp of permutations, carries counted and external layers in 96 bits 17.5 k, now 16.8 k (2^19
 // permutations: 253 -> 241 us; tiles, which leave out the internal layers' products, 203 us).
 namespace p2t {
-// Repairs left out so far. A borrow left as it is shows in the word it leaves: at least 2^64 - 2^38. So the largest high word
-// tells of them all (and of one right word in 2^26); a maximum goes to the other pipe than a carry kept in a register, and
-// the same holds for an addition to which its own carry is added at once: 27.1 -> 23.4 cycles a product. Carries left
-// out are counted.
-struct Missed {
-    uint32_t top, carries;
-    __device__ __forceinline__ bool any() const { return top >= 0xFFFFFFC0u || carries != 0; }
-};
-// reduce_limbs without the repair; z4 2^128 = -z4 2^32 for z4 < 32
-__device__ __forceinline__ uint64_t reduce(uint32_t z0, uint32_t z1, uint32_t z2, uint32_t z3, uint32_t z4, Missed& missed) {
-    uint32_t A, B0, B1, r0, r1;
-    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %3, %4;\n\taddc.u32 %0, t, 0;\n\taddc.cc.u32 %1, %4, %5;\n\taddc.u32 %2, %6, 0;\n\t}"
-        : "=&r"(A), "=&r"(B0), "=r"(B1) : "r"(z1), "r"(z2), "r"(z3), "r"(z4));
-    asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, %4, %5;" : "=&r"(r0), "=r"(r1) : "r"(z0), "r"(B0), "r"(A), "r"(B1));
-    missed.top = max(missed.top, r1);
-    return pack64(r0, r1);
-}
-__device__ __forceinline__ uint64_t reduce(unsigned __int128 f, Missed& missed) {
-    const uint64_t lo = (uint64_t)f, hi = (uint64_t)(f >> 64);
-    return reduce(lo32(lo), hi32(lo), lo32(hi), hi32(hi), 0, missed);
-}
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b, Missed& missed) { return reduce((unsigned __int128)a * b, missed); }
-__device__ __forceinline__ uint64_t mul_add(uint64_t a, uint64_t b, uint64_t c, Missed& missed) {
-    return reduce((unsigned __int128)a * b + c, missed);
-}
+using namespace fast;
 __device__ __forceinline__ uint64_t sbox7(uint64_t x, Missed& missed) {
     const uint64_t x2 = mul(x, x, missed), x4 = mul(x2, x2, missed), x3 = mul(x2, x, missed);
     return mul(x4, x3, missed);
-}
-// For code that waits for single results: a product less (the cross one doubled) takes 9 cycles off an S-box; where many run at a time,
-// the shifts cost more than the product.
-__device__ __forceinline__ uint64_t sqr(uint64_t a, Missed& missed) {
-    const uint32_t a0 = lo32(a), a1 = hi32(a);
-    const uint64_t e = (uint64_t)a0 * a0, f = (uint64_t)a1 * a1, o = (uint64_t)a0 * a1;
-    uint32_t z1 = hi32(e), z2 = lo32(f), z3 = hi32(f);
-    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-        : "+r"(z1), "+r"(z2), "+r"(z3) : "r"(lo32(o) << 1), "r"((uint32_t)(o >> 31)), "r"(hi32(o) >> 31));
-    return reduce(lo32(e), z1, z2, z3, 0, missed);
 }
 __device__ __forceinline__ uint64_t sbox7_soon(uint64_t x, Missed& missed) {
     const uint64_t x2 = sqr(x, missed), x4 = sqr(x2, missed), x3 = mul(x2, x, missed);
     return mul(x4, x3, missed);
 }
-// sums of words: 96 bits
-struct Sum {
-    uint32_t a, b, c;
-};
+// sums of words
 __device__ __forceinline__ Sum sum(uint64_t x, uint64_t y) {
     Sum r;
     asm("add.cc.u32 %0, %3, %5;\n\taddc.cc.u32 %1, %4, %6;\n\taddc.u32 %2, 0, 0;"
@@ -234,23 +197,12 @@ __device__ __forceinline__ Sum sum(Sum x, uint64_t y) {
         : "=&r"(r.a), "=&r"(r.b), "=r"(r.c) : "r"(x.a), "r"(x.b), "r"(x.c), "r"(lo32(y)), "r"(hi32(y)));
     return r;
 }
-// (b:a) + c EPS for c < 64; a carry out of b + c and a borrow of (b + c : a) - c are not repaired
-__device__ __forceinline__ uint64_t reduce(Sum x, Missed& missed) {
-    uint32_t r0, r1;
-    asm("add.cc.u32 %1, %4, %5;\n\taddc.u32 %2, %2, 0;\n\tsub.cc.u32 %0, %3, %5;\n\tsubc.u32 %1, %1, 0;"
-        : "=&r"(r0), "=&r"(r1), "+r"(missed.carries) : "r"(x.a), "r"(x.b), "r"(x.c));
-    missed.top = max(missed.top, r1);
-    return pack64(r0, r1);
-}
 // The external layer on the FP64 pipe, which the integer work leaves idle: the 32-bit halves of the words are whole numbers in
 // doubles (2^52 + x is the word 0x43300000 in front of x), their weighted sums (row sum 21) stay below 2^37, so every
 // operation is exact, and 2^52 + sum carries the sum in its mantissa again. What is left to the integer pipes are the two
 // words of each sum: 84 operations of the FP64 pipe take the place of 160 carry additions. A round with its S-boxes:
 // 1286 -> 1064 cycles a warp and scheduler (990 with the shorter reduction).
-constexpr uint32_t FP_ONE = 0x43300000u;   // high word of 2^52
-__device__ __forceinline__ double whole(uint32_t x) { return __hiloint2double((int)FP_ONE, (int)x); }
-// The constants' halves in front of round r (8: none) with what makes words of the sums: 2^52 on the low sum L, 2^52 + 2^32 - FP_ONE on
-// the high one H, so that FP_ONE in the high word of the first meets its complement in the low word of the second.
+// The constants' halves in front of round r (8: none), with what from_halves wants on the sums.
 struct RoundConstants {
     double half[9][8][2];
 };
@@ -259,8 +211,8 @@ constexpr RoundConstants round_constants() {
     RoundConstants c{};
     for (int r = 0; r < 9; r++)
         for (int i = 0; i < 8; i++) {
-            c.half[r][i][0] = 4503599627370496.0 + (double)(r < 8 ? rc[r][i] & 0xFFFFFFFFu : 0);
-            c.half[r][i][1] = 4503599627370496.0 + (double)(r < 8 ? rc[r][i] >> 32 : 0) + (4294967296.0 - (double)FP_ONE);
+            c.half[r][i][0] = LOW_HALF + (double)(r < 8 ? rc[r][i] & 0xFFFFFFFFu : 0);
+            c.half[r][i][1] = HIGH_HALF + (double)(r < 8 ? rc[r][i] >> 32 : 0);
         }
     return c;
 }
@@ -271,7 +223,7 @@ __device__ __forceinline__ void external_linear(uint64_t* s, int next_round, Mis
     for (int h = 0; h < 2; h++) {
         double v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = __dadd_rn(whole(h ? hi32(s[i]) : lo32(s[i])), -4503599627370496.0);
+        for (int i = 0; i < 8; i++) v[i] = __dadd_rn(whole(h ? hi32(s[i]) : lo32(s[i])), -TWO_52);
 #pragma unroll
         for (int q = 0; q < 8; q += 4) {   // M4 on each half
             const double t01 = __dadd_rn(v[q], v[q + 1]), t23 = __dadd_rn(v[q + 2], v[q + 3]), t = __dadd_rn(t01, t23);
@@ -290,12 +242,7 @@ __device__ __forceinline__ void external_linear(uint64_t* s, int next_round, Mis
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        Sum x;
-        x.a = (uint32_t)__double2loint(y[0][i]);
-        asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;"
-            : "=&r"(x.b), "=r"(x.c)
-            : "r"((uint32_t)__double2hiint(y[0][i])), "r"((uint32_t)__double2loint(y[1][i])), "r"((uint32_t)__double2hiint(y[1][i])), "n"(0u - FP_ONE - 1));
-        s[i] = reduce(x, missed);
+        s[i] = from_halves(y[0][i], y[1][i], missed);
     }
 }
 }  // namespace p2t

@@ -61,7 +61,10 @@ struct HashMonolith {
     template <class Load>
     static __device__ __forceinline__ void permute(uint64_t* s, Load load) {
         load(s);
-        gl::monolith_permute(s);
+        if (!gl::monolith_permute_throughput(s)) {
+            load(s);
+            gl::monolith_permute(s);
+        }
     }
     static const char* leaves_name() { return "monolith_hash_leaves"; }
     static const char* layer_name() { return "monolith_compress_layer"; }
