@@ -24,6 +24,7 @@
 #include <vector>
 #include "../same_point_kernels.cuh"
 #include "agl_transcript.hpp"
+#include "arrivals.hpp"
 #include "host_field.hpp"
 #include "scratch_pool.hpp"
 
@@ -147,7 +148,7 @@ public:
         if (scratch_) ScratchPool::give(scratch_, cudaStreamSynchronize(MB_STREAM) == cudaSuccess);
     }
     // Stages of the proof, eq tables of all passes, and the first pass, all queued; the sums of the first stage are in
-    // sums() after a stream synchronisation. claims_only: nothing after the first pass will be asked for; share: later stages
+    // sums() after wait(). claims_only: nothing after the first pass will be asked for; share: later stages
     // return the values of their rounds' polynomial, else each leaf's sums.
     int init(int M, int arity, const uint64_t* h_pts, int kind, const uint64_t* d_w0, const uint64_t* d_w1, bool claims_only, bool share) {
         M_ = M; share_ = share; k_ = arity; kind_ = kind; w0_ = d_w0; w1_ = d_w1;
@@ -218,6 +219,7 @@ public:
         a.lo_bits = lo_bits; a.hi_bits = rest - lo_bits; a.in_bits = inside; a.first_bits = stages_[0].rounds;
         a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = stages_[0].wl; a.wh_off = stages_[0].wh; a.low_off = low_off;
         a.partial = b_.partial; a.g6 = b_.g6; a.counter = b_.counter; a.out = h_sums_;
+        expect_sums(stages_[0]);
         // eight warps a block, a warp per high index: a power of two of blocks, so that no warp has more of them
         int gx = 1;
         while (2 * gx <= cap && (size_t)16 * gx <= ((size_t)1 << a.hi_bits)) gx *= 2;
@@ -230,6 +232,8 @@ public:
     }
     // The polynomial of the first stage's rounds, once alpha is known.
     int first_share(E2 alpha) {
+        expect_values(stages_[0]);
+        sums_words_ = 0;
         MB_KERNEL("same_point_share");
         sp::first_share_kernel<<<M_, sp::BLK, 0, MB_STREAM>>>(h_sums_, stages_[0].rounds, b_.pts, k_, alpha, b_.scale, scratch_.dev, scratch_.host);
         return finish_async();
@@ -246,7 +250,10 @@ public:
         a.tabs = b_.tabs; a.leaf_words = leaf_words_; a.wl_off = s.wl; a.wh_off = s.wh;
         a.partial = b_.partial; a.counter = b_.counter;
         a.out = !share_ || i == 0 || i + 1 == stages_.size() ? h_sums_ : nullptr;   // for the first share; for the reveals
+        if (a.out != nullptr) expect_sums(s);
+        else sums_words_ = 0;
         if (share_ && i > 0) {
+            expect_values(s);
             a.pts = b_.pts; a.arity = k_; a.first = s.first; a.bound = stages_[i - 1].rounds;
             a.scale = b_.scale; a.acc = scratch_.dev; a.u = scratch_.host;
             for (int j = 0; j < a.bound; j++) a.r[j] = r[count - a.bound + j];
@@ -293,11 +300,25 @@ public:
         }
         return finish_async();
     }
+    // The results of the pass queued last.
+    int wait() const {
+        if (value_words_) {
+            int rc = await_words(scratch_.host, value_words_);
+            if (rc != MB_OK) return rc;
+        }
+        return await_words(h_sums_, sums_words_);
+    }
     const std::vector<Stage>& stages() const { return stages_; }
     const uint64_t* sums() const { return h_sums_; }   // [leaf][2^rounds][2] of the stage queued last; share: of the first or the last
     const uint64_t* values() const { return scratch_.host; }   // [3^rounds][2] of the stage queued last
 
 private:
+    void expect_sums(const Stage& s) { expect_words(h_sums_, sums_words_ = ((size_t)2 << s.rounds) * M_); }
+    void expect_values(const Stage& s) {
+        value_words_ = 2;
+        for (int j = 0; j < s.rounds; j++) value_words_ *= 3;
+        expect_words(scratch_.host, value_words_);
+    }
     template <int B, int SRC, class W>
     static void launch(bool share, dim3 grid, size_t smem, const sp::FoldArgs& a, const W& w) {
         if (share) sp::fold_pass_kernel<B, SRC, true, W><<<grid, sp::BLK, smem, MB_STREAM>>>(a, w);
@@ -314,7 +335,7 @@ private:
             }
     }
     int M_ = 0, k_ = 0, kind_ = 0, max_blocks_ = 1;
-    size_t words_ = 1, leaf_words_ = 0;
+    size_t words_ = 1, leaf_words_ = 0, sums_words_ = 0, value_words_ = 0;   // the last two: of the pass queued last
     const uint64_t *w0_ = nullptr, *w1_ = nullptr;
     uint64_t *h_sums_ = nullptr, *cur_ = nullptr;
     bool flip_ = false, share_ = false;
@@ -333,7 +354,8 @@ int same_point_claims(int M, int arity, const uint64_t* h_pts, int kind, const u
     SamePointDevice dev;
     int rc = dev.init(M, arity, h_pts, kind, d_w0, d_w1, true, false);
     if (rc != MB_OK) return rc;
-    MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+    rc = dev.wait();
+    if (rc != MB_OK) return rc;
     const int b = dev.stages()[0].rounds;
     for (int i = 0; i < M; i++) {
         E2 g[1 << sp::MAX_B];
@@ -394,7 +416,8 @@ int rounds_by_leaf(SamePointDevice& dev, int M, int arity, const uint64_t* h_pts
                 at += n;
             }
         }
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        int rc = dev.wait();
+        if (rc != MB_OK) return rc;
         for (size_t x = 0; x < (size_t)M * size; x++) g[x] = E2{dev.sums()[2 * x], dev.sums()[2 * x + 1]};
         for (int j = 0; j < B; j++) {
             const int round = st.first + j, half = size >> (j + 1);
@@ -469,7 +492,8 @@ int rounds_by_share(SamePointDevice& dev, int M, int arity, E2 alpha, AglTranscr
         }
         if (rc != MB_OK) return rc;
         t.begin_append(SP_LABEL(L_MSG));   // while the pass runs
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+        rc = dev.wait();
+        if (rc != MB_OK) return rc;
         int size = 1;
         for (int j = 0; j < st.rounds; j++) size *= 3;
         for (int x = 0; x < size; x++) u[x] = E2{dev.values()[2 * x], dev.values()[2 * x + 1]};

@@ -12,6 +12,7 @@
 #include "../basefold_kernels.cuh"
 #include "../eq_kernels.cuh"
 #include "../merkle_kernels.cuh"
+#include "arrivals.hpp"
 #include "host_tree_top.hpp"
 #include "gl_transcript.hpp"
 #include "pair_sumcheck.cuh"
@@ -258,8 +259,9 @@ public:
         }
         return pass();
     }
-    // The oracle of the current round, c0 c1 c2 (six words); the stream must have been synchronised since the last call that
-    // queued a pass (init or fold).
+    // The sums of the pass queued last, if any, are there.
+    int wait() const { return g_.empty() && stage_ < stages_.size() ? await_words(sums_, (size_t)2 << stages_[stage_].rounds) : MB_OK; }
+    // The oracle of the current round, c0 c1 c2 (six words); after wait().
     void oracle(uint64_t* out6) {
         const Stage& st = stages_[stage_];
         if (g_.empty()) {
@@ -310,6 +312,7 @@ private:
         a.fb = fb; a.v = nv_ - st.first; a.rounds = st.rounds;
         a.wl = tabs_.p + st.wl; a.wh = tabs_.p + st.wh;
         a.acc = acc_; a.sums = sums_;
+        expect_words(sums_, (size_t)2 << st.rounds);
         a.in = in_; a.out = nullptr;
         if (fb && stage_ + 1 < stages_.size()) {
             DevBuf& t = tables_[stage_ & 1];

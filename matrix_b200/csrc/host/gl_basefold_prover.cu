@@ -13,7 +13,7 @@
 // B200: the claimed value is read off the first oracle (eval = p(0) + p(1), one
 // pass fewer), the inner sumcheck runs several rounds per pass over the
 // bit-reversed evaluations (OpenSumcheck), the codeword is folded by the kernels
-// that hash its leaves, each round issues them back to back and synchronises
+// that hash its leaves, each round issues them back to back and waits
 // once, and the query phase is one gather kernel and one copy.
 #include "gl_basefold_common.cuh"
 
@@ -44,7 +44,8 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     if (rc != MB_OK) return rc;
     t.observe_hash(cm.root);   // while the first pass runs
     for (int i = 0; i < nv; i++) t.observe_ext2(Ext2{point[2 * i], point[2 * i + 1]});
-    MB_CUDA(cudaStreamSynchronize(MB_STREAM));
+    rc = sc.wait();
+    if (rc != MB_OK) return rc;
     // oracle 0 and the claimed value eval = p(0) + p(1) = 2 c0 + c1 + c2
     sc.oracle(p_oracles);
     {
@@ -76,20 +77,22 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     for (int round = 0; round < nv - 1; round++) {
         Ext2 ch = t.sample_challenge_ext2();
         gl::E2 r{ch.c0, ch.c1};
-        // kernels write their results straight into pinned host memory: a round is its launches and one stream
-        // synchronisation, no copy command
+        // kernels write their results straight into pinned host memory: a round is its launches and one wait for them, no copy
+        // command
         rc = sc.fold(r);
         if (rc != MB_OK) return rc;
         // codeword fold with this round's table level, and its tree up to the layer the host takes over
         const size_t leaves = cw_pairs / 2;
         const mk::FoldSource f{round == 0 ? cm.d_codeword.p : fcw[round - 1]->p, table.device_level_ptr(round), fcw[round]->p, r};
+        const size_t top = host_top(cm.hash), top_nodes = leaves < top ? leaves : top;
+        expect_words(nodes, 4 * top_nodes);
         rc = queue_fold_tree(cm.hash, round == 0, f, ftree[round]->p, leaves, nodes);
+        if (rc == MB_OK) rc = await_words(nodes, 4 * top_nodes);
+        if (rc == MB_OK) rc = sc.wait();
         if (rc != MB_OK) return rc;
-        MB_CUDA(cudaStreamSynchronize(MB_STREAM));
         uint64_t* po = p_oracles + 6 * (size_t)(round + 1);
         sc.oracle(po);
-        const size_t top = host_top(cm.hash);
-        rc = host_finish_top(cm.hash, nodes, leaves < top ? leaves : top, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
+        rc = host_finish_top(cm.hash, nodes, top_nodes, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
                              ftree[round]->p, leaves, p_roots + 4 * (size_t)round, MB_STREAM);
         if (rc != MB_OK) return rc;
         for (int k = 0; k < 3; k++) t.observe_ext2(Ext2{po[2 * k], po[2 * k + 1]});

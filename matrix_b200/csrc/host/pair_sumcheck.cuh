@@ -18,6 +18,7 @@
 #include "../common.cuh"
 #include "../pair_kernels.cuh"
 #include "../pair_mma_kernels.cuh"
+#include "arrivals.hpp"
 #include "host_field.hpp"
 #include "scratch_pool.hpp"
 
@@ -295,6 +296,8 @@ private:
             p.wl = tabs_ + b.wl; p.wh = tabs_ + b.wh;
         }
         p.acc = scratch_.dev; p.sums = pin_;
+        arriving_ = 2 * (size_t)K_ * (last ? 2 * tn_ : (size_t)1 << (2 * gb));
+        expect_words(pin_, arriving_);
         if (!last && blocks_[block_].mma) {
             int rc = launch_mma(gb, weighted, p, fw);
             if (rc != MB_OK) return rc;
@@ -360,6 +363,7 @@ private:
         const size_t w = tn_ * (base_ ? 1 : 2);
         if (2 * w * K_ > ScratchPool::WORDS) return MB_ERR_UNSUPPORTED;
         pending_ = true;
+        arriving_ = 0;   // the caller's words need not be canonical
         if (together_) {
             MB_CUDA(cudaMemcpyAsync(pin_, a_, 16 * w, cudaMemcpyDeviceToHost, MB_STREAM));
             return MB_OK;
@@ -377,7 +381,7 @@ private:
     // Results of the pass queued last.
     int wait() {
         if (bad_ != MB_OK || !pending_) return bad_;
-        if (cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
+        if (arriving_ ? await_words(pin_, arriving_) != MB_OK : cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
         pending_ = false;
         if (pin_[ERROR_WORD] != 0) return failed(MB_ERR_CUDA);   // a wait of a pass on the tensor cores ran out
         if (block_ < blocks_.size()) return MB_OK;
@@ -506,7 +510,7 @@ private:
     }
 
     const uint64_t *a_ = nullptr, *b_ = nullptr;
-    size_t stride_ = 0;
+    size_t stride_ = 0, arriving_ = 0;   // words of pin_ that the pass queued last writes
     int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0, bad_ = MB_OK;
     bool base_ = false, together_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
     std::vector<Block> blocks_;

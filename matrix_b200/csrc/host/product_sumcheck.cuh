@@ -147,6 +147,7 @@ private:
         p.v = n_ - (last ? n_ - tail_vars_ : blocks_[block_].first);
         p.acc = scratch_.dev; p.sums = pin_;
         loaded_ = false;
+        arriving_ = 0;
         if (last) {
             p.out = pin_;
             if (fb == 0) return copy(p.v);
@@ -156,6 +157,8 @@ private:
             p.out = t;
             flip_ = !flip_;
         }
+        arriving_ = 2 * (last ? (size_t)d_ << p.v : blocks_[block_].mma ? (size_t)pr::TRI_ENTRIES : (size_t)1 << (blocks_[block_].rounds * d_));
+        expect_words(pin_, arriving_);
         if (!last && blocks_[block_].mma) {
             int rc = launch_mma(p, fw);
             if (rc != MB_OK) return rc;
@@ -232,7 +235,7 @@ private:
     }
     int wait() {
         if (bad_ != MB_OK) return bad_;
-        if (cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
+        if (arriving_ ? await_words(pin_, arriving_) != MB_OK : cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
         return failed(pin_[ERROR_WORD] != 0 ? MB_ERR_CUDA : MB_OK);
     }
     // The sums of the current block.
@@ -271,7 +274,7 @@ private:
     }
 
     const uint64_t* in_ = nullptr;
-    size_t stride_ = 0;
+    size_t stride_ = 0, arriving_ = 0;   // as in PairSumcheck
     int d_ = 0, n_ = 0, cap_ = 1, round_ = 0, side_ = 0, tail_vars_ = 0, bad_ = MB_OK;
     bool base_ = false, flip_ = false, loaded_ = false;
     std::vector<Block> blocks_;
