@@ -239,39 +239,75 @@ __device__ __forceinline__ bool monolith_permute_throughput(uint64_t* s) {
     return !missed.any();
 }
 
-// ---- one permutation spread over 16 lanes ----------------------------------------
+// ---- one permutation spread over 16 lanes, or over a warp --------------------------------------
 // For layers too small to fill the machine, where the latency of a permutation is what counts: lane i < 12 holds word i.
-// A linear layer is twelve shuffles of each half against the lane's row of the circulant (two chains of twelve
-// multiply-adds instead of 288), the bars run in lanes 0..3, the bricks take the neighbour's word by a shuffle. About 2 us
-// instead of 15 to 20 us for a permutation in one thread. All 32 lanes of the warp must call; lane16 = lane & 15.
+// A linear layer is twelve shuffles of each half against the lane's row of the circulant (instead of 288 multiply-adds), the bars
+// run in lanes 0..3, the bricks take the neighbour's word by a shuffle. With a whole warp, the first sixteen lanes form the sums of the
+// low halves and the other sixteen those of the high ones, and each hands the other its sum: half the shuffles and products. Rare
+// repairs are left out; a warp that missed one runs the exact form, a permutation a thread. All 32 lanes of the warp must call.
+// All layers above 2^8 digests 29.5 -> 23.6 us with the warp form where a block has a node a warp.
 static __device__ const uint64_t g_mono_rc[MONO_ROUNDS + 1][MONO_W] = GLMONO_RC_INIT;   // per-lane reads
 // C[(j - i) mod 12] = g_mono_row[12 - i + j]
 static __device__ const uint32_t g_mono_row[2 * MONO_W] = {7, 23, 8, 26, 13, 10, 9, 7, 6, 22, 21, 8, 7, 23, 8, 26, 13, 10, 9, 7, 6, 22, 21, 8};
-__device__ __forceinline__ uint64_t mono_concrete_coop(uint64_t x, const uint32_t (&m)[MONO_W], uint64_t rc) {
-    uint64_t L = lo32(rc), H = hi32(rc);
+template <bool WARP>
+__device__ __forceinline__ uint64_t mono_concrete_coop(uint64_t x, int lane, const uint32_t (&m)[MONO_W], uint64_t rc, fast::Missed& missed) {
     const uint32_t xl = lo32(x), xh = hi32(x);
+    uint64_t L, H;
+    if constexpr (WARP) {
+        const bool high = lane >= 16;
+        const uint32_t half = high ? xh : xl;
+        uint64_t s[2] = {high ? hi32(rc) : lo32(rc), 0};
 #pragma unroll
-    for (int j = 0; j < MONO_W; j++) {
-        L = madwide(__shfl_sync(0xffffffffu, xl, j, 16), m[j], L);
-        H = madwide(__shfl_sync(0xffffffffu, xh, j, 16), m[j], H);
+        for (int j = 0; j < MONO_W; j++) s[j & 1] = madwide(__shfl_sync(0xffffffffu, half, j, 16), m[j], s[j & 1]);
+        const uint64_t mine = s[0] + s[1];
+        const uint64_t other = pack64(__shfl_xor_sync(0xffffffffu, lo32(mine), 16), __shfl_xor_sync(0xffffffffu, hi32(mine), 16));
+        L = high ? other : mine;
+        H = high ? mine : other;
+    } else {
+        uint64_t l[2] = {lo32(rc), 0}, h[2] = {hi32(rc), 0};
+#pragma unroll
+        for (int j = 0; j < MONO_W; j++) {
+            l[j & 1] = madwide(__shfl_sync(0xffffffffu, xl, j, 16), m[j], l[j & 1]);
+            h[j & 1] = madwide(__shfl_sync(0xffffffffu, xh, j, 16), m[j], h[j & 1]);
+        }
+        L = l[0] + l[1];
+        H = h[0] + h[1];
     }
-    return reduce_limb_sums(L, H);
+    fast::Sum s;
+    s.a = lo32(L);
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;" : "=&r"(s.b), "=r"(s.c) : "r"(hi32(L)), "r"(lo32(H)), "r"(hi32(H)));
+    return fast::reduce(s, missed);
 }
-__device__ __forceinline__ uint64_t monolith_permute_coop16(uint64_t x, int lane16) {
+static __device__ __noinline__ uint64_t monolith_permute_gathered(uint64_t x, int lane16) {
+    uint64_t s[MONO_W];
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) s[j] = pack64(__shfl_sync(0xffffffffu, lo32(x), j, 16), __shfl_sync(0xffffffffu, hi32(x), j, 16));
+    monolith_permute(s);
+#pragma unroll
+    for (int j = 0; j < MONO_W; j++) x = j == lane16 ? s[j] : x;
+    return x;
+}
+// x: word lane mod 16 (WARP: in two copies), zero from word 12 on
+template <bool WARP>
+__device__ __forceinline__ uint64_t monolith_permute_lanes(uint64_t x, int lane) {
+    const uint64_t in = x;
+    const int lane16 = lane & 15;
     const bool live = lane16 < MONO_W;
+    fast::Missed missed{0, 0};
     uint32_t m[MONO_W];   // the lane's row of the circulant
 #pragma unroll
     for (int j = 0; j < MONO_W; j++) m[j] = live ? g_mono_row[MONO_W - lane16 + j] : 0;
-    x = mono_concrete_coop(x, m, 0);
+    x = mono_concrete_coop<WARP>(x, lane, m, 0, missed);
 #pragma unroll 1
     for (int r = 1; r <= MONO_ROUNDS; r++) {
         const uint64_t b = mono_bar(canon(x));
         x = lane16 < 4 ? b : x;
         const uint64_t prev = pack64(__shfl_up_sync(0xffffffffu, lo32(x), 1, 16), __shfl_up_sync(0xffffffffu, hi32(x), 1, 16));
-        const uint64_t y = mul_add(prev, prev, x);
+        const uint64_t y = fast::mul_add(prev, prev, x, missed);
         x = lane16 > 0 ? y : x;
-        x = mono_concrete_coop(x, m, (live && r < MONO_ROUNDS) ? g_mono_rc[r][lane16] : 0);
+        x = mono_concrete_coop<WARP>(x, lane, m, (live && r < MONO_ROUNDS) ? g_mono_rc[r][lane16] : 0, missed);
     }
+    if (__any_sync(0xffffffffu, missed.any())) return monolith_permute_gathered(in, lane16);
     return x;
 }
 #endif

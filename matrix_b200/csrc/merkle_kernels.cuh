@@ -32,15 +32,26 @@ constexpr int BLOCK = 128;
 
 // Hash policies. permute(load): the permutation of the state that load(s) writes (it may be asked for again).
 // coop(x, l): the permutation spread over LANES lanes, lane l holding word l. COOP_NODES: layers of at most this many
-// nodes take the spread form. WARP: there is a form with a permutation a warp, warp(x, lane, a copy of warp_table()).
+// nodes take the spread form. warp(x, lane, table, ready): a permutation a warp, word lane mod LANES in every copy; ready() is called before the
+// table, a Table in shared memory, is used.
 struct HashPoseidon2 {
     static constexpr int WIDTH = 8, LANES = 8, MIN_BLOCKS = 6;
     static constexpr size_t COOP_NODES = (size_t)1 << 12;
     static __device__ __forceinline__ uint64_t coop(uint64_t x, int l) { return gl::poseidon2_permute_coop8(x, l); }
-    static constexpr bool WARP = true;
-    using WarpTable = P2Warp;
-    static __device__ __forceinline__ const WarpTable& warp_table() { return g_p2_warp; }
-    static __device__ __forceinline__ uint64_t warp(uint64_t x, int lane, const WarpTable& w) { return poseidon2_permute_warp(x, lane, w); }
+    struct Table : P2Warp {
+        // in shared memory by asynchronous copies; whole blocks call
+        __device__ __forceinline__ void begin() {
+            const char* from = reinterpret_cast<const char*>(&g_p2_warp);
+            for (unsigned i = 16 * threadIdx.x; i < sizeof(P2Warp); i += 16 * blockDim.x) tc::copy16(tc::smem_u32(this) + i, from + i);
+            tc::copy_commit();
+        }
+        static __device__ __forceinline__ void end() {
+            tc::copy_wait<0>();
+            __syncthreads();
+        }
+    };
+    template <class Ready>
+    static __device__ __forceinline__ uint64_t warp(uint64_t x, int lane, const Table& w, Ready ready) { return poseidon2_permute_warp(x, lane, w, ready); }
     template <class Load>
     static __device__ __forceinline__ void permute(uint64_t* s, Load load) {
         load(s);
@@ -55,9 +66,13 @@ struct HashPoseidon2 {
 struct HashMonolith {
     static constexpr int WIDTH = 12, LANES = 16, MIN_BLOCKS = 4;
     static constexpr size_t COOP_NODES = (size_t)1 << 12;
-    static __device__ __forceinline__ uint64_t coop(uint64_t x, int l) { return gl::monolith_permute_coop16(x, l); }
-    static constexpr bool WARP = false;
-    struct WarpTable { uint64_t none; };
+    static __device__ __forceinline__ uint64_t coop(uint64_t x, int l) { return gl::monolith_permute_lanes<false>(x, l); }
+    struct Table {
+        __device__ __forceinline__ void begin() {}
+        static __device__ __forceinline__ void end() { __syncthreads(); }
+    };
+    template <class Ready>
+    static __device__ __forceinline__ uint64_t warp(uint64_t x, int lane, const Table&, Ready) { return gl::monolith_permute_lanes<true>(x, lane); }
     template <class Load>
     static __device__ __forceinline__ void permute(uint64_t* s, Load load) {
         load(s);
@@ -205,7 +220,7 @@ compress_layer_coop_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict
 // the top layer.
 // What a small layer costs is one permutation's latency, and issue slots as soon as more than one warp per scheduler
 // works on it: a block holds at most 16 permutations, so a layer of 4096 nodes is spread over 256 blocks. A layer with as few nodes in a
-// block as warps takes the form with a permutation a warp, where the hash has one.
+// block as warps takes the form with a permutation a warp.
 // Blocks are whole warps (the permutations shuffle with the full mask): threads beyond the block's groups compute on zeros
 // and store nothing.
 enum TreeSource { NODES, LEAF_BASE, LEAF_EXT, FOLD_BASE, FOLD_EXT };
@@ -213,18 +228,15 @@ template <class H, TreeSource SRC>
 __global__ void __launch_bounds__(256)
 tree_up_coop_kernel(const FoldSource f, uint64_t* dst, size_t size, int levels, size_t copies, uint64_t* last_out) {
     __shared__ uint64_t node[16 * 4];
-    __shared__ typename H::WarpTable table;
-    if constexpr (H::WARP) {   // read after the barrier below, or after the first layer's
-        const uint64_t* from = reinterpret_cast<const uint64_t*>(&H::warp_table());
-        for (unsigned i = threadIdx.x; i < sizeof(table) / 8; i += blockDim.x) reinterpret_cast<uint64_t*>(&table)[i] = from[i];
-    }
+    __shared__ __align__(16) typename H::Table table;
+    table.begin();
     size_t n = (size_t)1 << (levels - 1);   // this block's nodes of the current layer
     const size_t warps = blockDim.x / 32;
     const auto whole_warps = [](size_t m) { return ((m * H::LANES + 31) & ~(size_t)31) / H::LANES; };
     uint64_t x = 0;
     for (bool lowest = true;; lowest = false) {
-        const bool wide = H::WARP && n <= warps;
-        const int lanes = wide ? 32 : H::LANES, l = threadIdx.x & (lanes - 1), w = wide ? l & 7 : l;
+        const bool wide = n <= warps;
+        const int lanes = wide ? 32 : H::LANES, l = threadIdx.x & (lanes - 1), w = l & (H::LANES - 1);   // w: the lane's word
         const size_t g = threadIdx.x / lanes, k = (size_t)blockIdx.x * n + g;
         const bool live = g < n, in_use = wide ? live : g < whole_warps(n);   // whole warps drop out as the layers shrink
         if (!lowest) {
@@ -236,26 +248,27 @@ tree_up_coop_kernel(const FoldSource f, uint64_t* dst, size_t size, int levels, 
                 x = (live && w < 2) ? f.in[2 * k + w] : 0;
             } else if (SRC == LEAF_EXT) {
                 x = (live && w < 4) ? f.in[4 * k + w] : 0;
-            } else {
-                if (live && l < 2) {   // one element per lane, then four words in four lanes
-                    const gl::E2 e = folded_element<SRC == FOLD_BASE>(f, 2 * k + l, gl::mul_small(f.r.c1, 7));
+            } else {   // one element per lane of the first two, then a word per lane
+                gl::E2 e{0, 0};
+                if (live && l < 2) {
+                    e = folded_element<SRC == FOLD_BASE>(f, 2 * k + l, gl::mul_small(f.r.c1, 7));
                     gl::e2_store(f.out + 2 * (2 * k + l), e);
                 }
-                __syncwarp();
-                x = (live && w < 4) ? f.out[4 * k + w] : 0;
+                const uint64_t c0 = p2_from_lane(e.c0, (threadIdx.x & 31 & ~(lanes - 1)) + ((w >> 1) & 1)),
+                               c1 = p2_from_lane(e.c1, (threadIdx.x & 31 & ~(lanes - 1)) + ((w >> 1) & 1));
+                x = w < 4 ? (w & 1 ? c1 : c0) : 0;
             }
         }
-        if (H::WARP && lowest && wide) __syncthreads();
         if (in_use) {
-            if constexpr (H::WARP) x = wide ? H::warp(x, l, table) : H::coop(x, l);
-            else x = H::coop(x, l);
-            x = gl::canon(x);
+            // all warps are in use in a lowest layer of this form
+            x = gl::canon(wide ? H::warp(x, l, table, [&] { if (lowest) H::Table::end(); }) : H::coop(x, l));
         }
         if (live && l < 4) {
             for (size_t c = 0; c < copies; c++) dst[4 * (c * size + k) + l] = x;
         }
         if (n == 1) break;
-        __syncthreads();             // the pairs of the layer below have been read
+        if (lowest && !wide) H::Table::end();
+        else __syncthreads();            // the pairs of the layer below have been read
         if (live && l < 4) node[4 * g + l] = x;
         __syncthreads();
         dst += 4 * size * copies;
@@ -369,14 +382,16 @@ inline size_t launch_tree_up(const FoldSource& f, uint64_t*& dst, size_t size, s
                              size_t stop) {
     int levels = 1;
     while ((size >> levels) >= stop && (size >> levels) >= 1) levels++;
-    if (H::WARP && levels > 5 && levels <= 8) levels -= 3;   // the rest have a node a warp throughout
+    if (levels > 5 && levels <= 8) levels -= 3;   // the rest have a node a warp throughout
     if (levels > 5) levels = 5;
     const size_t top = size >> (levels - 1);
+    // a warp a node up to four nodes a block, LANES lanes above that
     size_t t = (size_t)H::LANES << (levels - 1);
-    if (H::WARP) t = levels > 2 ? 128 : (size_t)32 << (levels - 1);
+    if (levels <= 3) t = (size_t)32 << (levels - 1);
+    else if (t < 128) t = 128;
     {
         MB_KERNEL_ON("tree_up", st);
-        tree_up_coop_kernel<H, SRC><<<(unsigned)top, (unsigned)(t < 32 ? 32 : t), 0, st>>>(f, dst, size, levels, copies, top == stop ? root_out : nullptr);
+        tree_up_coop_kernel<H, SRC><<<(unsigned)top, (unsigned)t, 0, st>>>(f, dst, size, levels, copies, top == stop ? root_out : nullptr);
     }
     for (; size > top; size /= 2) dst += 4 * size * copies;
     return top;

@@ -116,8 +116,9 @@ __device__ __forceinline__ gl::Acc p2_product(uint64_t a, uint64_t b) {
     const uint64_t lo = (uint64_t)f, hi = (uint64_t)(f >> 64);
     return gl::Acc{gl::lo32(lo), gl::hi32(lo), gl::lo32(hi), gl::hi32(hi), 0};
 }
-// x: word lane mod 8, in four copies; the same on return. w: g_p2_warp, in shared memory. All 32 lanes call.
-__device__ __forceinline__ uint64_t poseidon2_permute_warp(uint64_t x, int lane, const P2Warp& w) {
+// x: word lane mod 8, in four copies; the same on return. w: g_p2_warp, in shared memory once ready() has been called. All 32 lanes call.
+template <class Ready>
+__device__ __forceinline__ uint64_t poseidon2_permute_warp(uint64_t x, int lane, const P2Warp& w, Ready ready) {
     const uint64_t in = x;
     const int lane8 = lane & 7;
     gl::p2t::Missed missed{0, 0};
@@ -125,6 +126,7 @@ __device__ __forceinline__ uint64_t poseidon2_permute_warp(uint64_t x, int lane,
 #pragma unroll 1
     for (int r = 0; r < 3; r++) x = gl::p2_coop_external(gl::p2t::sbox7_soon(x, missed), lane8, gl::g_p2_rc_ext[r + 1][lane8], missed);
     x = gl::p2t::sbox7_soon(x, missed);
+    ready();
     gl::Acc sum = gl::acc_from(w.c[lane]), odd = gl::acc_zero();
 #pragma unroll
     for (int m = 0; m < 8; m += 2) {

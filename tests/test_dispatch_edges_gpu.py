@@ -144,6 +144,26 @@ def test_small_poseidon2_trees(gl, oracle, log_leaves, ext):
     assert np.array_equal(d_t.to_numpy(), exp)
 
 
+@pytest.mark.parametrize("log_leaves", [0, 1, 2, 3, 4, 6, 9, 13])
+@pytest.mark.parametrize("ext", [False, True])
+def test_small_monolith_trees(gl, oracle, log_leaves, ext):
+    """Sixteen lanes a permutation and a warp a permutation, and (2^13 leaves) a layer a thread each in front of them; words at the ends of
+    their range, and a leaf that needs the exact form: after the first linear layer (rows 4 and 5: 6 22 .., 7 6 ..) its words 4 and 5
+    are 2^48 and 0, and 2^96 has no low word."""
+    leaves, width = 1 << log_leaves, 4 if ext else 2
+    cw = field_elems(191 + log_leaves, leaves * width).reshape(leaves, width)
+    cw[0], cw[leaves // 2] = GL_P - 1, 2**32 - 1
+    cw[leaves - 1] = 0
+    y = pow(6 * 6 - 7 * 22, -1, GL_P) * -7 * 2**48 % GL_P   # 6 x + 22 y = 2^48, 7 x + 6 y = 0
+    cw[leaves - 1, :2] = -6 * pow(7, -1, GL_P) * y % GL_P, y
+    d_cw, d_t = DeviceBuffer.from_numpy(gl, cw.reshape(-1)), DeviceBuffer(gl, 32 * (2 * leaves - 1))
+    assert (gl.monolith_merkle_tree_ext2_ffi if ext else gl.monolith_merkle_tree_gl_ffi)(d_cw.ptr, d_t.ptr, leaves) == 0
+    exp = np.zeros(4 * (2 * leaves - 1), dtype=np.uint64)
+    with pyoracle.merkle_hash(1):
+        oracle.oracle_bf_merkle_tree(cw.ctypes.data, leaves, int(ext), exp.ctypes.data)
+    assert np.array_equal(d_t.to_numpy(), exp)
+
+
 @pytest.mark.parametrize("log_n,m", [(8, 6), (9, 6), (9, 9), (10, 8), (13, 12), (17, 17), (18, 6), (19, 12), (20, 15),
                                      (22, 6), (22, 7), (22, 9), (24, 10), (24, 11), (24, 13), (25, 11), (25, 12)])
 def test_partial_evaluation_rows(oracle, gl, log_n, m):
