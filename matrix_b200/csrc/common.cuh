@@ -39,6 +39,29 @@ inline int finish_sync() {
 }
 inline int finish_async() { return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ERR_CUDA; }
 
+// Launches of a chain of short kernels on one stream: launch_chained lets a kernel's blocks come up once every block of the one before it
+// has called chain_next() or ended; chain_begin() (the first thing a kernel does, or after work on constants alone) waits for
+// all of that one's writes. Every kernel of a chain calls chain_begin() in every thread, so a kernel's end stands for all before
+// it. chain_next() belongs to the last part of a kernel: blocks that come up while the SMs are unevenly full stay where they are put.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Number of SMs of the current device (148 on B200), cached per thread.
 inline int sm_count() {
     static thread_local int cached_dev = -1, cached = 0;
