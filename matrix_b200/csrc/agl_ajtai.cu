@@ -3,6 +3,8 @@
 // almost-goldilocks-cuda-rs/cuda/wrapper.cu:1095-1204,1663-1670).
 #include "ajtai_kernels.cuh"
 #include "ajtai_tc.cuh"
+#include "host/arrivals.hpp"
+#include "host/scratch_pool.hpp"
 
 using namespace mb;
 using namespace mb::aj;
@@ -157,7 +159,9 @@ int commit_s8_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T,
     err[0] = err[1] = 0;
     uint64_t* partial = nullptr;
     MB_CUDA(pool_alloc((void**)&partial, chunks * 3 * TC_MAX_PLANES * TC_ROWS * D * sizeof(uint64_t)));
-    int rc = MB_OK;
+    mbhost::ScratchBlock done = mbhost::ScratchPool::take();
+    int rc = done ? MB_OK : MB_ERR_CUDA;
+    if (done) mbhost::expect_words(done.host, 1);
     for (int p0 = 0; p0 < planes && rc == MB_OK; p0 += TC_PASS_PLANES) {
         const int np = planes - p0 < TC_PASS_PLANES ? planes - p0 : TC_PASS_PLANES;
         {
@@ -169,13 +173,16 @@ int commit_s8_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T,
         if (rc != MB_OK) break;
         {
             MB_KERNEL("ajtai_reduce_tc");
-            reduce_tc_partials_kernel<<<(unsigned)(np * plane_words / 32), 32 * TC_RED_SLICES, 0, MB_STREAM>>>(
-                partial, chunks, np, d_out + (size_t)p0 * plane_words);
+            const bool last = p0 + TC_PASS_PLANES >= planes;
+            launch_chained(reduce_tc_partials_kernel, (unsigned)(np * plane_words / 32), 32 * TC_RED_SLICES, 0, MB_STREAM, partial, chunks, np,
+                           d_out + (size_t)p0 * plane_words, reinterpret_cast<unsigned*>(done.dev), last ? done.host : nullptr);
         }
         rc = finish_async();
     }
-    const int synced = finish_sync();   // also after a failed launch: nothing may still write to err or partial
-    if (rc == MB_OK) rc = synced;
+    // after a failed launch nothing may still write to err or partial
+    if (rc == MB_OK) rc = mbhost::await_words(done.host, 1);
+    else cudaStreamSynchronize(MB_STREAM);
+    mbhost::ScratchPool::give(done, rc == MB_OK);
     pool_free(partial);
     if (rc != MB_OK) return rc;
     if (err[1]) return MB_ERR_CUDA;

@@ -401,16 +401,34 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
             for (int x = t; x < (int)(2 * TC_SBO / 16); x += WS_THREADS)
                 reinterpret_cast<uint4*>(A_base + b * A_SLOT + 14 * TC_SBO)[x] = make_uint4(0, 0, 0, 0);
     }
+    bool failed = false;
+    int bad_digit = 0;
+    int copies_issued = 0;   // copy warp: stages whose bulk copy has gone out
+    auto tma_issue = [&](int stage) {   // one thread: the A image of `stage` into its ring slot
+        const uint32_t bar = smem_u32(&bar_tma[stage % A_SLOTS]);
+        const uint32_t dst = smem_u32(A_base + (stage % A_SLOTS) * A_SLOT);
+        const uint8_t* src = d_T + (((j0 / TC_STAGE_COLS) + (uint64_t)stage) * 3 + (uint64_t)group) * TCP_A_IMAGE;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)TCP_A_IMAGE) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(dst), "l"(src), "r"((uint32_t)TCP_A_IMAGE), "r"(bar) : "memory");
+    };
     if (t == 0) {
         for (int b = 0; b < NB; b++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_full[b])), "r"(WS_BUILD_WARPS));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_empty[b])));
         }
-        for (int q = 0; q < WS_A_SLOTS_MAX; q++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_tma[q])));
+        for (int q = 0; q < WS_A_SLOTS_MAX; q++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_afree[q])));
-        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (t == 32 * WS_COPY_WARP) {
+        for (int q = 0; q < WS_A_SLOTS_MAX; q++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_tma[q])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (TILED) {   // the ring fills while the block comes up
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            for (; copies_issued < A_SLOTS && copies_issued < n_stages; copies_issued++) tma_issue(copies_issued);
+        }
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)), "r"(tmem_cols));
@@ -421,19 +439,6 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_base_sh;
-    bool failed = false;
-    int bad_digit = 0;
-    int copies_issued = 0;   // copy warp: stages whose bulk copy has gone out
-
-    auto tma_issue = [&](int stage) {   // one thread: the A image of `stage` into its ring slot
-        const uint32_t bar = smem_u32(&bar_tma[stage % A_SLOTS]);
-        const uint32_t dst = smem_u32(A_base + (stage % A_SLOTS) * A_SLOT);
-        const uint8_t* src = d_T + (((j0 / TC_STAGE_COLS) + (uint64_t)stage) * 3 + (uint64_t)group) * TCP_A_IMAGE;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)TCP_A_IMAGE) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(dst), "l"(src), "r"((uint32_t)TCP_A_IMAGE), "r"(bar) : "memory");
-    };
-
     // the MMAs that last read the buffer of stage sidx (those of stage sidx - NB) are done: one lane polls
     auto buffer_free = [&](int sidx) {
         if (sidx < NB) return true;
@@ -596,7 +601,7 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
     } else if (warp == WS_COPY_WARP) {
         // ================= copies of the A images (tiled source) =================
         if (TILED && lane == 0) {
-            for (int st = 0; st < n_stages; st++) {
+            for (int st = copies_issued; st < n_stages; st++) {
                 // the slot held stage st - A_SLOTS; its MMAs are done when the issuer's commit to the slot's barrier lands
                 if (st >= A_SLOTS && !mbar_wait(smem_u32(&bar_afree[st % A_SLOTS]), (uint32_t)((st / A_SLOTS - 1) & 1))) { failed = true; break; }
                 tma_issue(st);
@@ -646,6 +651,7 @@ commit_tc_ws_kernel(const uint32_t* __restrict__ d_key, const uint64_t* __restri
             mbar_wait(smem_u32(&bar_tma[st % A_SLOTS]), (uint32_t)((st / A_SLOTS) & 1));
     }
     asm volatile("tcgen05.fence::after_thread_sync;");
+    chain_next();
 
     if (!failed && n_stages > 0 && warp < 16) {
         // Accumulator row m = 8 il + b holds byte plane b of matrix row il; a warp reads 32 rows (four values of
@@ -778,10 +784,14 @@ inline size_t tc_pipe_smem_bytes(int np) {
 // out[p][i][r] = sum over chunks of partial[chunk][group = i / 14][p][i % 14][r]. A block owns 32 outputs and deals
 // the chunks to sixteen warps: one thread per output read its chunks one after the other on a quarter of the SMs
 // (18.5 us for 98 chunks x 3 planes, 84 us for 542 chunks).
+// done (may be null): a word of page-locked memory that the block which is through last clears, after all results (`through` counts
+// them, zero before and after): the caller sees that 3.4 us before a synchronisation returns.
 constexpr int TC_RED_SLICES = 16;
 static __global__ void __launch_bounds__(32 * TC_RED_SLICES)
-reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, int np, uint64_t* __restrict__ out) {
+reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, int np, uint64_t* __restrict__ out, unsigned* through,
+                          uint64_t* done) {
     __shared__ uint64_t sums[TC_RED_SLICES][32];
+    chain_begin();
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
     const size_t k = (size_t)blockIdx.x * 32 + lane;   // 32 divides the width np * 42 * 64
     const int p = (int)(k / (KAPPA * D)), i = (int)((k / D) % KAPPA), r = (int)(k % D);
@@ -796,6 +806,15 @@ reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, i
 #pragma unroll
         for (int q = 1; q < TC_RED_SLICES; q++) a = agl::add(a, sums[q][lane]);
         out[k] = agl::canon(a);
+        if (done != nullptr) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0 && atomicAdd(through, 1u) == gridDim.x - 1) {
+                *through = 0;
+                __threadfence_system();
+                *(volatile uint64_t*)done = 0;
+            }
+        }
     }
 }
 
