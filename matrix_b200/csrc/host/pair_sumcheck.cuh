@@ -225,6 +225,7 @@ public:
 private:
     static constexpr size_t ERROR_WORD = ScratchPool::WORDS - 2;
     static constexpr size_t MMA_MIN = (size_t)1 << 14;
+    static constexpr size_t SMALL_TILES = 64;   // folds of fewer tiles of 256 elements than half the SMs: pair_small_kernel
     struct Block {
         int first, rounds;
         size_t wl, wh;      // word offsets of the eq tables
@@ -302,11 +303,22 @@ private:
             int rc = launch_mma(gb, weighted, p, fw);
             if (rc != MB_OK) return rc;
         } else {
-            const size_t tiles = (((size_t)1 << p.v) + pr::BLK - 1) / pr::BLK;
-            const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);
-            MB_KERNEL("pair_pass");
-            if (fb) base_ ? launch<true, true>(gb, weighted, grid, p, fw) : launch<true, false>(gb, weighted, grid, p, fw);
-            else base_ ? launch<false, true>(gb, weighted, grid, p, fw) : launch<false, false>(gb, weighted, grid, p, fw);
+            const size_t n = (size_t)1 << p.v, tiles = (n + pr::BLK - 1) / pr::BLK;
+            if (fb && tiles * K_ <= SMALL_TILES) {
+                // threads an element: as many as have two inputs each and leave half as many blocks as SMs (with as many as
+                // SMs the blocks' atomics on the same sums take longer than the products saved: 2^20 elements 282 -> 280 us a proof)
+                int s = 0;
+                while (s + 1 < fb && (n << (s + 1)) / (pr::BLK / 2) * K_ <= (size_t)sm_count() / 2) s++;
+                const size_t tile = (pr::BLK / 2) >> s;
+                const dim3 few((unsigned)((n + tile - 1) / tile), K_);
+                MB_KERNEL("pair_pass");
+                base_ ? launch_small<true>(gb, weighted, few, p, s, fw) : launch_small<false>(gb, weighted, few, p, s, fw);
+            } else {
+                const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);
+                MB_KERNEL("pair_pass");
+                if (fb) base_ ? launch<true, true>(gb, weighted, grid, p, fw) : launch<true, false>(gb, weighted, grid, p, fw);
+                else base_ ? launch<false, true>(gb, weighted, grid, p, fw) : launch<false, false>(gb, weighted, grid, p, fw);
+            }
         }
         if (p.out && !last) {   // the folded tables are the next pass's input
             a_ = p.out;
@@ -331,6 +343,21 @@ private:
             case 2: launch_w<FOLD, BASE, 2>(weighted, grid, p, fw); break;
             case 3: launch_w<FOLD, BASE, 3>(weighted, grid, p, fw); break;
             default: launch_w<FOLD, BASE, 4>(weighted, grid, p, fw); break;
+        }
+    }
+    template <bool BASE, int GB>
+    static void launch_small_w(bool weighted, dim3 grid, const pr::PairArgs& p, int s, const pr::FoldWeights<F>& fw) {
+        if (weighted) pr::pair_small_kernel<F, GB, BASE, true><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+        else pr::pair_small_kernel<F, GB, BASE, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+    }
+    template <bool BASE>
+    static void launch_small(int gb, bool weighted, dim3 grid, const pr::PairArgs& p, int s, const pr::FoldWeights<F>& fw) {
+        switch (gb) {
+            case 0: launch_small_w<BASE, 0>(false, grid, p, s, fw); break;
+            case 1: launch_small_w<BASE, 1>(weighted, grid, p, s, fw); break;
+            case 2: launch_small_w<BASE, 2>(weighted, grid, p, s, fw); break;
+            case 3: launch_small_w<BASE, 3>(weighted, grid, p, s, fw); break;
+            default: launch_small_w<BASE, 4>(weighted, grid, p, s, fw); break;
         }
     }
     template <bool FOLD, bool BASE, bool WEIGHTED>

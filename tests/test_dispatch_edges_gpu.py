@@ -53,6 +53,13 @@ def test_sumcheck_rounds_gl(gl, d, nv, base):
     gl_sumcheck_matches_oracle(gl, nv, d, base)
 
 
+# passes that fold a few tiles, several threads an element: one to eight of them, whole tiles and parts, below, at and above 64 tiles of 256
+# elements over the instances
+@pytest.mark.parametrize("K,nv", [(1, 11), (1, 12), (1, 17), (2, 10), (3, 13), (7, 12), (16, 10), (16, 14), (24, 9), (31, 12), (33, 13), (64, 11)])
+def test_small_folds(K, nv):
+    batched_matches_oracle(K, nv, 0)
+
+
 @pytest.mark.parametrize("d", [6, 7, 8])
 @pytest.mark.parametrize("blocks", [1, 148, 149, 600])   # a block per SM, and more
 def test_many_tables(gl, oracle, d, blocks):
