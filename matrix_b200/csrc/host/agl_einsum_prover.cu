@@ -169,13 +169,12 @@ int agl_einsum_prove_device_ffi(int num_operands, const mb_einsum_operand* ops, 
             lift_kernel<<<grid_for((size_t)1 << o.n, 256, 8), 256, 0, MB_STREAM>>>(o.d_src, dst, (size_t)1 << o.n);
             rc = finish_async();
         } else if (!o.d_lut_lo) {
-            // the fixed variables are the operand's low bits: a plain partial evaluation, then into place
-            uint64_t* out = sc.get((size_t)2 << (o.n - 1));
-            uint64_t* tmp = sc.get((size_t)2 << (o.n - 1));
-            if (!out || !tmp) return MB_ERR_CUDA;
-            rc = pe::partial_eval<AglBase, AglExt2>(o.d_src, out, tmp, d_small + r_off[k], o.n, o.m, MB_STREAM);
-            if (rc == MB_OK && cudaMemcpyAsync(dst, out, (size_t)16 << mine, cudaMemcpyDeviceToDevice, MB_STREAM) != cudaSuccess)
-                rc = MB_ERR_CUDA;
+            // the fixed variables are the operand's low bits: a plain partial evaluation, in place
+            const int passes = pe::plan<AglBase, AglExt2>(o.d_src, o.n, o.m).passes;
+            uint64_t* out = passes > 2 ? sc.get((size_t)2 << (o.n - 1)) : nullptr;
+            uint64_t* tmp = passes > 1 ? sc.get((size_t)2 << (o.n - 1)) : nullptr;
+            if ((passes > 2 && !out) || (passes > 1 && !tmp)) return MB_ERR_CUDA;
+            rc = pe::partial_eval<AglBase, AglExt2>(o.d_src, out, tmp, d_small + r_off[k], o.n, o.m, MB_STREAM, dst);
         } else {
             const uint64_t* eq_ptr = d_small + one_off;
             if (o.m) {

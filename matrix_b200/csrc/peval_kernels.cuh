@@ -248,25 +248,38 @@ inline void launch_levels(const uint64_t* in, uint64_t* out, const uint64_t* r, 
     }
 }
 
-// d_in: 2^log_n elements of FIn; result: 2^(log_n - m) elements of FOut in
-// d_out. d_tmp: scratch of at least 2^(log_n - min(m, K_MAX)) FOut elements
-// (unused when m <= K_MAX). d_in is not modified unless it aliases d_out/d_tmp.
-template <class FIn, class FOut>
-inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, const uint64_t* d_r, int log_n, int m,
-                        cudaStream_t st) {
-    if (log_n < 0 || log_n > 40 || m < 0 || m > log_n || !d_in || !d_out || (m > 0 && !d_r)) return MB_ERR_ARG;
-    if (m == 0) return MB_OK;
-    // dot_rows_kernel reads pairs of elements, and eight warps of 64 elements or more make a block
-    int first_vars = 0;
+struct Plan {
+    int first_vars = 0;   // bound by the first pass on the tensor cores or by rows, 0: K_MAX a pass from the start
     bool mma = false;
+    int passes = 0;
+};
+template <class FIn, class FOut>
+inline Plan plan(const uint64_t* d_in, int log_n, int m) {
+    Plan p;
+    // dot_rows_kernel reads pairs of elements, and eight warps of 64 elements or more make a block
     if constexpr (FIn::NW == 1 && FOut::NW == 2)
         if (m >= 6 && log_n >= 9 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) {
-            first_vars = dot_mma_vars(log_n, m);
-            mma = first_vars > 0;
-            if (!mma) first_vars = dot_rows_vars(log_n, m);
+            p.first_vars = dot_mma_vars(log_n, m);
+            p.mma = p.first_vars > 0;
+            if (!p.mma) p.first_vars = dot_rows_vars(log_n, m);
         }
-    int passes = first_vars ? 1 + (m - first_vars + K_MAX - 1) / K_MAX : (m + K_MAX - 1) / K_MAX;
-    if (passes > 1 && !d_tmp) return MB_ERR_ARG;
+    p.passes = p.first_vars ? 1 + (m - p.first_vars + K_MAX - 1) / K_MAX : (m + K_MAX - 1) / K_MAX;
+    return p;
+}
+
+// d_in: 2^log_n elements of FIn; result: 2^(log_n - m) elements of FOut in
+// d_out. d_tmp: scratch of at least 2^(log_n - min(m, K_MAX)) FOut elements
+// (unused when m <= K_MAX). d_in is not modified unless it aliases d_out/d_tmp. d_last (may be null): the result goes there, and
+// d_out is scratch of three passes and more, d_tmp of two and more (null otherwise).
+template <class FIn, class FOut>
+inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, const uint64_t* d_r, int log_n, int m,
+                        cudaStream_t st, uint64_t* d_last = nullptr) {
+    if (log_n < 0 || log_n > 40 || m < 0 || m > log_n || !d_in || (!d_out && !d_last) || (m > 0 && !d_r)) return MB_ERR_ARG;
+    if (m == 0) return MB_OK;
+    const Plan how = plan<FIn, FOut>(d_in, log_n, m);
+    const int first_vars = how.first_vars, passes = how.passes;
+    const bool mma = how.mma;
+    if ((passes > 1 && !d_tmp) || (passes > 2 && !d_out)) return MB_ERR_ARG;
     // ping-pong so that the last pass lands in d_out
     uint64_t* bufs[2] = {d_out, d_tmp};
     int which = (passes % 2 == 1) ? 0 : 1;
@@ -276,7 +289,7 @@ inline int partial_eval(const uint64_t* d_in, uint64_t* d_out, uint64_t* d_tmp, 
     while (left > 0) {
         int k = first && first_vars ? first_vars : left < K_MAX ? left : K_MAX;
         size_t n_out = (size_t)1 << (cur_log - k);
-        uint64_t* dst = bufs[which];
+        uint64_t* dst = left == k && d_last ? d_last : bufs[which];
         bool done = false;
         if constexpr (FIn::NW == 1 && FOut::NW == 2) {
             if (first && mma) {
