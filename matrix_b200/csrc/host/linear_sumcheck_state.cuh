@@ -80,7 +80,7 @@ public:
         if (d == 2 && num_vars > 0) {
             pair_.reset(new typename PairOf<typename Ext::T>::type);
             const size_t words = n_ * (base_field ? 1 : 2);
-            return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0, true);
+            return pair_->init(d_tables, d_tables + words, 0, 1, num_vars, base_field, nullptr, 0);
         }
         products_ = Product::handles(d) && num_vars > 0;
         if (products_ && num_vars <= Product::limit(d)) {

@@ -93,11 +93,8 @@ public:
         pool_free(tabs_);
     }
     // a, b: instance 0's device tables of 2^n elements (never written), instances inst_stride words apart; base: base
-    // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. together: b follows a in one allocation
-    // (addresses alone do not say so: two allocations may touch). Queues the first pass.
-    int init(const uint64_t* a, const uint64_t* b, size_t inst_stride, int K, int n, bool base, const uint64_t* eq_pt, int eq_vars,
-             bool together = false) {
-        together_ = together;
+    // field words, else (c0, c1). eq_pt: host, eq_vars (c0, c1) pairs, or null. Queues the first pass.
+    int init(const uint64_t* a, const uint64_t* b, size_t inst_stride, int K, int n, bool base, const uint64_t* eq_pt, int eq_vars) {
         a_ = a; b_ = b; stride_ = inst_stride; K_ = K; n_ = n; base_ = base;
         pt_.resize(eq_vars);
         for (int i = 0; i < eq_vars; i++) pt_[i] = H::canon(E2{eq_pt[2 * i], eq_pt[2 * i + 1]});
@@ -390,15 +387,11 @@ private:
         const size_t w = tn_ * (base_ ? 1 : 2);
         if (2 * w * K_ > ScratchPool::WORDS) return MB_ERR_UNSUPPORTED;
         pending_ = true;
-        arriving_ = 0;   // the caller's words need not be canonical
-        if (together_) {
-            MB_CUDA(cudaMemcpyAsync(pin_, a_, 16 * w, cudaMemcpyDeviceToHost, MB_STREAM));
-            return MB_OK;
-        }
-        for (int k = 0; k < K_; k++)
-            for (int s = 0; s < 2; s++)
-                MB_CUDA(cudaMemcpyAsync(pin_ + (2 * k + s) * w, (s ? b_ : a_) + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
-        return MB_OK;
+        arriving_ = 2 * w * K_;
+        expect_words(pin_, arriving_);
+        MB_KERNEL("pair_tables");
+        pr::send_tables_kernel<F><<<dim3((unsigned)((w + pr::BLK - 1) / pr::BLK), 2 * K_), pr::BLK, 0, MB_STREAM>>>(a_, b_, stride_, w, pin_);
+        return finish_async();
     }
     // A pass that could not be queued or did not finish leaves nothing to go on from: every later call returns its error too.
     int failed(int rc) {
@@ -408,7 +401,7 @@ private:
     // Results of the pass queued last.
     int wait() {
         if (bad_ != MB_OK || !pending_) return bad_;
-        if (arriving_ ? await_words(pin_, arriving_) != MB_OK : cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
+        if (await_words(pin_, arriving_) != MB_OK) return failed(MB_ERR_CUDA);
         pending_ = false;
         if (pin_[ERROR_WORD] != 0) return failed(MB_ERR_CUDA);   // a wait of a pass on the tensor cores ran out
         if (block_ < blocks_.size()) return MB_OK;
@@ -539,7 +532,7 @@ private:
     const uint64_t *a_ = nullptr, *b_ = nullptr;
     size_t stride_ = 0, arriving_ = 0;   // words of pin_ that the pass queued last writes
     int K_ = 1, n_ = 0, cap_ = 1, round_ = 0, tail_first_ = 0, bad_ = MB_OK;
-    bool base_ = false, together_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
+    bool base_ = false, flip_ = false, pending_ = false, host_ = false, weighted_ = false, have_w_ = false, words_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;
     std::vector<E2> pt_, r_, scale_, m_, w_, ta_, tb_;

@@ -224,9 +224,11 @@ private:
     // tables that no pass has folded come as they are
     int copy(int v) {
         const size_t w = ((size_t)1 << v) * (base_ ? 1 : 2);
-        for (int k = 0; k < d_; k++)
-            MB_CUDA(cudaMemcpyAsync(pin_ + w * k, in_ + stride_ * k, 8 * w, cudaMemcpyDeviceToHost, MB_STREAM));
-        return MB_OK;
+        arriving_ = w * d_;
+        expect_words(pin_, arriving_);
+        MB_KERNEL("product_tables");
+        pr::send_tables_kernel<F><<<dim3((unsigned)((w + pr::BLK - 1) / pr::BLK), d_), pr::BLK, 0, MB_STREAM>>>(in_, in_ + stride_, 2 * stride_, w, pin_);
+        return finish_async();
     }
     // As PairSumcheck: after a failure every later call fails.
     int failed(int rc) {
@@ -235,7 +237,7 @@ private:
     }
     int wait() {
         if (bad_ != MB_OK) return bad_;
-        if (arriving_ ? await_words(pin_, arriving_) != MB_OK : cudaStreamSynchronize(MB_STREAM) != cudaSuccess) return failed(MB_ERR_CUDA);
+        if (await_words(pin_, arriving_) != MB_OK) return failed(MB_ERR_CUDA);
         return failed(pin_[ERROR_WORD] != 0 ? MB_ERR_CUDA : MB_OK);
     }
     // The sums of the current block.

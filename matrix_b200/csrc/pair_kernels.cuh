@@ -260,6 +260,15 @@ __device__ __forceinline__ typename F::E2 fold_element(const uint64_t* p, size_t
     }
 }
 
+// Small tables as they are, canonical, to page-locked memory: w words of table 2 k + s from (s ? b : a) + stride k. (A copy command
+// and a synchronisation took 4 us longer, and as many commands as there were tables.)
+template <class F>
+__global__ void __launch_bounds__(BLK)
+send_tables_kernel(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, size_t stride, size_t w, uint64_t* out) {
+    const uint64_t* p = (blockIdx.y & 1 ? b : a) + stride * (blockIdx.y >> 1);
+    for (size_t x = (size_t)blockIdx.x * BLK + threadIdx.x; x < w; x += (size_t)gridDim.x * BLK) out[blockIdx.y * w + x] = F::canon(p[x]);
+}
+
 // FOLD: there are challenges to fold (a.fb of them); GB: rounds of the next block (0: fold and store only). BASE: input
 // words of the base field.
 template <class F, bool FOLD, int GB, bool BASE, bool WEIGHTED>
