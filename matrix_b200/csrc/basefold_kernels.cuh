@@ -62,6 +62,7 @@ bit_reverse_tiled_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__
     const int mid_bits = log_n - 2 * T;
     const size_t n = (size_t)1 << log_n;
     const size_t num_tiles = (size_t)1 << mid_bits;
+    chain_begin();
     for (size_t m = blockIdx.x; m < num_tiles; m += gridDim.x) {
         const size_t rm = bit_reverse(m, mid_bits);
         // element (h, l): index = h << (log_n - T) | m << T | l
@@ -70,6 +71,7 @@ bit_reverse_tiled_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__
             tile[h][l] = gl::canon(in[((size_t)h << (log_n - T)) | (m << T) | (size_t)l]);
         }
         __syncthreads();
+        if (m + gridDim.x >= num_tiles) chain_next();
         // rev(index) = rev(l) << (log_n - T) | rev(m) << T | rev(h); write runs over rev(h)
         for (int e = threadIdx.x; e < 4096; e += blockDim.x) {
             int rl = e >> T, rh = e & 63;
@@ -82,13 +84,15 @@ bit_reverse_tiled_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__
     }
 }
 
-// Small sizes: direct gather.
+// Small sizes: direct gather, on as many SMs as there are blocks of 256 elements.
 static __global__ void bit_reverse_copy_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int log_n,
                                         int copies) {
     const size_t n = (size_t)1 << log_n;
     const size_t step = (size_t)gridDim.x * blockDim.x;
+    chain_begin();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
         uint64_t v = gl::canon(in[bit_reverse(i, log_n)]);
+        if (i + step >= n) chain_next();
         for (int c = 0; c < copies; c++) out[(size_t)c * n + i] = v;
     }
 }
@@ -129,6 +133,7 @@ bit_pass_kernel(const uint64_t* in, uint64_t* out, int log_n, int bit_lo, int nb
     const int cbits = TILE_LOG - nbits, mid_bits = bit_lo - cbits, t = threadIdx.x;
     const auto pad = [](int e) { return e + (e >> 4); };
     const size_t num_tiles = (size_t)1 << (log_n - TILE_LOG);
+    chain_begin();
     for (size_t k = blockIdx.x; k < num_tiles; k += gridDim.x) {
         const size_t mid = k & (((size_t)1 << mid_bits) - 1), high = k >> mid_bits;
         const size_t base = (high << (bit_lo + nbits)) | (mid << cbits);
@@ -154,6 +159,7 @@ bit_pass_kernel(const uint64_t* in, uint64_t* out, int log_n, int bit_lo, int nb
 #pragma unroll
             for (int j = 0; j < 16; j++) tile[pad(e0 | (j << p))] = v[j];
         }
+        if (k + gridDim.x >= num_tiles) chain_next();
         __syncthreads();
 #pragma unroll 8
         for (int e = t; e < N; e += BLOCK) out[addr(e)] = gl::canon(tile[pad(e)]);
@@ -173,6 +179,7 @@ bit_layers_kernel(const uint64_t* in, uint64_t* out, int log_n, int bit_lo, int 
     const int mid_bits = bit_lo - cbits;
     const size_t num_tiles = (size_t)1 << (log_n - tile_log);
     const size_t cmask = ((size_t)1 << cbits) - 1;
+    chain_begin();
     for (size_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         size_t mid = t & (((size_t)1 << mid_bits) - 1), high = t >> mid_bits;
         size_t base = (high << (bit_lo + nbits)) | (mid << cbits);

@@ -48,12 +48,12 @@ __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wai
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 template <class... P, class... A>
-inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute early{};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
+    c.gridDim = grid;
     c.blockDim = dim3(block);
     c.dynamicSmemBytes = smem;
     c.stream = st;

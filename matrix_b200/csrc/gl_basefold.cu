@@ -36,7 +36,7 @@ int run_layers(const uint64_t* in, uint64_t* out, int log_n, int first_bit, int 
             if (TILE_LOG - nbits > bit) break;   // a first pass of fewer bits than a tile
             {
                 MB_KERNEL_ON("bit_layers", st);
-                bit_pass_kernel<Op><<<grid, BLOCK, smem, st>>>(src, out, log_n, bit, nbits);
+                launch_chained(bit_pass_kernel<Op>, (unsigned)grid, BLOCK, smem, st, src, out, log_n, bit, nbits);
             }
             src = out;
             bit += nbits;
@@ -55,7 +55,7 @@ int run_layers(const uint64_t* in, uint64_t* out, int log_n, int first_bit, int 
         int grid = (int)(tiles < (size_t)sm_count() * 4 ? tiles : (size_t)sm_count() * 4);
         {
             MB_KERNEL_ON("bit_layers", st);
-            bit_layers_kernel<Op><<<grid, BLOCK, smem, st>>>(src, out, log_n, bit, nbits, cbits);
+            launch_chained(bit_layers_kernel<Op>, (unsigned)grid, BLOCK, smem, st, src, out, log_n, bit, nbits, cbits);
         }
         src = out;
         bit += nbits;
@@ -64,19 +64,21 @@ int run_layers(const uint64_t* in, uint64_t* out, int log_n, int first_bit, int 
     return finish_async();
 }
 
+// By tiles from here on: below, a tile of 4096 elements is one block's work on one SM of few
+constexpr int REVERSE_TILED_FROM = 18;
 int bit_reverse_out_of_place(const uint64_t* in, uint64_t* out, int log_n, int copies, cudaStream_t st) {
     size_t n = (size_t)1 << log_n;
-    if (log_n >= 12) {
+    if (log_n >= REVERSE_TILED_FROM) {
         size_t tiles = (size_t)1 << (log_n - 12);
         int grid = (int)(tiles < (size_t)sm_count() * 4 ? tiles : (size_t)sm_count() * 4);
         {
             MB_KERNEL_ON("bit_reverse_tiled", st);
-            bit_reverse_tiled_kernel<<<grid, 256, 0, st>>>(in, out, log_n, copies);
+            launch_chained(bit_reverse_tiled_kernel, (unsigned)grid, 256, 0, st, in, out, log_n, copies);
         }
     } else {
         {
             MB_KERNEL_ON("bit_reverse_copy", st);
-            bit_reverse_copy_kernel<<<gs(n), BLOCK, 0, st>>>(in, out, log_n, copies);
+            launch_chained(bit_reverse_copy_kernel, (unsigned)gs(n), BLOCK, 0, st, in, out, log_n, copies);
         }
     }
     return finish_async();

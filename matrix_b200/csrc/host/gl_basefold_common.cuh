@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(pr::BLK)
 open_pass_kernel(const OpenPassArgs a, const __grid_constant__ pr::FoldWeights<pr::GlF> fw) {
     using F = pr::GlF;
     __shared__ gl::E2 sm[pr::BLK];
+    chain_begin();
     const int t = threadIdx.x, m = blockIdx.y, sb = a.v - a.rounds;
     const size_t ns = (size_t)1 << sb, n = (size_t)1 << a.v;
     gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
@@ -220,6 +221,7 @@ open_pass_kernel(const OpenPassArgs a, const __grid_constant__ pr::FoldWeights<p
     if (ns > pr::BLK) x = gl::E2{gl::acc_reduce_wide(s0), gl::acc_reduce_wide(s1)};
     if (sb > 0 && (size_t)t < ns) x = F::fma(pr::load_weight<F>(a.wl + 4 * t), x, gl::E2{0, 0});
     gl::E2 total[1] = {x};
+    chain_next();
     if (!pr::grid_sum<F, 1>(total, 0, sm, a.acc + pr::grid_words(1) * m)) return;
     if (t == 0) pr::store2(a.sums + 2 * m, sm[0].c0, sm[0].c1);
 }
@@ -331,9 +333,8 @@ private:
         const dim3 grid(rows < GX ? (unsigned)rows : GX, 1u << a.rounds);
         {
             MB_KERNEL_ON("open_pass", MB_STREAM);
-            if (!fb) open_pass_kernel<false, true><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
-            else if (stage_ == 1) open_pass_kernel<true, true><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
-            else open_pass_kernel<true, false><<<grid, pr::BLK, 0, MB_STREAM>>>(a, fw);
+            const auto k = !fb ? open_pass_kernel<false, true> : stage_ == 1 ? open_pass_kernel<true, true> : open_pass_kernel<true, false>;
+            launch_chained(k, grid, pr::BLK, 0, MB_STREAM, a, fw);
         }
         if (a.out) in_ = a.out;
         return finish_async();

@@ -19,6 +19,8 @@
 
 namespace mbhost {
 
+constexpr size_t QUERY_WORD = 1024;   // of an opening's scratch block: the queries' indices
+
 // open_ext2 (basefold.rs:578-863). Writes the proof as
 //   eval[2] | oracles[nv][3][2] | folded_roots[nv-1][4] | final_codeword[2^lr][2] |
 //   per query: index, nv value pairs [2][2], path in the commitment tree,
@@ -116,14 +118,18 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
 
     // queries: all indices first (basefold.rs:2321-2326), then one gather
     if (num_queries > 0) {
-        std::vector<uint64_t> idx(num_queries);
-        for (int q = 0; q < num_queries; q++) idx[q] = t.sample_challenge() % (uint64_t)(cw_len / 2);
+        // the kernel reads the indices where the host leaves them, as far as there is room
+        uint64_t* host_idx = pin.p + QUERY_WORD;
+        const bool direct = num_queries <= (int)(ScratchPool::WORDS - QUERY_WORD);
+        std::vector<uint64_t> idx(direct ? 0 : num_queries);
+        if (!direct) host_idx = idx.data();
+        for (int q = 0; q < num_queries; q++) host_idx[q] = t.sample_challenge() % (uint64_t)(cw_len / 2);
         size_t qw = query_words(nv, lr);
         DevBuf d_idx, d_q;
-        rc = d_idx.alloc(num_queries);
+        rc = direct ? MB_OK : d_idx.alloc(num_queries);
         if (rc == MB_OK) rc = d_q.alloc(qw * num_queries);
         if (rc != MB_OK) return rc;
-        MB_CUDA(cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(uint64_t) * num_queries, cudaMemcpyHostToDevice, MB_STREAM));
+        if (!direct) MB_CUDA(cudaMemcpyAsync(d_idx.p, idx.data(), sizeof(uint64_t) * num_queries, cudaMemcpyHostToDevice, MB_STREAM));
         QueryLevels lv;
         lv.nv = nv; lv.lr = lr;
         lv.commit_cw = cm.d_codeword.p;
@@ -131,7 +137,7 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
         for (int i = 0; i <= nv - 2; i++) { lv.fcw[i] = fcw[i]->p; lv.ftree[i] = ftree[i]->p; }
         {
             MB_KERNEL_ON("query_gather", MB_STREAM);
-            query_gather_kernel<<<num_queries, 128, 0, MB_STREAM>>>(lv, d_idx.p, d_q.p, qw);
+            query_gather_kernel<<<num_queries, 128, 0, MB_STREAM>>>(lv, direct ? host_idx : d_idx.p, d_q.p, qw);
         }
         if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
         MB_CUDA(cudaMemcpyAsync(p_queries, d_q.p, sizeof(uint64_t) * qw * num_queries, cudaMemcpyDeviceToHost, MB_STREAM));
