@@ -436,15 +436,28 @@ public:
                 MB_KERNEL_ON("table_invert", MB_STREAM);
                 table_invert_kernel<<<grid_for(total, 256, 8), 256, 0, MB_STREAM>>>(d_entries.p, total);
             }
-            rc = finish_sync();
+            // the levels that an opening folds on the host
+            host_first = (size_t)num_rounds;
+            while (host_first > 0 && level_sizes[host_first - 1] <= 2 * host_leaves(1)) host_first--;
+            const size_t from = host_first < level_offsets.size() ? level_offsets[host_first] : total;
+            host_entries.resize(2 * (total - from));
+            if (!host_entries.empty() && cudaMemcpyAsync(host_entries.data(), d_entries.p + 2 * from, 8 * host_entries.size(), cudaMemcpyDeviceToHost,
+                                                         MB_STREAM) != cudaSuccess)
+                rc = MB_ERR_CUDA;
+            const int done = finish_sync();
+            if (rc == MB_OK) rc = done;
         }
         cudaFreeHost(h);
         return rc;
     }
     const uint64_t* device_level_ptr(int level) const { return d_entries.p + 2 * level_offsets[level]; }
 
+    // the same in host memory, for levels of at most 2 host_leaves entries
+    const uint64_t* host_level(int level) const { return host_entries.data() + 2 * (level_offsets[level] - level_offsets[host_first]); }
+
     int num_vars = 0, log_rate = 0, rounds = 0;
-    size_t entries = 0;
+    size_t entries = 0, host_first = 0;
+    std::vector<uint64_t> host_entries;
     std::vector<size_t> level_offsets, level_sizes;
     DevBuf d_entries;
 };

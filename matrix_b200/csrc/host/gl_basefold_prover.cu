@@ -14,10 +14,22 @@
 // pass fewer), the inner sumcheck runs several rounds per pass over the
 // bit-reversed evaluations (OpenSumcheck), the codeword is folded by the kernels
 // that hash its leaves, each round issues them back to back and waits
-// once, and the query phase is one gather kernel and one copy.
+// once, the last few rounds are folded and hashed by the host (host_leaves),
+// and the query phase is one gather kernel and one copy.
 #include "gl_basefold_common.cuh"
 
 namespace mbhost {
+
+// out[i], i < n: the codeword `in` folded on r (entries: its table level)
+static void fold_on_host(const uint64_t* in, const uint64_t* entries, gl::E2 r, uint64_t* out, size_t n) {
+    const uint64_t r1w = gl::mul_small(r.c1, 7);
+    for (size_t i = 0; i < n; i++) {
+        const gl::E2 e = bf::fold_pair_ext(gl::E2{in[4 * i], in[4 * i + 1]}, gl::E2{in[4 * i + 2], in[4 * i + 3]},
+                                           make_ulonglong2(entries[2 * i], entries[2 * i + 1]), r, r1w);
+        out[2 * i] = e.c0;
+        out[2 * i + 1] = e.c1;
+    }
+}
 
 constexpr size_t QUERY_WORD = 1024;   // of an opening's scratch block: the queries' indices
 
@@ -38,8 +50,23 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     uint64_t* p_queries = p_final + ((size_t)2 << lr);
 
     ScopedScratch pin;   // sums of the inner sumcheck (32 words), a tree's last device layer (from word 64)
-    uint64_t* top_staging = pinned_arena(4 * (HOST_TOP - 1) * (size_t)nv);   // host-hashed tree tops on their way up
+    // The first round of the host's own: its codeword is folded, and hashed, from a copy of the one before. (Never round 0; nv - 1: none.)
+    const auto leaves_of = [&](int round) { return cw_len >> (round + 2); };
+    int host_round = 1;
+    while (host_round < nv - 1 && leaves_of(host_round) > host_leaves(cm.hash)) host_round++;
+    const bool on_host = host_round < nv - 1;
+    const size_t copy_words = on_host ? 8 * leaves_of(host_round) : 0;
+    // host-hashed tree tops on their way up; the copy; the host's rounds: by round the codeword (a pair of elements a leaf), the tree
+    std::vector<size_t> own(nv, 0);
+    size_t own_words = 0;
+    for (int i = host_round; i < nv - 1; i++) {
+        own[i] = own_words;
+        own_words += 4 * leaves_of(i) + 4 * (2 * leaves_of(i) - 1);
+    }
+    const size_t staging_words = 4 * (HOST_TOP - 1) * (size_t)nv;
+    uint64_t* top_staging = pinned_arena(staging_words + copy_words + own_words);
     if (!pin.p || !top_staging) return MB_ERR_CUDA;
+    uint64_t *copied = top_staging + staging_words, *host_rounds = copied + copy_words;
     uint64_t* nodes = pin.p + 64;
     OpenSumcheck sc;
     int rc = sc.init(cm.d_bh_evals.p, nv, point, pin.p, pin.b.dev);
@@ -62,7 +89,7 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     std::vector<std::unique_ptr<DevBuf>> fcw(nv), ftree(nv - 1);
     {
         size_t len = cw_len / 2;
-        for (int i = 0; i < nv; i++) {
+        for (int i = 0; i < (on_host ? host_round : nv); i++) {
             fcw[i].reset(new DevBuf);
             rc = fcw[i]->alloc(2 * len);
             if (rc != MB_OK) return rc;
@@ -83,22 +110,46 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
         // command
         rc = sc.fold(r);
         if (rc != MB_OK) return rc;
+        uint64_t* po = p_oracles + 6 * (size_t)(round + 1);
+        uint64_t* root = p_roots + 4 * (size_t)round;
+        if (round >= host_round) {   // beside a pass of the inner sumcheck, if the fold queued one
+            if (round == host_round) rc = await_words(copied, copy_words);
+            if (rc != MB_OK) return rc;
+            const size_t n_leaves = leaves_of(round);
+            uint64_t *cw = host_rounds + own[round], *tree = cw + 4 * n_leaves;
+            fold_on_host(round == host_round ? copied : host_rounds + own[round - 1], table.host_level(round), r, cw, 2 * n_leaves);
+            static const uint64_t none[4] = {0, 0, 0, 0};
+            for (size_t k = 0; k < n_leaves; k++) std::memcpy(tree + 4 * k, host_compress(cm.hash, cw + 4 * k, none).w, 32);
+            host_hash_top(cm.hash, tree, n_leaves, tree + 4 * n_leaves, root);
+            rc = sc.wait();
+            if (rc != MB_OK) return rc;
+            sc.oracle(po);
+            for (int k = 0; k < 3; k++) t.observe_ext2(Ext2{po[2 * k], po[2 * k + 1]});
+            t.observe_hash(root);
+            cw_pairs /= 2;
+            continue;
+        }
         // codeword fold with this round's table level, and its tree up to the layer the host takes over
         const size_t leaves = cw_pairs / 2;
         const mk::FoldSource f{round == 0 ? cm.d_codeword.p : fcw[round - 1]->p, table.device_level_ptr(round), fcw[round]->p, r};
         const size_t top = host_top(cm.hash), top_nodes = leaves < top ? leaves : top;
         expect_words(nodes, 4 * top_nodes);
         rc = queue_fold_tree(cm.hash, round == 0, f, ftree[round]->p, leaves, nodes);
+        if (rc == MB_OK && round + 1 == host_round && on_host) {
+            expect_words(copied, copy_words);
+            MB_KERNEL_ON("send_tables", MB_STREAM);
+            pr::send_tables_kernel<pr::GlF><<<1, pr::BLK, 0, MB_STREAM>>>(fcw[round]->p, nullptr, 0, copy_words, copied);
+            if (cudaGetLastError() != cudaSuccess) rc = MB_ERR_CUDA;
+        }
         if (rc == MB_OK) rc = await_words(nodes, 4 * top_nodes);
         if (rc == MB_OK) rc = sc.wait();
         if (rc != MB_OK) return rc;
-        uint64_t* po = p_oracles + 6 * (size_t)(round + 1);
         sc.oracle(po);
         rc = host_finish_top(cm.hash, nodes, top_nodes, top_staging + 4 * (HOST_TOP - 1) * (size_t)round,
-                             ftree[round]->p, leaves, p_roots + 4 * (size_t)round, MB_STREAM);
+                             ftree[round]->p, leaves, root, MB_STREAM);
         if (rc != MB_OK) return rc;
         for (int k = 0; k < 3; k++) t.observe_ext2(Ext2{po[2 * k], po[2 * k + 1]});
-        t.observe_hash(p_roots + 4 * (size_t)round);
+        t.observe_hash(root);
         cw_pairs /= 2;
     }
 
@@ -106,14 +157,16 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     {
         Ext2 ch = t.sample_challenge_ext2();
         gl::E2 r{ch.c0, ch.c1};
-        {
+        if (on_host) {
+            fold_on_host(host_rounds + own[nv - 2], table.host_level(nv - 1), r, p_final, cw_pairs);
+        } else {
             MB_KERNEL_ON("fold_ext2", MB_STREAM);
             bf::fold_ext2_kernel<<<grid_for(cw_pairs, 256, 8), 256, 0, MB_STREAM>>>(
                 fcw[nv - 2]->p, table.device_level_ptr(nv - 1), r, fcw[nv - 1]->p, cw_pairs);
         }
         if (cudaGetLastError() != cudaSuccess) return MB_ERR_CUDA;
-        MB_CUDA(cudaMemcpyAsync(p_final, fcw[nv - 1]->p, sizeof(uint64_t) * ((size_t)2 << lr), cudaMemcpyDeviceToHost,
-                                MB_STREAM));
+        if (!on_host)
+            MB_CUDA(cudaMemcpyAsync(p_final, fcw[nv - 1]->p, sizeof(uint64_t) * ((size_t)2 << lr), cudaMemcpyDeviceToHost, MB_STREAM));
     }
 
     // queries: all indices first (basefold.rs:2321-2326), then one gather
@@ -125,7 +178,7 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
         if (!direct) host_idx = idx.data();
         for (int q = 0; q < num_queries; q++) host_idx[q] = t.sample_challenge() % (uint64_t)(cw_len / 2);
         size_t qw = query_words(nv, lr);
-        DevBuf d_idx, d_q;
+        DevBuf d_idx, d_q, d_own;   // d_own: the host's rounds
         rc = direct ? MB_OK : d_idx.alloc(num_queries);
         if (rc == MB_OK) rc = d_q.alloc(qw * num_queries);
         if (rc != MB_OK) return rc;
@@ -134,7 +187,15 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
         lv.nv = nv; lv.lr = lr;
         lv.commit_cw = cm.d_codeword.p;
         lv.commit_tree = cm.d_tree.p;
-        for (int i = 0; i <= nv - 2; i++) { lv.fcw[i] = fcw[i]->p; lv.ftree[i] = ftree[i]->p; }
+        if (on_host) {
+            rc = d_own.alloc(own_words);
+            if (rc != MB_OK) return rc;
+            MB_CUDA(cudaMemcpyAsync(d_own.p, host_rounds, sizeof(uint64_t) * own_words, cudaMemcpyHostToDevice, MB_STREAM));
+        }
+        for (int i = 0; i <= nv - 2; i++) {
+            lv.fcw[i] = i < host_round ? fcw[i]->p : d_own.p + own[i];
+            lv.ftree[i] = i < host_round ? ftree[i]->p : d_own.p + own[i] + 4 * leaves_of(i);
+        }
         {
             MB_KERNEL_ON("query_gather", MB_STREAM);
             query_gather_kernel<<<num_queries, 128, 0, MB_STREAM>>>(lv, direct ? host_idx : d_idx.p, d_q.p, qw);

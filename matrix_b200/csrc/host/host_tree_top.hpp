@@ -1,7 +1,7 @@
 // Host hashing of the top of a Merkle tree (Poseidon2 or Monolith over Goldilocks, as the device trees).
 //
-// The last levels of a tree are bound by the latency of one permutation per level on the device (about 8 us with the
-// 8-lane Poseidon2, 2 us with the 16-lane Monolith); a host core runs a permutation in 0.6 or 0.2 us. So a round's
+// The last levels of a tree are bound by the latency of one permutation per level on the device (about 5 us with
+// a warp's Poseidon2, 2 us with its Monolith); a host core runs a permutation in 0.6 or 0.2 us. So a round's
 // tree stops on the device at a layer of host_top(hash) digests (mk::build_tree's `stop`), which the kernel leaves in pinned
 // memory, and the host hashes the levels above: 15 or 31 permutations, then one small upload puts them into the device tree
 // for the query phase (host_finish_top, gl_basefold_common.cuh).
@@ -30,6 +30,11 @@ inline Digest host_compress(int hash, const Digest& l, const Digest& r) { return
 // where a level costs the device as long as its nodes cost the host
 constexpr size_t host_top(int hash) { return hash ? 32 : 16; }
 constexpr size_t HOST_TOP = 32;   // the largest of them
+
+// The last rounds of an opening, whose trees have at most this many leaves, are the host's: a whole tree of them costs it less
+// than the launches, the wait (8.8 us) and the levels that would be left for the device. Openings at 2^8, 40 queries, limits of
+// 4, 8 and 16 leaves with Poseidon2: 325, 312 and 303 us (379 without host rounds); of 16, 32 and 64 with Monolith: 205, 197, 205.
+constexpr size_t host_leaves(int hash) { return hash ? 32 : 16; }
 
 // nodes: a layer of `count` digests (a power of two). upper receives the count - 1 digests of the layers above it,
 // layer by layer as the tree stores them (count / 2, count / 4, ..., 1); root receives the last one.

@@ -94,6 +94,14 @@ def test_basefold_sizes(gl, nv, lr, nq):
     monolith_basefold_matches_oracle(gl, nv, lr, nq)
 
 
+@pytest.mark.parametrize("nv,lr,nq", [(3, 0, 2), (4, 4, 3), (4, 5, 3), (3, 6, 2), (6, 1, 0), (9, 1, 12)])
+def test_basefold_rounds_of_the_host(gl, nv, lr, nq):
+    """The host folds and hashes the rounds of few leaves: one round, several, none, in either hash."""
+    basefold_matches_oracle(gl, nv, lr, nq)
+    if nq:   # (the other test ends with openings that the wrong hash must not verify)
+        monolith_basefold_matches_oracle(gl, nv, lr, nq)
+
+
 def test_poseidon2_with_a_missed_carry(gl, oracle):
     """The throughput form adds without the rare carry and borrow repairs and redoes a permutation that needed one. The
     first round constant makes lane 0 of this state 2^48 before its S-box, whose square is a power of two that does;
