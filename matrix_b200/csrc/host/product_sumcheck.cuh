@@ -56,7 +56,6 @@ public:
         if (!scratch_) return MB_ERR_CUDA;
         pin_ = scratch_.host;
         pin_[ERROR_WORD] = 0;
-        cap_ = sm_count() * (d == 1 ? 8 : 2);
         return failed(pass());
     }
     // Every round that is left is the host's: tables() has them.
@@ -163,15 +162,11 @@ private:
             int rc = launch_mma(p, fw);
             if (rc != MB_OK) return rc;
         } else {
-            const size_t tiles = ((size_t)1 << p.v) / (d_ == 1 ? pr::BLK : pr::PTILE);
             const int gb = last ? 0 : blocks_[block_].rounds;
-            // 2^9 sums: half as many blocks as SMs, or their atomics take longer than the products (2^14 elements: 30 -> 27 us)
-            const size_t most = gb * d_ >= 9 ? cap_ / 4 : cap_;
-            const unsigned grid = last ? (tiles ? (unsigned)tiles : 1u) : (unsigned)(tiles < most ? tiles : most);
             MB_KERNEL("product_pass");
-            if (d_ == 1) launch_d<1>(gb, fb > 0, grid, p, fw);
-            else if (d_ == 3) launch_d<3>(gb, fb > 0, grid, p, fw);
-            else launch_d<4>(gb, fb > 0, grid, p, fw);
+            if (d_ == 1) launch_one(gb, fb > 0, p, fw);
+            else if (d_ == 3) launch_three(gb, fb > 0, p, fw);
+            else launch_four(gb, fb > 0, p, fw);
         }
         if (fb) {
             base_ = false;
@@ -201,25 +196,52 @@ private:
         if (q.fb) return base_ ? launch_mma_as<true, true>(grid, p, fw) : launch_mma_as<true, false>(grid, p, fw);
         return base_ ? launch_mma_as<false, true>(grid, p, fw) : launch_mma_as<false, false>(grid, p, fw);
     }
-    template <int D, int GB>
-    void launch(bool fold, unsigned grid, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
+    template <int GB>
+    void launch_one(bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
+        const size_t tiles = ((size_t)1 << p.v) / pr::BLK, most = GB > 0 ? 8 * (size_t)sm_count() : tiles;
+        const unsigned grid = tiles == 0 ? 1u : (unsigned)(tiles < most ? tiles : most);
         if (fold) {
-            if (base_) pr::product_pass_kernel<F, D, GB, true, true><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
-            else pr::product_pass_kernel<F, D, GB, true, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
+            if (base_) pr::product_pass_kernel<F, GB, true, true><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
+            else pr::product_pass_kernel<F, GB, true, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
         } else if constexpr (GB > 0) {
-            if (base_) pr::product_pass_kernel<F, D, GB, false, true><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
-            else pr::product_pass_kernel<F, D, GB, false, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
+            if (base_) pr::product_pass_kernel<F, GB, false, true><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
+            else pr::product_pass_kernel<F, GB, false, false><<<grid, pr::BLK, 0, MB_STREAM>>>(p, fw);
         }
     }
-    template <int D>
-    void launch_d(int gb, bool fold, unsigned grid, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
+    void launch_one(int gb, bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
         switch (gb) {
-            case 0: launch<D, 0>(fold, grid, p, fw); break;
-            case 1: launch<D, 1>(fold, grid, p, fw); break;
-            case 2: launch<D, 2>(fold, grid, p, fw); break;
-            case 3: if constexpr (D != 4) launch<D, 3>(fold, grid, p, fw); break;
-            default: if constexpr (D == 1) launch<D, 4>(fold, grid, p, fw); break;
+            case 0: launch_one<0>(fold, p, fw); break;
+            case 1: launch_one<1>(fold, p, fw); break;
+            case 2: launch_one<2>(fold, p, fw); break;
+            case 3: launch_one<3>(fold, p, fw); break;
+            default: launch_one<4>(fold, p, fw); break;
         }
+    }
+    template <int D, int GB, int PT>
+    void launch_tiles(bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
+        const size_t n = (size_t)1 << p.v, tiles = n > PT ? n / PT : 1;
+        const unsigned grid = GB > 0 ? (unsigned)((tiles + pr::PRODUCT_CLUSTER - 1) / pr::PRODUCT_CLUSTER * pr::PRODUCT_CLUSTER) : (unsigned)tiles;
+        const int s = !fold || PT > 16 ? 0 : p.fb > 2 ? 2 : p.fb - 1;   // a thread folds two inputs or more
+        if (fold) {
+            if (base_) pr::product_tile_kernel<F, D, GB, true, true, PT><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+            else pr::product_tile_kernel<F, D, GB, true, false, PT><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+        } else if constexpr (GB > 0) {
+            if (base_) pr::product_tile_kernel<F, D, GB, false, true, PT><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+            else pr::product_tile_kernel<F, D, GB, false, false, PT><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);
+        }
+    }
+    // Tiles of 16 elements for three tables of up to 2^13 elements, of 64 for 2^14: a whole proof at 2^13 takes 99 or 101 us, at 2^14 117 or
+    // 113 (four blocks an SM of the smaller ones wait for one another's sums). Four tables have at most 2^13: 123 or 127 us there.
+    static constexpr int SMALL_TILES_TO = 13;
+    void launch_three(int gb, bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {   // two rounds: of 2^9 elements
+        if (gb == 0) launch_tiles<3, 0, 16>(fold, p, fw);
+        else if (gb == 2) launch_tiles<3, 2, 16>(fold, p, fw);
+        else if (p.v <= SMALL_TILES_TO) launch_tiles<3, 3, 16>(fold, p, fw);
+        else launch_tiles<3, 3, 64>(fold, p, fw);
+    }
+    void launch_four(int gb, bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
+        if (gb == 0) launch_tiles<4, 0, 16>(fold, p, fw);
+        else launch_tiles<4, 2, 16>(fold, p, fw);
     }
     // tables that no pass has folded come as they are
     int copy(int v) {
@@ -277,7 +299,7 @@ private:
 
     const uint64_t* in_ = nullptr;
     size_t stride_ = 0, arriving_ = 0;   // as in PairSumcheck
-    int d_ = 0, n_ = 0, cap_ = 1, round_ = 0, side_ = 0, tail_vars_ = 0, bad_ = MB_OK;
+    int d_ = 0, n_ = 0, round_ = 0, side_ = 0, tail_vars_ = 0, bad_ = MB_OK;
     bool base_ = false, flip_ = false, loaded_ = false;
     std::vector<Block> blocks_;
     size_t block_ = 0;

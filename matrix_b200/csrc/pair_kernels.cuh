@@ -226,7 +226,35 @@ struct FoldWeights {
     typename F::Pre w[1 << MAX_B];   // eq vector of the challenges to fold, bit k: challenge k
 };
 
-// element y of the folded table: a dot product with the eq vector of fb challenges (two or more inputs, read in pairs)
+// `inputs` terms (two or more, read in pairs) of a folded element from term m0 on, loose: a dot product with the eq vector
+template <class F, bool BASE, int UNROLL>
+__device__ __forceinline__ typename F::E2 fold_part(const uint64_t* q, int m0, int inputs, const FoldWeights<F>& fw) {
+    using E2 = typename F::E2;
+    gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
+#pragma unroll UNROLL
+    for (int m = 0; m < inputs; m += 2) {
+        const typename F::Pre &u = fw.w[m0 + m], &w = fw.w[m0 + m + 1];
+        if constexpr (BASE) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(q + m);
+            gl::acc_mul(s0, u.c0, v.x);
+            gl::acc_mul(s1, u.c1, v.x);
+            gl::acc_mul(s0, w.c0, v.y);
+            gl::acc_mul(s1, w.c1, v.y);
+        } else {
+            const E2 v = load2<E2>(q + 2 * m), z = load2<E2>(q + 2 * m + 2);
+            gl::acc_mul(s0, u.c0, v.c0);
+            gl::acc_mul(s0, u.c1w, v.c1);
+            gl::acc_mul(s1, u.c0, v.c1);
+            gl::acc_mul(s1, u.c1, v.c0);
+            gl::acc_mul(s0, w.c0, z.c0);
+            gl::acc_mul(s0, w.c1w, z.c1);
+            gl::acc_mul(s1, w.c0, z.c1);
+            gl::acc_mul(s1, w.c1, z.c0);
+        }
+    }
+    return E2{F::red(s0), F::red(s1)};
+}
+// element y of the folded table
 template <class F, bool FOLD, bool BASE>
 __device__ __forceinline__ typename F::E2 fold_element(const uint64_t* p, size_t y, int fb, const FoldWeights<F>& fw) {
     using E2 = typename F::E2;
@@ -234,30 +262,16 @@ __device__ __forceinline__ typename F::E2 fold_element(const uint64_t* p, size_t
         if constexpr (BASE) return E2{p[y], 0};
         else return load2<E2>(p + 2 * y);
     } else {
-        gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
-        const uint64_t* q = p + ((BASE ? y : 2 * y) << fb);
-#pragma unroll 2
-        for (int m = 0; m < (1 << fb); m += 2) {
-            if constexpr (BASE) {
-                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(q + m);
-                gl::acc_mul(s0, fw.w[m].c0, x.x);
-                gl::acc_mul(s1, fw.w[m].c1, x.x);
-                gl::acc_mul(s0, fw.w[m + 1].c0, x.y);
-                gl::acc_mul(s1, fw.w[m + 1].c1, x.y);
-            } else {
-                const E2 x = load2<E2>(q + 2 * m), z = load2<E2>(q + 2 * m + 2);
-                gl::acc_mul(s0, fw.w[m].c0, x.c0);
-                gl::acc_mul(s0, fw.w[m].c1w, x.c1);
-                gl::acc_mul(s1, fw.w[m].c0, x.c1);
-                gl::acc_mul(s1, fw.w[m].c1, x.c0);
-                gl::acc_mul(s0, fw.w[m + 1].c0, z.c0);
-                gl::acc_mul(s0, fw.w[m + 1].c1w, z.c1);
-                gl::acc_mul(s1, fw.w[m + 1].c0, z.c1);
-                gl::acc_mul(s1, fw.w[m + 1].c1, z.c0);
-            }
-        }
-        return E2{F::canon(F::red(s0)), F::canon(F::red(s1))};
+        const E2 e = fold_part<F, BASE, 2>(p + ((BASE ? y : 2 * y) << fb), 0, 1 << fb, fw);
+        return E2{F::canon(e.c0), F::canon(e.c1)};
     }
+}
+// the sum of 2^s neighbouring threads' parts, canonical
+template <class F>
+__device__ __forceinline__ typename F::E2 fold_join(typename F::E2 e, int s) {
+    for (int off = 1; off < (1 << s); off <<= 1)
+        e = F::add(e, typename F::E2{__shfl_xor_sync(0xffffffffu, e.c0, off), __shfl_xor_sync(0xffffffffu, e.c1, off)});
+    return typename F::E2{F::canon(e.c0), F::canon(e.c1)};
 }
 
 // Small tables as they are, canonical, to page-locked memory: w words of table 2 k + s from (s ? b : a) + stride k. (A copy command
@@ -385,38 +399,12 @@ pair_small_kernel(const PairArgs a, int s, const __grid_constant__ FoldWeights<F
     const int t = threadIdx.x, k = blockIdx.y, tile = (BLK / 2) >> s, part = t & ((1 << s) - 1), f = t >> s, x = f & (tile - 1);
     const bool second = f >= tile;   // of the second table
     const size_t n = (size_t)1 << a.v, first = (size_t)blockIdx.x * tile, y = first + x;
-    gl::Acc s0 = gl::acc_zero(), s1 = gl::acc_zero();
+    E2 e{0, 0};
     if (y < n) {
         const int inputs = 1 << (a.fb - s), m0 = part * inputs;   // at least two
-        const uint64_t* q = (second ? a.b : a.a) + a.in_stride * k + (((BASE ? y : 2 * y) << a.fb) + (BASE ? m0 : 2 * m0));
-#pragma unroll 4
-        for (int m = 0; m < inputs; m += 2) {
-            const typename F::Pre &u = fw.w[m0 + m], &w = fw.w[m0 + m + 1];
-            if constexpr (BASE) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(q + m);
-                gl::acc_mul(s0, u.c0, v.x);
-                gl::acc_mul(s1, u.c1, v.x);
-                gl::acc_mul(s0, w.c0, v.y);
-                gl::acc_mul(s1, w.c1, v.y);
-            } else {
-                const E2 v = load2<E2>(q + 2 * m), z = load2<E2>(q + 2 * m + 2);
-                gl::acc_mul(s0, u.c0, v.c0);
-                gl::acc_mul(s0, u.c1w, v.c1);
-                gl::acc_mul(s1, u.c0, v.c1);
-                gl::acc_mul(s1, u.c1, v.c0);
-                gl::acc_mul(s0, w.c0, z.c0);
-                gl::acc_mul(s0, w.c1w, z.c1);
-                gl::acc_mul(s1, w.c0, z.c1);
-                gl::acc_mul(s1, w.c1, z.c0);
-            }
-        }
+        e = fold_part<F, BASE, 4>((second ? a.b : a.a) + a.in_stride * k + (((BASE ? y : 2 * y) << a.fb) + (BASE ? m0 : 2 * m0)), m0, inputs, fw);
     }
-    E2 e{F::red(s0), F::red(s1)};
-    for (int off = 1; off < (1 << s); off <<= 1) {
-        const E2 o{__shfl_xor_sync(0xffffffffu, e.c0, off), __shfl_xor_sync(0xffffffffu, e.c1, off)};
-        e = F::add(e, o);
-    }
-    e = E2{F::canon(e.c0), F::canon(e.c1)};
+    e = fold_join<F>(e, s);
     if (part == 0) {
         if (y < n && a.out != nullptr) store2(a.out + ((size_t)4 << a.v) * k + 2 * ((second ? n : 0) + y), e.c0, e.c1);
         if constexpr (GB > 0) {

@@ -44,10 +44,6 @@ __device__ __forceinline__ void transpose_bytes(const uint64_t (&f)[8], uint64_t
     }
 }
 
-__device__ __forceinline__ void cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // A row without the tensor cores, from the operand (bytes of eq(x) are its bytes for i = 0): after a wait that ran out.
 template <class F>
 static __device__ __noinline__ typename F::E2 plain_row(const uint64_t* in, const uint8_t* op, int n) {
@@ -176,7 +172,7 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
             else share[t] = e;
         }
         if (slices > 1) {
-            cluster_sync();
+            tc::cluster_sync();
             const uint32_t mine = DM_ROWS / slices;
             if ((uint32_t)t < mine) {
                 const uint32_t row = slice * mine + t;
@@ -190,7 +186,7 @@ dot_mma_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, cons
                 }
                 pr::store2(out + 2 * (first + row), F::canon(e.c0), F::canon(e.c1));
             }
-            cluster_sync();
+            tc::cluster_sync();
         }
     }
     tc::copy_wait<0>();

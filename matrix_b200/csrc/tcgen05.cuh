@@ -57,6 +57,11 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // barrier of `threads` threads of a block, id from 1
 __device__ __forceinline__ void named_sync(uint32_t threads, uint32_t id = 1) { asm volatile("bar.sync %1, %0;" ::"r"(threads), "r"(id) : "memory"); }
+// all threads of the cluster: what they wrote to shared memory is there for the others
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // bounded: false after `polls` polls. MB_TC_POLLS: 0 in a test build, where every wait of a kernel but Issued::drain runs out at once.
 #ifndef MB_TC_POLLS
