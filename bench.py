@@ -1341,9 +1341,9 @@ def run_basefold(args):
     node_bytes = big_nodes(leaves_commit) * (64 + 32 * copies) + sum(big_nodes(m // world) for m in big_folded) * 96
     hash_ms = sum(kernels.get(k, (0, 0))[1] for k in ("hash_leaves", "compress_layer", "tree_up"))
     perms_per_s = (leaves_commit + leaves_folded + nodes_per_step) * prof_steps / (hash_ms * 1e-3) if hash_ms else 0.0
-    # of a permutation's thread: Poseidon2 10870 a thread each (profiles/poseidon2_permute_batch_ncu.md), 8640 to 9630 in tiles, where
-    # 85 % of the permutations are at 2^24 (profiles/bench_basefold_launches.md)
-    inst_per_perm = 9090.0 if args.hash == "poseidon2" else 5615.0
+    # of a permutation's thread: Poseidon2 6960 to 7260 in tiles, where 97 % of the permutations are at 2^24
+    # (profiles/bench_basefold_launches.md); Monolith 4400 (profiles/tensor_core_field_kernels_ncu.md)
+    inst_per_perm = 7050.0 if args.hash == "poseidon2" else 4400.0
     sm_hz = 1e6 * (clocks.get("sm_mhz") or 1965.0)
     if dom is not None:
         cnt, ms = kernels[dom]
@@ -1370,8 +1370,8 @@ def run_basefold(args):
                         "traffic_note": "bytes per launch (average), scaled from the capture in profiles/bench_basefold_launches.md",
                         "launches": cnt, "avg_launch_ms": ms / cnt, "share_of_kernel_time": ms / total_kernel_ms,
                         "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % prof_steps,
-                        "note": ("Poseidon2 hashing: ~380 modular multiplications per 32-byte digest and thread, the internal "
-                                 "rounds' linear algebra on the tensor cores (520 below 2^20 nodes a layer), bound by the "
+                        "note": ("Poseidon2 hashing: ~350 modular multiplications per 32-byte digest and thread, the internal "
+                                 "rounds' linear algebra on the tensor cores (520 below 2^16 nodes a layer), bound by the "
                                  "integer pipes, not HBM; permutations/s is the meaningful rate") if args.hash == "poseidon2"
                         else "Monolith hashing: bound by the integer pipes, not HBM; permutations/s is the meaningful rate",
                         "permutations_per_s": perms_per_s,

@@ -8,7 +8,7 @@
 //                     cost next to nothing there (a pass that folds words to 2^16 elements takes 15 us, 26 without; 2^11 and fewer
 //                     elements a table are less than a tile).
 //   rounds per block  otherwise 4: a round more doubles the products per element (2^B), which pays while a launch and a
-//                     synchronisation (about 12 us) cost more than they do, and with at most 64 instances these passes have at
+//                     synchronisation or wait (9 to 12 us) cost more than they do, and with at most 64 instances these passes have at
 //                     most 2^17 elements. In every case bounded by what the host then has to fold, K 4^B entries.
 //   host tables       2^t elements per table with K 2^t <= 512: the rest of a proof on them takes a core about as long
 //                     as one more pass and its synchronisation.
