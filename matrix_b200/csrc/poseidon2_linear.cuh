@@ -85,7 +85,7 @@ constexpr P2Linear P2_LINEAR = p2_linear();
 // product; every lane makes the S-boxes itself. R_(r+1) without u_r's part is whole one round ahead, so its reduction and its
 // shuffle run beside the S-box, and the chain from u_r to u_(r+1) is the S-box alone: 9.1 k cycles a permutation against 12.0 k
 // with eight lanes (13.3 k with lane 0's S-box output sent round), at one warp a scheduler.
-struct P2Warp {
+struct alignas(16) P2Warp {   // copied 16 bytes at a time
     uint64_t z[8][32], c[32], u[23][32], own[22];   // by lane; own[q]: u_q to R_(q+1), which u[q] leaves out
 };
 constexpr P2Warp p2_warp(const P2Linear& p) {
@@ -99,6 +99,7 @@ constexpr P2Warp p2_warp(const P2Linear& p) {
     for (int q = 1; q < 22; q++) w.own[q] = p.row[q + 1][8 + q];
     return w;
 }
+static_assert(sizeof(P2Warp) % 16 == 0, "whole copies");
 static __device__ const P2Warp g_p2_warp = p2_warp(P2_LINEAR);
 
 __device__ __forceinline__ uint64_t p2_from_lane(uint64_t x, int lane) {

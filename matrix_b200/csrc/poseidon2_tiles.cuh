@@ -60,7 +60,7 @@ __host__ __device__ constexpr P2Step p2_step(int i) {
 // where a step's operand lies, in rows of 32 bytes
 __host__ __device__ constexpr uint32_t p2_at(int i) { return i == 0 ? 0 : p2_at(i - 1) + p2_step(i - 1).columns; }
 constexpr uint32_t P2_TABLE_ROWS = p2_at(P2_STEPS);
-struct P2Table {
+struct alignas(16) P2Table {   // read 16 bytes at a time
     uint64_t word[4 * P2_TABLE_ROWS];
 };
 // Byte i of a symbol adds byte b of 2^(8 i) times its coefficient to column b: byte i of word [row of the column][symbol].
@@ -84,6 +84,7 @@ constexpr P2Table p2_table(const P2Linear& p) {
     }
     return t;
 }
+static_assert(sizeof(P2Table) % 16 == 0, "whole units");
 static __device__ const P2Table g_p2_table = p2_table(P2_LINEAR);
 
 // shared memory: the table, a column of ones and the constants for it (two stages), the tiles' operands (z, chunks 0 .. 3; 4 and 5 go

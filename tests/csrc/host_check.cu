@@ -12,6 +12,7 @@
 #include "host/gl_monolith_host.hpp"
 #include "host/host_tree_top.hpp"
 #include "agl_mcommit.cuh"
+#include "poseidon2_tiles.cuh"
 
 extern "C" {
 uint64_t hc_gl_add(uint64_t a, uint64_t b) { return gl::add(a, b); }
@@ -59,6 +60,10 @@ void hc_mcm_shake(const uint32_t* seed, uint32_t counter, const uint32_t* nonce,
 }
 void hc_mcm_key_block(const uint32_t* seed, uint32_t kind, uint32_t row, uint64_t col, uint32_t b, uint64_t* vals) {
     mcm::key_block8(seed, kind, row, col, b, vals);
+}
+// alignment and size of the tables that kernels read 16 bytes at a time
+void hc_p2_tables(size_t* o) {
+    o[0] = alignof(mb::mk::P2Warp); o[1] = sizeof(mb::mk::P2Warp); o[2] = alignof(mb::mk::P2Table); o[3] = sizeof(mb::mk::P2Table);
 }
 void hc_poseidon2(uint64_t* s) { gl::poseidon2_permute(s); }
 // the host-side form (transcripts, tree tops) and the reductions underneath both host permutations

@@ -10,6 +10,14 @@ from .conftest import GL_P
 RC0 = 0xdd5743e7f2a5a5d9   # Poseidon2's first constant of lane 0
 
 
+def test_device_tables_are_aligned(hostcheck):
+    """The tables of the tiles and of the permutation a warp are copied by 16-byte loads: their type has to say so, or where they lie
+    depends on their neighbours in the translation unit."""
+    o = (ctypes.c_size_t * 4)()
+    hostcheck.hc_p2_tables(o)
+    assert o[0] >= 16 and o[2] >= 16 and o[1] % 16 == 0 and o[3] % 16 == 0
+
+
 def _states(width, p):
     rnd = random.Random(31)
     edge = [0, 1, p - 1, p, 2**64 - 1, 2**32 - 1, 2**32, 2**63]
