@@ -160,8 +160,9 @@ int commit_s8_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T,
     uint64_t* partial = nullptr;
     MB_CUDA(pool_alloc((void**)&partial, chunks * 3 * TC_MAX_PLANES * TC_ROWS * D * sizeof(uint64_t)));
     mbhost::ScratchBlock done = mbhost::ScratchPool::take();
-    int rc = done ? MB_OK : MB_ERR_CUDA;
     if (done) mbhost::expect_words(done.host, 1);
+    else cudaGetLastError();   // without a block the call ends with a synchronisation
+    int rc = MB_OK;
     for (int p0 = 0; p0 < planes && rc == MB_OK; p0 += TC_PASS_PLANES) {
         const int np = planes - p0 < TC_PASS_PLANES ? planes - p0 : TC_PASS_PLANES;
         {
@@ -179,9 +180,12 @@ int commit_s8_tc(const uint32_t* d_key, const uint64_t* d_M, const uint8_t* d_T,
         }
         rc = finish_async();
     }
-    // after a failed launch nothing may still write to err or partial
-    if (rc == MB_OK) rc = mbhost::await_words(done.host, 1);
-    else cudaStreamSynchronize(MB_STREAM);
+    if (rc == MB_OK && done) {
+        rc = mbhost::await_words(done.host, 1);
+    } else {   // also after a failed launch: nothing may still write to err or partial
+        const bool synced = cudaStreamSynchronize(MB_STREAM) == cudaSuccess;
+        if (!synced) rc = MB_ERR_CUDA;
+    }
     mbhost::ScratchPool::give(done, rc == MB_OK);
     pool_free(partial);
     if (rc != MB_OK) return rc;

@@ -1,5 +1,5 @@
-"""A pass that gave up a bounded wait, seen from the host: the library's own objects linked with a stand-in for the CUDA runtime,
-so no GPU is needed and none is made to fail."""
+"""A pass that gave up a bounded wait, and scratch that cannot be had, seen from the host: the library's own objects linked with a
+stand-in for the CUDA runtime, so no GPU is needed and none is made to fail."""
 import ctypes
 import os
 import subprocess
@@ -11,7 +11,7 @@ from matrix_b200 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 MB_ERR_CUDA = -1
-UNITS = ["gl_memory.cu", "prof.cu", "host/exchange.cu", "host/gl_batched_prover.cu"]
+UNITS = ["gl_memory.cu", "prof.cu", "host/exchange.cu", "host/gl_batched_prover.cu", "agl_ajtai.cu"]
 
 
 @pytest.fixture(scope="module")
@@ -98,3 +98,21 @@ def test_scratch_is_kept_after_a_good_proof(lib):
     s = Handle(lib, 2, 13)
     assert lib.fake_scratch_allocated() == counts[0]
     s.close()
+
+
+@pytest.mark.parametrize("planes", [1, 3, 4, 5, 9])   # one pass over the matrix, and several
+def test_ajtai_commitment_without_scratch(lib, planes):
+    """A commitment needs a scratch block for nothing but an earlier answer: without one it synchronises."""
+    allocated, holders = lib.fake_scratch_allocated(), []
+    while lib.fake_scratch_allocated() == allocated:   # every block kept from earlier proofs is in use
+        holders.append(Handle(lib, 1, 12))
+    key, digits, out = np.ones(8, dtype=np.uint32), np.ones(40 * 64 * planes, dtype=np.int8), np.zeros(42 * 64 * planes, dtype=np.uint64)
+    args = [ctypes.c_void_p(x.ctypes.data) for x in (key, digits)] + [ctypes.c_uint64(40), planes, ctypes.c_uint64(0), ctypes.c_void_p(out.ctypes.data)]
+    before = lib.fake_synchronised()
+    lib.fake_no_scratch(1)
+    rcs = [lib.ajtai_commit_s8_ffi(*args) for _ in range(2)]
+    lib.fake_no_scratch(0)
+    assert rcs == [0, 0] and lib.fake_synchronised() == before + 2
+    for h in holders:
+        h.close()
+    assert lib.ajtai_commit_s8_ffi(*args) == 0
