@@ -10,9 +10,11 @@
 #define BLOCKS 64
 static uint64_t* blocks[BLOCKS];
 static int fail_next, launched, allocated, freed, no_scratch, last_error, synchronised;
+static unsigned device_flags;
 
 void fake_fail_next_wait(void) { fail_next = 1; launched = 0; }
 void fake_no_scratch(int on) { no_scratch = on; }
+void fake_device_flags(unsigned flags) { device_flags = flags; }
 int fake_synchronised(void) { return synchronised; }
 int fake_scratch_allocated(void) { return allocated; }
 int fake_scratch_freed(void) { return freed; }
@@ -59,6 +61,7 @@ int cudaMemsetAsync_ptsz(void* d, int v, size_t n, void* st) { memset(d, v, n); 
 int cudaLaunchKernel_ptsz(void) { launched = 1; return 0; }
 int cudaLaunchKernelExC_ptsz(void) { launched = 1; return 0; }
 int cudaFuncSetAttribute(void) { return 0; }
+int cudaGetDeviceFlags(unsigned* f) { *f = device_flags; return 0; }
 int cudaGetDevice(int* d) { *d = 0; return 0; }
 int cudaSetDevice(int d) { return 0; }
 int cudaGetDeviceCount(int* n) { *n = 1; return 0; }

@@ -1,8 +1,9 @@
-"""A pass that gave up a bounded wait, and scratch that cannot be had, seen from the host: the library's own objects linked with a
-stand-in for the CUDA runtime, so no GPU is needed and none is made to fail."""
+"""A pass that gave up a bounded wait, scratch that cannot be had, and the caller's way of waiting, seen from the host: the library's
+own objects linked with a stand-in for the CUDA runtime, so no GPU is needed and none is made to fail."""
 import ctypes
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -116,3 +117,21 @@ def test_ajtai_commitment_without_scratch(lib, planes):
     for h in holders:
         h.close()
     assert lib.ajtai_commit_s8_ffi(*args) == 0
+
+
+def test_waits_of_a_caller_that_does_not_spin(lib):
+    """Device flags of blocking synchronisation (4) or yielding (2): a wait for words is the synchronisation that they are for. No word
+    arrives here, so the others (0 and 1) use up their polls, a third of a millisecond or more each, in front of it."""
+    key, digits, out = np.ones(8, dtype=np.uint32), np.ones(8 * 64, dtype=np.int8), np.zeros(42 * 64, dtype=np.uint64)
+    args = [ctypes.c_void_p(x.ctypes.data) for x in (key, digits)] + [ctypes.c_uint64(8), 1, ctypes.c_uint64(0), ctypes.c_void_p(out.ctypes.data)]
+    took = {}
+    for flags in (0, 1, 2, 4, 4 | 8):   # 8: mapped host memory, no way of waiting
+        lib.fake_device_flags(flags)
+        assert lib.ajtai_commit_s8_ffi(*args) == 0
+        before, t = lib.fake_synchronised(), time.thread_time()
+        for _ in range(40):
+            assert lib.ajtai_commit_s8_ffi(*args) == 0
+        took[flags] = time.thread_time() - t
+        assert lib.fake_synchronised() == before + 40
+    lib.fake_device_flags(0)
+    assert max(took[2], took[4], took[12]) < min(took[0], took[1]) / 4, took
