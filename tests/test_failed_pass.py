@@ -22,7 +22,10 @@ def lib(tmp_path_factory):
     objs = [os.path.join(build.OBJ, u.replace("/", "_") + ".o") for u in UNITS]
     fake = out[:-3] + ".o"
     subprocess.check_call(["gcc", "-O1", "-w", "-fPIC", "-c", os.path.join(HERE, "csrc", "fake_cudart.c"), "-o", fake])
-    subprocess.check_call(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", out] + objs + [fake, "-lrt", "-lpthread"])
+    only = out[:-3] + ".map"   # statics of inline functions are unique in a process otherwise: the product's scratch pool would get these blocks
+    with open(only, "w") as f:
+        f.write("{ global: fake_*; gl_*; ajtai_*; local: *; };")
+    subprocess.check_call(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-Wl,--version-script," + only, "-o", out] + objs + [fake, "-lrt", "-lpthread"])
     lib = ctypes.CDLL(out)
     u64 = ctypes.c_uint64
     lib.gl_batched_state_set_alpha.argtypes = lib.gl_batched_state_fold.argtypes = [ctypes.c_void_p, u64, u64]
