@@ -6,15 +6,18 @@
 #ifdef __CUDACC__
 namespace gl {
 namespace fast {
-// Repairs left out so far. A borrow left as it is shows in the word it leaves: at least 2^64 - 2^38. So the largest high word
-// tells of them all (and of one right word in 2^26); a maximum goes to the other pipe than a carry kept in a register, and
-// the same holds for an addition to which its own carry is added at once: 27.1 -> 23.4 cycles a product. Carries left
-// out are counted.
+// Repairs left out so far. A borrow left as it is shows in the word it leaves: a high word of at least 2^32 - 1 - z4 (below). So
+// the largest high word tells of them all, and of z4 + 1 right words in 2^32; a maximum goes to the other pipe than a carry kept in
+// a register, and the same holds for an addition to which its own carry is added at once: 27.1 -> 23.4 cycles a product. Carries
+// left out are counted.
 struct Missed {
     uint32_t top, carries;
-    __device__ __forceinline__ bool any() const { return top >= 0xFFFFFFC0u || carries != 0; }
+    // most: the largest z4 of the reductions so far. What is told of for nothing costs a whole exact permutation: with 63 here, a layer of
+    // 2^14 permutations took 39 us instead of 23 one time in eight.
+    __device__ __forceinline__ bool any(uint32_t most = 0) const { return top >= 0xFFFFFFFFu - most || carries != 0; }
 };
-// reduce_limbs without the repair; z4 2^128 = -z4 2^32 for z4 < 32
+// reduce_limbs without the repair; z4 2^128 = -z4 2^32. (A : z0) - (B1 : B0) borrows if A is less than B1 or B1 + 1, and B1 is z4 or, with
+// A at least 1 then, z4 + 1: the high word comes out at 2^32 - 1 - z4 or above. Likewise in a sum (z4 = 0).
 __device__ __forceinline__ uint64_t reduce(uint32_t z0, uint32_t z1, uint32_t z2, uint32_t z3, uint32_t z4, Missed& missed) {
     uint32_t A, B0, B1, r0, r1;
     asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %3, %4;\n\taddc.u32 %0, t, 0;\n\taddc.cc.u32 %1, %4, %5;\n\taddc.u32 %2, %6, 0;\n\t}"

@@ -169,7 +169,7 @@ GLF void poseidon2_permute(uint64_t* s) {
 // other), which overlap to about 1.4. Against the exact form:
 //   * the last repair of a reduction is left out. It is needed when a 64-bit word comes out below a 33-bit subtrahend (or
 //     a sum of eight words has a high word within 64 of 2^32): about once in 2^31 products. Missed tells, and the caller runs the
-//     exact form on the same input (one permutation in a hundred thousand, by the words that only look like it);
+//     exact form on the same input (one permutation in four million, half of them by words that only look like it);
 //   * the sums of the internal layer are sums of whole words in 96 bits, three carry additions each; the external layers are on
 //     the FP64 pipe.
 // Exact form 25.3 k cycles per warp of permutations, carries counted and external layers in 96 bits 17.5 k, now 16.8 k (2^19

@@ -155,7 +155,8 @@ __device__ __forceinline__ uint64_t poseidon2_permute_warp(uint64_t x, int lane,
     x = lane8 ? x : u;
 #pragma unroll 1
     for (int r = 4; r < 8; r++) x = gl::p2_coop_external(gl::p2t::sbox7_soon(x, missed), lane8, r < 7 ? gl::g_p2_rc_ext[r + 1][lane8] : 0, missed);
-    if (__any_sync(0xffffffffu, missed.any())) return gl::poseidon2_permute_gathered(in, lane8);
+    if (__any_sync(0xffffffffu, missed.any(29)))   // a row: at most thirty products
+        return gl::poseidon2_permute_gathered(in, lane8);
     return x;
 }
 
