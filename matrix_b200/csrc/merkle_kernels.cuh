@@ -288,8 +288,9 @@ tree_up_coop_kernel(const FoldSource f, uint64_t* dst, size_t size, int levels, 
     if (last_out != nullptr && threadIdx.x < 4) last_out[4 * (size_t)blockIdx.x + threadIdx.x] = x;
 }
 
-// Full permutation of n width-8 states (poseidon2_hash_batch_ffi).
-static __global__ void __launch_bounds__(BLOCK, 8)
+// Full permutation of n width-8 states (poseidon2_hash_batch_ffi). The compiler's own 80 registers, no spills; held to 64 for eight blocks
+// an SM 136 bytes of them go to memory (calls of 1, 2^14 and 2^20 states 27.8, 26.2 and 481 us there, 26.2, 24.8 and 476 here).
+static __global__ void __launch_bounds__(BLOCK)
 permute_batch_kernel(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, size_t n) {
     const size_t step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += step) {
@@ -365,8 +366,8 @@ poseidon2_tiles_kernel(const FoldSource f, uint64_t* __restrict__ dst, size_t n,
     __syncthreads();
     if (t < 32) tc::tmem_free(tmem_sm, 512);
 }
-// Layers of this many permutations and more go in tiles (us, a thread each and in tiles): 2^15 25 and 25, 2^16 42 and 35, 2^17 75 and 57,
-// 2^18 134 and 117, 2^19 245 and 203, 2^20 487 and 383. One tile an SM takes 20 us whatever their number (2^13 and 2^14: a thread each 19).
+// Layers of this many permutations and more go in tiles (us, a thread each and in tiles): 2^15 25.7 and 26.7, 2^16 42.6 and 36.9, 2^17 66 and
+// 57, 2^18 123 and 105, 2^19 236 and 192, 2^20 469 and 377. One tile an SM takes 23 us whatever their number (2^13 and 2^14: a thread each 20).
 constexpr size_t P2_TILES_FROM = (size_t)1 << 16;
 template <TreeSource SRC>
 inline void launch_poseidon2_tiles(const FoldSource& f, uint64_t* dst, size_t n, size_t copies, cudaStream_t st) {
