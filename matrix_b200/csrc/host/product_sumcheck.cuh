@@ -219,8 +219,9 @@ private:
     }
     template <int D, int GB, int PT>
     void launch_tiles(bool fold, const pr::ProductArgs& p, const pr::FoldWeights<F>& fw) const {
-        const size_t n = (size_t)1 << p.v, tiles = n > PT ? n / PT : 1;
-        const unsigned grid = GB > 0 ? (unsigned)((tiles + pr::PRODUCT_CLUSTER - 1) / pr::PRODUCT_CLUSTER * pr::PRODUCT_CLUSTER) : (unsigned)tiles;
+        // with sums 2^9 elements or more, at least four clusters; else the host's tables, 2^7 or 2^8
+        static_assert(512 / PT % pr::PRODUCT_CLUSTER == 0 && 128 % PT == 0, "whole clusters, whole tiles");
+        const unsigned grid = (unsigned)(((size_t)1 << p.v) / PT);
         const int s = !fold || PT > 16 ? 0 : p.fb > 2 ? 2 : p.fb - 1;   // a thread folds two inputs or more
         if (fold) {
             if (base_) pr::product_tile_kernel<F, D, GB, true, true, PT><<<grid, pr::BLK, 0, MB_STREAM>>>(p, s, fw);

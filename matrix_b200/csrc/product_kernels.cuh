@@ -52,6 +52,7 @@ product_pass_kernel(const ProductArgs a, const __grid_constant__ FoldWeights<F> 
 // a pass are those of its clusters. (Every thread with its own products of the first two, tiles of 64, half as many blocks as SMs so that their atomics
 // did not take longer than the products: three extension tables of 2^14, fold and three rounds 28.4 -> 15.6 us, of 2^11 13.9 -> 10.8,
 // the last fold 8.2 -> 7.2; a proof over tables of 2^14 136 -> 113, over four of 2^13 160 -> 123.)
+// n is a multiple of PT, and of 8 PT where there are sums.
 constexpr int PRODUCT_CLUSTER = 8;
 template <class F, int D, int GB, bool FOLD, bool BASE, int PT>
 __global__ void __launch_bounds__(BLK) __cluster_dims__(GB > 0 ? PRODUCT_CLUSTER : 1, 1, 1)
@@ -70,7 +71,7 @@ product_tile_kernel(const ProductArgs a, int s, const __grid_constant__ FoldWeig
         const int part = t & ((1 << s) - 1), k = (t >> s) / PT, x = (t >> s) % PT;
         const size_t g = (size_t)blockIdx.x * PT + x;
         E2 e{0, 0};
-        if (k < D && g < n) {
+        if (k < D) {
             const uint64_t* q = a.in + a.stride * k;
             if constexpr (FOLD) {
                 const int inputs = 1 << (a.fb - s), m0 = part * inputs;   // at least two
@@ -81,7 +82,7 @@ product_tile_kernel(const ProductArgs a, int s, const __grid_constant__ FoldWeig
         }
         if constexpr (FOLD) e = fold_join<F>(e, s);
         if (k < D && part == 0) {
-            if (g < n && a.out != nullptr) store2(a.out + 2 * (n * k + g), e.c0, e.c1);
+            if (a.out != nullptr) store2(a.out + 2 * (n * k + g), e.c0, e.c1);
             sf[k][x] = e;
             if (k == D - 1) sw[x] = F::times_w(e.c1);
         }
@@ -120,7 +121,6 @@ product_tile_kernel(const ProductArgs a, int s, const __grid_constant__ FoldWeig
             if (t < h) work[t] = F::add(work[t], work[t + h]);
         }
         tc::cluster_sync();
-        const bool alone = gridDim.x == CL;
         for (int u0 = 0; u0 < E; u0 += BLK) {   // eight threads an entry, one a block
             const int u = u0 + t, from = u % CL, entry = (int)(blockIdx.x % CL) * (E / CL) + u / CL;
             E2 e{0, 0};
@@ -130,13 +130,10 @@ product_tile_kernel(const ProductArgs a, int s, const __grid_constant__ FoldWeig
                 asm volatile("ld.shared::cluster.v2.u64 {%0, %1}, [%2];" : "=l"(e.c0), "=l"(e.c1) : "r"(at) : "memory");
             }
             e = fold_join<F>(e, 3);
-            if (u < E && from == 0) {
-                if (alone) store2(a.sums + 2 * entry, e.c0, e.c1);
-                else grid_add(a.acc, E, blockIdx.x / CL, entry, e.c0, e.c1);
-            }
+            if (u < E && from == 0) grid_add(a.acc, E, blockIdx.x / CL, entry, e.c0, e.c1);
         }
         tc::cluster_sync();   // the others have read this block's
-        if (alone || !grid_last(a.acc, &last, gridDim.x)) return;
+        if (!grid_last(a.acc, &last, gridDim.x)) return;
         for (int e = t; e < E; e += BLK) {
             const E2 x = grid_take<F>(a.acc, E, e);
             store2(a.sums + 2 * e, x.c0, x.c1);

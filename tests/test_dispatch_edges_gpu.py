@@ -60,8 +60,8 @@ def test_small_folds(K, nv):
     batched_matches_oracle(K, nv, 0)
 
 
-# three and four tables by tiles of 16 elements: few tiles, whole clusters of eight and more than one, and folds of two, three and no challenges
-@pytest.mark.parametrize("d,nv", [(3, 10), (3, 11), (3, 12), (3, 13), (4, 9), (4, 11), (4, 12), (4, 15)])
+# three and four tables by tiles of 16 elements: from four clusters of eight blocks on (2^9 elements), and folds of two, three and no challenges
+@pytest.mark.parametrize("d,nv", [(3, 9), (3, 10), (3, 11), (3, 12), (3, 13), (4, 9), (4, 11), (4, 12), (4, 15)])
 @pytest.mark.parametrize("base", [True, False])
 def test_small_products(gl, d, nv, base):
     gl_sumcheck_matches_oracle(gl, nv, d, base)
