@@ -31,7 +31,9 @@ static void fold_on_host(const uint64_t* in, const uint64_t* entries, gl::E2 r, 
     }
 }
 
-constexpr size_t QUERY_WORD = 1024;   // of an opening's scratch block: the queries' indices
+// Of an opening's scratch block: sums of the inner sumcheck from word 0, a tree's last device layer from NODE_WORD, the queries' indices.
+constexpr size_t NODE_WORD = 64, QUERY_WORD = 1024;
+static_assert((size_t)2 << pr::MAX_B <= NODE_WORD && NODE_WORD + 4 * HOST_TOP <= QUERY_WORD && QUERY_WORD < ScratchPool::WORDS, "one after another");
 
 // open_ext2 (basefold.rs:578-863). Writes the proof as
 //   eval[2] | oracles[nv][3][2] | folded_roots[nv-1][4] | final_codeword[2^lr][2] |
@@ -49,7 +51,7 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     uint64_t* p_final = p_roots + (size_t)(nv - 1) * 4;
     uint64_t* p_queries = p_final + ((size_t)2 << lr);
 
-    ScopedScratch pin;   // sums of the inner sumcheck (32 words), a tree's last device layer (from word 64)
+    ScopedScratch pin;
     // The first round of the host's own: its codeword is folded, and hashed, from a copy of the one before. (Never round 0; nv - 1: none.)
     const auto leaves_of = [&](int round) { return cw_len >> (round + 2); };
     int host_round = 1;
@@ -67,7 +69,7 @@ int open_ext2(const BasefoldCommitment& cm, const uint64_t* point, const Basefol
     uint64_t* top_staging = pinned_arena(staging_words + copy_words + own_words);
     if (!pin.p || !top_staging) return MB_ERR_CUDA;
     uint64_t *copied = top_staging + staging_words, *host_rounds = copied + copy_words;
-    uint64_t* nodes = pin.p + 64;
+    uint64_t* nodes = pin.p + NODE_WORD;
     OpenSumcheck sc;
     int rc = sc.init(cm.d_bh_evals.p, nv, point, pin.p, pin.b.dev);
     if (rc != MB_OK) return rc;

@@ -110,6 +110,12 @@ def test_basefold_rounds_of_the_host(gl, nv, lr, nq):
         monolith_basefold_matches_oracle(gl, nv, lr, nq)
 
 
+@pytest.mark.parametrize("nq", [7168, 7169])
+def test_basefold_queries_beyond_the_scratch_block(gl, nq):
+    """Up to 7168 query indices are read where the host leaves them, more go up in a buffer."""
+    basefold_matches_oracle(gl, 3, 1, nq)
+
+
 def test_poseidon2_with_a_missed_carry(gl, oracle):
     """The throughput form adds without the rare carry and borrow repairs and redoes a permutation that needed one. The
     first round constant makes lane 0 of this state 2^48 before its S-box, whose square is a power of two that does;
