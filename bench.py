@@ -319,7 +319,7 @@ def run_batched(args):
     if cnt:
         total_bytes = (2 * 2 * K * m * 8 + 2 * sum(2 * K * (m >> (3 * r)) * 16 for r in range(1, n_loc // 3 + 1))) * psteps
         ach = total_bytes / (kms * 1e-3) / 1e9
-        roofline = {"kernel": "pair_mma + pair_pass", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+        roofline = {"kernel": "pair_mma + pair_pass + pair_small", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                     "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "launches": cnt,
                     "avg_launch_ms": kms / cnt,
                     "timed_in": "a separate pass of %d steps with CUDA events around every launch (not the timed region)" % psteps,
@@ -906,7 +906,7 @@ def basefold_config(nv, hash_name, world):
 
 def pass_times(kernels):
     """Launches and milliseconds of the passes over two tables, on the tensor cores and below their sizes."""
-    both = [kernels[k] for k in ("pair_mma", "pair_pass") if k in kernels]
+    both = [kernels[k] for k in ("pair_mma", "pair_pass", "pair_small") if k in kernels]
     return sum(c for c, _ in both), sum(ms for _, ms in both)
 
 
@@ -1084,7 +1084,7 @@ def part_sumcheck(lib, args, peak, peak_kind):
     whole = alg_bytes / (ms * 1e-3) / 1e9
     out = {"metric": "field-elems/s: sumcheck of f*g over 2^%d points, Goldilocks" % nv, "value": d * n / (ms * 1e-3), "unit": UNIT,
            "ms": ms, "config": {"workload": "sumcheck nv=%d d=2" % nv},
-           "roofline": {"kernel": "pair_mma + pair_pass (all passes of a proof)", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
+           "roofline": {"kernel": "pair_mma + pair_pass + pair_small (all passes of a proof)", "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                         "frac": ach / peak, "traffic": None, "peak_kind": peak_kind, "avg_launch_ms": pass_ms / cnt, "launches": cnt,
                         "timed_in": "a proof of its own with CUDA events around every launch (not the timed region)",
                         "note": "three or four rounds per pass, fold and sums on the tensor cores; latency bound after the first two",

@@ -308,7 +308,7 @@ private:
                 while (s + 1 < fb && (n << (s + 1)) / (pr::BLK / 2) * K_ <= (size_t)sm_count() / 2) s++;
                 const size_t tile = (pr::BLK / 2) >> s;
                 const dim3 few((unsigned)((n + tile - 1) / tile), K_);
-                MB_KERNEL("pair_pass");
+                MB_KERNEL("pair_small");
                 base_ ? launch_small<true>(gb, weighted, few, p, s, fw) : launch_small<false>(gb, weighted, few, p, s, fw);
             } else {
                 const dim3 grid(tiles < (size_t)cap_ ? (unsigned)tiles : (unsigned)cap_, K_);

@@ -163,7 +163,7 @@ private:
             if (rc != MB_OK) return rc;
         } else {
             const int gb = last ? 0 : blocks_[block_].rounds;
-            MB_KERNEL("product_pass");
+            MB_KERNEL(d_ == 1 ? "product_pass" : "product_tile");
             if (d_ == 1) launch_one(gb, fb > 0, p, fw);
             else if (d_ == 3) launch_three(gb, fb > 0, p, fw);
             else launch_four(gb, fb > 0, p, fw);
