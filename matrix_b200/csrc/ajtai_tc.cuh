@@ -785,7 +785,8 @@ inline size_t tc_pipe_smem_bytes(int np) {
 // the chunks to sixteen warps: one thread per output read its chunks one after the other on a quarter of the SMs
 // (18.5 us for 98 chunks x 3 planes, 84 us for 542 chunks).
 // done (may be null): a word of page-locked memory that the block which is through last clears, after all results (`through` counts
-// them, zero before and after): the caller sees that 3.4 us before a synchronisation returns.
+// them, zero before and after): the caller sees that 3.4 us before a synchronisation returns, and may then give both words to another
+// stream. So the store to done stays the last access to either, behind the fence.
 constexpr int TC_RED_SLICES = 16;
 static __global__ void __launch_bounds__(32 * TC_RED_SLICES)
 reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, int np, uint64_t* __restrict__ out, unsigned* through,
@@ -812,7 +813,7 @@ reduce_tc_partials_kernel(const uint64_t* __restrict__ partial, size_t chunks, i
             if (lane == 0 && atomicAdd(through, 1u) == gridDim.x - 1) {
                 *through = 0;
                 __threadfence_system();
-                *(volatile uint64_t*)done = 0;
+                *(volatile uint64_t*)done = 0;   // nothing after this
             }
         }
     }

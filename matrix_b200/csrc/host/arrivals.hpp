@@ -1,7 +1,8 @@
 // Waiting for results that a kernel writes straight into page-locked memory. The words are canonical residues, so a word of all ones is
 // none of them: the host sets them to that before the launch and looks until every one has changed. That sees a pass's sums 3.4 us
 // before a stream synchronisation returns (launch, empty kernel and wait: 8.8 against 12.1 us). The kernel may still be on its
-// way out then, which the stream's order hides from later work on it; who gives memory to other streams synchronises first.
+// way out then, which the stream's order hides from later work on it; who gives memory to other streams synchronises first, or waits
+// for a word that the kernel stores behind everything else, fenced.
 // A caller whose device flags ask for yielding or blocking waits gets the synchronisation instead.
 // A pass that takes longer than the polls, fails, or gives up one of its own waits (it writes no sums then) ends with a synchronisation.
 #pragma once

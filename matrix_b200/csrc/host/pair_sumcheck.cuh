@@ -222,7 +222,9 @@ public:
 private:
     static constexpr size_t ERROR_WORD = ScratchPool::WORDS - 2;
     static constexpr size_t MMA_MIN = (size_t)1 << 14;
-    static constexpr size_t SMALL_TILES = 64;   // folds of fewer tiles of 256 elements than half the SMs: pair_small_kernel
+    // Folds of at most this many tiles of 256 elements, over all instances: pair_small_kernel. Limits of 32 to 128 measure the same (all
+    // rounds of three instances of 2^15: 168 us; of five of 2^14: 165), 16 and 256 one or two per cent more (172 and 170, 168 and 167).
+    static constexpr size_t SMALL_TILES = 64;
     struct Block {
         int first, rounds;
         size_t wl, wh;      // word offsets of the eq tables

@@ -1,8 +1,9 @@
 // Scratch of a prover's passes: a page-locked block for results that kernels write straight to the host, and a device block
 // for the sums over blocks, which is zero whenever no kernel is using it (a kernel's last block puts it back,
 // pair_kernels.cuh). Allocating and clearing the two takes longer than a small proof, so freed pairs are kept (at most
-// MAX_KEPT, the rest go back to the driver). Any thread may take or give one; the owner has synchronised with whatever
-// wrote the blocks before it gives them back, and discards them if that went wrong.
+// MAX_KEPT, the rest go back to the driver). Any thread may take or give one. When the owner gives a pair back, nothing
+// may touch it any more: it has synchronised with whatever wrote the blocks, or has waited for a word whose store was the last access
+// to either of them, behind a fence (reduce_tc_partials_kernel). It discards them if that went wrong.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -45,7 +46,7 @@ public:
         }
         return b;
     }
-    // After the stream that used it was synchronised; clean: that went well, the device block is zero again.
+    // Once nothing touches it any more (above); clean: that went well, the device block is zero again.
     static void give(ScratchBlock b, bool clean) {
         if (!b) return;
         ScratchPool& p = instance();
