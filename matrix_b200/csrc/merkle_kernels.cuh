@@ -13,7 +13,8 @@
 // wrapper.cu:1894-1987). Digests are written canonical.
 //
 // Large layers are bound by the integer pipes (about 520 modular multiplications for every 32-byte Poseidon2 digest), not
-// by HBM: one fully parallel launch per layer, a permutation per thread. The leaves of a folded codeword are hashed by
+// by HBM: one fully parallel launch per layer, Poseidon2's from P2_TILES_FROM permutations on in tiles of 128
+// (poseidon2_tiles.cuh), smaller ones and Monolith's a permutation per thread. The leaves of a folded codeword are hashed by
 // the thread that folds them, so a folded codeword is written once and not read back for its tree.
 // Small layers are bound by the latency of one permutation: several lanes share a permutation, and a launch covers up to five
 // levels (the leaf layer, with its fold, among them). The launches of a tree are a chain (common.cuh): the next one's blocks come up while

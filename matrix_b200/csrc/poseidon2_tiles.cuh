@@ -11,7 +11,8 @@
 // and the other words, from all the operands so far, once these are read. Every wait is bounded; once one ran out, the whole
 // block takes the exact form.
 // Four tiles, because a tile is 128 threads of up to 128 registers and three leave schedulers idle (3237 us below).
-// Bound by the integer pipes (ncu: 0.7 of the multiply pipe, 0.53 of the other, about 0.5 of the issue slots). Layers of 2^23 permutations:
+// Bound by the integer pipes (ncu, 2^22 leaves: 0.67 of the multiply pipe, 0.51 of the logic pipe, 0.56 of the issue slots, 6940
+// instructions a permutation). Layers of 2^23 permutations:
 // 3426 us (14.9 k cycles a warp of permutations and scheduler) with six tiles of which two at a time had tensor memory, six products
 // by hand in four rounds, every S-box output reduced apart and external layers of carry additions; 2917 us (12.7 k) now.
 #pragma once
