@@ -172,7 +172,7 @@ GLF void poseidon2_permute(uint64_t* s) {
 //     exact form on the same input (one permutation in four million, half of them by words that only look like it);
 //   * the sums of the internal layer are sums of whole words in 96 bits, three carry additions each; the external layers are on
 //     the FP64 pipe.
-// Exact form 25.3 k cycles per warp of permutations, carries counted and external layers in 96 bits 17.5 k, now 16.5 k (2^19
+// Exact form 25.3 k cycles per warp of permutations, carries counted and external layers in 96 bits 17.5 k, now 16.2 k (2^19
 // permutations: 253 -> 236 us; tiles, which leave out the internal layers' products, 192 us).
 namespace p2t {
 using namespace fast;
